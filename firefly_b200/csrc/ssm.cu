@@ -11,9 +11,11 @@
 // linear attention: a_t = diag(alpha_t) with alpha from a low-rank projection (`low_rank_decay_kernel`), b = 1.
 //
 // The state lives in the request's state slot in 32-bit and is carried from step to step; a fresh request
-// starts from zeros.  Decays, steps, S and every sum are 32-bit.  A sequence's tokens are walked in order
-// with the same order of additions however the prompt was cut into steps.
+// starts from zeros.  Decays, steps, S and every sum are 32-bit.  Steps of few tokens walk a sequence token by token;
+// bfloat16 prompts are taken a chunk of tokens at a time, whose sums are formed in another order, as right.
+#include "chunk_scan.cuh"
 #include "common.cuh"
+#include "scan_wide.cuh"
 
 namespace ff {
 
@@ -183,176 +185,558 @@ struct ScanArgs {
     float q_scale;                               // q is multiplied by this as it is read (behind the activation)
 };
 
-constexpr int SCAN_CHUNK = 8;
-constexpr int SCAN_MAX_THREADS = 512;
-
-// How the recurrence is laid out for key size N and value size V: the key size it is instantiated for (NP),
-// the threads that share a value column (PARTS, each with NP / PARTS key channels in registers), over how many
-// blocks a head's value columns are split (vsplit, Vb columns each) and the threads of a block.  A token costs a
-// thread NP / PARTS steps of a serial chain, so long keys get many threads a column and the columns of a head go
-// to several blocks.  (Sixteen threads a column were tried for keys of 128: a head of 64 columns then needs two
-// blocks of 512 threads, eight sequences of 32 heads no longer fit the GPU at once, and the prompt pass was slower.)
-struct ScanPlan { int NP, PARTS, vsplit, Vb, threads; };
-static inline bool scan_plan(int N, int V, ScanPlan* p) {
-    if (N <= 0 || N > 256 || V <= 0 || V > 256) return false;
-    p->NP = N <= 16 ? 16 : (N <= 32 ? 32 : (N <= 64 ? 64 : (N <= 128 ? 128 : 256)));
-    p->PARTS = p->NP >= 32 ? 8 : 4;
-    const int max_cols = SCAN_MAX_THREADS / p->PARTS;
-    p->vsplit = (V + max_cols - 1) / max_cols;
-    p->Vb = (V + p->vsplit - 1) / p->vsplit;
-    p->threads = ((p->Vb * p->PARTS + 31) / 32) * 32;
-    return true;
-}
-
-// One block per (sequence, head, share of the value columns).  Value column j is held by PARTS neighbouring
-// threads, each with NP / PARTS key channels of column j in registers.
-// PF: the next chunk's inputs are asked for (into registers) before the current chunk is computed, so their
-// latency hides behind the recurrence; it needs a block with enough threads for SCAN_PFQ q and k values and
-// SCAN_PFV v values each a chunk (the launcher checks), else the chunk is staged when it is needed.
-constexpr int SCAN_PFQ = 2, SCAN_PFV = 1;
-
-// CD: mode 2, a decay per key channel (staged beside q and k).
-template <typename T, int NP, int PARTS, bool PF, bool CD>
-__global__ void __launch_bounds__(SCAN_MAX_THREADS, 2) scalar_decay_scan_kernel(
+// One block per (sequence, head, VB value columns), token by token (scan_wide.cuh).  A chunk's q, k, v and decays are staged in
+// 32-bit in one of two buffers; the next chunk's are asked for before the current one is walked and staged behind it, so
+// a chunk has one barrier.  CD: mode 2, a decay per key channel (staged beside q and k).
+// This is the kernel for steps of few tokens, for 32-bit inputs, for inputs that pass SiLU (both factors of every product
+// would have to be split, and on sums that lean to one side, as those of SiLU's do, the tensor cores' cut-off leaves 8e-7 where
+// this one leaves 1e-7) and for sizes that the chunked ones do not take.  Against one column a thread: 758 -> 279 us
+// for three sequences of 1501, 1000 and 700 tokens with 16 heads of 64 x 128, 1256 -> 745 us for 4 x 2048 tokens, SiLU, 8 heads
+// of 128 x 128.
+template <typename T, int NP, bool CD>
+__global__ void __launch_bounds__(WS_THREADS) scalar_decay_scan_kernel(
     ScanArgs A, float* __restrict__ state, size_t state_stride, int state_off, const int* __restrict__ cu_q,
     const int* __restrict__ state_slots, const int* __restrict__ seq_fresh, float* __restrict__ o /*[T, heads*V]*/,
-    int heads, int N, int V, int Vb) {
+    int heads, int N, int V) {
     pdl_prologue();
-    constexpr int KP = NP / PARTS;
-    static_assert(KP % 4 == 0, "a thread reads its key channels four at a time");
-    __shared__ __align__(16) float s_q[SCAN_CHUNK][NP], s_k[SCAN_CHUNK][NP];
-    __shared__ __align__(16) float s_cd[CD ? SCAN_CHUNK : 1][CD ? NP : 4];
-    __shared__ float s_v[SCAN_CHUNK][128];
-    __shared__ float s_a[SCAN_CHUNK], s_d[SCAN_CHUNK];
-    const int s = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, nthr = blockDim.x;
-    const int jl = tid / PARTS, part = tid % PARTS;
-    const int j0 = blockIdx.z * Vb, j = j0 + jl;
+    using WS = WideState<NP>;
+    constexpr int CH = WS::CH, VB = WS::VB, PQ = CH * NP / WS_THREADS, PV = (CH * VB + WS_THREADS - 1) / WS_THREADS;
+    static_assert(CH * NP % WS_THREADS == 0, "a thread stages the same number of elements");
+    __shared__ __align__(16) float s_q[2][CH][NP], s_k[2][CH][NP], s_cd[CD ? 2 : 1][CD ? CH : 1][CD ? NP : 4];
+    __shared__ __align__(16) f32x2 s_v[2][CH][VB];        // each value twice
+    __shared__ float s_a[2][CH], s_d[2][CH];
+    const int s = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
+    const int j0 = blockIdx.z * VB;
     const int t0 = cu_q[s], t1 = cu_q[s + 1];
-    const bool live = jl < Vb && j < V;
-    const bool fresh = seq_fresh[s] != 0;
-    // a block's share of a head's state is kept as its threads hold it: register i of thread tid at i * threads + tid
-    float* S_g = state + (size_t)state_slots[s] * state_stride + state_off +
-                 ((size_t)h * gridDim.z + blockIdx.z) * KP * nthr;
-    float S[KP];
-#pragma unroll
-    for (int i = 0; i < KP; ++i) S[i] = fresh ? 0.f : S_g[(size_t)i * nthr + tid];
+    WS w;
+    w.place(tid);
+    float* S_g = state + (size_t)state_slots[s] * state_stride + state_off + (size_t)h * V * NP;
+    w.load(S_g, j0, V, seq_fresh[s] != 0);
     const int group = h / A.heads_per_group;
     const T* qp = pdl_fresh((const T*)A.q) + A.q_off + (size_t)group * N;
     const T* kp = pdl_fresh((const T*)A.k) + A.k_off + (size_t)group * N;
     const T* vp = pdl_fresh((const T*)A.v) + A.v_off + (size_t)h * V + j0;
     const T* stepp = pdl_fresh((const T*)A.step);
     const float* cdp = CD ? pdl_fresh(A.channel_decay) + A.cd_off + (size_t)h * N : nullptr;
-    const int cols = min(Vb, V - j0);
+    const int cols = min(VB, V - j0);
     float a_const = 1.f, rate = 0.f, sbias = 0.f, skip = 0.f;
     if (A.mode == 0) a_const = A.decay[h];
     else if (!CD) { rate = expf(A.a_log[h]); sbias = A.step_bias[h]; skip = A.skip ? A.skip[h] : 0.f; }
-    // the values a thread stages: element u of a thread is flat index tid + u * threads of the chunk's [8][NP] or [8][cols]
-    float rq[PF ? SCAN_PFQ : 1], rk[PF ? SCAN_PFQ : 1], rv[PF ? SCAN_PFV : 1], rcd[PF && CD ? SCAN_PFQ : 1], rstep = 0.f;
+    // element u of a thread is flat index tid + u * threads of the chunk's [CH][NP] or [CH][VB]
+    T rq[PQ], rk[PQ], rv[PV], rstep = from_float<T>(0.f);
+    float rcd[CD ? PQ : 1];
     auto fetch = [&](int c0) {
-        const int n = min(SCAN_CHUNK, t1 - c0);
+        const int n = min(CH, t1 - c0);
 #pragma unroll
-        for (int u = 0; u < SCAN_PFQ; ++u) {
-            const int idx = tid + u * nthr, c = idx / NP, i = idx - c * NP;
-            const bool ok = idx < SCAN_CHUNK * NP && c < n && i < N;
-            rq[u] = ok ? to_float(qp[(size_t)(c0 + c) * A.q_stride + i]) : 0.f;
-            rk[u] = ok ? to_float(kp[(size_t)(c0 + c) * A.k_stride + i]) : 0.f;
+        for (int u = 0; u < PQ; ++u) {
+            const int idx = tid + u * WS_THREADS, c = idx / NP, i = idx % NP;
+            const bool ok = c < n && i < N;
+            rq[u] = ok ? qp[(size_t)(c0 + c) * A.q_stride + i] : from_float<T>(0.f);
+            rk[u] = ok ? kp[(size_t)(c0 + c) * A.k_stride + i] : from_float<T>(0.f);
             if constexpr (CD) rcd[u] = ok ? cdp[(size_t)(c0 + c) * A.cd_stride + i] : 0.f;
         }
 #pragma unroll
-        for (int u = 0; u < SCAN_PFV; ++u) {
-            const int idx = tid + u * nthr, c = idx / cols, jj = idx - c * cols;
-            rv[u] = (idx < SCAN_CHUNK * cols && c < n) ? to_float(vp[(size_t)(c0 + c) * A.v_stride + jj]) : 0.f;
+        for (int u = 0; u < PV; ++u) {
+            const int idx = tid + u * WS_THREADS, c = idx / VB, jj = idx % VB;
+            rv[u] = (idx < CH * VB && c < n && jj < cols) ? vp[(size_t)(c0 + c) * A.v_stride + jj] : from_float<T>(0.f);
         }
-        if (A.mode == 1 && tid < n) rstep = to_float(stepp[(size_t)(c0 + tid) * A.step_stride + A.step_off + h]);
+        if (A.mode == 1 && tid < n) rstep = stepp[(size_t)(c0 + tid) * A.step_stride + A.step_off + h];
     };
-    if constexpr (PF) fetch(t0);
-    for (int c0 = t0; c0 < t1; c0 += SCAN_CHUNK) {
-        const int n = min(SCAN_CHUNK, t1 - c0);
-        __syncthreads();
-        // staging: the chunk's q, k, v, decays and input scales in 32-bit
-        if (tid < SCAN_CHUNK) {
-            float a = a_const, b = 1.f;
-            if (A.mode == 1 && tid < n) {
-                const float raw = PF ? rstep : to_float(stepp[(size_t)(c0 + tid) * A.step_stride + A.step_off + h]);
-                const float dt = softplus_f(raw + sbias);
-                a = expf(-rate * dt);
-                b = dt;
-            }
-            s_a[tid] = a;
-            s_d[tid] = b;
+    auto stage = [&](int b, int n) {
+#pragma unroll
+        for (int u = 0; u < PQ; ++u) {
+            const int idx = tid + u * WS_THREADS;
+            const float qv = to_float(rq[u]), kv = to_float(rk[u]);
+            (&s_q[b][0][0])[idx] = (A.act ? silu_f(qv) : qv) * A.q_scale;
+            (&s_k[b][0][0])[idx] = A.act ? silu_f(kv) : kv;
+            if constexpr (CD) (&s_cd[b][0][0])[idx] = rcd[u];
         }
-        if constexpr (PF) {
 #pragma unroll
-            for (int u = 0; u < SCAN_PFQ; ++u) {
-                const int idx = tid + u * nthr;
-                if (idx < SCAN_CHUNK * NP) {
-                    (&s_q[0][0])[idx] = (A.act ? silu_f(rq[u]) : rq[u]) * A.q_scale;
-                    (&s_k[0][0])[idx] = A.act ? silu_f(rk[u]) : rk[u];
-                    if constexpr (CD) (&s_cd[0][0])[idx] = rcd[u];
-                }
+        for (int u = 0; u < PV; ++u) {
+            const float raw = to_float(rv[u]), vv = A.act ? silu_f(raw) : raw;
+            if (CH * VB % WS_THREADS == 0 || tid + u * WS_THREADS < CH * VB) (&s_v[b][0][0])[tid + u * WS_THREADS] = f2_pack(vv, vv);
+        }
+        if (!CD && tid < CH) {
+            float a = a_const, d = 1.f;
+            if (A.mode == 1 && tid < n) {
+                d = softplus_f(to_float(rstep) + sbias);
+                a = expf(-rate * d);
             }
+            s_a[b][tid] = a;
+            s_d[b][tid] = d;
+        }
+    };
+    const int first = w.first();
+    const bool owns = w.part < CH * WS_COLS;             // with more threads a column than sums the rest hold copies
+    float* oh = o + (size_t)h * V + j0;
+    if (t0 < t1) {
+        fetch(t0);
+        stage(0, min(CH, t1 - t0));
+    }
+    __syncthreads();
+    int b = 0;
+    for (int c0 = t0; c0 < t1; c0 += CH, b ^= 1) {
+        const int n = min(CH, t1 - c0);
+        if (c0 + CH < t1) fetch(c0 + CH);
+        auto token = [&](int c, float* part) {
+            f32x2 v[WS_COLS];
+            WS::values(&s_v[b][c][w.jl * WS_COLS], v);
+            if (!CD && A.mode == 1) {
+                const f32x2 d = f2_pack(s_d[b][c], s_d[b][c]);
 #pragma unroll
-            for (int u = 0; u < SCAN_PFV; ++u) {
-                const int idx = tid + u * nthr, c = idx / cols, jj = idx - c * cols;
-                if (idx < SCAN_CHUNK * cols) s_v[c][jj] = A.act ? silu_f(rv[u]) : rv[u];
+                for (int x = 0; x < WS_COLS; ++x) v[x] = f2_mul(v[x], d);
+            }
+            w.template token<CD, false>(s_q[b][c], s_k[b][c], CD ? s_cd[b][c] : nullptr, CD ? 1.f : s_a[b][c], v, part);
+        };
+        if (n == CH) {
+            float part[CH * WS_COLS];
+#pragma unroll
+            for (int c = 0; c < CH; ++c) token(c, part + c * WS_COLS);
+            w.reduce_chunk(part);
+#pragma unroll
+            for (int r = 0; r < WS::OUTS; ++r) {
+                const int at = first + r, c = at / WS_COLS, jj = w.jl * WS_COLS + at % WS_COLS;
+                if (owns && j0 + jj < V)
+                    oh[(size_t)(c0 + c) * heads * V + jj] = skip != 0.f ? part[r] + skip * f2_low(s_v[b][c][jj]) : part[r];
             }
         } else {
-            for (int idx = tid; idx < SCAN_CHUNK * NP; idx += nthr) {
-                const int c = idx / NP, i = idx - c * NP;
-                float qv = 0.f, kv = 0.f, cdv = 0.f;
-                if (c < n && i < N) {
-                    qv = to_float(qp[(size_t)(c0 + c) * A.q_stride + i]);
-                    kv = to_float(kp[(size_t)(c0 + c) * A.k_stride + i]);
-                    if (A.act) { qv = silu_f(qv); kv = silu_f(kv); }
-                    qv *= A.q_scale;
-                    if constexpr (CD) cdv = cdp[(size_t)(c0 + c) * A.cd_stride + i];
-                }
-                s_q[c][i] = qv;
-                s_k[c][i] = kv;
-                if constexpr (CD) s_cd[c][i] = cdv;
+            for (int c = 0; c < n; ++c) {
+                float part[WS_COLS];
+                token(c, part);
+                const float y = w.reduce(part);
+                const int jj = w.jl * WS_COLS + w.col();
+                if (w.part < 4 && j0 + jj < V)
+                    oh[(size_t)(c0 + c) * heads * V + jj] = skip != 0.f ? y + skip * f2_low(s_v[b][c][jj]) : y;
             }
-            for (int idx = tid; idx < SCAN_CHUNK * cols; idx += nthr) {
-                const int c = idx / cols, jj = idx - c * cols;
-                float vv = 0.f;
-                if (c < n) {
-                    vv = to_float(vp[(size_t)(c0 + c) * A.v_stride + jj]);
-                    if (A.act) vv = silu_f(vv);
+        }
+        if (c0 + CH < t1) stage(b ^ 1, min(CH, t1 - c0 - CH));
+        __syncthreads();
+    }
+    w.store(S_g, j0, V);
+}
+
+// ------------------------------------------------------------------- the recurrence, a chunk of tokens at a time --
+// Modes 0 and 1 over prompts, bfloat16 inputs that are read as they are.  With L_t the sum of the logarithms of the decays up
+// to token t of a chunk and S the state in front of it:
+//
+//   P_ts = (q_t . k_s) exp(L_t - L_s) b_s   for s <= t
+//   o_t  = exp(L_t) S^T q_t + sum_s P_ts v_s
+//   S   <- exp(L_end) S + sum_s exp(L_end - L_s) b_s k_s v_s^T
+//
+// Every exponent is a difference that is never positive, formed from sums held in twice 32 bits, so it is as right as the
+// product of the decays it stands for.  The four sums over key channels or tokens run on the tensor cores in 32-bit
+// out of bfloat16 products (chunk_mma.cuh); S never leaves the registers.
+// P, the decays' sums and what follows from them do not hold S: a first kernel forms them for all chunks of the step at once and
+// leaves them as records in scratch memory.  The second one walks a sequence's chunks: one block per (sequence, head, VB = 16 W
+// value columns), whose warps hold S^T as the accumulators of mma.sync; the same registers are, split, the left operand of
+// S^T q, so the state goes nowhere between the products.
+// Measured on 4 x 2048 tokens, 32 heads of 128 x 64: token by token with one column a thread 1552 us; the two kernels 33 + 143.
+// From SCAN_CHUNK_MIN tokens a sequence (average of a step) on it is the faster one (us, chunked / token by token wide, 32 heads of
+// 128 x 64: eight sequences of 16 16.1 / 12.7, of 32 16.6 / 22.4, of 64 22.7 / 41.7; one of 32 9.3 / 10.3, of 64 11.4 / 18.3).
+constexpr int SC_C = 32;                                  // tokens a chunk
+constexpr int SCAN_CHUNK_MIN = 32;
+// The same for a decay per key channel (us, 16 heads of 64 x 128: eight sequences of 64 34.9 / 23.8, of 96 22.3 / 34.5 with records of
+// their own block; one of 96 10.1 / 18.3).
+constexpr int CHANNEL_CHUNK_MIN = 80;
+constexpr int SC_PP = SC_C + 8;
+
+struct ScanRecord {
+    bf16 P[3][SC_C * SC_PP];
+    float e[SC_C], w[SC_C], end[4];                       // exp(L_t), exp(L_end - L_s) b_s, exp(L_end)
+};
+static_assert(sizeof(ScanRecord) % 16 == 0, "a record is copied in 16-byte pieces");
+
+// The first kernel: a block per (chunk, group of heads that share q and k).  Three of its warps multiply q with k once for the
+// group; then four heads at a time, a warp a head sums up the decays and each tile of the product is scaled for each head.
+template <int NK>
+__global__ void __launch_bounds__(128) scalar_decay_prepare_kernel(ScanArgs A, ScanRecord* __restrict__ recs, const int* __restrict__ cu_q,
+                                                                   int n_seqs, int heads) {
+    pdl_prologue();
+    constexpr int QP = NK + 8;
+    __shared__ __align__(16) bf16 sq[SC_C * QP], sk[SC_C * QP];
+    __shared__ float lh[4][SC_C], ll[4][SC_C], sb[4][SC_C], pw[4][SC_C + 1];
+    int s, chunk;
+    chunk_of_record<SC_C>(cu_q, n_seqs, blockIdx.x, s, chunk);
+    if (chunk < 0) return;
+    const int group = blockIdx.y, row0 = cu_q[s] + chunk * SC_C, n = min(SC_C, cu_q[s + 1] - row0);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c2 = (lane & 3) * 2;
+    const int row_a = (lane & 7) + ((lane >> 3) & 1) * 8, col_a = (lane >> 4) * 8;
+    const int row_b = (lane & 7) + (lane >> 4) * 8, col_b = ((lane >> 3) & 1) * 8;
+    const bf16* qp = pdl_fresh((const bf16*)A.q) + A.q_off + (size_t)group * NK;
+    const bf16* kp = pdl_fresh((const bf16*)A.k) + A.k_off + (size_t)group * NK;
+    const bf16* stepp = pdl_fresh((const bf16*)A.step) + A.step_off;
+    for (int idx = threadIdx.x; idx < SC_C * (NK / 8); idx += 128) {
+        const int r = idx / (NK / 8), c = (idx % (NK / 8)) * 8;
+        const bool in = r < n;
+        cm_copy16(sq + r * QP + c, qp + (size_t)(row0 + (in ? r : 0)) * A.q_stride + c, in);
+        cm_copy16(sk + r * QP + c, kp + (size_t)(row0 + (in ? r : 0)) * A.k_stride + c, in);
+    }
+    cm_copy_commit();
+    // P's tiles: rows (tokens) 16 mt.., columns (keys) 16 nh..; keys behind the tokens are not formed
+    const int mt = warp >> 1, nh = warp & 1;
+    float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+    for (int h0 = 0; h0 < A.heads_per_group; h0 += 4) {
+        if (h0 + warp < A.heads_per_group) {              // the decays of a head, one token a lane
+            const int h = group * A.heads_per_group + h0 + warp;
+            ScanRecord* rec = recs + (size_t)blockIdx.x * heads + h;
+            const bool in = lane < n;
+            if (A.mode == 1) {
+                const float rate = expf(A.a_log[h]);
+                const float dt = in ? softplus_f(to_float(stepp[(size_t)(row0 + lane) * A.step_stride + h]) + A.step_bias[h]) : 0.f;
+                // at most e^-200 a token: 0 in 32 bits, and the sums stay exact enough to be subtracted from one another
+                double L = in ? (double)(-rate * dt < -200.f ? -200.f : -rate * dt) : 0.0;
+#pragma unroll
+                for (int off = 1; off < 32; off <<= 1) {
+                    const double up = __shfl_up_sync(0xffffffffu, L, off);
+                    if (lane >= off) L += up;
                 }
-                s_v[c][jj] = vv;
+                const double Lend = __shfl_sync(0xffffffffu, L, 31);
+                const float hi = (float)L;
+                lh[warp][lane] = hi;
+                ll[warp][lane] = (float)(L - (double)hi);
+                sb[warp][lane] = dt;
+                rec->e[lane] = expf(hi) * A.q_scale;
+                rec->w[lane] = dt * expf((float)(Lend - L));
+                if (lane == 0) rec->end[0] = expf((float)Lend);
+            } else {                                      // powers of the constant decay, for any sign and zero
+                const double a = (double)A.decay[h];
+                double p = 1.0;
+                for (int r = 0; r < lane; ++r) p *= a;
+                pw[warp][lane] = (float)p;
+                if (lane == 31) pw[warp][32] = (float)(p * a);
+                __syncwarp();
+                rec->e[lane] = pw[warp][lane + 1] * A.q_scale;
+                rec->w[lane] = in ? pw[warp][n - 1 - lane] : 0.f;
+                if (lane == 0) rec->end[0] = pw[warp][n];
+            }
+        }
+        if (h0 == 0) {
+            cm_copy_wait<0>();
+            __syncthreads();
+            if (nh <= mt) {
+#pragma unroll
+                for (int kk = 0; kk < NK / 16; ++kk) {
+                    uint32_t a[1][4], b[1][4];
+                    cm_ldsm4(a[0], sq + (mt * 16 + row_a) * QP + kk * 16 + col_a);
+                    cm_ldsm4(b[0], sk + (nh * 16 + row_b) * QP + kk * 16 + col_b);
+                    cm_mma_rows(acc, acc, a, b);
+                }
+            }
+        } else __syncthreads();
+        if (nh <= mt) {
+            for (int hw = 0; hw < min(4, A.heads_per_group - h0); ++hw) {
+                const int h = group * A.heads_per_group + h0 + hw;
+                bf16* Pd = recs[(size_t)blockIdx.x * heads + h].P[0];
+#pragma unroll
+                for (int nt = 0; nt < 2; ++nt) {
+#pragma unroll
+                    for (int r = 0; r < 2; ++r) {
+                        const int t = mt * 16 + g + r * 8, u = nh * 16 + nt * 8 + c2;
+                        float x[2];
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            const int us = u + e;
+                            float d = 0.f;
+                            if (us <= t) d = A.mode == 0 ? pw[hw][t - us] : expf((lh[hw][t] - lh[hw][us]) + (ll[hw][t] - ll[hw][us])) * sb[hw][us];
+                            // a key behind the token counts nothing, whatever its product is
+                            x[e] = us <= t ? acc[nt][r * 2 + e] * (d * A.q_scale) : 0.f;
+                        }
+                        uint32_t p0, p1, p2;
+                        cm_split3(x[0], x[1], p0, p1, p2);
+                        uint32_t* dst = reinterpret_cast<uint32_t*>(Pd + t * SC_PP + u);
+                        dst[0] = p0;
+                        dst[SC_C * SC_PP / 2] = p1;
+                        dst[SC_C * SC_PP] = p2;
+                    }
+                }
             }
         }
         __syncthreads();
-        if constexpr (PF) {
-            if (c0 + SCAN_CHUNK < t1) fetch(c0 + SCAN_CHUNK);
+    }
+}
+
+template <int NK, int W>
+struct ScanChunkSmem {
+    static constexpr int QP = NK + 8, VP = 16 * W + 8;    // row pitches: 16-byte pieces of 8 rows lie in different banks
+    struct Stage { ScanRecord rec; bf16 q[SC_C * QP], k[SC_C * QP], v[SC_C * VP]; };
+    Stage stage[3];                                       // walked, there, on its way
+    float xch[2][2 * W][8][32];
+};
+
+// The second kernel; two warps hold the keys' halves of 16 value columns and exchange their shares of S^T q, each for the tokens (16
+// of 32) that the other goes on with, as in chunk_scan.cuh.
+template <int NK, int W>
+__global__ void __launch_bounds__(64 * W + CS_LOADERS) scalar_decay_chunk_kernel(
+    ScanArgs A, const ScanRecord* recs_, float* __restrict__ state, size_t state_stride, int state_off, const int* __restrict__ cu_q,
+    const int* __restrict__ state_slots, const int* __restrict__ seq_fresh, float* __restrict__ o /*[T, heads*V]*/,
+    int heads, int V) {
+    pdl_prologue();
+    using SM = ScanChunkSmem<NK, W>;
+    constexpr int QP = SM::QP, VP = SM::VP, PP = SC_PP, NT = NK / 16, VB = 16 * W;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    SM& sm = *reinterpret_cast<SM*>(smem_raw);
+    const int s = blockIdx.x, h = blockIdx.y, j0 = blockIdx.z * VB;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int t0 = cu_q[s], len = cu_q[s + 1] - t0, chunks = (len + SC_C - 1) / SC_C;
+    if (warp >= 2 * W) {
+        // ---- the warps that load
+        const int pt = threadIdx.x - 64 * W, group = h / A.heads_per_group;
+        const ScanRecord* recs = pdl_fresh(recs_) + (size_t)chunk_first_record<SC_C>(t0, s) * heads + h;
+        const bf16* qp = pdl_fresh((const bf16*)A.q) + A.q_off + (size_t)group * NK;
+        const bf16* kp = pdl_fresh((const bf16*)A.k) + A.k_off + (size_t)group * NK;
+        const bf16* vp = pdl_fresh((const bf16*)A.v) + A.v_off + (size_t)h * V + j0;
+        auto load = [&](int i) {                          // ask for chunk i's record and q, k, v (zeros behind the sequence's end)
+            if (i < chunks) {
+                typename SM::Stage& st = sm.stage[i % 3];
+                const int n = len - i * SC_C;
+                const size_t row0 = (size_t)(t0 + i * SC_C);
+                const unsigned char* src = reinterpret_cast<const unsigned char*>(recs + (size_t)i * heads);
+#pragma unroll 8
+                for (int p = pt; p < (int)(sizeof(ScanRecord) / 16); p += CS_LOADERS)
+                    cm_copy16(reinterpret_cast<unsigned char*>(&st.rec) + p * 16, src + p * 16, true);
+#pragma unroll 4
+                for (int idx = pt; idx < SC_C * (NK / 8); idx += CS_LOADERS) {
+                    const int r = idx / (NK / 8), c = (idx % (NK / 8)) * 8;
+                    const bool in = r < n;
+                    const size_t row = in ? row0 + r : (size_t)t0;
+                    cm_copy16(st.q + r * QP + c, qp + row * A.q_stride + c, in);
+                    cm_copy16(st.k + r * QP + c, kp + row * A.k_stride + c, in);
+                }
+                for (int idx = pt; idx < SC_C * (VB / 8); idx += CS_LOADERS) {
+                    const int r = idx / (VB / 8), c = (idx % (VB / 8)) * 8;
+                    const bool in = r < n && j0 + c < V;
+                    cm_copy16(st.v + r * VP + c, vp + (in ? (row0 + r) * A.v_stride + c : 0), in);
+                }
+            }
+            cm_copy_commit();
+        };
+        load(0);
+        load(1);
+        for (int i = 0; i < chunks; ++i) {
+            cm_copy_wait<1>();
+            __syncthreads();                              // chunk i is there, and everybody is done with chunk i - 1
+            load(i + 2);
+        }
+        cm_copy_wait<0>();
+        return;
+    }
+    // ---- the warps that hold S^T
+    const int tile = warp % W, half = warp / W, other = tile + (1 - half) * W, k0 = half * (NK / 2);
+    const int g = lane >> 2, c2 = (lane & 3) * 2;
+    // where ldmatrix finds the four 8 x 8 tiles of a lane's row: the second one 8 rows down and the third 8 columns on (a),
+    // or the second 8 columns on and the third 8 rows down (b)
+    const int row_a = (lane & 7) + ((lane >> 3) & 1) * 8, col_a = (lane >> 4) * 8;
+    const int row_b = (lane & 7) + (lane >> 4) * 8, col_b = ((lane >> 3) & 1) * 8;
+    float* S_g = state + (size_t)state_slots[s] * state_stride + state_off + (size_t)h * V * NK + k0;      // [V][NK]
+    const bool fresh = seq_fresh[s] != 0;
+    const int jr[2] = {j0 + tile * 16 + g, j0 + tile * 16 + g + 8};
+    float S[NT][4];
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            S[nt][e] = (fresh || jr[e >> 1] >= V) ? 0.f : S_g[(size_t)jr[e >> 1] * NK + nt * 8 + c2 + (e & 1)];
+    }
+    const int ld = heads * V, t_own = half * 16 + c2;
+    float* op = o + (size_t)(t0 + t_own) * ld + (size_t)h * V + jr[0];
+    const bool all_cols = j0 + VB <= V;
+    const float skip = (A.mode == 1 && A.skip) ? A.skip[h] : 0.f;
+    for (int i = 0; i < chunks; ++i) {
+        __syncthreads();
+        const typename SM::Stage& st = sm.stage[i % 3];
+        const int n = min(SC_C, len - i * SC_C);
+        float acc[4][4], low[4][4];                       // o^T, and the sum of its small terms
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[nt][e] = low[nt][e] = 0.f;
+        }
+        // S^T q
+#pragma unroll
+        for (int kk = 0; kk < NK / 32; ++kk) {
+            uint32_t a[3][4], r[1][4];
+            cm_split3(S[2 * kk][0], S[2 * kk][1], a[0][0], a[1][0], a[2][0]);
+            cm_split3(S[2 * kk][2], S[2 * kk][3], a[0][1], a[1][1], a[2][1]);
+            cm_split3(S[2 * kk + 1][0], S[2 * kk + 1][1], a[0][2], a[1][2], a[2][2]);
+            cm_split3(S[2 * kk + 1][2], S[2 * kk + 1][3], a[0][3], a[1][3], a[2][3]);
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                cm_ldsm4(r[0], st.q + (t * 16 + row_b) * QP + k0 + kk * 16 + col_b);
+                cm_mma_rows(&acc[2 * t], &low[2 * t], a, r);
+            }
+        }
+        float own[2][4], own_low[2][4];                   // the own sixteen tokens
+        {
+            float (*mine)[32] = sm.xch[i & 1][warp];
+            const float (*theirs)[32] = sm.xch[i & 1][other];
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) mine[nt * 4 + e][lane] = half ? acc[nt][e] + low[nt][e] : acc[2 + nt][e] + low[2 + nt][e];
+            }
+            cm_barrier(1 + tile, 64);
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt) {
+                const float2 e2 = *reinterpret_cast<const float2*>(&st.rec.e[nt * 8 + t_own]);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    own[nt][e] = ((half ? acc[2 + nt][e] + low[2 + nt][e] : acc[nt][e] + low[nt][e]) + theirs[nt * 4 + e][lane]) * ((e & 1) ? e2.y : e2.x);
+                    own_low[nt][e] = 0.f;
+                }
+            }
+        }
+        // the chunk's values, V^T: 16 value columns x 32 tokens
+        uint32_t va[2][1][4];
+        bool odd = false;
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            cm_ldsm4t(va[b][0], st.v + (b * 16 + row_b) * VP + tile * 16 + col_b);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) odd |= cm_not_finite(va[b][0][r]);
+        }
+        if (!__any_sync(0xffffffffu, odd)) {
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                if (b <= half) {                          // tokens of the first half do not see keys of the second
+                    uint32_t r[3][4];
+#pragma unroll
+                    for (int p = 0; p < 3; ++p) cm_ldsm4(r[p], st.rec.P[p] + (half * 16 + row_b) * PP + b * 16 + col_b);
+                    cm_mma_rows(own, own_low, va[b], r);
+                }
+            }
+        } else {
+            // a value that is not finite must not reach the tokens in front of it through a product with zero
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int t = nt * 8 + t_own + (e & 1), col = tile * 16 + g + (e >> 1) * 8;
+                    for (int u = 0; u <= t; ++u) {
+                        float pv = 0.f;
+                        for (int p = 2; p >= 0; --p) pv += to_float(st.rec.P[p][t * PP + u]);
+                        own[nt][e] += pv * to_float(st.v[u * VP + col]);
+                    }
+                }
+            }
+        }
+        // the skip term: V^T lies in the registers of a left operand as an accumulator does
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            float* d = &own[r >> 1][(r & 1) * 2];
+            const float* l = &own_low[r >> 1][(r & 1) * 2];
+            const uint32_t v = half ? va[1][0][r] : va[0][0][r];
+            d[0] = d[0] + l[0];
+            d[1] = d[1] + l[1];
+            if (skip != 0.f) { d[0] += skip * cm_lo(v); d[1] += skip * cm_hi(v); }
+        }
+        if (n == SC_C && all_cols) {
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) op[(size_t)(nt * 8 + (e & 1)) * ld + (e >> 1) * 8] = own[nt][e];
+            }
+        } else {
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (nt * 8 + t_own + (e & 1) < n && jr[e >> 1] < V) op[(size_t)(nt * 8 + (e & 1)) * ld + (e >> 1) * 8] = own[nt][e];
+            }
+        }
+        op += (size_t)SC_C * ld;
+        // S <- end S + sum_s (w_s v_s) k_s
+        const float end = st.rec.end[0];
+        uint32_t wa[2][3][4];
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const float2 w2 = *reinterpret_cast<const float2*>(&st.rec.w[b * 16 + (r >> 1) * 8 + c2]);
+                cm_split3(cm_lo(va[b][0][r]) * w2.x, cm_hi(va[b][0][r]) * w2.y, wa[b][0][r], wa[b][1][r], wa[b][2][r]);
+            }
         }
 #pragma unroll
-        for (int c = 0; c < SCAN_CHUNK; ++c) {
-            if (c < n) {
-                const float vj = live ? s_v[c][jl] : 0.f;
-                const float a = s_a[c], bv = s_d[c] * vj;
-                float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+        for (int m = 0; m < NK / 32; ++m) {
+            float sl[2][4];
 #pragma unroll
-                for (int i = 0; i < KP; i += 4) {
-                    // thread `part` holds key channels 4 PARTS m + 4 part + e (m = i / 4, e < 4)
-                    const int at = i * PARTS + part * 4;
-                    const float4 q4 = *reinterpret_cast<const float4*>(&s_q[c][at]);
-                    const float4 k4 = *reinterpret_cast<const float4*>(&s_k[c][at]);
-                    float4 d4 = make_float4(a, a, a, a);
-                    if constexpr (CD) d4 = *reinterpret_cast<const float4*>(&s_cd[c][at]);
-                    S[i]     = d4.x * S[i]     + k4.x * bv;  a0 += q4.x * S[i];
-                    S[i + 1] = d4.y * S[i + 1] + k4.y * bv;  a1 += q4.y * S[i + 1];
-                    S[i + 2] = d4.z * S[i + 2] + k4.z * bv;  a2 += q4.z * S[i + 2];
-                    S[i + 3] = d4.w * S[i + 3] + k4.w * bv;  a3 += q4.w * S[i + 3];
-                }
-                float acc = (a0 + a1) + (a2 + a3);
+            for (int nt = 0; nt < 2; ++nt) {
 #pragma unroll
-                for (int off = 1; off < PARTS; off <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-                if (live && part == 0) o[(size_t)(c0 + c) * heads * V + (size_t)h * V + j] = acc + skip * vj;
+                for (int e = 0; e < 4; ++e) { S[2 * m + nt][e] *= end; sl[nt][e] = 0.f; }
             }
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                uint32_t r[1][4];
+                cm_ldsm4t(r[0], st.k + (b * 16 + row_a) * QP + k0 + m * 16 + col_a);
+                cm_mma_rows(&S[2 * m], sl, wa[b], r);
+            }
+            cm_add(S[2 * m], sl[0]);
+            cm_add(S[2 * m + 1], sl[1]);
         }
     }
 #pragma unroll
-    for (int i = 0; i < KP; ++i) S_g[(size_t)i * nthr + tid] = S[i];
+    for (int nt = 0; nt < NT; ++nt) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (jr[e >> 1] < V) S_g[(size_t)jr[e >> 1] * NK + nt * 8 + c2 + (e & 1)] = S[nt][e];
+    }
+}
+
+// Mode 2 over bfloat16 prompts: sixteen tokens at a time (chunk_scan.cuh).  This is the first kernel: a block per (a few records,
+// head).
+template <int NK>
+__global__ void __launch_bounds__(2 * NK) channel_decay_prepare_kernel(ScanArgs A, ChunkRecord<NK, false>* __restrict__ recs,
+                                                                       const int* __restrict__ cu_q, int n_seqs, int n_records,
+                                                                       int per_block, int heads) {
+    pdl_prologue();
+    __shared__ __align__(16) float sq[CS_C * NK], sk[CS_C * NK], sa[CS_C * NK];
+    __shared__ __align__(16) ChunkHalves<NK, false> halves;
+    const int h = blockIdx.y, group = h / A.heads_per_group, tid = threadIdx.x;
+    const int row = tid / (NK / 8), col = tid % (NK / 8) * 8;
+    const bf16* qp = pdl_fresh((const bf16*)A.q) + A.q_off + (size_t)group * NK + col;
+    const bf16* kp = pdl_fresh((const bf16*)A.k) + A.k_off + (size_t)group * NK + col;
+    const float* cdp = pdl_fresh(A.channel_decay) + A.cd_off + (size_t)h * NK + col;
+    const int r0 = blockIdx.x * per_block, r1 = min(n_records, r0 + per_block);
+    int s, chunk, left = 0;
+    uint4 qv, kv;
+    float4 d0, d1;
+    auto fetch = [&](int r) {
+        chunk_of_record(cu_q, n_seqs, r, s, chunk);
+        qv = kv = make_uint4(0, 0, 0, 0);
+        d0 = d1 = make_float4(1.f, 1.f, 1.f, 1.f);
+        if (chunk < 0) return;
+        const int t0 = cu_q[s] + chunk * CS_C;
+        left = cu_q[s + 1] - t0;
+        if (row < left) {
+            qv = *reinterpret_cast<const uint4*>(qp + (size_t)(t0 + row) * A.q_stride);
+            kv = *reinterpret_cast<const uint4*>(kp + (size_t)(t0 + row) * A.k_stride);
+            d0 = *reinterpret_cast<const float4*>(cdp + (size_t)(t0 + row) * A.cd_stride);
+            d1 = *reinterpret_cast<const float4*>(cdp + (size_t)(t0 + row) * A.cd_stride + 4);
+        }
+    };
+    fetch(r0);
+    for (int r = r0; r < r1; ++r) {
+        const bool any = chunk >= 0;
+        if (any) {
+            float xq[8], xk[8];
+            chunk_unpack(qv, xq);
+            chunk_unpack(kv, xk);
+            const float xa[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) xq[i] *= A.q_scale;
+            chunk_stage8(sq + row * NK + col, xq);
+            chunk_stage8(sk + row * NK + col, xk);
+            chunk_stage8(sa + row * NK + col, xa);
+        }
+        __syncthreads();
+        if (r + 1 < r1) fetch(r + 1);
+        ChunkRecord<NK, false>* rec = recs + (size_t)r * heads + h;
+        if (any) {
+            chunk_scaled_rows<NK, false, false>(rec, halves, sq, sk, sa);
+            chunk_near_pairs<NK, false, false>(sq, sk, sa, nullptr, [&](int t, int u, float x, float) { chunk_put(rec->P[0], t, u, x); });
+        }
+        __syncthreads();
+        if (any) chunk_far_pairs<NK, false>(halves, [&](int t, int u, float x, float) { chunk_put_far(rec->P[0], t, u, x); });
+    }
 }
 
 // ------------------------------------------------------------------- decays from a low-rank projection --
@@ -542,39 +926,93 @@ FF_EXPORT int ff_conv_state_update(const void* in, int dtype, int in_stride, int
 
 // floats of a request's state for `heads` heads of key size N and value size V (-1: sizes not supported)
 FF_EXPORT long long ff_scan_state_floats(int heads, int N, int V) {
-    ScanPlan p;
-    if (!scan_plan(N, V, &p)) return -1;
-    return (long long)heads * p.vsplit * (p.NP / p.PARTS) * p.threads;
+    const int NP = ws_key_size(N);
+    if (!NP || V <= 0 || V > 256) return -1;
+    return (long long)heads * V * NP;
+}
+
+// Whether a step's recurrence runs a chunk at a time: bfloat16 prompts, long enough on average, sizes that the tiles take and
+// layouts that 16-byte copies take.  One decay per head and token (its inputs read as they are), or one per key channel.
+static bool scalar_chunk_sizes(int mode, int act, int T, int n_seqs, int N, int V) {
+    return mode != 2 && !act && (long long)T >= (long long)SCAN_CHUNK_MIN * n_seqs && (N == 64 || N == 128) && V % 8 == 0;
+}
+static bool channel_chunk_sizes(int mode, int act, int T, int n_seqs, int N, int V) {
+    return mode == 2 && !act && (long long)T >= (long long)CHANNEL_CHUNK_MIN * n_seqs && (N == 64 || N == 128) && V % 8 == 0;
+}
+static bool scan_layout_in_chunks(const ScanArgs& A, int heads) {
+    auto aligned = [](const void* p, int stride, int off, int per) { return ((uintptr_t)p & 15) == 0 && stride % per == 0 && off % per == 0; };
+    return heads % A.heads_per_group == 0 && aligned(A.q, A.q_stride, A.q_off, 8) && aligned(A.k, A.k_stride, A.k_off, 8) &&
+           aligned(A.v, A.v_stride, A.v_off, 8) && (A.mode != 2 || aligned(A.channel_decay, A.cd_stride, A.cd_off, 4));
+}
+
+// Bytes of scratch memory that a step of T tokens can use (0: none; without it the token-by-token kernel runs).
+FF_EXPORT long long ff_scan_scratch_bytes(int dtype, int mode, int act, int T, int n_seqs, int heads, int N, int V) {
+    if (dtype != 1 || T <= 0 || n_seqs <= 0 || heads <= 0 || V <= 0 || V > 256) return 0;
+    if (scalar_chunk_sizes(mode, act, T, n_seqs, N, V)) return chunk_records<SC_C>(T, n_seqs) * heads * (long long)sizeof(ScanRecord);
+    if (!channel_chunk_sizes(mode, act, T, n_seqs, N, V)) return 0;
+    return chunk_records(T, n_seqs) * heads * (long long)(N == 64 ? sizeof(ChunkRecord<64, false>) : sizeof(ChunkRecord<128, false>));
+}
+
+template <int NK>
+static int scan_chunk_launch(const ScanArgs& A, float* state, long long state_stride, int state_off, const int* cu_q, const int* state_slots,
+                             const int* seq_fresh, float* o, int T, int n_seqs, int heads, int V, void* scratch, cudaStream_t stream) {
+    ScanRecord* recs = (ScanRecord*)scratch;
+    FF_LAUNCH(scalar_decay_prepare_kernel<NK>, dim3((unsigned)chunk_records<SC_C>(T, n_seqs), heads / A.heads_per_group), 128, 0, stream, A, recs,
+              cu_q, n_seqs, heads);
+#define FF_SCAN_CHUNK(W)                                                                                                \
+    do {                                                                                                                \
+        const dim3 grid(n_seqs, heads, (V + 16 * W - 1) / (16 * W));                                                    \
+        const size_t smem = chunk_even_smem(sizeof(ScanChunkSmem<NK, W>), (long long)grid.x * grid.y * grid.z);         \
+        FF_SMEM_LIMIT((scalar_decay_chunk_kernel<NK, W>), 227 * 1024);                                                  \
+        FF_LAUNCH((scalar_decay_chunk_kernel<NK, W>), grid, 64 * W + CS_LOADERS, smem, stream,                          \
+                  A, recs, state, (size_t)state_stride, state_off, cu_q, state_slots, seq_fresh, o, heads, V);          \
+    } while (0)
+    // 64 value columns a block if that gives most SMs a block, else 32
+    if ((long long)n_seqs * heads * ((V + 63) / 64) >= 100) FF_SCAN_CHUNK(4);
+    else FF_SCAN_CHUNK(2);
+#undef FF_SCAN_CHUNK
+    FF_LAUNCH_CHECK();
+    return 0;
+}
+
+template <int NK>
+static int channel_chunk_launch(const ScanArgs& A, const ChunkScanArgs& B, int T, int n_seqs, void* scratch, cudaStream_t stream) {
+    const int n_records = (int)chunk_records(T, n_seqs), per_block = chunk_records_a_block((long long)n_records * B.heads);
+    FF_LAUNCH(channel_decay_prepare_kernel<NK>, dim3((n_records + per_block - 1) / per_block, B.heads), 2 * NK, 0, stream, A,
+              (ChunkRecord<NK, false>*)scratch, B.cu_q, n_seqs, n_records, per_block, B.heads);
+    return chunk_scan_launch<NK, false>(B, n_seqs, stream);
 }
 
 template <typename T>
 static int scan_launch(const ScanArgs& A, float* state, long long state_stride, int state_off, const int* cu_q,
-                       const int* state_slots, const int* seq_fresh, float* o, int n_seqs, int heads, int N, int V,
-                       cudaStream_t stream) {
-    ScanPlan p;
-    if (!scan_plan(N, V, &p)) return FF_ERR_UNSUPPORTED;
-    dim3 grid(n_seqs, heads, p.vsplit);
-    const bool pf = SCAN_CHUNK * p.NP <= SCAN_PFQ * p.threads && SCAN_CHUNK * p.Vb <= SCAN_PFV * p.threads;
-#define FF_SCAN_ONE(NP, PARTS, PF, CD)                                                                                  \
-    FF_LAUNCH((scalar_decay_scan_kernel<T, NP, PARTS, PF, CD>), grid, p.threads, 0, stream, A, state,                   \
-              (size_t)state_stride, state_off, cu_q, state_slots, seq_fresh, o, heads, N, V, p.Vb)
-#define FF_SCAN(NP, PARTS)                                                                                              \
+                       const int* state_slots, const int* seq_fresh, float* o, int T_tot, int n_seqs, int heads, int N, int V,
+                       void* scratch, long long scratch_bytes, cudaStream_t stream) {
+    if (!ws_key_size(N) || V <= 0 || V > 256) return FF_ERR_UNSUPPORTED;
+    if constexpr (sizeof(T) == 2) {
+        const long long need = ff_scan_scratch_bytes(1, A.mode, A.act, T_tot, n_seqs, heads, N, V);
+        if (need > 0 && scratch && scratch_bytes >= need && scan_layout_in_chunks(A, heads)) {
+            if (A.mode != 2) {
+                if (N == 64) return scan_chunk_launch<64>(A, state, state_stride, state_off, cu_q, state_slots, seq_fresh, o, T_tot, n_seqs, heads, V, scratch, stream);
+                return scan_chunk_launch<128>(A, state, state_stride, state_off, cu_q, state_slots, seq_fresh, o, T_tot, n_seqs, heads, V, scratch, stream);
+            }
+            const ChunkScanArgs B{scratch, (const bf16*)A.v, A.v_stride, A.v_off, state, state_stride, state_off, V * N, cu_q, state_slots, seq_fresh, o, heads, V};
+            return N == 64 ? channel_chunk_launch<64>(A, B, T_tot, n_seqs, scratch, stream) : channel_chunk_launch<128>(A, B, T_tot, n_seqs, scratch, stream);
+        }
+    }
+#define FF_SCAN_ONE(NP, CD)                                                                                             \
+    FF_LAUNCH((scalar_decay_scan_kernel<T, NP, CD>), dim3(n_seqs, heads, (V + WideState<NP>::VB - 1) / WideState<NP>::VB), \
+              WS_THREADS, 0, stream, A, state, (size_t)state_stride, state_off, cu_q, state_slots, seq_fresh, o, heads, N, V)
+#define FF_SCAN(NP)                                                                                                     \
     do {                                                                                                                \
-        if (A.mode == 2) {                                                                                              \
-            if (pf) FF_SCAN_ONE(NP, PARTS, true, true);                                                                 \
-            else FF_SCAN_ONE(NP, PARTS, false, true);                                                                   \
-        } else {                                                                                                        \
-            if (pf) FF_SCAN_ONE(NP, PARTS, true, false);                                                                \
-            else FF_SCAN_ONE(NP, PARTS, false, false);                                                                  \
-        }                                                                                                               \
+        if (A.mode == 2) FF_SCAN_ONE(NP, true);                                                                         \
+        else FF_SCAN_ONE(NP, false);                                                                                    \
     } while (0)
-    switch (p.NP) {
-        case 16: FF_SCAN(16, 4); break;
-        case 32: FF_SCAN(32, 8); break;
-        case 64: FF_SCAN(64, 8); break;
-        case 128: FF_SCAN(128, 8); break;
-        case 256: FF_SCAN(256, 8); break;
-        default: return FF_ERR_UNSUPPORTED;
+    switch (ws_key_size(N)) {
+        case 16: FF_SCAN(16); break;
+        case 32: FF_SCAN(32); break;
+        case 64: FF_SCAN(64); break;
+        case 128: FF_SCAN(128); break;
+        default: FF_SCAN(256); break;
     }
 #undef FF_SCAN
 #undef FF_SCAN_ONE
@@ -589,15 +1027,15 @@ FF_EXPORT int ff_scalar_decay_scan(const void* q, int q_stride, int q_off, const
                                    const float* channel_decay, int cd_stride, int cd_off, float q_scale, float* state,
                                    long long state_stride, int state_off, const int* cu_q, const int* state_slots,
                                    const int* seq_fresh, float* o, int T, int n_seqs, int heads, int N, int V,
-                                   cudaStream_t stream) {
+                                   void* scratch, long long scratch_bytes, cudaStream_t stream) {
     if (T <= 0 || n_seqs <= 0) return 0;
     if (heads_per_group <= 0 || mode < 0 || mode > 2 || (mode == 2 && !channel_decay)) return FF_ERR_BAD_ARG;
     ScanArgs A{q, q_stride, q_off, k, k_stride, k_off, v, v_stride, v_off, heads_per_group, act, decay,
                step, step_stride, step_off, step_bias, a_log, skip, mode, channel_decay, cd_stride, cd_off, q_scale};
     if (dtype == 0)
-        return scan_launch<float>(A, state, state_stride, state_off, cu_q, state_slots, seq_fresh, o, n_seqs, heads, N, V, stream);
+        return scan_launch<float>(A, state, state_stride, state_off, cu_q, state_slots, seq_fresh, o, T, n_seqs, heads, N, V, scratch, scratch_bytes, stream);
     if (dtype == 1)
-        return scan_launch<bf16>(A, state, state_stride, state_off, cu_q, state_slots, seq_fresh, o, n_seqs, heads, N, V, stream);
+        return scan_launch<bf16>(A, state, state_stride, state_off, cu_q, state_slots, seq_fresh, o, T, n_seqs, heads, N, V, scratch, scratch_bytes, stream);
     return FF_ERR_BAD_ARG;
 }
 

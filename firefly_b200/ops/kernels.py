@@ -905,6 +905,29 @@ def wkv_state_dim(dim: int) -> int:
     return 32 if dim <= 32 else (64 if dim <= 64 else 128)
 
 
+@functools.lru_cache(maxsize=4096)
+def _recurrence_scratch_bytes(module: str, entry: str, *sizes: int) -> int:
+    fn = getattr(_lib(module), entry)
+    fn.restype = ctypes.c_longlong
+    return int(fn(*[c_int(x) for x in sizes]))
+
+
+def _recurrence_scratch(ctx, module: str, entry: str, *sizes: int):
+    """Scratch memory for a recurrence that takes a step's prompts a chunk at a time: (pointer, bytes), nothing when the step
+    is none for it or the context has no workspace (the token-by-token kernel runs then)."""
+    ws = getattr(ctx, "workspace", None)
+    need = _recurrence_scratch_bytes(module, entry, *sizes) if ws is not None else 0
+    if need <= 0:
+        return c_void_p(0), ctypes.c_longlong(0)
+    return _p(ws.get("scan.records", (-(-need // 4),), torch.float32)), ctypes.c_longlong(need)
+
+
+def _count_preparing(scratch) -> None:
+    global LAUNCHES
+    if scratch[0].value:
+        LAUNCHES += 1     # the kernel that prepares the chunks
+
+
 def wkv_scan(rkvg, dlog, w0, u, state, prev_off: int, x, ctx, o, heads: int, dim: int) -> None:
     """The recurrence, token by token, one block per (sequence, head).  rkvg [4,T,heads*dim] (r, k, v, gate
     projections; the gate is not read here), dlog float32 [T,heads*dim] (the decay's inner logarithm without
@@ -1286,26 +1309,19 @@ def low_rank_decay(low, w: torch.Tensor, bias: torch.Tensor, tau: float, alpha: 
 SCAN_MAX_KEY, SCAN_MAX_VALUE = 256, 256
 
 
-def scan_plan(N: int, V: int):
-    """(key size the kernel is built for, threads that share a value column, blocks a head's columns are split
-    over, columns a block, threads a block): the recurrence kernel's layout for key size N and value size V
-    (the twin of `scan_plan` in csrc/ssm.cu; `scan_state_floats_of_kernel` is the kernel's own figure)."""
+def scan_key_size(N: int, V: int) -> int:
+    """The key size the recurrence kernel is built for that serves key size N (the twin of `ws_key_size` in
+    csrc/scan_wide.cuh; `scan_state_floats_of_kernel` is the kernel's own figure)."""
     if not (0 < N <= SCAN_MAX_KEY and 0 < V <= SCAN_MAX_VALUE):
         raise KernelError(f"recurrence: key size {N} / value size {V} not supported "
                           f"(up to {SCAN_MAX_KEY} / {SCAN_MAX_VALUE})")
-    pad = 16 if N <= 16 else (32 if N <= 32 else (64 if N <= 64 else (128 if N <= 128 else 256)))
-    parts = 8 if pad >= 32 else 4
-    max_cols = 512 // parts
-    vsplit = -(-V // max_cols)
-    vb = -(-V // vsplit)
-    return pad, parts, vsplit, vb, -(-(vb * parts) // 32) * 32
+    return 16 if N <= 16 else (32 if N <= 32 else (64 if N <= 64 else (128 if N <= 128 else 256)))
 
 
 def scan_state_floats(heads: int, N: int, V: int) -> int:
-    """Floats of a request's state for `heads` heads of key size N and value size V, in the recurrence
-    kernel's own layout (sizes rounded up to what the kernel is instantiated for)."""
-    pad, parts, vsplit, _, threads = scan_plan(N, V)
-    return heads * vsplit * (pad // parts) * threads
+    """Floats of a request's state for `heads` heads of key size N and value size V: [heads, V, N], N rounded up to what
+    the kernel is instantiated for."""
+    return heads * V * scan_key_size(N, V)
 
 
 def scan_state_floats_of_kernel(heads: int, N: int, V: int) -> int:
@@ -1496,7 +1512,8 @@ def head_norm_gate(o: torch.Tensor, gate, weight: torch.Tensor, eps: float, y: t
 def scalar_decay_scan(q, k, v, state: torch.Tensor, state_off: int, ctx, o: torch.Tensor, heads: int, N: int, V: int, *,
                       heads_per_group: int = 1, silu_inputs: bool = False, decay: Optional[torch.Tensor] = None,
                       step=None, step_bias=None, a_log=None, skip=None, channel_decay=None, q_scale: float = 1.0) -> None:
-    """S = a S + b k v^T, o = S^T q (+ skip * v) per head, token by token, one block per (sequence, head).
+    """S = a S + b k v^T, o = S^T q (+ skip * v) per head, token by token or (bfloat16 prompts, with ``ctx.workspace`` for scratch
+    memory) a chunk of tokens at a time.
     ``q``, ``k``, ``v``: (matrix [T, *], first column); a q/k row holds [groups, N], a v row [heads, V].
     Either ``decay`` float32 [heads] (a constant, b = 1), ``channel_decay`` = (float32 matrix, first column) whose rows
     hold [heads, N] decays (S = diag(a) S + k v^T), or ``step`` = (matrix, first column) with ``step_bias``,
@@ -1516,13 +1533,15 @@ def scalar_decay_scan(q, k, v, state: torch.Tensor, state_off: int, ctx, o: torc
     sm, s0 = step if step is not None else (None, 0)
     if mode == 1:
         assert sm.dtype == qm.dtype and step_bias is not None and a_log is not None
+    scratch = _recurrence_scratch(ctx, "ssm", "ff_scan_scratch_bytes", _dt(qm), mode, 1 if silu_inputs else 0, T, ctx.num_seqs, heads, N, V)
     _check(_lib("ssm").ff_scalar_decay_scan(
         _p(qm), c_int(qm.stride(0)), c_int(q0), _p(km), c_int(km.stride(0)), c_int(k0), _p(vm), c_int(vm.stride(0)),
         c_int(v0), c_int(_dt(qm)), c_int(heads_per_group), c_int(1 if silu_inputs else 0), c_int(mode), _p(decay),
         _p(sm), c_int(sm.stride(0) if sm is not None else 0), c_int(s0), _p(step_bias), _p(a_log), _p(skip),
         _p(cm), c_int(cm.stride(0) if cm is not None else 0), c_int(cd0), c_float(q_scale), _p(state),
         ctypes.c_longlong(state.stride(0)), c_int(state_off), _p(ctx.cu_q), _p(ctx.state_slots), _p(ctx.seq_fresh),
-        _p(o), c_int(T), c_int(ctx.num_seqs), c_int(heads), c_int(N), c_int(V), _stream()), "scalar_decay_scan")
+        _p(o), c_int(T), c_int(ctx.num_seqs), c_int(heads), c_int(N), c_int(V), *scratch, _stream()), "scalar_decay_scan")
+    _count_preparing(scratch)
 
 
 def gated_rms_norm(o: torch.Tensor, gate, weight: torch.Tensor, eps: float, y: torch.Tensor, parts: int,
