@@ -11,14 +11,15 @@
 // with q and k made unit vectors per head on the way in (x / sqrt(sum x^2 + unit_eps), q also times q_scale),
 // beta_t = sigmoid(raw beta) and g_t[i] = exp(-exp(A_log_h) * softplus(a_t[i] + dt_bias[i])).  Everything behind
 // the projections is 32-bit.  The state lives in the request's state slot and is carried from step to step; a
-// fresh request starts from zeros.  A sequence's tokens are walked in order with the same order of additions
-// however the prompt was cut into steps.
+// fresh request starts from zeros.  Steps of few tokens walk a sequence token by token; bfloat16 prompts are taken a chunk
+// of tokens at a time, whose sums are formed in another order, as right.
 //
 // One block per (sequence, head, share of the value columns).  Value column j is held by PARTS neighbouring
 // threads, each with NP / PARTS key channels of column j in registers; the two sums over key channels of a
 // token (the prediction and the read-out) are joined over those threads by shuffles.  For keys of 128 and more a
 // thread holds the same key channels of two neighbouring columns: what it reads of the staged q, k and g serves
 // both, and a head needs half the blocks.
+#include "chunk_scan.cuh"
 #include "common.cuh"
 
 namespace ff {
@@ -77,15 +78,20 @@ __global__ void __launch_bounds__(DR_MAX_THREADS) delta_rule_scan_kernel(
 #pragma unroll
     for (int x = 0; x < VJ; ++x) live[x] = jl * VJ + x < Vb && j0 + jl * VJ + x < V;
     const bool fresh = seq_fresh[s] != 0;
-    // a block's share of a head's state is kept as its threads hold it: register (x, i) of thread tid at
-    // (x * KP + i) * threads + tid
-    float* S_g = state + (size_t)state_slots[s] * state_stride + state_off +
-                 ((size_t)h * gridDim.z + blockIdx.z) * KP * VJ * nthr;
+    // a head's state lies in the slot as [V][NP], whatever kernel wrote it
+    float* S_g = state + (size_t)state_slots[s] * state_stride + state_off + (size_t)h * V * NP;
+    const bool vec = ((uintptr_t)S_g & 15) == 0;
     float S[VJ][KP];
 #pragma unroll
     for (int x = 0; x < VJ; ++x) {
 #pragma unroll
-        for (int i = 0; i < KP; ++i) S[x][i] = fresh ? 0.f : S_g[(size_t)(x * KP + i) * nthr + tid];
+        for (int i = 0; i < KP; i += 4) {
+            // thread `part` holds key channels 4 PARTS m + 4 part + e (m = i / 4, e < 4)
+            const float* p = S_g + (size_t)(j0 + jl * VJ + x) * NP + i * PARTS + part * 4;
+            float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (!fresh && live[x]) r = vec ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
+            S[x][i] = r.x; S[x][i + 1] = r.y; S[x][i + 2] = r.z; S[x][i + 3] = r.w;
+        }
     }
     const int group = h / A.heads_per_group;
     const T* qp = pdl_fresh((const T*)A.q) + A.q_off + (size_t)group * N;
@@ -243,7 +249,122 @@ __global__ void __launch_bounds__(DR_MAX_THREADS) delta_rule_scan_kernel(
 #pragma unroll
     for (int x = 0; x < VJ; ++x) {
 #pragma unroll
-        for (int i = 0; i < KP; ++i) S_g[(size_t)(x * KP + i) * nthr + tid] = S[x][i];
+        for (int i = 0; i < KP; i += 4) {
+            float* p = S_g + (size_t)(j0 + jl * VJ + x) * NP + i * PARTS + part * 4;
+            if (!live[x]) continue;
+            if (vec) *reinterpret_cast<float4*>(p) = make_float4(S[x][i], S[x][i + 1], S[x][i + 2], S[x][i + 3]);
+            else { p[0] = S[x][i]; p[1] = S[x][i + 1]; p[2] = S[x][i + 2]; p[3] = S[x][i + 3]; }
+        }
+    }
+}
+
+// Prompts in bfloat16, sixteen tokens at a time (chunk_scan.cuh): the first kernel, a block per (a few records, head).  It makes
+// q and k unit vectors, forms the decays, the products of pairs of tokens, and the inverse of the unit lower triangle by
+// forward substitution, a column a thread.
+// 4 x 2048 tokens, 8 heads of 128 x 128: token by token 1373 us, the two kernels 135 + 216.
+template <int NK>
+__global__ void __launch_bounds__(2 * NK) delta_prepare_kernel(DeltaArgs A, ChunkRecord<NK, true>* __restrict__ recs,
+                                                               const int* __restrict__ cu_q, int n_seqs, int n_records, int per_block, int heads) {
+    pdl_prologue();
+    __shared__ __align__(16) float sq[CS_C * NK], sk[CS_C * NK], sa[CS_C * NK];
+    __shared__ __align__(16) ChunkHalves<NK, true> halves;
+    __shared__ float sM[CS_C][CS_C + 1], s_beta[CS_C];
+    const int h = blockIdx.y, group = h / A.heads_per_group, tid = threadIdx.x;
+    const int row = tid / (NK / 8), col = tid % (NK / 8) * 8;
+    const bf16* qp = pdl_fresh((const bf16*)A.q) + A.q_off + (size_t)group * NK + col;
+    const bf16* kp = pdl_fresh((const bf16*)A.k) + A.k_off + (size_t)group * NK + col;
+    const bf16* bp = pdl_fresh((const bf16*)A.beta) + A.beta_off + h;
+    const float* ap = pdl_fresh(A.a) + A.a_off + (A.decay_per_head ? (size_t)h : (size_t)h * NK + col);
+    const float rate = expf(A.a_log[h]);
+    float bias[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) bias[i] = A.dt_bias[A.decay_per_head ? h : h * NK + col + i];
+    const int r0 = blockIdx.x * per_block, r1 = min(n_records, r0 + per_block);
+    int s, chunk, left = 0;
+    uint4 qv, kv;
+    float4 d0, d1;
+    float braw = 0.f;
+    auto fetch = [&](int r) {
+        chunk_of_record(cu_q, n_seqs, r, s, chunk);
+        qv = kv = make_uint4(0, 0, 0, 0);
+        d0 = d1 = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (chunk < 0) return;
+        const int t0 = cu_q[s] + chunk * CS_C;
+        left = cu_q[s + 1] - t0;
+        if (row < left) {
+            qv = *reinterpret_cast<const uint4*>(qp + (size_t)(t0 + row) * A.q_stride);
+            kv = *reinterpret_cast<const uint4*>(kp + (size_t)(t0 + row) * A.k_stride);
+            const float* a = ap + (size_t)(t0 + row) * A.a_stride;
+            if (A.decay_per_head) d0.x = *a;
+            else {
+                d0 = *reinterpret_cast<const float4*>(a);
+                d1 = *reinterpret_cast<const float4*>(a + 4);
+            }
+            if (col == 0) braw = to_float(bp[(size_t)(t0 + row) * A.beta_stride]);
+        }
+    };
+    fetch(r0);
+    for (int r = r0; r < r1; ++r) {
+        const bool any = chunk >= 0, in = row < left;
+        ChunkRecord<NK, true>* rec = recs + (size_t)r * heads + h;
+        if (any) {
+            float xq[8], xk[8], xa[8];
+            chunk_unpack(qv, xq);
+            chunk_unpack(kv, xk);
+            float qq = 0.f, kk = 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) { qq += xq[i] * xq[i]; kk += xk[i] * xk[i]; }
+#pragma unroll
+            for (int off = 1; off < NK / 8; off <<= 1) {
+                qq += __shfl_xor_sync(0xffffffffu, qq, off);
+                kk += __shfl_xor_sync(0xffffffffu, kk, off);
+            }
+            const float fq = A.q_scale / sqrtf(qq + A.unit_eps), fk = 1.0f / sqrtf(kk + A.unit_eps);
+            const float d[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
+            if (A.decay_per_head) {
+                const float gd = in ? expf(-rate * dr_softplus(d[0] + bias[0])) : 1.f;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) xa[i] = gd;
+            } else {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) xa[i] = in ? expf(-rate * dr_softplus(d[i] + bias[i])) : 1.f;
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) { xq[i] *= fq; xk[i] *= fk; }
+            chunk_stage8(sq + row * NK + col, xq);
+            chunk_stage8(sk + row * NK + col, xk);
+            chunk_stage8(sa + row * NK + col, xa);
+            if (col == 0) s_beta[row] = in ? 1.0f / (1.0f + expf(-braw)) : 0.f;
+        }
+        __syncthreads();
+        if (r + 1 < r1) fetch(r + 1);
+        if (any) {
+            chunk_scaled_rows<NK, true, false>(rec, halves, sq, sk, sa);
+            chunk_near_pairs<NK, true, false>(sq, sk, sa, nullptr, [&](int t, int u, float x, float y) {
+                chunk_put(rec->P[0], t, u, x);
+                sM[t][u] = s_beta[t] * y;
+            });
+        }
+        __syncthreads();
+        if (any) {
+            chunk_far_pairs<NK, true>(halves, [&](int t, int u, float x, float y) {
+                chunk_put_far(rec->P[0], t, u, x);
+                sM[t][u] = s_beta[t] * y;
+            });
+        }
+        __syncthreads();
+        if (any && tid < CS_C) {
+            float x[CS_C];
+#pragma unroll
+            for (int t = 0; t < CS_C; ++t) {
+                float y = t == tid ? s_beta[t] : 0.f;
+#pragma unroll
+                for (int u = 0; u < t; ++u) y -= sM[t][u] * x[u];
+                x[t] = y;
+                chunk_put(rec->TB[0], t, tid, y);
+            }
+        }
+        __syncthreads();
     }
 }
 
@@ -280,7 +401,31 @@ using namespace ff;
 FF_EXPORT long long ff_delta_state_floats(int heads, int N, int V) {
     DeltaPlan p;
     if (!delta_plan(N, V, &p)) return -1;
-    return (long long)heads * p.vsplit * (p.NP / p.PARTS) * p.VJ * p.threads;
+    return (long long)heads * V * p.NP;
+}
+
+// Tokens a sequence (average of a step) from which chunks are taken (us, chunked / token by token, 8 heads of 128 x 128: eight sequences
+// of 32 37.9 / 23.5, of 64 24.9 / 44.2; one of 64 17.4 / 43.7).
+constexpr int DELTA_CHUNK_MIN = 48;
+
+// Bytes of scratch memory that a step of T tokens can use (0: none; without it the token-by-token kernel runs).
+FF_EXPORT long long ff_delta_scratch_bytes(int dtype, int T, int n_seqs, int heads, int N, int V) {
+    if (dtype != 1 || T <= 0 || n_seqs <= 0 || (long long)T < (long long)DELTA_CHUNK_MIN * n_seqs || (N != 64 && N != 128) || V <= 0 || V > 256 || V % 8) return 0;
+    return chunk_records(T, n_seqs) * heads * (long long)(N == 64 ? sizeof(ChunkRecord<64, true>) : sizeof(ChunkRecord<128, true>));
+}
+
+static bool delta_layout_in_chunks(const DeltaArgs& A) {
+    auto aligned = [](const void* p, int stride, int off, int per) { return ((uintptr_t)p & 15) == 0 && stride % per == 0 && off % per == 0; };
+    return aligned(A.q, A.q_stride, A.q_off, 8) && aligned(A.k, A.k_stride, A.k_off, 8) && aligned(A.v, A.v_stride, A.v_off, 8) &&
+           (A.decay_per_head || aligned(A.a, A.a_stride, A.a_off, 4));
+}
+
+template <int NK>
+static int delta_chunk_launch(const DeltaArgs& A, const ChunkScanArgs& B, int T, int n_seqs, void* scratch, cudaStream_t stream) {
+    const int n_records = (int)chunk_records(T, n_seqs), per_block = chunk_records_a_block((long long)n_records * B.heads);
+    FF_LAUNCH(delta_prepare_kernel<NK>, dim3((n_records + per_block - 1) / per_block, B.heads), 2 * NK, 0, stream, A,
+              (ChunkRecord<NK, true>*)scratch, B.cu_q, n_seqs, n_records, per_block, B.heads);
+    return chunk_scan_launch<NK, true>(B, n_seqs, stream);
 }
 
 template <typename T>
@@ -313,11 +458,16 @@ FF_EXPORT int ff_delta_rule_scan(const void* q, int q_stride, int q_off, const v
                                  const float* a_log, int decay_per_head, int heads_per_group, float q_scale, float unit_eps, float* state,
                                  long long state_stride, int state_off, const int* cu_q, const int* state_slots,
                                  const int* seq_fresh, float* o, int T, int n_seqs, int heads, int N, int V,
-                                 cudaStream_t stream) {
+                                 void* scratch, long long scratch_bytes, cudaStream_t stream) {
     if (T <= 0 || n_seqs <= 0) return 0;
     if (heads_per_group <= 0 || heads % heads_per_group) return FF_ERR_BAD_ARG;
     DeltaArgs A{q, q_stride, q_off, k, k_stride, k_off, v, v_stride, v_off, beta, beta_stride, beta_off,
                 a, a_stride, a_off, dt_bias, a_log, heads_per_group, q_scale, unit_eps, decay_per_head ? 1 : 0};
+    const long long need = ff_delta_scratch_bytes(dtype, T, n_seqs, heads, N, V);
+    if (need > 0 && scratch && scratch_bytes >= need && delta_layout_in_chunks(A)) {
+        const ChunkScanArgs B{scratch, (const bf16*)v, v_stride, v_off, state, state_stride, state_off, V * N, cu_q, state_slots, seq_fresh, o, heads, V};
+        return N == 64 ? delta_chunk_launch<64>(A, B, T, n_seqs, scratch, stream) : delta_chunk_launch<128>(A, B, T, n_seqs, scratch, stream);
+    }
     if (dtype == 0)
         return delta_launch<float>(A, state, state_stride, state_off, cu_q, state_slots, seq_fresh, o, n_seqs, heads, N, V, stream);
     if (dtype == 1)

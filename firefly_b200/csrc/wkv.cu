@@ -8,9 +8,11 @@
 //
 // The state (S and the last x of the sequence) lives in 32-bit in the request's state slot and
 // is carried from step to step; a fresh request starts from zeros.  Everything that enters the
-// recurrence is 32-bit: decays, the bonus u, S, the sums.  Tokens are walked one after the other,
-// each with the same order of additions, so the result does not depend on how a prompt was cut into steps.
+// recurrence is 32-bit: decays, the bonus u, S, the sums.  Steps of few tokens walk a sequence token by token; bfloat16
+// prompts are taken a chunk of tokens at a time, whose sums are formed in another order, as right.
+#include "chunk_scan.cuh"
 #include "common.cuh"
+#include "scan_wide.cuh"
 
 namespace ff {
 
@@ -48,119 +50,203 @@ __global__ void tanh_cast_kernel(const float* __restrict__ in, TO* __restrict__ 
     if (idx < total) out[idx] = from_float<TO>(tanhf(in[idx]));
 }
 
-constexpr int WKV_CHUNK = 8;     // tokens whose r, k, w are staged in shared memory at a time
-// threads that share a column of S, each with a share of its key channels (a block has DIM * parts threads).
-// Eight were tried up to head size 64 and were slower than four (1.30 against 1.11 ms for eight prompts of 2048).
-constexpr int wkv_parts(int dim) { return 4; }
-
-// One block per (sequence, head).  A column j of S (value channel j) is held by WKV_PARTS neighbouring
-// threads, each with DIM / WKV_PARTS key channels in registers, so a token costs DIM / WKV_PARTS steps of the
-// serial chain and two or three shuffles.  The bonus term's factors p_i = r_i u_i k_i are formed while a chunk is
-// staged, so the inner loop has one multiply-add for it.
-//   o_j = sum_i (r_i S_ij + p_i v_j);   S_ij <- w_i S_ij + k_i v_j
-template <typename T, int DIM, int WKV_PARTS>
-__global__ void __launch_bounds__(DIM * WKV_PARTS) wkv_scan_kernel(
-    const T* __restrict__ rkvg /*[4,T,HD]*/, const float* __restrict__ dlog /*[T,HD]*/,
+// One block per (sequence, head, VB value channels), token by token (scan_wide.cuh): a thread holds four columns of S and
+// reads r, k and w of its key channels once for all four.  A chunk's r, k, v and decays are staged in 32-bit in one of two
+// buffers, asked for before the chunk in front is walked.  The bonus term's sum p = sum_i r_i u_i k_i is formed on the way, a
+// thread's share of it from the u of its own key channels.
+//   o_j = sum_i r_i S_ij + p v_j;   S_ij <- w_i S_ij + k_i v_j
+// Against one column a thread 518 -> 185 us for a sequence of 999 tokens, 16 heads of 64.
+template <typename T, int DIM>
+__global__ void __launch_bounds__(WS_THREADS) wkv_scan_kernel(
+    const T* __restrict__ rkvg_ /*[4,T,HD]*/, const float* __restrict__ dlog_ /*[T,HD]*/,
     const float* __restrict__ w0, const float* __restrict__ u, float* __restrict__ state, size_t state_stride,
-    int prev_off, const T* __restrict__ x, int W, const int* __restrict__ cu_q,
+    int prev_off, const T* __restrict__ x_, int W, const int* __restrict__ cu_q,
     const int* __restrict__ state_slots, const int* __restrict__ seq_fresh, float* __restrict__ o /*[T,HD]*/,
     int Ttot, int heads, int dim) {
     pdl_prologue();
-    constexpr int KP = DIM / WKV_PARTS;          // key channels a thread holds
-    __shared__ __align__(16) float s_r[WKV_CHUNK][DIM], s_k[WKV_CHUNK][DIM], s_w[WKV_CHUNK][DIM], s_p[WKV_CHUNK][DIM];
-    __shared__ float s_v[WKV_CHUNK][DIM];
-    const int s = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
-    // thread `part` of a column holds key channels 4 WKV_PARTS m + 4 part + e (m < KP / 4, e < 4): the parts of a
-    // column then read neighbouring 16-byte pieces of shared memory, which lie in different banks
-    const int j = tid / WKV_PARTS, part = tid % WKV_PARTS;
-    auto chan = [&](int i) { return (i >> 2) * (4 * WKV_PARTS) + part * 4 + (i & 3); };
+    using WS = WideState<DIM>;
+    constexpr int CH = WS::CH, VB = WS::VB < DIM ? WS::VB : DIM, PQ = CH * DIM / WS_THREADS, PV = CH * VB / WS_THREADS;
+    static_assert(CH * DIM % WS_THREADS == 0 && CH * VB % WS_THREADS == 0 && WS_THREADS % DIM == 0, "a thread stages one channel of the same number of tokens");
+    __shared__ __align__(16) float s_r[2][CH][DIM], s_k[2][CH][DIM], s_w[2][CH][DIM];
+    __shared__ __align__(16) f32x2 s_v[2][CH][VB];             // each value twice
+    const int s = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, j0 = blockIdx.z * VB;
     const int t0 = cu_q[s], t1 = cu_q[s + 1];
     const int HD = heads * dim;
-    const bool live = j < dim;
     float* st = state + (size_t)state_slots[s] * state_stride;
-    // A head's state is kept in the slot as this kernel's threads hold it: element (register i, thread tid) at
-    // i * blockDim + tid, DIM * DIM floats a head, so that loading and storing it is coalesced.  Only this kernel
-    // reads it, and a layer always runs the same instantiation.
     float* S_g = st + (size_t)h * DIM * DIM;
-    const bool fresh = seq_fresh[s] != 0;
-    float S[KP];
+    const bool holds = tid < WS::PARTS * (VB / WS_COLS);       // heads of 32: more threads than columns
+    WS w;
+    w.place(tid);
+    w.load(S_g, j0, holds ? dim : 0, seq_fresh[s] != 0);
+    f32x2 ub[WS::KP / 2];
 #pragma unroll
-    for (int i = 0; i < KP; ++i) S[i] = (live && chan(i) < dim && !fresh) ? S_g[i * (DIM * WKV_PARTS) + tid] : 0.f;
-    // staging: thread c < dim takes channel c of every token of a chunk.  The next chunk's values are asked
-    // for (into registers) before the current chunk is computed, so their latency hides behind the recurrence.
-    const bool stager = tid < DIM, s_live = tid < dim;
-    const float w0c = (stager && s_live) ? w0[h * dim + tid] : 0.f;
-    const float uc = (stager && s_live) ? u[h * dim + tid] : 0.f;
-    const T* r_in = rkvg;
-    const T* k_in = rkvg + (size_t)Ttot * HD;
-    const T* v_in = rkvg + (size_t)2 * Ttot * HD;
-    T rn[WKV_CHUNK], kn[WKV_CHUNK], vn[WKV_CHUNK];
-    float dn[WKV_CHUNK];
+    for (int m = 0; m < WS::KP / 2; ++m) {
+        const int i = (m >> 1) * 4 * WS::PARTS + w.part * 4 + (m & 1) * 2;
+        ub[m] = f2_pack(i < dim ? u[h * dim + i] : 0.f, i + 1 < dim ? u[h * dim + i + 1] : 0.f);
+    }
+    const T* r_in = pdl_fresh(rkvg_) + (size_t)h * dim;
+    const T* k_in = r_in + (size_t)Ttot * HD;
+    const T* v_in = k_in + (size_t)Ttot * HD + j0;
+    const float* d_in = pdl_fresh(dlog_) + (size_t)h * dim;
+    const int ch = tid % DIM;                                  // the thread's channel of every token it stages
+    const float w0c = ch < dim ? w0[h * dim + ch] : 0.f;
+    T rn[PQ], kn[PQ], vn[PV];
+    float dn[PQ];
     auto fetch = [&](int c0) {
+        const int n = min(CH, t1 - c0);
 #pragma unroll
-        for (int c = 0; c < WKV_CHUNK; ++c) {
-            const bool in = stager && s_live && c0 + c < t1;
-            const size_t at = in ? (size_t)(c0 + c) * HD + h * dim + tid : 0;
-            rn[c] = in ? r_in[at] : from_float<T>(0.f);
-            kn[c] = in ? k_in[at] : from_float<T>(0.f);
-            vn[c] = in ? v_in[at] : from_float<T>(0.f);
-            dn[c] = in ? dlog[at] : 0.f;
+        for (int p = 0; p < PQ; ++p) {
+            const int c = (tid + p * WS_THREADS) / DIM;
+            const bool in = c < n && ch < dim;
+            const size_t at = in ? (size_t)(c0 + c) * HD + ch : 0;
+            rn[p] = in ? r_in[at] : from_float<T>(0.f);
+            kn[p] = in ? k_in[at] : from_float<T>(0.f);
+            dn[p] = in ? d_in[at] : 0.f;
+        }
+#pragma unroll
+        for (int p = 0; p < PV; ++p) {
+            const int idx = tid + p * WS_THREADS, c = idx / VB, jj = idx % VB;
+            vn[p] = (c < n && j0 + jj < dim) ? v_in[(size_t)(c0 + c) * HD + jj] : from_float<T>(0.f);
         }
     };
-    fetch(t0);
-    for (int c0 = t0; c0 < t1; c0 += WKV_CHUNK) {
-        const int n = min(WKV_CHUNK, t1 - c0);
-        __syncthreads();
-        if (stager) {
+    auto stage = [&](int b) {
 #pragma unroll
-            for (int c = 0; c < WKV_CHUNK; ++c) {
-                const bool in = s_live && c < n;
-                const float rv = to_float(rn[c]), kv = to_float(kn[c]);
-                s_r[c][tid] = rv;
-                s_k[c][tid] = kv;
-                s_v[c][tid] = to_float(vn[c]);
-                s_w[c][tid] = in ? expf(-expf(dn[c] + w0c)) : 1.f;
-                s_p[c][tid] = rv * uc * kv;
-            }
+        for (int p = 0; p < PQ; ++p) {
+            const int idx = tid + p * WS_THREADS;
+            (&s_r[b][0][0])[idx] = to_float(rn[p]);
+            (&s_k[b][0][0])[idx] = to_float(kn[p]);
+            (&s_w[b][0][0])[idx] = expf(-expf(dn[p] + w0c));
         }
-        __syncthreads();
-        if (c0 + WKV_CHUNK < t1) fetch(c0 + WKV_CHUNK);
-        // Four partial sums shorten the chain inside a token.  (Computing all eight places of a chunk without a
-        // branch, the places past the portion's end staged as values that leave S alone, was no faster for
-        // prompts, 1.07 against 1.11 ms, and made a step of single tokens half again as slow.)  What bounds a
-        // token is the shared-memory pipe: every thread reads r, k, w and p of its sixteen channels.
 #pragma unroll
-        for (int c = 0; c < WKV_CHUNK; ++c) {
-            if (c < n) {
-                const float vj = s_v[c][j];
-                float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-#pragma unroll
-                for (int i = 0; i < KP; i += 4) {
-                    const int at = i * WKV_PARTS + part * 4;      // = chan(i), i a multiple of 4
-                    const float4 r4 = *reinterpret_cast<const float4*>(&s_r[c][at]);
-                    const float4 k4 = *reinterpret_cast<const float4*>(&s_k[c][at]);
-                    const float4 w4 = *reinterpret_cast<const float4*>(&s_w[c][at]);
-                    const float4 p4 = *reinterpret_cast<const float4*>(&s_p[c][at]);
-                    a0 += r4.x * S[i] + p4.x * vj;     S[i]     = w4.x * S[i]     + k4.x * vj;
-                    a1 += r4.y * S[i + 1] + p4.y * vj; S[i + 1] = w4.y * S[i + 1] + k4.y * vj;
-                    a2 += r4.z * S[i + 2] + p4.z * vj; S[i + 2] = w4.z * S[i + 2] + k4.z * vj;
-                    a3 += r4.w * S[i + 3] + p4.w * vj; S[i + 3] = w4.w * S[i + 3] + k4.w * vj;
-                }
-                float acc = (a0 + a1) + (a2 + a3);
-                acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-                acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-                if (WKV_PARTS == 8) acc += __shfl_xor_sync(0xffffffffu, acc, 4);
-                if (live && part == 0) o[(size_t)(c0 + c) * HD + h * dim + j] = acc;
-            }
-        }
+        for (int p = 0; p < PV; ++p) (&s_v[b][0][0])[tid + p * WS_THREADS] = f2_pack(to_float(vn[p]), to_float(vn[p]));
+    };
+    const int vj = holds ? w.jl * WS_COLS : 0, first = w.first();
+    float* oh = o + (size_t)h * dim + j0;
+    if (t0 < t1) {
+        fetch(t0);
+        stage(0);
     }
+    __syncthreads();
+    int b = 0;
+    for (int c0 = t0; c0 < t1; c0 += CH, b ^= 1) {
+        const int n = min(CH, t1 - c0);
+        if (c0 + CH < t1) fetch(c0 + CH);
+        auto token = [&](int c, float* part) {
+            f32x2 v[WS_COLS];
+            WS::values(&s_v[b][c][vj], v);
+            w.template token<true, true>(s_r[b][c], s_k[b][c], s_w[b][c], 1.f, v, part);
+            f32x2 p2 = 0ull;
 #pragma unroll
-    for (int i = 0; i < KP; ++i) S_g[i * (DIM * WKV_PARTS) + tid] = (live && chan(i) < dim) ? S[i] : 0.f;
+            for (int m = 0; m < WS::KP / 4; ++m) {
+                const int at = m * 4 * WS::PARTS + w.part * 4;
+                const ulonglong2 r2 = *reinterpret_cast<const ulonglong2*>(&s_r[b][c][at]);
+                const ulonglong2 k2 = *reinterpret_cast<const ulonglong2*>(&s_k[b][c][at]);
+                p2 = f2_fma(f2_mul(r2.x, ub[2 * m]), k2.x, p2);
+                p2 = f2_fma(f2_mul(r2.y, ub[2 * m + 1]), k2.y, p2);
+            }
+            const float p = f2_sum(p2);
+#pragma unroll
+            for (int x = 0; x < WS_COLS; ++x) part[x] += p * f2_low(v[x]);
+        };
+        if (n == CH) {
+            float part[CH * WS_COLS];
+#pragma unroll
+            for (int c = 0; c < CH; ++c) token(c, part + c * WS_COLS);
+            w.reduce_chunk(part);
+#pragma unroll
+            for (int r = 0; r < WS::OUTS; ++r) {
+                const int at = first + r, jj = w.jl * WS_COLS + at % WS_COLS;
+                if (holds && j0 + jj < dim) oh[(size_t)(c0 + at / WS_COLS) * HD + jj] = part[r];
+            }
+        } else {
+            for (int c = 0; c < n; ++c) {
+                float part[WS_COLS];
+                token(c, part);
+                const float y = w.reduce(part);
+                const int jj = w.jl * WS_COLS + w.col();
+                if (holds && w.part < 4 && j0 + jj < dim) oh[(size_t)(c0 + c) * HD + jj] = y;
+            }
+        }
+        if (c0 + CH < t1) stage(b ^ 1);
+        __syncthreads();
+    }
+    w.store(S_g, j0, holds ? dim : 0);
     // the sequence's last input row, for the first token of its next step
-    if (h == 0 && t1 > t0) {
-        const T* last = x + (size_t)(t1 - 1) * W;
-        for (int i = tid; i < W; i += DIM * WKV_PARTS) st[prev_off + i] = to_float(last[i]);
-        static_assert(WKV_PARTS == 4 || WKV_PARTS == 8, "the sum over a column's threads is two or three shuffles");
+    if (h == 0 && blockIdx.z == 0 && t1 > t0) {
+        const T* last = pdl_fresh(x_) + (size_t)(t1 - 1) * W;
+        for (int i = tid; i < W; i += WS_THREADS) st[prev_off + i] = to_float(last[i]);
+    }
+}
+
+// Prompts in bfloat16, sixteen tokens at a time (chunk_scan.cuh): the first kernel, a block per (a few records, head).  The
+// read-out sees the state in front of the token's own decay and write; the bonus term is the diagonal of P.
+template <int NK>
+__global__ void __launch_bounds__(2 * NK) wkv_prepare_kernel(const bf16* rkvg, const float* dlog, const float* __restrict__ w0,
+                                                             const float* __restrict__ u, ChunkRecord<NK, false>* __restrict__ recs,
+                                                             float* __restrict__ state, size_t state_stride, int prev_off, const bf16* x, int W,
+                                                             const int* __restrict__ cu_q, const int* __restrict__ state_slots, int n_seqs,
+                                                             int n_records, int per_block, int Ttot, int heads) {
+    pdl_prologue();
+    __shared__ __align__(16) float sr[CS_C * NK], sk[CS_C * NK], sw[CS_C * NK], su[NK];
+    __shared__ __align__(16) ChunkHalves<NK, false> halves;
+    const int h = blockIdx.y, HD = heads * NK, tid = threadIdx.x;
+    const int row = tid / (NK / 8), col = tid % (NK / 8) * 8;
+    const bf16* rp = pdl_fresh(rkvg) + h * NK + col;
+    const bf16* kp = rp + (size_t)Ttot * HD;
+    const float* dp = pdl_fresh(dlog) + h * NK + col;
+    float w0c[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) w0c[i] = w0[h * NK + col + i];
+    if (tid < NK) su[tid] = u[h * NK + tid];
+    const int r0 = blockIdx.x * per_block, r1 = min(n_records, r0 + per_block);
+    int s, chunk, t0 = 0, left = 0;
+    uint4 rv, kv;
+    float4 d0, d1;
+    auto fetch = [&](int r) {
+        chunk_of_record(cu_q, n_seqs, r, s, chunk);
+        rv = kv = make_uint4(0, 0, 0, 0);
+        d0 = d1 = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (chunk < 0) return;
+        t0 = cu_q[s] + chunk * CS_C;
+        left = cu_q[s + 1] - t0;
+        if (row < left) {
+            const size_t at = (size_t)(t0 + row) * HD;
+            rv = *reinterpret_cast<const uint4*>(rp + at);
+            kv = *reinterpret_cast<const uint4*>(kp + at);
+            d0 = *reinterpret_cast<const float4*>(dp + at);
+            d1 = *reinterpret_cast<const float4*>(dp + at + 4);
+        }
+    };
+    fetch(r0);
+    for (int r = r0; r < r1; ++r) {
+        const bool any = chunk >= 0, in = row < left;
+        if (any) {
+            float xr[8], xk[8], xw[8];
+            chunk_unpack(rv, xr);
+            chunk_unpack(kv, xk);
+            const float d[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) xw[i] = in ? expf(-expf(d[i] + w0c[i])) : 1.f;
+            chunk_stage8(sr + row * NK + col, xr);
+            chunk_stage8(sk + row * NK + col, xk);
+            chunk_stage8(sw + row * NK + col, xw);
+        }
+        __syncthreads();
+        const int seq = s, first_row = t0, rows = left;
+        if (r + 1 < r1) fetch(r + 1);
+        ChunkRecord<NK, false>* rec = recs + (size_t)r * heads + h;
+        if (any) {
+            chunk_scaled_rows<NK, false, true>(rec, halves, sr, sk, sw);
+            chunk_near_pairs<NK, false, true>(sr, sk, sw, su, [&](int t, int i, float y, float) { chunk_put(rec->P[0], t, i, y); });
+            // the sequence's last input row, for the first token of its next step
+            if (h == 0 && rows <= CS_C) {
+                const bf16* last = pdl_fresh(x) + (size_t)(first_row + rows - 1) * W;
+                float* prev = state + (size_t)state_slots[seq] * state_stride + prev_off;
+                for (int i = tid; i < W; i += 2 * NK) prev[i] = to_float(last[i]);
+            }
+        }
+        __syncthreads();
+        if (any) chunk_far_pairs<NK, false>(halves, [&](int t, int i, float y, float) { chunk_put_far(rec->P[0], t, i, y); });
     }
 }
 
@@ -218,10 +304,9 @@ static int wkv_scan_launch(const void* rkvg, const float* dlog, const float* w0,
                            long long state_stride, int prev_off, const void* x, int W, const int* cu_q,
                            const int* state_slots, const int* seq_fresh, float* o, int Ttot, int n_seqs, int heads,
                            int dim, cudaStream_t stream) {
-    dim3 grid(n_seqs, heads);
 #define FF_WKV(D)                                                                                                  \
-    FF_LAUNCH((wkv_scan_kernel<T, D, wkv_parts(D)>), grid, D * wkv_parts(D), 0, stream, (const T*)rkvg, dlog, w0, u, state, (size_t)state_stride, \
-              prev_off, (const T*)x, W, cu_q, state_slots, seq_fresh, o, Ttot, heads, dim)
+    FF_LAUNCH((wkv_scan_kernel<T, D>), dim3(n_seqs, heads, (dim + min(D, WideState<D>::VB) - 1) / min(D, WideState<D>::VB)), WS_THREADS, 0, stream, \
+              (const T*)rkvg, dlog, w0, u, state, (size_t)state_stride, prev_off, (const T*)x, W, cu_q, state_slots, seq_fresh, o, Ttot, heads, dim)
     if (dim <= 32) FF_WKV(32);
     else if (dim <= 64) FF_WKV(64);
     else if (dim <= 128) FF_WKV(128);
@@ -234,11 +319,39 @@ static int wkv_scan_launch(const void* rkvg, const float* dlog, const float* w0,
 // the head size the recurrence kernel is instantiated for (its state keeps that many squared floats a head)
 FF_EXPORT int ff_wkv_state_dim(int dim) { return dim <= 32 ? 32 : (dim <= 64 ? 64 : (dim <= 128 ? 128 : -1)); }
 
+// Tokens a sequence (average of a step) from which chunks are taken (us, chunked / token by token, 32 heads of 64: eight sequences of
+// 64 37.5 / 26.6, of 96 30.4 / 38.7; one of 96 12.1 / 21.0).
+constexpr int WKV_CHUNK_MIN = 80;
+
+// Bytes of scratch memory that a step of T tokens can use (0: none; without it the token-by-token kernel runs).
+FF_EXPORT long long ff_wkv_scratch_bytes(int dtype, int T, int n_seqs, int heads, int dim) {
+    if (dtype != 1 || T <= 0 || n_seqs <= 0 || (long long)T < (long long)WKV_CHUNK_MIN * n_seqs || (dim != 64 && dim != 128)) return 0;
+    return chunk_records(T, n_seqs) * heads * (long long)(dim == 64 ? sizeof(ChunkRecord<64, false>) : sizeof(ChunkRecord<128, false>));
+}
+
+template <int D>
+static int wkv_chunk_launch(const bf16* rkvg, const float* dlog, const float* w0, const float* u, int prev_off, const bf16* x, int W,
+                            const ChunkScanArgs& B, int Ttot, int n_seqs, void* scratch, cudaStream_t stream) {
+    const int n_records = (int)chunk_records(Ttot, n_seqs), per_block = chunk_records_a_block((long long)n_records * B.heads);
+    FF_LAUNCH(wkv_prepare_kernel<D>, dim3((n_records + per_block - 1) / per_block, B.heads), 2 * D, 0, stream, rkvg, dlog, w0, u,
+              (ChunkRecord<D, false>*)scratch, B.state, (size_t)B.state_stride, prev_off, x, W, B.cu_q, B.state_slots, n_seqs, n_records, per_block,
+              Ttot, B.heads);
+    return chunk_scan_launch<D, false>(B, n_seqs, stream);
+}
+
 FF_EXPORT int ff_wkv_scan(const void* rkvg, int dtype, const float* dlog, const float* w0, const float* u, float* state,
                           long long state_stride, int prev_off, const void* x, int W, const int* cu_q,
                           const int* state_slots, const int* seq_fresh, float* o, int Ttot, int n_seqs, int heads,
-                          int dim, cudaStream_t stream) {
+                          int dim, void* scratch, long long scratch_bytes, cudaStream_t stream) {
     if (Ttot <= 0 || n_seqs <= 0) return 0;
+    const long long need = ff_wkv_scratch_bytes(dtype, Ttot, n_seqs, heads, dim);
+    if (need > 0 && scratch && scratch_bytes >= need && (((uintptr_t)rkvg | (uintptr_t)dlog) & 15) == 0) {
+        const bf16* in = (const bf16*)rkvg;
+        const int HD = heads * dim;
+        const ChunkScanArgs B{scratch, in + (size_t)2 * Ttot * HD, HD, 0, state, state_stride, 0, dim * dim, cu_q, state_slots, seq_fresh, o, heads, dim};
+        if (dim == 64) return wkv_chunk_launch<64>(in, dlog, w0, u, prev_off, (const bf16*)x, W, B, Ttot, n_seqs, scratch, stream);
+        return wkv_chunk_launch<128>(in, dlog, w0, u, prev_off, (const bf16*)x, W, B, Ttot, n_seqs, scratch, stream);
+    }
     if (dtype == 0)
         return wkv_scan_launch<float>(rkvg, dlog, w0, u, state, state_stride, prev_off, x, W, cu_q, state_slots,
                                       seq_fresh, o, Ttot, n_seqs, heads, dim, stream);

@@ -929,7 +929,7 @@ def _count_preparing(scratch) -> None:
 
 
 def wkv_scan(rkvg, dlog, w0, u, state, prev_off: int, x, ctx, o, heads: int, dim: int) -> None:
-    """The recurrence, token by token, one block per (sequence, head).  rkvg [4,T,heads*dim] (r, k, v, gate
+    """The recurrence, token by token or (bfloat16 prompts, with ``ctx.workspace`` for scratch memory) a chunk of tokens at a time.  rkvg [4,T,heads*dim] (r, k, v, gate
     projections; the gate is not read here), dlog float32 [T,heads*dim] (the decay's inner logarithm without
     its offset w0), state float32 [slots, prev_off + W] with prev_off >= heads * wkv_state_dim(dim)^2 (read unless
     the request is fresh, written back in the kernel's own order, the portion's last row of x saved at prev_off),
@@ -941,10 +941,12 @@ def wkv_scan(rkvg, dlog, w0, u, state, prev_off: int, x, ctx, o, heads: int, dim
     assert o.shape == (T, HD) and o.dtype == torch.float32 and state.dtype == torch.float32
     assert w0.dtype == u.dtype == torch.float32 and w0.numel() == HD and u.numel() == HD
     assert state.shape[1] >= prev_off + W and prev_off >= heads * wkv_state_dim(dim) ** 2
+    scratch = _recurrence_scratch(ctx, "wkv", "ff_wkv_scratch_bytes", _dt(rkvg), T, ctx.num_seqs, heads, dim)
     _check(_lib("wkv").ff_wkv_scan(_p(rkvg), c_int(_dt(rkvg)), _p(dlog), _p(w0), _p(u), _p(state),
                                   ctypes.c_longlong(state.stride(0)), c_int(prev_off), _p(x), c_int(W), _p(ctx.cu_q),
                                   _p(ctx.state_slots), _p(ctx.seq_fresh), _p(o), c_int(T), c_int(ctx.num_seqs),
-                                  c_int(heads), c_int(dim), _stream()), "wkv_scan")
+                                  c_int(heads), c_int(dim), *scratch, _stream()), "wkv_scan")
+    _count_preparing(scratch)
 
 
 def wkv_out(o, gate, norm_w, eps: float, y, heads: int, dim: int) -> None:
@@ -1437,25 +1439,12 @@ def head_gate(att: torch.Tensor, gate, y: torch.Tensor, heads: int, d: int, dv: 
 
 # --------------------------------------------------------------------------- #
 # the gated delta rule with a decay per key channel (csrc/delta_rule.cu)
-def delta_plan(N: int, V: int):
-    """(key size the kernel is built for, threads that share a value column, blocks a head's columns are split over,
-    columns a block, threads a block): the twin of `delta_plan` in csrc/delta_rule.cu (`delta_state_floats` is the
-    kernel's own figure)."""
+def delta_state_floats_plan(heads: int, N: int, V: int) -> int:
+    """Floats of a request's state for `heads` heads of key size N and value size V (worked out on the host): [heads, V, N], N
+    rounded up to what the kernel is instantiated for (`delta_state_floats` is the kernel's own figure)."""
     if not (0 < N <= 256 and 0 < V <= 256):
         raise KernelError(f"delta rule: key size {N} / value size {V} not supported (up to 256 each)")
-    pad = 16 if N <= 16 else (32 if N <= 32 else (64 if N <= 64 else (128 if N <= 128 else 256)))
-    parts = 16 if pad >= 128 else (8 if pad >= 32 else 4)
-    vj = 2 if pad >= 128 else 1                 # value columns a thread
-    max_cols = 512 // parts * vj
-    vsplit = -(-V // max_cols)
-    vb = -(-V // vsplit)
-    return pad, parts, vsplit, vb, -(-(-(-vb // vj) * parts) // 32) * 32
-
-
-def delta_state_floats_plan(heads: int, N: int, V: int) -> int:
-    """Floats of a request's state for `heads` heads of key size N and value size V (worked out on the host)."""
-    pad, parts, vsplit, _, threads = delta_plan(N, V)
-    return heads * vsplit * (pad // parts) * (2 if pad >= 128 else 1) * threads
+    return heads * V * scan_key_size(N, V)
 
 
 def delta_state_floats(heads: int, N: int, V: int) -> int:
@@ -1471,7 +1460,8 @@ def delta_state_floats(heads: int, N: int, V: int) -> int:
 def delta_rule_scan(q, k, v, beta, a, dt_bias: torch.Tensor, a_log: torch.Tensor, state: torch.Tensor, state_off: int,
                     ctx, o: torch.Tensor, heads: int, N: int, V: int, *, heads_per_group: int = 1, q_scale: float = 1.0,
                     unit_eps: float = 1e-6, decay_per_head: bool = False) -> None:
-    """S = diag(g) S; u = beta (v - S^T k); S += k u^T; o = S^T q per head, token by token.  ``q``, ``k``, ``v``,
+    """S = diag(g) S; u = beta (v - S^T k); S += k u^T; o = S^T q per head, token by token or (bfloat16 prompts, with
+    ``ctx.workspace`` for scratch memory) a chunk of tokens at a time.  ``q``, ``k``, ``v``,
     ``beta``, ``a``: (matrix [T, *], first column); a q/k row holds [groups, N] (made unit vectors here, q also times
     ``q_scale``), a v row [heads, V], a beta row [heads] (its sigmoid is taken here), an ``a`` row float32
     [heads, N] with g = exp(-exp(a_log) softplus(a + dt_bias)) (``decay_per_head``: an ``a`` row is [heads], dt_bias
@@ -1485,12 +1475,14 @@ def delta_rule_scan(q, k, v, beta, a, dt_bias: torch.Tensor, a_log: torch.Tensor
     assert dt_bias.dtype == a_log.dtype == torch.float32 and a_log.numel() == heads
     assert dt_bias.numel() == (heads if decay_per_head else heads * N)
     assert o.dtype == torch.float32 and o.shape == (T, heads * V) and state.dtype == torch.float32
+    scratch = _recurrence_scratch(ctx, "delta_rule", "ff_delta_scratch_bytes", _dt(qm), T, ctx.num_seqs, heads, N, V)
     _check(_lib("delta_rule").ff_delta_rule_scan(
         _p(qm), c_int(qm.stride(0)), c_int(q0), _p(km), c_int(km.stride(0)), c_int(k0), _p(vm), c_int(vm.stride(0)),
         c_int(v0), _p(bm), c_int(bm.stride(0)), c_int(b0), c_int(_dt(qm)), _p(am), c_int(am.stride(0)), c_int(a0),
         _p(dt_bias), _p(a_log), c_int(1 if decay_per_head else 0), c_int(heads_per_group), c_float(q_scale), c_float(unit_eps), _p(state),
         ctypes.c_longlong(state.stride(0)), c_int(state_off), _p(ctx.cu_q), _p(ctx.state_slots), _p(ctx.seq_fresh),
-        _p(o), c_int(T), c_int(ctx.num_seqs), c_int(heads), c_int(N), c_int(V), _stream()), "delta_rule_scan")
+        _p(o), c_int(T), c_int(ctx.num_seqs), c_int(heads), c_int(N), c_int(V), *scratch, _stream()), "delta_rule_scan")
+    _count_preparing(scratch)
 
 
 def head_norm_gate(o: torch.Tensor, gate, weight: torch.Tensor, eps: float, y: torch.Tensor, heads: int, V: int,
