@@ -1,0 +1,184 @@
+"""The recurrences a chunk of tokens at a time (csrc/ssm.cu, csrc/wkv.cu, csrc/delta_rule.cu over csrc/chunk_scan.cuh) against
+the same recurrence token by token in 64 bits: lengths around the chunk sizes of 16 and 32, key sizes of 64 and 128, value
+sizes that fill no block of columns, decays from none to all, and numbers that are not finite.
+
+Tolerance of the outputs' norm: 2^-24 (32 + L) for sequences of up to L tokens.  Every number and sum is 32-bit; a decay is rounded
+once, and what a state keeps of a token passed at most L of them, each off by 2^-24 at most; the sums over key channels and
+tokens, of terms of random sign, stay below 32 roundings."""
+import math
+from types import SimpleNamespace
+
+import pytest
+import torch
+import torch.nn.functional as F
+
+from firefly_b200.engine.context import Workspace
+from firefly_b200.ops import kernels as K
+
+pytestmark = pytest.mark.gpu
+BF = torch.bfloat16
+LENS = [(15, 16, 17, 400), (31, 32, 33, 330), (1, 260), (112, 128, 144)]
+
+
+def _ctx(lens, fresh):
+    n = len(lens)
+    cu = torch.tensor([0, *torch.tensor(lens).cumsum(0).tolist()], dtype=torch.int32, device="cuda")
+    return SimpleNamespace(cu_q=cu, num_seqs=n, state_slots=torch.arange(n, 0, -1, dtype=torch.int32, device="cuda"),
+                           seq_fresh=torch.full((n,), fresh, dtype=torch.int32, device="cuda"), workspace=Workspace("cuda"))
+
+
+def _walk(q, k, v, decay, beta=None, bonus=None, S=None):
+    """One sequence in 64 bits: q, k, decay [T, h, N], v [T, h, V]."""
+    q, k, v, decay = (x.double() for x in (q, k, v, decay))
+    T, h, N = q.shape
+    S = torch.zeros(h, N, v.shape[-1], dtype=torch.float64, device=q.device) if S is None else S
+    o = torch.empty_like(v)
+    for t in range(T):
+        if bonus is not None:
+            w = k[t][:, :, None] * v[t][:, None]
+            o[t] = torch.einsum("hn,hnv->hv", q[t], S + bonus.double()[:, :, None] * w)
+            S = S * decay[t][:, :, None] + w
+            continue
+        S = S * decay[t][:, :, None]
+        u = v[t] if beta is None else beta[t].double()[:, None] * (v[t] - torch.einsum("hn,hnv->hv", k[t], S))
+        S = S + k[t][:, :, None] * u[:, None]
+        o[t] = torch.einsum("hn,hnv->hv", q[t], S)
+    return o, S
+
+
+def _check(call, inputs, lens, heads, V, T, bonus=None):
+    """A step of prompts on fresh slots, then one of single tokens behind them, against `_walk`."""
+    n, tol = len(lens), 2.0 ** -24 * (32 + max(lens))
+    o, o1 = torch.empty(T, heads * V, device="cuda"), torch.empty(n, heads * V, device="cuda")
+    before = K.LAUNCHES
+    call(0, T, _ctx(lens, 1), o)
+    assert K.LAUNCHES == before + 2                        # the chunks' two kernels ran
+    call(T, T + n, _ctx([1] * n, 0), o1)                   # token by token, from the state that the chunks left
+    at = 0
+    for i, L in enumerate(lens):
+        want, S = _walk(*inputs(at, at + L), bonus=bonus)
+        assert (o[at:at + L].view_as(want).double() - want).norm() <= tol * want.norm()
+        want, _ = _walk(*inputs(T + i, T + i + 1), bonus=bonus, S=S)
+        assert (o1[i].view_as(want).double() - want).norm() <= tol * want.norm()
+        at += L
+
+
+def _rand(seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return lambda *s: torch.randn(*s, generator=g, device="cuda")
+
+
+@pytest.mark.parametrize("lens", LENS)
+@pytest.mark.parametrize("N,V,heads,groups,mode", [(64, 64, 4, 1, "step"), (128, 40, 6, 3, "step"), (128, 128, 2, 2, "constant"),
+                                                   (64, 72, 3, 3, "channel"), (128, 8, 2, 2, "channel")])
+def test_decay_scans(lens, N, V, heads, groups, mode):
+    rn = _rand(N + V)
+    T, n = sum(lens), len(lens)
+    x = rn(T + n, heads * V + 2 * groups * N).to(BF)
+    raw = rn(T + n, heads).to(BF)
+    bias, a_log, skip = rn(heads) - 2, rn(heads) + 1, rn(heads)
+    const = torch.tensor([-0.5, 0.999], device="cuda")
+    # per channel: from keeping everything to forgetting everything at once
+    alpha = torch.sigmoid(6 * rn(T + n, heads * N)) ** 2
+    alpha[:, 0], alpha[:, 1] = 0.0, 1.0
+    state = torch.full((n + 1, K.scan_state_floats(heads, N, V)), 7.0, device="cuda")
+    kw = {"step": lambda a, b: dict(step=(raw[a:b], 0), step_bias=bias, a_log=a_log, skip=skip), "constant": lambda a, b: dict(decay=const),
+          "channel": lambda a, b: dict(channel_decay=(alpha[a:b], 0), q_scale=0.125)}[mode]
+
+    def values(a, b):
+        return x[a:b, : heads * V].double().view(b - a, heads, V)
+
+    def call(a, b, ctx, o):
+        K.scalar_decay_scan((x[a:b], heads * V), (x[a:b], heads * V + groups * N), (x[a:b], 0), state, 0, ctx, o, heads, N, V,
+                            heads_per_group=heads // groups, **kw(a, b))
+        if mode == "step":                                 # the skip term is taken off again
+            o.copy_((o.double() - (skip.double()[None, :, None] * values(a, b)).view(b - a, -1)).float())
+
+    def inputs(a, b):
+        xx, v = x[a:b].double(), values(a, b)
+        q, k = (xx[:, heads * V + i * groups * N:][:, : groups * N].view(b - a, groups, N).repeat_interleave(heads // groups, 1) for i in (0, 1))
+        if mode == "step":
+            s = F.softplus(raw[a:b].double() + bias.double(), threshold=1e9)
+            return q, k * s[:, :, None], v, torch.exp(-torch.exp(a_log.double()) * s)[:, :, None].expand_as(k)
+        if mode == "constant":
+            return q, k, v, const.double()[None, :, None].expand_as(k)
+        return q * 0.125, k, v, alpha[a:b].view(b - a, heads, N)
+    _check(call, inputs, lens, heads, V, T)
+
+
+@pytest.mark.parametrize("lens", LENS)
+@pytest.mark.parametrize("dim,heads", [(64, 3), (128, 2)])
+def test_wkv_scan(lens, dim, heads):
+    rn = _rand(dim)
+    T, n, hd = sum(lens), len(lens), heads * dim
+    rkvg, rkvg1 = rn(4, T, hd).to(BF), rn(4, n, hd).to(BF)
+    dlog, w0, u = rn(T + n, hd), 2.5 * rn(hd) - 2, rn(hd)
+    x = rn(T + n, 48).to(BF)
+    state = torch.full((n + 1, heads * dim * dim + 48), 7.0, device="cuda")
+
+    def call(a, b, ctx, o):
+        K.wkv_scan(rkvg if a == 0 else rkvg1, dlog[a:b].contiguous(), w0, u, state, heads * dim * dim, x[a:b].contiguous(), ctx, o, heads, dim)
+        assert torch.equal(state[ctx.state_slots.long(), heads * dim * dim:], x[a:b][ctx.cu_q[1:].long() - 1].float())
+
+    def inputs(a, b):
+        r = (rkvg[:, a:b] if a < T else rkvg1[:, a - T:b - T]).reshape(4, b - a, heads, dim)
+        return r[0], r[1], r[2], torch.exp(-torch.exp(dlog[a:b].double() + w0.double())).view(b - a, heads, dim)
+    _check(call, inputs, lens, heads, dim, T, bonus=u.view(heads, dim))
+
+
+@pytest.mark.parametrize("lens", LENS)
+@pytest.mark.parametrize("N,V,heads,per_group,per_head", [(64, 40, 4, 2, False), (128, 128, 2, 1, False), (128, 72, 2, 2, True)])
+def test_delta_rule_scan(lens, N, V, heads, per_group, per_head):
+    rn = _rand(N + V + per_head)
+    T, n, G = sum(lens), len(lens), heads // per_group
+    x, beta = rn(T + n, 2 * G * N + heads * V).to(BF), (2 * rn(T + n, heads)).to(BF)
+    wide = heads if per_head else heads * N
+    a_raw, bias, a_log = 3 * rn(T + n, wide), rn(wide) - 1, rn(heads)
+    state = torch.full((n + 1, K.delta_state_floats_plan(heads, N, V)), 7.0, device="cuda")
+    assert K.delta_state_floats(heads, N, V) == K.delta_state_floats_plan(heads, N, V)
+
+    def call(a, b, ctx, o):
+        xs, bs, rs = x[a:b], beta[a:b], a_raw[a:b]
+        K.delta_rule_scan((xs, 0), (xs, G * N), (xs, 2 * G * N), (bs, 0), (rs, 0), bias, a_log, state, 0, ctx, o, heads, N, V,
+                          heads_per_group=per_group, q_scale=N ** -0.5, unit_eps=1e-6, decay_per_head=per_head)
+
+    def inputs(a, b):
+        xx = x[a:b].double()
+        q, k = (xx[:, i * G * N:][:, : G * N].view(b - a, G, N).repeat_interleave(per_group, 1) for i in (0, 1))
+        q, k = (y / torch.sqrt((y * y).sum(-1, keepdim=True) + 1e-6) for y in (q, k))
+        s = F.softplus(a_raw[a:b].double() + bias.double(), threshold=1e9).view(b - a, heads, -1).expand(b - a, heads, N)
+        return (q * N ** -0.5, k, xx[:, 2 * G * N:].view(b - a, heads, V), torch.exp(-torch.exp(a_log.double())[None, :, None] * s),
+                torch.sigmoid(beta[a:b].double()))
+    _check(call, inputs, lens, heads, V, T)
+
+
+@pytest.mark.parametrize("bad", [math.nan, math.inf])
+@pytest.mark.parametrize("kind", ["step", "channel", "wkv", "delta"])
+def test_not_finite_values_stay_behind_their_token(kind, bad):
+    """A value that is not finite spoils its own column from its token on, as token by token, and nothing in front of it."""
+    rn = _rand(3)
+    T, N, V, at, col = 100, 64, 64, 37, 21
+    x = rn(T, 2 * N + V).to(BF)
+    x[at, 2 * N + col] = bad
+    zeros = lambda *s: torch.zeros(*s, device="cuda")  # noqa: E731
+    out = []
+    for workspace in (Workspace("cuda"), None):
+        ctx = _ctx([T], 1)
+        ctx.workspace = workspace
+        o, state = zeros(T, V), zeros(2, N * V + 8)
+        q, k, v = (x, 0), (x, N), (x, 2 * N)
+        if kind == "step":
+            K.scalar_decay_scan(q, k, v, state, 0, ctx, o, 1, N, V, step=(x, 0), step_bias=zeros(1), a_log=zeros(1))
+        elif kind == "channel":
+            K.scalar_decay_scan(q, k, v, state, 0, ctx, o, 1, N, V, channel_decay=(zeros(T, N) + 0.9, 0))
+        elif kind == "wkv":
+            rkvg = torch.stack([x[:, :N], x[:, N:2 * N], x[:, 2 * N:], x[:, :N]]).contiguous()
+            K.wkv_scan(rkvg, zeros(T, N), zeros(N), zeros(N) + 1, state, N * V, x[:, :8].contiguous(), ctx, o, 1, N)
+        else:
+            K.delta_rule_scan(q, k, v, (x, 0), (zeros(T, N), 0), zeros(N), zeros(1), state, 0, ctx, o, 1, N, V)
+        out.append(o)
+    chunked, walked = out
+    spoilt = ~torch.isfinite(walked)
+    assert torch.equal(~torch.isfinite(chunked), spoilt)
+    assert spoilt[at:, col].all() and not spoilt[:at].any() and not spoilt[:, :col].any()
+    assert (chunked[~spoilt] - walked[~spoilt]).norm() <= 2.0 ** -23 * (32 + T) * walked[~spoilt].norm()
