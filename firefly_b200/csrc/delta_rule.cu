@@ -393,6 +393,42 @@ __global__ void head_norm_gate_kernel(const float* o, const TG* gate, int gate_s
     }
 }
 
+// The same for heads of 64 or 128 values on 16 bytes: V / 4 lanes a head, four values each.
+template <typename T, typename TG, int LANES>
+__global__ void __launch_bounds__(256) head_norm_gate_vec_kernel(const float* o, const TG* gate, int gate_stride, int gate_off,
+                                                                 const float* __restrict__ w, float eps, T* __restrict__ y, int rows, int heads,
+                                                                 int gate_act) {
+    pdl_prologue();
+    o = pdl_fresh(o);
+    gate = pdl_fresh(gate);
+    constexpr int V = 4 * LANES;
+    const int row = (blockIdx.x * 256 + threadIdx.x) / LANES, i = threadIdx.x % LANES * 4;
+    const bool live = row < rows;
+    const int t = live ? row / heads : 0, h = live ? row - t * heads : 0;
+    struct alignas(4 * sizeof(TG)) FourG { TG v[4]; };
+    struct alignas(4 * sizeof(T)) Four { T v[4]; };
+    float4 ov = make_float4(0.f, 0.f, 0.f, 0.f);
+    FourG gv;
+    if (live) {
+        ov = *reinterpret_cast<const float4*>(o + (size_t)row * V + i);
+        gv = *reinterpret_cast<const FourG*>(gate + (size_t)t * gate_stride + gate_off + (size_t)h * V + i);
+    }
+    float ss = (ov.x * ov.x + ov.y * ov.y) + (ov.z * ov.z + ov.w * ov.w);
+#pragma unroll
+    for (int off = LANES / 2; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+    if (!live) return;
+    const float inv = 1.0f / sqrtf(ss / (float)V + eps);
+    const float4 w4 = *reinterpret_cast<const float4*>(w + i);
+    const float v[4] = {ov.x, ov.y, ov.z, ov.w}, wv[4] = {w4.x, w4.y, w4.z, w4.w};
+    Four out;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const float g = to_float(gv.v[e]), sg = 1.0f / (1.0f + expf(-g));
+        out.v[e] = from_float<T>(v[e] * inv * wv[e] * (gate_act ? g * sg : sg));
+    }
+    *reinterpret_cast<Four*>(y + (size_t)row * V + i) = out;
+}
+
 }  // namespace ff
 
 using namespace ff;
@@ -482,6 +518,23 @@ FF_EXPORT int ff_head_norm_gate(const float* o, const void* gate, int gate_dtype
     if (rows <= 0) return 0;
     const int warps = 4;
     const unsigned blocks = (unsigned)((rows + warps - 1) / warps);
+    const int es = dtype == 0 ? 4 : 2, eg = gate_dtype == 0 ? 4 : 2;
+    if ((V == 64 || V == 128) && (((uintptr_t)o | (uintptr_t)w) & 15) == 0 && ((uintptr_t)y & (4 * es - 1)) == 0 &&
+        ((uintptr_t)gate & (4 * eg - 1)) == 0 && gate_stride % 4 == 0 && gate_off % 4 == 0) {
+        const unsigned n = (unsigned)(((long long)rows * (V / 4) + 255) / 256);
+#define FF_HEAD_NORM(TT, TG)                                                                                                     \
+        do {                                                                                                                     \
+            if (V == 64) FF_LAUNCH((head_norm_gate_vec_kernel<TT, TG, 16>), n, 256, 0, stream, o, (const TG*)gate, gate_stride, gate_off, w, eps, (TT*)y, rows, heads, gate_act); \
+            else FF_LAUNCH((head_norm_gate_vec_kernel<TT, TG, 32>), n, 256, 0, stream, o, (const TG*)gate, gate_stride, gate_off, w, eps, (TT*)y, rows, heads, gate_act); \
+        } while (0)
+        if (dtype == 0 && gate_dtype == 0) FF_HEAD_NORM(float, float);
+        else if (dtype == 1 && gate_dtype == 0) FF_HEAD_NORM(bf16, float);
+        else if (dtype == 1 && gate_dtype == 1) FF_HEAD_NORM(bf16, bf16);
+        else return FF_ERR_BAD_ARG;
+#undef FF_HEAD_NORM
+        FF_LAUNCH_CHECK();
+        return 0;
+    }
     if (dtype == 0 && gate_dtype == 0)
         FF_LAUNCH((head_norm_gate_kernel<float, float>), blocks, warps * 32, 0, stream, o, (const float*)gate, gate_stride,
                   gate_off, w, eps, (float*)y, rows, heads, V, gate_act);

@@ -33,6 +33,7 @@ __device__ __forceinline__ float softplus_f(float z) { return z > 20.f ? z : log
 // (steps of few tokens get a thread a token, so that they still fill the GPU).
 constexpr int CONV_MAX_TAPS = 16;
 constexpr int CONV_SILU = 1, CONV_ADD_INPUT = 2;
+constexpr int CONV_AHEAD = 4;
 
 // TAPS > 0: the number of taps is known when the kernel is built (the window stays in registers); 0: any number
 // up to CONV_MAX_TAPS.
@@ -88,13 +89,27 @@ __global__ void causal_conv_silu_kernel(const T* in, int in_stride, int in_off,
             }
         }
     };
+    // The rows and sequences of CONV_AHEAD tokens are asked for together: with one at a time the walk waits for memory at every
+    // token (118 us on 8192 tokens of 4096 channels, whose bytes take 21).
     int s_prev = -1;
-    for (int t = tile0; t < tile1; ++t) {
-        const int s = token_seq[t];
+    float rows[CONV_AHEAD][VEC];
+    int seqs[CONV_AHEAD];
+    for (int tb = tile0; tb < tile1; tb += CONV_AHEAD) {
+#pragma unroll
+      for (int a = 0; a < CONV_AHEAD; ++a) {
+        const int t = min(tb + a, tile1 - 1);
+        seqs[a] = token_seq[t];
+        load_row(t, rows[a]);
+      }
+#pragma unroll
+      for (int a = 0; a < CONV_AHEAD; ++a) {
+        const int t = tb + a, s = seqs[a];
+        if (t >= tile1) break;
         if (t == tile0 || s != s_prev) fill_window(t, s);
         s_prev = s;
         float cur[VEC], acc[VEC];
-        load_row(t, cur);
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) cur[e] = rows[a][e];
 #pragma unroll
         for (int e = 0; e < VEC; ++e) acc[e] = bs[e];
 #pragma unroll
@@ -134,6 +149,7 @@ __global__ void causal_conv_silu_kernel(const T* in, int in_stride, int in_off,
                 for (int e = 0; e < VEC; ++e) win[j][e] = cur[e];
             }
         }
+      }
     }
 }
 
@@ -834,6 +850,75 @@ __global__ void gated_rms_norm_kernel(const float* o, const T* z, int z_stride, 
     }
 }
 
+// The same where a part is 128 to 4096 values in steps of 128 and everything lies on 16 bytes: TP threads a part (whole warps), each with
+// its values in registers between the sum and the writes, four at a time (the kernel above reads everything twice and has a
+// block of its own for every 256 values: 90 us on 8192 rows of 2048 values in 8 parts, whose bytes take 20).
+template <typename T, int TP>
+__global__ void __launch_bounds__(256) gated_rms_norm_vec_kernel(const float* o, const T* z, int z_stride, int z_off, const float* __restrict__ w,
+                                                                 float eps, T* __restrict__ y, int rows, int width, int parts, int order) {
+    pdl_prologue();
+    o = pdl_fresh(o);
+    z = pdl_fresh(z);
+    constexpr int MAXV = TP == 32 ? 8 : 4;
+    __shared__ float scratch[8];
+    const int per = width / parts, lane = threadIdx.x % TP;
+    const long long item = (long long)blockIdx.x * (256 / TP) + threadIdx.x / TP;       // row * parts + part
+    const bool live = item < (long long)rows * parts;
+    const int t = live ? (int)(item / parts) : 0, g = live ? (int)(item % parts) : 0;
+    const float* orow = o + (size_t)t * width + (size_t)g * per;
+    const T* zrow = z + (size_t)t * z_stride + z_off + (size_t)g * per;
+    struct alignas(4 * sizeof(T)) Four { T v[4]; };
+    float4 ov[MAXV];
+    Four zv[MAXV];
+#pragma unroll
+    for (int m = 0; m < MAXV; ++m) {
+        const int i = (m * TP + lane) * 4;
+        if (i < per) {
+            ov[m] = *reinterpret_cast<const float4*>(orow + i);
+            zv[m] = *reinterpret_cast<const Four*>(zrow + i);
+        }
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int m = 0; m < MAXV; ++m) {
+        if ((m * TP + lane) * 4 < per) {
+            if (order == 0) {
+                ov[m].x *= silu_f(to_float(zv[m].v[0]));
+                ov[m].y *= silu_f(to_float(zv[m].v[1]));
+                ov[m].z *= silu_f(to_float(zv[m].v[2]));
+                ov[m].w *= silu_f(to_float(zv[m].v[3]));
+            }
+            ss += (ov[m].x * ov[m].x + ov[m].y * ov[m].y) + (ov[m].z * ov[m].z + ov[m].w * ov[m].w);
+        }
+    }
+    ss = warp_sum(ss);
+    if constexpr (TP > 32) {                             // the block is one part: 256 threads
+        if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = ss;
+        __syncthreads();
+        ss = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) ss += scratch[i];
+    }
+    if (!live) return;
+    const float inv = 1.0f / sqrtf(ss / (float)per + eps);
+    T* yrow = y + (size_t)t * width + (size_t)g * per;
+#pragma unroll
+    for (int m = 0; m < MAXV; ++m) {
+        const int i = (m * TP + lane) * 4;
+        if (i < per) {
+            const float4 w4 = *reinterpret_cast<const float4*>(w + g * per + i);
+            const float wv[4] = {w4.x, w4.y, w4.z, w4.w}, v[4] = {ov[m].x, ov[m].y, ov[m].z, ov[m].w};
+            Four out;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float r = v[e] * inv * wv[e];
+                out.v[e] = from_float<T>(order == 0 ? r : r / (1.0f + expf(-to_float(zv[m].v[e]))));
+            }
+            *reinterpret_cast<Four*>(yrow + i) = out;
+        }
+    }
+}
+
 }  // namespace ff
 
 using namespace ff;
@@ -1066,6 +1151,21 @@ FF_EXPORT int ff_gated_rms_norm(const float* o, const void* z, int dtype, int z_
     if (parts <= 0 || width % parts || (order != 0 && order != 1)) return FF_ERR_BAD_ARG;
     const int per = width / parts;
     const int threads = per >= 1024 ? 256 : (per >= 256 ? 128 : 64);
+    const int es = dtype == 0 ? 4 : 2;
+    if (per % 128 == 0 && per <= 4096 && (((uintptr_t)o | (uintptr_t)w) & 15) == 0 && (((uintptr_t)z | (uintptr_t)y) & (4 * es - 1)) == 0 &&
+        z_stride % 4 == 0 && z_off % 4 == 0) {
+        const bool one_warp = per <= 1024;
+        const long long items = (long long)T * parts;
+        const unsigned blocks = (unsigned)(one_warp ? (items + 7) / 8 : items);
+#define FF_GATED_NORM(TT, TP) \
+        FF_LAUNCH((gated_rms_norm_vec_kernel<TT, TP>), blocks, 256, 0, stream, o, (const TT*)z, z_stride, z_off, w, eps, (TT*)y, T, width, parts, order)
+        if (dtype == 0) { if (one_warp) FF_GATED_NORM(float, 32); else FF_GATED_NORM(float, 256); }
+        else if (dtype == 1) { if (one_warp) FF_GATED_NORM(bf16, 32); else FF_GATED_NORM(bf16, 256); }
+        else return FF_ERR_BAD_ARG;
+#undef FF_GATED_NORM
+        FF_LAUNCH_CHECK();
+        return 0;
+    }
     if (dtype == 0)
         FF_LAUNCH((gated_rms_norm_kernel<float>), dim3(T, parts), threads, 0, stream, o, (const float*)z, z_stride, z_off, w, eps,
                   (float*)y, width, parts, order);

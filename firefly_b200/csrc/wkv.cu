@@ -42,6 +42,65 @@ __global__ void wkv_shift_mix_kernel(const T* __restrict__ x, const float* __res
     }
 }
 
+// The same for widths in steps of 8 on 16 bytes: eight channels a thread, whose five weights stay in registers over
+// MIX_TOKENS tokens (with one channel a thread the loads and stores are two bytes each: 52 us on 4900 rows of 2048, whose bytes take 19).
+constexpr int MIX_TOKENS = 4;
+template <typename T>
+__global__ void __launch_bounds__(128) wkv_shift_mix_vec_kernel(const T* x, const float* __restrict__ mu /*[5,W]*/, const float* state,
+                                                                size_t state_stride, int prev_off, const int* __restrict__ token_seq,
+                                                                const int* __restrict__ cu_q, const int* __restrict__ state_slots,
+                                                                const int* __restrict__ seq_fresh, T* __restrict__ mixes /*[5,T,W]*/, int Ttot, int W,
+                                                                int tokens) {
+    pdl_prologue();
+    x = pdl_fresh(x);
+    state = pdl_fresh(state);
+    struct alignas(16) Pack { T v[16 / sizeof(T)]; };
+    constexpr int PER = 16 / (int)sizeof(T), PACKS = 8 / PER;
+    const int i = (blockIdx.y * 128 + threadIdx.x) * 8;
+    if (i >= W) return;
+    const int tile0 = blockIdx.x * tokens, tile1 = min(Ttot, tile0 + tokens);
+    auto row = [&](int t, float v[8]) {
+#pragma unroll
+        for (int p = 0; p < PACKS; ++p) {
+            const Pack r = *reinterpret_cast<const Pack*>(x + (size_t)t * W + i + p * PER);
+#pragma unroll
+            for (int e = 0; e < PER; ++e) v[p * PER + e] = to_float(r.v[e]);
+        }
+    };
+    float m[5][8], prev[8], cur[8];
+#pragma unroll
+    for (int s = 0; s < 5; ++s) {
+        *reinterpret_cast<float4*>(m[s]) = *reinterpret_cast<const float4*>(mu + (size_t)s * W + i);
+        *reinterpret_cast<float4*>(m[s] + 4) = *reinterpret_cast<const float4*>(mu + (size_t)s * W + i + 4);
+    }
+    if (tile0 > 0) row(tile0 - 1, prev);
+    for (int t = tile0; t < tile1; ++t) {
+        const int s = token_seq[t];
+        row(t, cur);
+        if (t == cu_q[s]) {
+            const float* saved = state + (size_t)state_slots[s] * state_stride + prev_off + i;
+            const bool fresh = seq_fresh[s] != 0;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) prev[e] = fresh ? 0.f : saved[e];
+        }
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+#pragma unroll
+            for (int p = 0; p < PACKS; ++p) {
+                Pack r;
+#pragma unroll
+                for (int e = 0; e < PER; ++e) {
+                    const int c = p * PER + e;
+                    r.v[e] = from_float<T>(cur[c] + (prev[c] - cur[c]) * m[k][c]);
+                }
+                *reinterpret_cast<Pack*>(mixes + ((size_t)k * Ttot + t) * W + i + p * PER) = r;
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) prev[e] = cur[e];
+    }
+}
+
 // tanh of a 32-bit matrix, into the type of the product that follows
 template <typename TO>
 __global__ void tanh_cast_kernel(const float* __restrict__ in, TO* __restrict__ out, size_t total) {
@@ -269,6 +328,39 @@ __global__ void wkv_out_kernel(const float* __restrict__ o, const T* __restrict_
     }
 }
 
+// The same for heads of 64 or 128 on 16 bytes: dim / 4 lanes a head, four values each
+template <typename T, int LANES>
+__global__ void __launch_bounds__(256) wkv_out_vec_kernel(const float* o, const T* g, const float* __restrict__ norm, float eps,
+                                                          T* __restrict__ y, int Ttot, int heads) {
+    pdl_prologue();
+    o = pdl_fresh(o);
+    g = pdl_fresh(g);
+    constexpr int D = 4 * LANES;
+    const int row = (blockIdx.x * 256 + threadIdx.x) / LANES, i = threadIdx.x % LANES * 4;
+    const bool live = row < Ttot * heads;
+    struct alignas(4 * sizeof(T)) Four { T v[4]; };
+    float4 ov = make_float4(0.f, 0.f, 0.f, 0.f);
+    Four gv;
+    if (live) {
+        ov = *reinterpret_cast<const float4*>(o + (size_t)row * D + i);
+        gv = *reinterpret_cast<const Four*>(g + (size_t)row * D + i);
+    }
+    float ss = (ov.x * ov.x + ov.y * ov.y) + (ov.z * ov.z + ov.w * ov.w);
+#pragma unroll
+    for (int off = LANES / 2; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+    if (!live) return;
+    const float inv = 1.0f / sqrtf(ss / (float)D + eps);
+    const float4 w4 = *reinterpret_cast<const float4*>(norm + (row % heads) * D + i);
+    const float v[4] = {ov.x, ov.y, ov.z, ov.w}, wv[4] = {w4.x, w4.y, w4.z, w4.w};
+    Four out;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const float z = to_float(gv.v[e]);
+        out.v[e] = from_float<T>(v[e] * inv * wv[e] * (z / (1.0f + expf(-z))));
+    }
+    *reinterpret_cast<Four*>(y + (size_t)row * D + i) = out;
+}
+
 }  // namespace ff
 
 using namespace ff;
@@ -278,6 +370,18 @@ FF_EXPORT int ff_wkv_shift_mix(const void* x, int dtype, const float* mu, const 
                                const int* seq_fresh, void* mixes, int T, int W, cudaStream_t stream) {
     if (T <= 0) return 0;
     const int threads = W >= 1024 ? 256 : 128;
+    if (W % 8 == 0 && (((uintptr_t)x | (uintptr_t)mu | (uintptr_t)mixes) & 15) == 0 && (dtype == 0 || dtype == 1)) {
+        const int tokens = T >= 1024 ? MIX_TOKENS : 1;           // few tokens: a thread a token, so that they still fill the GPU
+        const dim3 grid((T + tokens - 1) / tokens, (W / 8 + 127) / 128);
+        if (dtype == 0)
+            FF_LAUNCH((wkv_shift_mix_vec_kernel<float>), grid, 128, 0, stream, (const float*)x, mu, state, (size_t)state_stride, prev_off,
+                      token_seq, cu_q, state_slots, seq_fresh, (float*)mixes, T, W, tokens);
+        else
+            FF_LAUNCH((wkv_shift_mix_vec_kernel<bf16>), grid, 128, 0, stream, (const bf16*)x, mu, state, (size_t)state_stride, prev_off,
+                      token_seq, cu_q, state_slots, seq_fresh, (bf16*)mixes, T, W, tokens);
+        FF_LAUNCH_CHECK();
+        return 0;
+    }
     if (dtype == 0)
         FF_LAUNCH((wkv_shift_mix_kernel<float>), T, threads, 0, stream, (const float*)x, mu, state, (size_t)state_stride,
                   prev_off, token_seq, cu_q, state_slots, seq_fresh, (float*)mixes, T, W);
@@ -366,6 +470,17 @@ FF_EXPORT int ff_wkv_out(const float* o, const void* g, int dtype, const float* 
     if (T <= 0) return 0;
     const long long warps = (long long)T * heads;
     const unsigned blocks = (unsigned)((warps + 3) / 4);
+    const int es = dtype == 0 ? 4 : 2;
+    if ((dim == 64 || dim == 128) && (dtype == 0 || dtype == 1) && (((uintptr_t)o | (uintptr_t)norm) & 15) == 0 &&
+        (((uintptr_t)g | (uintptr_t)y) & (4 * es - 1)) == 0) {
+        const unsigned n = (unsigned)((warps * (dim / 4) + 255) / 256);
+#define FF_WKV_OUT(TT, L) FF_LAUNCH((wkv_out_vec_kernel<TT, L>), n, 256, 0, stream, o, (const TT*)g, norm, eps, (TT*)y, T, heads)
+        if (dtype == 0) { if (dim == 64) FF_WKV_OUT(float, 16); else FF_WKV_OUT(float, 32); }
+        else { if (dim == 64) FF_WKV_OUT(bf16, 16); else FF_WKV_OUT(bf16, 32); }
+#undef FF_WKV_OUT
+        FF_LAUNCH_CHECK();
+        return 0;
+    }
     if (dtype == 0)
         FF_LAUNCH((wkv_out_kernel<float>), blocks, 128, 0, stream, o, (const float*)g, norm, eps, (float*)y, T, heads, dim);
     else if (dtype == 1)
