@@ -58,8 +58,13 @@ __global__ void causal_conv_silu_kernel(const T* in, int in_stride, int in_off,
 #pragma unroll
     for (int e = 0; e < VEC; ++e) {
         bs[e] = bias ? bias[c0 + e] : 0.f;
+        if constexpr (TAPS == 4 && VEC > 1) {         // a channel's four weights in one load (the launcher has seen to the alignment)
+            const float4 w4 = *reinterpret_cast<const float4*>(w + (size_t)(c0 + e) * 4);
+            wt[0][e] = w4.x; wt[1][e] = w4.y; wt[2][e] = w4.z; wt[3][e] = w4.w;
+        } else {
 #pragma unroll
-        for (int j = 0; j < MT; ++j) wt[j][e] = j < taps ? w[(size_t)(c0 + e) * taps + j] : 0.f;
+            for (int j = 0; j < MT; ++j) wt[j][e] = j < taps ? w[(size_t)(c0 + e) * taps + j] : 0.f;
+        }
     }
     auto load_row = [&](int tt, float* dst) {           // the inputs of token tt (a row of this step)
         const T* src = in + (size_t)tt * in_stride + in_off + c0;
@@ -97,9 +102,10 @@ __global__ void causal_conv_silu_kernel(const T* in, int in_stride, int in_off,
     for (int tb = tile0; tb < tile1; tb += CONV_AHEAD) {
 #pragma unroll
       for (int a = 0; a < CONV_AHEAD; ++a) {
-        const int t = min(tb + a, tile1 - 1);
-        seqs[a] = token_seq[t];
-        load_row(t, rows[a]);
+        if (tb + a < tile1) {
+          seqs[a] = token_seq[tb + a];
+          load_row(tb + a, rows[a]);
+        }
       }
 #pragma unroll
       for (int a = 0; a < CONV_AHEAD; ++a) {
@@ -853,13 +859,12 @@ __global__ void gated_rms_norm_kernel(const float* o, const T* z, int z_stride, 
 // The same where a part is 128 to 4096 values in steps of 128 and everything lies on 16 bytes: TP threads a part (whole warps), each with
 // its values in registers between the sum and the writes, four at a time (the kernel above reads everything twice and has a
 // block of its own for every 256 values: 90 us on 8192 rows of 2048 values in 8 parts, whose bytes take 20).
-template <typename T, int TP>
+template <typename T, int TP, int MAXV>
 __global__ void __launch_bounds__(256) gated_rms_norm_vec_kernel(const float* o, const T* z, int z_stride, int z_off, const float* __restrict__ w,
                                                                  float eps, T* __restrict__ y, int rows, int width, int parts, int order) {
     pdl_prologue();
     o = pdl_fresh(o);
     z = pdl_fresh(z);
-    constexpr int MAXV = TP == 32 ? 8 : 4;
     __shared__ float scratch[8];
     const int per = width / parts, lane = threadIdx.x % TP;
     const long long item = (long long)blockIdx.x * (256 / TP) + threadIdx.x / TP;       // row * parts + part
@@ -930,11 +935,12 @@ static int conv_launch(const void* in, int in_stride, int in_off, const float* w
                        cudaStream_t stream) {
     constexpr int V = 16 / (int)sizeof(T);
     const bool vec = taps >= 2 && taps <= 4 && C % V == 0 && in_off % V == 0 && in_stride % V == 0 &&
-                     (((uintptr_t)in | (uintptr_t)out) & 15) == 0;
+                     (((uintptr_t)in | (uintptr_t)out | (uintptr_t)w) & 15) == 0;
     const int per = vec ? V : 1;
     const int lanes = (C + per - 1) / per;
     const int threads = lanes >= 128 ? 128 : ((lanes + 31) / 32) * 32;
-    const int tile = T_ >= 4096 ? 16 : (T_ >= 512 ? 4 : 1);
+    // a thread's weights are read once for its tile of tokens; few tokens get small tiles, so that they still fill the GPU
+    const int tile = T_ >= 4096 ? 32 : (T_ >= 512 ? 4 : 1);
     dim3 grid((T_ + tile - 1) / tile, (lanes + threads - 1) / threads);
 #define FF_CONV(VV, TT)                                                                                              \
     FF_LAUNCH((causal_conv_silu_kernel<T, TO, VV, TT>), grid, threads, 0, stream, (const T*)in, in_stride, in_off, w, bias, \
@@ -1157,11 +1163,19 @@ FF_EXPORT int ff_gated_rms_norm(const float* o, const void* z, int dtype, int z_
         const bool one_warp = per <= 1024;
         const long long items = (long long)T * parts;
         const unsigned blocks = (unsigned)(one_warp ? (items + 7) / 8 : items);
-#define FF_GATED_NORM(TT, TP) \
-        FF_LAUNCH((gated_rms_norm_vec_kernel<TT, TP>), blocks, 256, 0, stream, o, (const TT*)z, z_stride, z_off, w, eps, (TT*)y, T, width, parts, order)
-        if (dtype == 0) { if (one_warp) FF_GATED_NORM(float, 32); else FF_GATED_NORM(float, 256); }
-        else if (dtype == 1) { if (one_warp) FF_GATED_NORM(bf16, 32); else FF_GATED_NORM(bf16, 256); }
+#define FF_GATED_NORM(TT, TP, MV) \
+        FF_LAUNCH((gated_rms_norm_vec_kernel<TT, TP, MV>), blocks, 256, 0, stream, o, (const TT*)z, z_stride, z_off, w, eps, (TT*)y, T, width, parts, order)
+#define FF_GATED_NORM_SIZE(TT)                                  \
+        do {                                                    \
+            if (!one_warp) FF_GATED_NORM(TT, 256, 4);           \
+            else if (per <= 256) FF_GATED_NORM(TT, 32, 2);      \
+            else if (per <= 512) FF_GATED_NORM(TT, 32, 4);      \
+            else FF_GATED_NORM(TT, 32, 8);                      \
+        } while (0)
+        if (dtype == 0) FF_GATED_NORM_SIZE(float);
+        else if (dtype == 1) FF_GATED_NORM_SIZE(bf16);
         else return FF_ERR_BAD_ARG;
+#undef FF_GATED_NORM_SIZE
 #undef FF_GATED_NORM
         FF_LAUNCH_CHECK();
         return 0;
