@@ -20,6 +20,15 @@
 namespace ff {
 
 __device__ __forceinline__ float silu_f(float z) { return z / (1.0f + expf(-z)); }
+// 1 / (1 + e^-z) for results that are rounded to 16 bits, without a division's branches: the hardware's reciprocal and one Newton step, right to the last bit or next to it;
+// 0 where e^-z is beyond 8e37.
+__device__ __forceinline__ float sigmoid_f(float z) {
+    const float d = 1.0f + expf(-z);
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+    r = fmaf(r, fmaf(-d, r, 1.0f), r);
+    return d > 8e37f ? 0.f : r;
+}
 __device__ __forceinline__ float softplus_f(float z) { return z > 20.f ? z : log1pf(expf(z)); }
 
 // ----------------------------------------------------------------------------- convolution --
@@ -38,7 +47,7 @@ constexpr int CONV_AHEAD = 4;
 // TAPS > 0: the number of taps is known when the kernel is built (the window stays in registers); 0: any number
 // up to CONV_MAX_TAPS.
 template <typename T, typename TO, int VEC, int TAPS>
-__global__ void causal_conv_silu_kernel(const T* in, int in_stride, int in_off,
+__global__ void __launch_bounds__(128, 4) causal_conv_silu_kernel(const T* in, int in_stride, int in_off,
                                         const float* __restrict__ w /*[C,taps]*/, const float* __restrict__ bias,
                                         const float* state, size_t state_stride, int conv_off,
                                         const int* __restrict__ token_seq, const int* __restrict__ cu_q,
@@ -107,6 +116,46 @@ __global__ void causal_conv_silu_kernel(const T* in, int in_stride, int in_off,
           load_row(tb + a, rows[a]);
         }
       }
+      auto finish = [&](int t, float (&acc)[VEC], const float (&cur)[VEC]) {
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) {
+            if (flags & CONV_SILU) acc[e] = sizeof(TO) == 4 ? silu_f(acc[e]) : acc[e] * sigmoid_f(acc[e]);
+            if (flags & CONV_ADD_INPUT) acc[e] += cur[e];
+        }
+        TO* dst = out + (size_t)t * C + c0;
+        if constexpr (VEC == 1) dst[0] = from_float<TO>(acc[0]);
+        else {
+            struct alignas(VEC * sizeof(TO)) Pack { TO v[VEC]; };
+            Pack raw;
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) raw.v[e] = from_float<TO>(acc[e]);
+            *reinterpret_cast<Pack*>(dst) = raw;
+        }
+      };
+      if constexpr (TAPS > 0) {
+        // all of them in the sequence the window belongs to: the inputs stand where they were read, nothing slides
+        if (tb + CONV_AHEAD <= tile1 && seqs[0] == s_prev && seqs[CONV_AHEAD - 1] == s_prev) {
+#pragma unroll
+          for (int a = 0; a < CONV_AHEAD; ++a) {
+            float acc[VEC];
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) acc[e] = bs[e];
+#pragma unroll
+            for (int j = 0; j < MT; ++j) {
+              const int from = a - (MT - 1) + j;            // row of this batch, or (negative) of the window
+#pragma unroll
+              for (int e = 0; e < VEC; ++e) acc[e] += wt[j][e] * (from >= 0 ? rows[from >= 0 ? from : 0][e] : win[from < 0 ? MT - 1 + from : 0][e]);
+            }
+            finish(tb + a, acc, rows[a]);
+          }
+#pragma unroll
+          for (int j = 0; j < MT - 1; ++j) {
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) win[j][e] = rows[CONV_AHEAD - (MT - 1) + j][e];
+          }
+          continue;
+        }
+      }
 #pragma unroll
       for (int a = 0; a < CONV_AHEAD; ++a) {
         const int t = tb + a, s = seqs[a];
@@ -115,9 +164,7 @@ __global__ void causal_conv_silu_kernel(const T* in, int in_stride, int in_off,
         s_prev = s;
         float cur[VEC], acc[VEC];
 #pragma unroll
-        for (int e = 0; e < VEC; ++e) cur[e] = rows[a][e];
-#pragma unroll
-        for (int e = 0; e < VEC; ++e) acc[e] = bs[e];
+        for (int e = 0; e < VEC; ++e) { cur[e] = rows[a][e]; acc[e] = bs[e]; }
 #pragma unroll
         for (int j = 0; j < MT - 1; ++j)
             if (j < taps - 1) {
@@ -130,20 +177,7 @@ __global__ void causal_conv_silu_kernel(const T* in, int in_stride, int in_off,
 #pragma unroll
                 for (int e = 0; e < VEC; ++e) acc[e] += wt[j][e] * cur[e];
             }
-#pragma unroll
-        for (int e = 0; e < VEC; ++e) {
-            if (flags & CONV_SILU) acc[e] = silu_f(acc[e]);
-            if (flags & CONV_ADD_INPUT) acc[e] += cur[e];
-        }
-        TO* dst = out + (size_t)t * C + c0;
-        if constexpr (VEC == 1) dst[0] = from_float<TO>(acc[0]);
-        else {
-            struct alignas(VEC * sizeof(TO)) Pack { TO v[VEC]; };
-            Pack raw;
-#pragma unroll
-            for (int e = 0; e < VEC; ++e) raw.v[e] = from_float<TO>(acc[e]);
-            *reinterpret_cast<Pack*>(dst) = raw;
-        }
+        finish(t, acc, cur);
         // slide: the oldest row leaves, the current one comes in
 #pragma unroll
         for (int j = 0; j < MT - 1; ++j) {
