@@ -172,6 +172,41 @@ __device__ __forceinline__ uint32_t exp2_bf16x2(float x0, float x1) {
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(y) : "f"(p1), "f"(p0));        // low half = p0
     return y;
 }
+// Pairs of 32-bit values in one register pair, and the steps of the softmax that work on them: half the
+// instructions of the element-by-element form, which were what the softmax warps spent their time on.
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+// 2^(x * scale + off), rounded to bfloat16 as exp2_bf16x2 does
+__device__ __forceinline__ uint32_t exp2_scaled(float x0, float x1, uint64_t scale2, uint64_t off2) {
+    uint64_t y;
+    float y0, y1;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(y) : "l"(pack2(x0, x1)), "l"(scale2), "l"(off2));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(y0), "=f"(y1) : "l"(y));
+    return exp2_bf16x2(y0, y1);
+}
+// a += low half of w, b += high half: bfloat16 to 32-bit is exact
+__device__ __forceinline__ void add_pair(uint32_t w, float& a, float& b) {
+    asm("{\n\t.reg .b16 x, y;\n\tmov.b32 {x, y}, %2;\n\tadd.rn.f32.bf16 %0, x, %0;\n\tadd.rn.f32.bf16 %1, y, %1;\n\t}"
+        : "+f"(a), "+f"(b) : "r"(w));
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+// largest of N values (a multiple of 8), four independent chains of three-input maxima
+template <int N>
+__device__ __forceinline__ float row_max(const float (&s)[N]) {
+    float m[4] = {s[0], s[1], s[2], s[3]};
+#pragma unroll
+    for (int i = 4; i < N - 4; i += 8)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) m[u] = max3(m[u], s[i + u], s[i + 4 + u]);
+    return fmaxf(max3(m[0], m[1], s[N - 4]), max3(max3(m[2], m[3], s[N - 3]), s[N - 2], s[N - 1]));
+}
 __device__ __forceinline__ void tm_st16(uint32_t taddr, const float (&v)[16]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
                  ::"r"(taddr), "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])),
@@ -392,7 +427,7 @@ attn_tc_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __restri
             tm_ld32_nowait(tm_Sj + 32, s + 32);
             tm_ld_wait();
             // mask (only tiles that touch the diagonal or a window's edge), then the row max of the raw
-            // scores with four independent chains; the scale (> 0) is applied later
+            // scores; the scale (> 0) is applied later
             if (early) {
 #pragma unroll
                 for (int i = 0; i < BN; ++i) {
@@ -410,10 +445,7 @@ attn_tc_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __restri
                     if (key < lo || key >= hi) s[i] = -CUDART_INF_F;
                 }
             }
-            float mx4[4] = {s[0], s[1], s[2], s[3]};
-#pragma unroll
-            for (int i = 4; i < BN; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], s[i]);
-            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * sl2;
+            const float mx = row_max<BN>(s) * sl2;
             // The reference max `m` follows the true row max lazily: it moves (and O is rescaled) only
             // when the true max has grown by more than 2^8 since, which keeps p <= 256 and makes the
             // rescale rare after the first tiles.
@@ -429,10 +461,11 @@ attn_tc_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __restri
             // values, the same numbers the P V product sees
             uint32_t w[BN / 2];
             float sum4[4] = {0.f, 0.f, 0.f, 0.f};
+            const uint64_t scale2 = pack2(sl2, sl2), neg_m2 = pack2(neg_m, neg_m);
 #pragma unroll
             for (int e = 0; e < BN / 2; ++e) {
-                w[e] = exp2_bf16x2(fmaf(s[2 * e], sl2, neg_m), fmaf(s[2 * e + 1], sl2, neg_m));
-                sum4[e & 3] += __uint_as_float(w[e] << 16) + __uint_as_float(w[e] & 0xffff0000u);
+                w[e] = exp2_scaled(s[2 * e], s[2 * e + 1], scale2, neg_m2);
+                add_pair(w[e], sum4[(e & 1) * 2], sum4[(e & 1) * 2 + 1]);
             }
             // Tensor memory is written only between products: the last P V must be complete before P
             // of this tile is stored (stores issued while it was still running gave wrong sums, although
@@ -607,6 +640,327 @@ attn_tc_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __restri
     }
 }
 
+// ------------------------------------------------------------ two row tiles a block --
+#define FF_ATC_PAIR (FF_HEAD_DIM <= 128)
+#if FF_ATC_PAIR
+#ifndef FF_PAIR_MIN
+#define FF_PAIR_MIN 296
+#endif
+constexpr int PN = 128;                              // keys per tile
+constexpr int PAIR_ROWS = 2 * BM;
+constexpr int PAIR_SLOTS = 5;                        // ring of K and V tiles: K0, V0, K1, V1, ...
+constexpr int PAIR_THREADS = 320;                    // warps 0-3 and 4-7 softmax of either row tile, 8 loads, 9 MMAs
+constexpr int PAIR_TILE_BYTES = PN * D * 2;
+constexpr int PAIR_PAGE_LIST = MAX_PAGE_LIST < 32 ? 32 : MAX_PAGE_LIST > 256 ? 256 : MAX_PAGE_LIST / 32 * 32;
+constexpr size_t PAIR_SMEM = 1024 + 2 * Q_BYTES + PAIR_SLOTS * PAIR_TILE_BYTES + 128 + PAIR_PAGE_LIST * 4;
+enum { PB_FULL = 0, PB_EMPTY = PB_FULL + PAIR_SLOTS, PB_S = PB_EMPTY + PAIR_SLOTS, PB_P = PB_S + 2, PB_Q = PB_P + 2,
+       PB_PAGES, PB_COUNT };
+static_assert(PB_COUNT * 8 <= 128, "barriers");
+
+__global__ void __launch_bounds__(PAIR_THREADS, 1)
+attn_tc_pair_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __restrict__ q, int q_stride,
+                    const int* __restrict__ block_table, int max_blocks, const int* __restrict__ cu_q,
+                    const int* __restrict__ ctx_lens, int n_seqs, bf16* __restrict__ out, int out_stride, int nq,
+                    int nkv, int block_size, int num_blocks, float scale_log2, int window, int* __restrict__ status,
+                    const float* __restrict__ sink) {
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    unsigned char* Qs = base;                                        // [row tile][PANELS][128][128 B]
+    unsigned char* KVs = Qs + 2 * Q_BYTES;                           // [slot][PANELS][128][128 B]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(KVs + PAIR_SLOTS * PAIR_TILE_BYTES);
+    int* s_pages = reinterpret_cast<int*>(bars + 16);
+    __shared__ int s_seq, s_tile, s_abort, s_tok0, s_qlen, s_ctx;
+    __shared__ uint32_t s_tmem;
+    const int G = nq / nkv;
+    const int kh = (int)(blockIdx.x % (unsigned)nkv);
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    volatile int* abort_flag = &s_abort;
+
+    if (threadIdx.x == 0) {
+        s_abort = 0;
+        for (int i = 0; i < PB_COUNT; ++i) mb_init(sa(&bars[i]), i >= PB_Q ? 8 : i >= PB_P ? 4 : 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    // All of the SM's tensor memory: taken after the kernels before this one are done, and before the next one may start.
+    if (warp == 9) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sa(&s_tmem)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    // the pairs of row tiles are handed out last first, as above
+    const int vtile = (int)(gridDim.x / (unsigned)nkv) - 1 - (int)(blockIdx.x / (unsigned)nkv);
+    if (warp == 0) {   // which sequence owns pair vtile (none: the grid is an upper bound)
+        int cum = 0, found_seq = -1, found_tile = 0;
+        for (int s0 = 0; s0 < n_seqs && found_seq < 0; s0 += 32) {
+            const int s = s0 + lane;
+            const int cnt = s < n_seqs ? ((cu_q[s + 1] - cu_q[s]) * G + PAIR_ROWS - 1) / PAIR_ROWS : 0;
+            int incl = cnt;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += v;
+            }
+            const int total = __shfl_sync(0xffffffffu, incl, 31);
+            const unsigned hit = __ballot_sync(0xffffffffu, cum + incl > vtile);
+            if (hit) {
+                const int l0 = __ffs(hit) - 1;
+                found_seq = s0 + l0;
+                found_tile = vtile - (cum + __shfl_sync(0xffffffffu, incl, l0) - __shfl_sync(0xffffffffu, cnt, l0));
+            }
+            cum += total;
+        }
+        if (lane == 0) {
+            s_seq = found_seq; s_tile = found_tile;
+            if (found_seq >= 0) {
+                const int a = cu_q[found_seq];
+                s_tok0 = a; s_qlen = cu_q[found_seq + 1] - a; s_ctx = ctx_lens[found_seq];
+            }
+        }
+    }
+    tc_before();
+    __syncthreads();
+    tc_after();
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const uint32_t tmem = s_tmem;
+    const uint32_t tm_S = tmem, tm_O = tmem + 2 * PN;                // S (then P) of either row tile, O of either
+    const int seq = s_seq;
+    const int ppt = PN / block_size, tph = (PAIR_PAGE_LIST / 2) / ppt;    // pages of a tile, tiles of half the ring
+
+    int n_tiles = 0, t_begin = 0, tok0 = 0, q_len = 0, ctx = 0, rows = 0, row0 = 0, kv_lo = 0, kv_hi = 1;
+    if (seq >= 0) {
+        tok0 = s_tok0; q_len = s_qlen; ctx = s_ctx;
+        rows = q_len * G; row0 = s_tile * PAIR_ROWS;
+        kv_hi = ctx + min(q_len - 1, (row0 + PAIR_ROWS - 1) / G) + 1;
+        kv_lo = first_visible_key(ctx + row0 / G, window);
+        t_begin = kv_lo / PN;
+        n_tiles = (kv_hi + PN - 1) / PN - t_begin;
+    }
+    const int n_half = row0 + BM < rows ? 2 : 1;                     // row tiles of this block that have rows
+    const int* bt = block_table + (size_t)max(seq, 0) * max_blocks;
+    const int last_page = (kv_hi - 1) / block_size, first_page = kv_lo / block_size;
+    auto fill_pages = [&](int first, int count, int who, int nthreads) {
+        for (int i = who; i < count * ppt; i += nthreads) {
+            const int tile = first + i / ppt;
+            const int pi = (t_begin + tile) * ppt + i % ppt;
+            const bool wanted = pi >= first_page && pi <= last_page;
+            int page = (wanted && pi < max_blocks) ? bt[pi] : -1;
+            if (page >= num_blocks) page = -1;
+            if (wanted && page < 0) atomicExch(status, 4);
+            s_pages[(tile % (2 * tph)) * ppt + i % ppt] = page;
+        }
+    };
+
+    if (warp < 8) {
+        const int half = warp >> 2;                                  // the row tile of this warp
+        const int r = threadIdx.x & 127;
+        const int t0 = row0 + half * BM;                             // the row tile's first row
+        const int rg = t0 + r;
+        const bool valid = rg < rows;
+        const int rgc = min(rg, max(rows - 1, 0));
+        const int token = rgc / G, head = kh * G + rgc % G;
+        uint4 qv[D / 8];
+        if (n_tiles > 0) {
+            const uint4* src = reinterpret_cast<const uint4*>(q + (size_t)(tok0 + token) * q_stride + (size_t)head * D);
+#pragma unroll
+            for (int ch = 0; ch < D / 8; ++ch) qv[ch] = valid ? __ldg(src + ch) : make_uint4(0u, 0u, 0u, 0u);
+        }
+        fill_pages(0, min(n_tiles, 2 * tph), threadIdx.x, 256);
+        __syncwarp();
+        if (lane == 0) mb_arrive(sa(&bars[PB_PAGES]));
+        if (n_tiles > 0) {
+#pragma unroll
+            for (int ch = 0; ch < D / 8; ++ch)
+                *reinterpret_cast<uint4*>(Qs + half * Q_BYTES + (ch >> 3) * (BM * 128) + r * 128 + (((ch & 7) ^ (r & 7)) << 4)) = qv[ch];
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mb_arrive(sa(&bars[PB_Q]));
+
+        if (half < n_half) {
+            const int pos = ctx + token;
+            const int hi = pos + 1;
+            const int lo = first_visible_key(pos, window);
+            const int first_pos = ctx + t0 / G;
+            const int full_lo = first_visible_key(ctx + min(q_len - 1, (t0 + BM - 1) / G), window);
+            const uint32_t lane_base = (uint32_t)(((warp & 3) * 32) << 16);
+            const uint32_t tm_s = tm_S + (uint32_t)(half * PN) + lane_base, tm_o = tm_O + (uint32_t)(half * D) + lane_base;
+            float m = sink ? sink[head] * LOG2E : -CUDART_INF_F, l = sink ? 1.f : 0.f;
+            const uint64_t scale2 = pack2(scale_log2, scale_log2);
+            bool ok = true;
+            for (int j = 0; j < n_tiles && ok; ++j) {
+                // S of this tile; the product P V of the tile before was issued ahead of it, so O is at rest as well
+                ok = mb_wait(sa(&bars[PB_S + half]), j & 1, status, abort_flag);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                tc_after();
+                const int key0 = (t_begin + j) * PN;
+                float s[PN];
+#pragma unroll
+                for (int c = 0; c < PN / 32; ++c) tm_ld32_nowait(tm_s + c * 32, s + c * 32);
+                tm_ld_wait();
+                if (key0 + PN > first_pos + 1 || key0 < full_lo) {
+#pragma unroll
+                    for (int i = 0; i < PN; ++i) {
+                        const int key = key0 + i;
+                        if (key < lo || key >= hi) s[i] = -CUDART_INF_F;
+                    }
+                }
+                const float mx = row_max<PN>(s) * scale_log2;
+                float corr = 1.0f;
+                if (mx > m + 8.0f || m == -CUDART_INF_F) {
+                    const float m_new = fmaxf(m, mx);
+                    corr = fast_exp2(m - (m_new == -CUDART_INF_F ? 0.f : m_new));
+                    m = m_new;
+                }
+                if (j > 0 && !__all_sync(0xffffffffu, corr == 1.0f)) {       // some row's reference max moved: rescale O
+#pragma unroll 1
+                    for (int c = 0; c < D / 16; ++c) {
+                        float v[16];
+                        tm_ld16(tm_o + c * 16, v);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) v[i] *= corr;
+                        tm_st16(tm_o + c * 16, v);
+                    }
+                }
+                const float neg_m = m == -CUDART_INF_F ? 0.f : -m;
+                const uint64_t neg_m2 = pack2(neg_m, neg_m);
+                float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int c = 0; c < PN / 32; ++c) {
+                    uint32_t w[16];
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) {
+                        w[e] = exp2_scaled(s[c * 32 + 2 * e], s[c * 32 + 2 * e + 1], scale2, neg_m2);
+                        add_pair(w[e], sum[(e & 1) * 2], sum[(e & 1) * 2 + 1]);
+                    }
+                    tm_st16u(tm_s + c * 16, w);                     // P over the first half of S, which is in registers
+                }
+                l = l * corr + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                tc_before();
+                __syncwarp();
+                if (lane == 0) mb_arrive(sa(&bars[PB_P + half]));
+            }
+            if (n_tiles > 0 && ok) {
+                ok = mb_wait(sa(&bars[PB_S + half]), n_tiles & 1, status, abort_flag);
+                ok = __all_sync(0xffffffffu, ok);
+            }
+            if (n_tiles > 0 && ok) {
+                tc_after();
+                const float inv = 1.0f / l;
+                bf16* dst = out + (size_t)(tok0 + token) * out_stride + (size_t)head * D;
+#pragma unroll 1
+                for (int c = 0; c < D / 16; ++c) {
+                    float v[16];
+                    tm_ld16(tm_o + c * 16, v);
+                    if (valid) {
+                        uint32_t w[8];
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            __nv_bfloat162 pp = __floats2bfloat162_rn(v[2 * i] * inv, v[2 * i + 1] * inv);
+                            w[i] = *reinterpret_cast<uint32_t*>(&pp);
+                        }
+                        *reinterpret_cast<uint4*>(dst + c * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+                        *reinterpret_cast<uint4*>(dst + c * 16 + 8) = make_uint4(w[4], w[5], w[6], w[7]);
+                    }
+                }
+            }
+        }
+    } else if (warp == 8) {
+        bool ok = n_tiles == 0 || mb_wait(sa(&bars[PB_PAGES]), 0, status, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
+        const int p = lane / PANELS, h = lane % PANELS;                  // this lane's page and panel of a tile
+        for (int c = 0; c < 2 * n_tiles && ok; ++c) {
+            const int j = c >> 1, kv = c & 1, slot = c % PAIR_SLOTS;
+            if (kv == 0 && j >= 2 * tph && j % tph == 0) {
+                // every tile of this half of the ring is loaded: the next tiles' page ids
+                fill_pages(j, min(tph, n_tiles - j), lane, 32);
+                __syncwarp();
+            }
+            const bool fine = mb_wait(sa(&bars[PB_EMPTY + slot]), ((c / PAIR_SLOTS) & 1) ^ 1, status, abort_flag);
+            ok = __all_sync(0xffffffffu, fine);
+            if (!ok) break;
+            unsigned char* st = KVs + (size_t)slot * PAIR_TILE_BYTES;
+            const int page = p < ppt ? s_pages[(j % (2 * tph)) * ppt + p] : -1;
+            const unsigned boxes = __ballot_sync(0xffffffffu, page >= 0);
+            unsigned absent = __ballot_sync(0xffffffffu, p < ppt && page < 0);
+            if (absent) {
+                // pages outside the visible range (at a row tile's first and last keys): zeros, since what
+                // the masked probabilities of zero are multiplied by has to be finite
+                for (; absent; absent &= absent - 1) {
+                    const int b = __ffs(absent) - 1;
+                    uint4* z = reinterpret_cast<uint4*>(st + (b % PANELS) * (PN * 128) + (b / PANELS) * block_size * 128);
+                    for (int i = lane; i < block_size * 8; i += 32) z[i] = make_uint4(0u, 0u, 0u, 0u);
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+            }
+            const uint32_t bar = sa(&bars[PB_FULL + slot]);
+            if (lane == 0) mb_expect_tx(bar, (uint32_t)(__popc(boxes) * block_size * 128));
+            __syncwarp();
+            if (page >= 0) {
+                const int y = ((page * FF_KV_PLANES + kv * (FF_KV_PLANES - 1)) * nkv + kh) * block_size;
+                tma_2d(sa(st + h * (PN * 128) + p * block_size * 128), &kv_map, h * 64, y, bar);
+            }
+        }
+    } else {
+        const uint32_t idesc_qk = idesc_bf16(PN, false);
+        const uint32_t idesc_pv = idesc_bf16(D, true);
+        const bool issue = lane == 0;
+        auto wait_full = [&](int c) -> bool {
+            return __all_sync(0xffffffffu, mb_wait(sa(&bars[PB_FULL + c % PAIR_SLOTS]), (c / PAIR_SLOTS) & 1, status, abort_flag));
+        };
+        auto issue_qk = [&](int t, int j) {
+            const uint32_t ks = sa(KVs + (size_t)((2 * j) % PAIR_SLOTS) * PAIR_TILE_BYTES);
+#pragma unroll
+            for (int k = 0; k < D / 16; ++k)
+                tc_mma(issue, tm_S + (uint32_t)(t * PN), desc_k_major(sa(Qs + t * Q_BYTES) + (k >> 2) * (BM * 128) + (k & 3) * 32),
+                       desc_k_major(ks + (k >> 2) * (PN * 128) + (k & 3) * 32), idesc_qk, k > 0 ? 1u : 0u);
+            tc_commit_to(issue, sa(&bars[PB_S + t]));
+            if (t == n_half - 1) tc_commit_to(issue, sa(&bars[PB_EMPTY + (2 * j) % PAIR_SLOTS]));
+            __syncwarp();
+        };
+        bool ok = n_tiles > 0 && __all_sync(0xffffffffu, mb_wait(sa(&bars[PB_Q]), 0, status, abort_flag));
+        if (ok) ok = wait_full(0);
+        if (ok) {
+            tc_after();
+            for (int t = 0; t < n_half; ++t) issue_qk(t, 0);
+        }
+        for (int j = 0; j < n_tiles && ok; ++j) {
+            const uint32_t vs = sa(KVs + (size_t)((2 * j + 1) % PAIR_SLOTS) * PAIR_TILE_BYTES);
+            for (int t = 0; t < n_half && ok; ++t) {
+                // the softmax of one row tile runs while the tensor cores work on the other
+                ok = __all_sync(0xffffffffu, mb_wait(sa(&bars[PB_P + t]), j & 1, status, abort_flag));
+                if (ok && t == 0) ok = wait_full(2 * j + 1);
+                if (!ok) break;
+                tc_after();
+#pragma unroll
+                for (int k = 0; k < PN / 16; ++k)
+                    tc_mma_a_tmem(issue, tm_O + (uint32_t)(t * D), tm_S + (uint32_t)(t * PN + k * 8),
+                                  desc_n_major(vs + k * 16 * 128, PN * 128), idesc_pv, (j > 0 || k > 0) ? 1u : 0u);
+                if (t == n_half - 1) tc_commit_to(issue, sa(&bars[PB_EMPTY + (2 * j + 1) % PAIR_SLOTS]));
+                if (j + 1 < n_tiles) {
+                    if (t == 0) ok = wait_full(2 * j + 2);
+                    if (!ok) break;
+                    tc_after();
+                    issue_qk(t, j + 1);
+                } else {
+                    tc_commit_to(issue, sa(&bars[PB_S + t]));           // the last product: O is complete
+                    __syncwarp();
+                }
+            }
+        }
+    }
+    tc_before();
+    __syncthreads();
+    if (warp == 9) {
+        __syncwarp();
+        tc_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    }
+}
+#endif  // FF_ATC_PAIR
+
 // Join of the shares: out[token, head, :] = sum_s w_s O_s / sum_s w_s l_s, w_s = 2^(m_s - max m), in
 // the order of the shares.  D / 4 threads own one (token, head) and four columns each (16-byte loads,
 // all shares' loads in flight together); a block of JOIN_THREADS takes as many pairs as fit it.
@@ -727,6 +1081,16 @@ FF_EXPORT int ff_attn_tc(const void* q, int q_stride, const void* cache, const i
     if (rc) return rc;
     TensorMapArg arg;
     std::memcpy(arg.bytes, &map, sizeof(map));
+#if FF_ATC_PAIR
+    const long long pairs = (((long long)total_tiles + n_seqs) / 2) * nkv;    // at least ceil(row tiles of a sequence / 2), summed
+    if (num_splits == 1 && !dist_bias && softcap == 0.f && (long long)total_tiles * nkv >= FF_PAIR_MIN && pairs < (1ll << 31)) {
+        FF_SMEM_LIMIT(attn_tc_pair_kernel, PAIR_SMEM);
+        FF_LAUNCH((attn_tc_pair_kernel), dim3((unsigned)pairs), PAIR_THREADS, PAIR_SMEM, stream, arg, (const bf16*)q, q_stride,
+                  block_table, max_blocks, cu_q, ctx_lens, n_seqs, (bf16*)out, out_stride, nq, nkv, block_size, num_blocks,
+                  scale * LOG2E, window, status, sink);
+        return 0;
+    }
+#endif
     if ((long long)total_tiles * nkv * num_splits >= (1ll << 31)) return FF_ERR_UNSUPPORTED;
     FF_LAUNCH((attn_tc_kernel), dim3((unsigned)(total_tiles * nkv * num_splits)), ATC_THREADS, ATC_SMEM, stream, arg,
               (const bf16*)q, q_stride, block_table, max_blocks, cu_q, ctx_lens, n_seqs, (bf16*)out, out_stride, nq, nkv,
