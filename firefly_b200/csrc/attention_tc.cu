@@ -133,6 +133,21 @@ __device__ __forceinline__ void tc_mma_a_tmem(bool issue, uint32_t d_tmem, uint3
                  "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
                  ::"r"(d_tmem), "r"(a_tmem), "l"(db), "r"(idesc), "r"(acc), "r"((uint32_t)issue) : "memory");
 }
+// the same two with the operands' descriptors as their low words and the high word that all of them share
+__device__ __forceinline__ void tc_mma_lo(bool issue, uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi,
+                                          uint32_t idesc, uint32_t acc) {
+    asm volatile("{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\tmov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %3};\n\t"
+                 "setp.ne.b32 p, %5, 0;\n\tsetp.ne.b32 q, %6, 0;\n\t"
+                 "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p;\n\t}"
+                 ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(acc), "r"((uint32_t)issue) : "memory");
+}
+__device__ __forceinline__ void tc_mma_a_tmem_lo(bool issue, uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t hi,
+                                                 uint32_t idesc, uint32_t acc) {
+    asm volatile("{\n\t.reg .pred p, q;\n\t.reg .b64 b;\n\tmov.b64 b, {%2, %3};\n\t"
+                 "setp.ne.b32 p, %5, 0;\n\tsetp.ne.b32 q, %6, 0;\n\t"
+                 "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n\t}"
+                 ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(hi), "r"(idesc), "r"(acc), "r"((uint32_t)issue) : "memory");
+}
 __device__ __forceinline__ void tm_ld16(uint32_t taddr, float (&v)[16]) {
     uint32_t r[16];
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
@@ -904,52 +919,74 @@ attn_tc_pair_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __r
             }
         }
     } else {
-        const uint32_t idesc_qk = idesc_bf16(PN, false);
-        const uint32_t idesc_pv = idesc_bf16(D, true);
+        // Everything the products are addressed by is the same in all lanes and is added up from 32-bit bases: with
+        // 64-bit descriptors made anew for every product the issue of a tile took longer than its execution.
+        constexpr uint32_t DESC_HI = (uint32_t)((1024 >> 4) | (1u << 14) | (2u << 29));
+        const uint32_t idesc_qk = idesc_bf16(PN, false), idesc_pv = idesc_bf16(D, true);
+        const int nt = __shfl_sync(0xffffffffu, n_tiles, 0);
+        const bool two = __shfl_sync(0xffffffffu, n_half, 0) == 2;
         const bool issue = lane == 0;
-        auto wait_full = [&](int c) -> bool {
-            return __all_sync(0xffffffffu, mb_wait(sa(&bars[PB_FULL + c % PAIR_SLOTS]), (c / PAIR_SLOTS) & 1, status, abort_flag));
+        const uint32_t q_lo = (sa(Qs) >> 4) | (1u << 16), kv_k = (sa(KVs) >> 4) | (1u << 16),
+                       kv_v = (sa(KVs) >> 4) | ((uint32_t)((PN * 128) >> 4) << 16);
+        auto wait_full = [&](int slot, uint32_t parity) -> bool {
+            return __all_sync(0xffffffffu, mb_wait(sa(&bars[PB_FULL + slot]), parity, status, abort_flag));
         };
-        auto issue_qk = [&](int t, int j) {
-            const uint32_t ks = sa(KVs + (size_t)((2 * j) % PAIR_SLOTS) * PAIR_TILE_BYTES);
+        auto qk = [&](int t, int slot, bool last) {
+            const uint32_t a0 = q_lo + (uint32_t)(t * (Q_BYTES >> 4)), b0 = kv_k + (uint32_t)slot * (PAIR_TILE_BYTES >> 4);
 #pragma unroll
             for (int k = 0; k < D / 16; ++k)
-                tc_mma(issue, tm_S + (uint32_t)(t * PN), desc_k_major(sa(Qs + t * Q_BYTES) + (k >> 2) * (BM * 128) + (k & 3) * 32),
-                       desc_k_major(ks + (k >> 2) * (PN * 128) + (k & 3) * 32), idesc_qk, k > 0 ? 1u : 0u);
+                tc_mma_lo(issue, tm_S + (uint32_t)(t * PN), a0 + (k >> 2) * ((BM * 128) >> 4) + (k & 3) * 2,
+                          b0 + (k >> 2) * ((PN * 128) >> 4) + (k & 3) * 2, DESC_HI, idesc_qk, k > 0 ? 1u : 0u);
             tc_commit_to(issue, sa(&bars[PB_S + t]));
-            if (t == n_half - 1) tc_commit_to(issue, sa(&bars[PB_EMPTY + (2 * j) % PAIR_SLOTS]));
-            __syncwarp();
+            if (last) tc_commit_to(issue, sa(&bars[PB_EMPTY + slot]));
         };
-        bool ok = n_tiles > 0 && __all_sync(0xffffffffu, mb_wait(sa(&bars[PB_Q]), 0, status, abort_flag));
-        if (ok) ok = wait_full(0);
+        auto pv = [&](int t, int slot, bool last, bool acc) {
+            const uint32_t b0 = kv_v + (uint32_t)slot * (PAIR_TILE_BYTES >> 4);
+#pragma unroll
+            for (int k = 0; k < PN / 16; ++k)
+                tc_mma_a_tmem_lo(issue, tm_O + (uint32_t)(t * D), tm_S + (uint32_t)(t * PN + k * 8), b0 + k * ((16 * 128) >> 4),
+                                 DESC_HI, idesc_pv, (acc || k > 0) ? 1u : 0u);
+            if (last) tc_commit_to(issue, sa(&bars[PB_EMPTY + slot]));
+        };
+        bool ok = nt > 0 && __all_sync(0xffffffffu, mb_wait(sa(&bars[PB_Q]), 0, status, abort_flag));
+        if (ok) ok = wait_full(0, 0);
         if (ok) {
             tc_after();
-            for (int t = 0; t < n_half; ++t) issue_qk(t, 0);
+            qk(0, 0, !two);
+            if (two) qk(1, 0, true);
         }
-        for (int j = 0; j < n_tiles && ok; ++j) {
-            const uint32_t vs = sa(KVs + (size_t)((2 * j + 1) % PAIR_SLOTS) * PAIR_TILE_BYTES);
-            for (int t = 0; t < n_half && ok; ++t) {
-                // the softmax of one row tile runs while the tensor cores work on the other
-                ok = __all_sync(0xffffffffu, mb_wait(sa(&bars[PB_P + t]), j & 1, status, abort_flag));
-                if (ok && t == 0) ok = wait_full(2 * j + 1);
+        int slot = 0;
+        uint32_t phase = 0;
+        auto next_slot = [&] { if (++slot == PAIR_SLOTS) { slot = 0; phase ^= 1u; } };
+        for (int j = 0; j < nt && ok; ++j) {
+            // the softmax of one row tile runs while the tensor cores work on the other
+            ok = __all_sync(0xffffffffu, mb_wait(sa(&bars[PB_P]), j & 1, status, abort_flag));
+            next_slot();
+            const int v_slot = slot;
+            if (ok) ok = wait_full(slot, phase);
+            if (!ok) break;
+            tc_after();
+            pv(0, v_slot, !two, j > 0);
+            const bool more = j + 1 < nt;
+            if (more) {
+                next_slot();
+                ok = wait_full(slot, phase);
                 if (!ok) break;
                 tc_after();
-#pragma unroll
-                for (int k = 0; k < PN / 16; ++k)
-                    tc_mma_a_tmem(issue, tm_O + (uint32_t)(t * D), tm_S + (uint32_t)(t * PN + k * 8),
-                                  desc_n_major(vs + k * 16 * 128, PN * 128), idesc_pv, (j > 0 || k > 0) ? 1u : 0u);
-                if (t == n_half - 1) tc_commit_to(issue, sa(&bars[PB_EMPTY + (2 * j + 1) % PAIR_SLOTS]));
-                if (j + 1 < n_tiles) {
-                    if (t == 0) ok = wait_full(2 * j + 2);
-                    if (!ok) break;
-                    tc_after();
-                    issue_qk(t, j + 1);
-                } else {
-                    tc_commit_to(issue, sa(&bars[PB_S + t]));           // the last product: O is complete
-                    __syncwarp();
-                }
+                qk(0, slot, !two);
+            } else {
+                tc_commit_to(issue, sa(&bars[PB_S]));               // the last product: O is complete
+            }
+            if (two) {
+                ok = __all_sync(0xffffffffu, mb_wait(sa(&bars[PB_P + 1]), j & 1, status, abort_flag));
+                if (!ok) break;
+                tc_after();
+                pv(1, v_slot, true, j > 0);
+                if (more) qk(1, slot, true);
+                else tc_commit_to(issue, sa(&bars[PB_S + 1]));
             }
         }
+        __syncwarp();
     }
     tc_before();
     __syncthreads();
