@@ -207,13 +207,6 @@ __device__ __forceinline__ void add_pair(uint32_t w, float& a, float& b) {
     asm("{\n\t.reg .b16 x, y;\n\tmov.b32 {x, y}, %2;\n\tadd.rn.f32.bf16 %0, x, %0;\n\tadd.rn.f32.bf16 %1, y, %1;\n\t}"
         : "+f"(a), "+f"(b) : "r"(w));
 }
-// Barrier `id` of two warps; true if `ok` is in all of their threads, so that they leave a loop together.
-__device__ __forceinline__ bool both_ok(int id, bool ok) {
-    uint32_t r;
-    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 q, %1, 0;\n\tbar.red.and.pred p, %2, 64, q;\n\tselp.b32 %0, 1, 0, p;\n\t}"
-                 : "=r"(r) : "r"((uint32_t)ok), "r"(id) : "memory");
-    return r != 0;
-}
 __device__ __forceinline__ float max3(float a, float b, float c) {
     float r;
     asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
@@ -670,12 +663,12 @@ attn_tc_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __restri
 #endif
 constexpr int PN = 128;                              // keys per tile
 constexpr int PAIR_ROWS = 2 * BM;
-constexpr int PAIR_SLOTS = 4;                        // ring of K and V tiles: K0, V0, K1, V1, ...
-constexpr int PAIR_THREADS = 576;                    // warps 0-7 and 8-15 softmax of either row tile, 16 loads, 17 MMAs
+constexpr int PAIR_SLOTS = 5;                        // ring of K and V tiles: K0, V0, K1, V1, ...
+constexpr int PAIR_THREADS = 320;                    // warps 0-3 and 4-7 softmax of either row tile, 8 loads, 9 MMAs
 constexpr int PAIR_TILE_BYTES = PN * D * 2;
 constexpr int PAIR_PAGE_LIST = MAX_PAGE_LIST < 32 ? 32 : MAX_PAGE_LIST > 256 ? 256 : MAX_PAGE_LIST / 32 * 32;
-constexpr size_t PAIR_SMEM = 1024 + 2 * Q_BYTES + PAIR_SLOTS * PAIR_TILE_BYTES + 128 + PAIR_PAGE_LIST * 4 + 2 * 2 * 2 * BM * 4;
-enum { PB_FULL = 0, PB_EMPTY = PB_FULL + PAIR_SLOTS, PB_S = PB_EMPTY + PAIR_SLOTS, PB_P = PB_S + 2, PB_Q = PB_P + 2,
+constexpr size_t PAIR_SMEM = 1024 + 2 * Q_BYTES + PAIR_SLOTS * PAIR_TILE_BYTES + 128 + PAIR_PAGE_LIST * 4;
+enum { PB_FULL = 0, PB_EMPTY = PB_FULL + PAIR_SLOTS, PB_S = PB_EMPTY + PAIR_SLOTS, PB_P = PB_S + 2, PB_Q = PB_P + 4,
        PB_PAGES, PB_COUNT };
 static_assert(PB_COUNT * 8 <= 128, "barriers");
 
@@ -691,7 +684,6 @@ attn_tc_pair_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __r
     unsigned char* KVs = Qs + 2 * Q_BYTES;                           // [slot][PANELS][128][128 B]
     uint64_t* bars = reinterpret_cast<uint64_t*>(KVs + PAIR_SLOTS * PAIR_TILE_BYTES);
     int* s_pages = reinterpret_cast<int*>(bars + 16);
-    float* s_max = reinterpret_cast<float*>(s_pages + PAIR_PAGE_LIST);   // [row tile][tile & 1][key half][128]
     __shared__ int s_seq, s_tile, s_abort, s_tok0, s_qlen, s_ctx;
     __shared__ uint32_t s_tmem;
     const int G = nq / nkv;
@@ -701,12 +693,12 @@ attn_tc_pair_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __r
 
     if (threadIdx.x == 0) {
         s_abort = 0;
-        for (int i = 0; i < PB_COUNT; ++i) mb_init(sa(&bars[i]), i >= PB_Q ? 16 : i >= PB_P ? 8 : 1);
+        for (int i = 0; i < PB_COUNT; ++i) mb_init(sa(&bars[i]), i >= PB_Q ? 8 : i >= PB_P ? 4 : 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
     // All of the SM's tensor memory: taken after the kernels before this one are done, and before the next one may start.
-    if (warp == 17) {
+    if (warp == 9) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sa(&s_tmem)), "r"(512u) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -773,79 +765,62 @@ attn_tc_pair_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __r
         }
     };
 
-    if (warp < 16) {
-        // A row of S is shared by two threads, one to either half of the tile's keys: four softmax warps to a
-        // scheduler instead of two, which hides the latencies that a thread meets on its own.
-        const int half = warp >> 3, kh2 = (warp >> 2) & 1;           // the row tile, the half of its keys
-        const int r = (warp & 3) * 32 + lane;
+    if (warp < 8) {
+        const int half = warp >> 2;                                  // the row tile of this warp
+        const int r = threadIdx.x & 127;
         const int t0 = row0 + half * BM;                             // the row tile's first row
         const int rg = t0 + r;
         const bool valid = rg < rows;
         const int rgc = min(rg, max(rows - 1, 0));
         const int token = rgc / G, head = kh * G + rgc % G;
-        constexpr int QC = D / 16;                                   // 16-byte pieces of half a row
-        uint4 qv[QC];
+        uint4 qv[D / 8];
         if (n_tiles > 0) {
-            const uint4* src = reinterpret_cast<const uint4*>(q + (size_t)(tok0 + token) * q_stride + (size_t)head * D) + kh2 * QC;
+            const uint4* src = reinterpret_cast<const uint4*>(q + (size_t)(tok0 + token) * q_stride + (size_t)head * D);
 #pragma unroll
-            for (int ch = 0; ch < QC; ++ch) qv[ch] = valid ? __ldg(src + ch) : make_uint4(0u, 0u, 0u, 0u);
+            for (int ch = 0; ch < D / 8; ++ch) qv[ch] = valid ? __ldg(src + ch) : make_uint4(0u, 0u, 0u, 0u);
         }
-        fill_pages(0, min(n_tiles, 2 * tph), threadIdx.x, 512);
+        fill_pages(0, min(n_tiles, 2 * tph), threadIdx.x, 256);
         __syncwarp();
         if (lane == 0) mb_arrive(sa(&bars[PB_PAGES]));
         if (n_tiles > 0) {
 #pragma unroll
-            for (int i = 0; i < QC; ++i) {
-                const int ch = kh2 * QC + i;
-                *reinterpret_cast<uint4*>(Qs + half * Q_BYTES + (ch >> 3) * (BM * 128) + r * 128 + (((ch & 7) ^ (r & 7)) << 4)) = qv[i];
-            }
+            for (int ch = 0; ch < D / 8; ++ch)
+                *reinterpret_cast<uint4*>(Qs + half * Q_BYTES + (ch >> 3) * (BM * 128) + r * 128 + (((ch & 7) ^ (r & 7)) << 4)) = qv[ch];
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (lane == 0) mb_arrive(sa(&bars[PB_Q]));
 
         if (half < n_half) {
-            constexpr int KEYS = PN / 2;
             const int pos = ctx + token;
             const int hi = pos + 1;
             const int lo = first_visible_key(pos, window);
             const int first_pos = ctx + t0 / G;
             const int full_lo = first_visible_key(ctx + min(q_len - 1, (t0 + BM - 1) / G), window);
             const uint32_t lane_base = (uint32_t)(((warp & 3) * 32) << 16);
-            const uint32_t tm_s = tm_S + (uint32_t)(half * PN) + lane_base;
-            const uint32_t tm_o = tm_O + (uint32_t)(half * D + kh2 * (D / 2)) + lane_base;     // this thread's columns of O
-            float* x_mine = s_max + (half * 4 + kh2) * BM + r;
-            float* x_other = s_max + (half * 4 + (kh2 ^ 1)) * BM + r;
-            const int bar_id = 1 + half * 4 + (warp & 3);            // the two warps that share 32 rows
-            const bool has_sink = sink != nullptr;
-            float m = has_sink ? sink[head] * LOG2E : -CUDART_INF_F, l = has_sink && kh2 == 0 ? 1.f : 0.f;
+            const uint32_t tm_s = tm_S + (uint32_t)(half * PN) + lane_base, tm_o = tm_O + (uint32_t)(half * D) + lane_base;
+            float m = sink ? sink[head] * LOG2E : -CUDART_INF_F, l = sink ? 1.f : 0.f;
             const uint64_t scale2 = pack2(scale_log2, scale_log2);
             bool ok = true;
             for (int j = 0; j < n_tiles && ok; ++j) {
                 // S of this tile; the product P V of the tile before was issued ahead of it, so O is at rest as well
                 ok = mb_wait(sa(&bars[PB_S + half]), j & 1, status, abort_flag);
                 ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
                 tc_after();
-                const int key0 = (t_begin + j) * PN + kh2 * KEYS;
-                float s[KEYS];
+                const int key0 = (t_begin + j) * PN;
+                float s[PN];
 #pragma unroll
-                for (int c = 0; c < KEYS / 32; ++c) tm_ld32_nowait(tm_s + kh2 * KEYS + c * 32, s + c * 32);
+                for (int c = 0; c < PN / 32; ++c) tm_ld32_nowait(tm_s + c * 32, s + c * 32);
                 tm_ld_wait();
-                if (key0 + KEYS > first_pos + 1 || key0 < full_lo) {
+                if (key0 + PN > first_pos + 1 || key0 < full_lo) {
 #pragma unroll
-                    for (int i = 0; i < KEYS; ++i) {
+                    for (int i = 0; i < PN; ++i) {
                         const int key = key0 + i;
                         if (key < lo || key >= hi) s[i] = -CUDART_INF_F;
                     }
                 }
-                float mx = row_max<KEYS>(s);
-                // The other half's maximum.  Behind this barrier both warps have also read S, over which P is written.
-                x_mine[(j & 1) * 2 * BM] = mx;
-                tc_before();
-                ok = both_ok(bar_id, ok);
-                if (!ok) break;
-                tc_after();
-                mx = fmaxf(mx, x_other[(j & 1) * 2 * BM]) * scale_log2;
+                const float mx = row_max<PN>(s) * scale_log2;
                 float corr = 1.0f;
                 if (mx > m + 8.0f || m == -CUDART_INF_F) {
                     const float m_new = fmaxf(m, mx);
@@ -854,7 +829,7 @@ attn_tc_pair_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __r
                 }
                 if (j > 0 && !__all_sync(0xffffffffu, corr == 1.0f)) {       // some row's reference max moved: rescale O
 #pragma unroll 1
-                    for (int c = 0; c < D / 32; ++c) {
+                    for (int c = 0; c < D / 16; ++c) {
                         float v[16];
                         tm_ld16(tm_o + c * 16, v);
 #pragma unroll
@@ -866,33 +841,37 @@ attn_tc_pair_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __r
                 const uint64_t neg_m2 = pack2(neg_m, neg_m);
                 float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-                for (int c = 0; c < KEYS / 32; ++c) {
+                for (int c = 0; c < PN / 32; ++c) {
                     uint32_t w[16];
 #pragma unroll
                     for (int e = 0; e < 16; ++e) {
                         w[e] = exp2_scaled(s[c * 32 + 2 * e], s[c * 32 + 2 * e + 1], scale2, neg_m2);
                         add_pair(w[e], sum[(e & 1) * 2], sum[(e & 1) * 2 + 1]);
                     }
-                    tm_st16u(tm_s + kh2 * (KEYS / 2) + c * 16, w);   // P over the first half of S
+                    tm_st16u(tm_s + c * 16, w);                     // P over the first half of S, which is in registers
+                    if (c == PN / 64 - 1) {                         // half of the keys: their products may start
+                        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                        tc_before();
+                        __syncwarp();
+                        if (lane == 0) mb_arrive(sa(&bars[PB_P + half]));
+                    }
                 }
                 l = l * corr + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 tc_before();
                 __syncwarp();
-                if (lane == 0) mb_arrive(sa(&bars[PB_P + half]));
+                if (lane == 0) mb_arrive(sa(&bars[PB_P + 2 + half]));
             }
-            if (n_tiles > 0) {
-                ok = ok && mb_wait(sa(&bars[PB_S + half]), n_tiles & 1, status, abort_flag);
+            if (n_tiles > 0 && ok) {
+                ok = mb_wait(sa(&bars[PB_S + half]), n_tiles & 1, status, abort_flag);
                 ok = __all_sync(0xffffffffu, ok);
-                x_mine[(n_tiles & 1) * 2 * BM] = l;                  // the buffer of the tile before the last
-                ok = both_ok(bar_id, ok);
             }
             if (n_tiles > 0 && ok) {
                 tc_after();
-                const float inv = 1.0f / (kh2 ? x_other[(n_tiles & 1) * 2 * BM] + l : l + x_other[(n_tiles & 1) * 2 * BM]);
-                bf16* dst = out + (size_t)(tok0 + token) * out_stride + (size_t)head * D + kh2 * (D / 2);
+                const float inv = 1.0f / l;
+                bf16* dst = out + (size_t)(tok0 + token) * out_stride + (size_t)head * D;
 #pragma unroll 1
-                for (int c = 0; c < D / 32; ++c) {
+                for (int c = 0; c < D / 16; ++c) {
                     float v[16];
                     tm_ld16(tm_o + c * 16, v);
                     if (valid) {
@@ -908,7 +887,7 @@ attn_tc_pair_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __r
                 }
             }
         }
-    } else if (warp == 16) {
+    } else if (warp == 8) {
         bool ok = n_tiles == 0 || mb_wait(sa(&bars[PB_PAGES]), 0, status, abort_flag);
         ok = __all_sync(0xffffffffu, ok);
         const int p = lane / PANELS, h = lane % PANELS;                  // this lane's page and panel of a tile
@@ -967,13 +946,20 @@ attn_tc_pair_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __r
             tc_commit_to(issue, sa(&bars[PB_S + t]));
             if (last) tc_commit_to(issue, sa(&bars[PB_EMPTY + slot]));
         };
-        auto pv = [&](int t, int slot, bool last, bool acc) {
+        // O += P V of row tile t, the first half of the keys as soon as their P is there
+        auto pv = [&](int t, int slot, int j, bool last) -> bool {
             const uint32_t b0 = kv_v + (uint32_t)slot * (PAIR_TILE_BYTES >> 4);
 #pragma unroll
-            for (int k = 0; k < PN / 16; ++k)
-                tc_mma_a_tmem_lo(issue, tm_O + (uint32_t)(t * D), tm_S + (uint32_t)(t * PN + k * 8), b0 + k * ((16 * 128) >> 4),
-                                 DESC_HI, idesc_pv, (acc || k > 0) ? 1u : 0u);
+            for (int h = 0; h < 2; ++h) {
+                if (!__all_sync(0xffffffffu, mb_wait(sa(&bars[PB_P + 2 * h + t]), j & 1, status, abort_flag))) return false;
+                tc_after();
+#pragma unroll
+                for (int k = h * (PN / 32); k < (h + 1) * (PN / 32); ++k)
+                    tc_mma_a_tmem_lo(issue, tm_O + (uint32_t)(t * D), tm_S + (uint32_t)(t * PN + k * 8), b0 + k * ((16 * 128) >> 4),
+                                     DESC_HI, idesc_pv, (j > 0 || k > 0) ? 1u : 0u);
+            }
             if (last) tc_commit_to(issue, sa(&bars[PB_EMPTY + slot]));
+            return true;
         };
         bool ok = nt > 0 && __all_sync(0xffffffffu, mb_wait(sa(&bars[PB_Q]), 0, status, abort_flag));
         if (ok) ok = wait_full(0, 0);
@@ -987,14 +973,12 @@ attn_tc_pair_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __r
         auto next_slot = [&] { if (++slot == PAIR_SLOTS) { slot = 0; phase ^= 1u; } };
         for (int j = 0; j < nt && ok; ++j) {
             // the softmax of one row tile runs while the tensor cores work on the other
-            ok = __all_sync(0xffffffffu, mb_wait(sa(&bars[PB_P]), j & 1, status, abort_flag));
             next_slot();
             const int v_slot = slot;
-            if (ok) ok = wait_full(slot, phase);
-            if (!ok) break;
-            tc_after();
-            pv(0, v_slot, !two, j > 0);
             const bool more = j + 1 < nt;
+            ok = wait_full(slot, phase);
+            if (ok) ok = pv(0, v_slot, j, !two);
+            if (!ok) break;
             if (more) {
                 next_slot();
                 ok = wait_full(slot, phase);
@@ -1005,10 +989,8 @@ attn_tc_pair_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __r
                 tc_commit_to(issue, sa(&bars[PB_S]));               // the last product: O is complete
             }
             if (two) {
-                ok = __all_sync(0xffffffffu, mb_wait(sa(&bars[PB_P + 1]), j & 1, status, abort_flag));
+                ok = pv(1, v_slot, j, true);
                 if (!ok) break;
-                tc_after();
-                pv(1, v_slot, true, j > 0);
                 if (more) qk(1, slot, true);
                 else tc_commit_to(issue, sa(&bars[PB_S + 1]));
             }
@@ -1017,7 +999,7 @@ attn_tc_pair_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __r
     }
     tc_before();
     __syncthreads();
-    if (warp == 17) {
+    if (warp == 9) {
         __syncwarp();
         tc_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
