@@ -667,10 +667,10 @@ constexpr int PAIR_SLOTS = 5;                        // ring of K and V tiles: K
 constexpr int PAIR_THREADS = 320;                    // warps 0-3 and 4-7 softmax of either row tile, 8 loads, 9 MMAs
 constexpr int PAIR_TILE_BYTES = PN * D * 2;
 constexpr int PAIR_PAGE_LIST = MAX_PAGE_LIST < 32 ? 32 : MAX_PAGE_LIST > 256 ? 256 : MAX_PAGE_LIST / 32 * 32;
-constexpr size_t PAIR_SMEM = 1024 + 2 * Q_BYTES + PAIR_SLOTS * PAIR_TILE_BYTES + 128 + PAIR_PAGE_LIST * 4;
+constexpr size_t PAIR_SMEM = 1024 + 2 * Q_BYTES + PAIR_SLOTS * PAIR_TILE_BYTES + 256 + PAIR_PAGE_LIST * 4;
 enum { PB_FULL = 0, PB_EMPTY = PB_FULL + PAIR_SLOTS, PB_S = PB_EMPTY + PAIR_SLOTS, PB_P = PB_S + 2, PB_Q = PB_P + 4,
        PB_PAGES, PB_COUNT };
-static_assert(PB_COUNT * 8 <= 128, "barriers");
+static_assert(PB_COUNT * 8 <= 256, "barriers");
 
 __global__ void __launch_bounds__(PAIR_THREADS, 1)
 attn_tc_pair_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __restrict__ q, int q_stride,
@@ -683,7 +683,7 @@ attn_tc_pair_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __r
     unsigned char* Qs = base;                                        // [row tile][PANELS][128][128 B]
     unsigned char* KVs = Qs + 2 * Q_BYTES;                           // [slot][PANELS][128][128 B]
     uint64_t* bars = reinterpret_cast<uint64_t*>(KVs + PAIR_SLOTS * PAIR_TILE_BYTES);
-    int* s_pages = reinterpret_cast<int*>(bars + 16);
+    int* s_pages = reinterpret_cast<int*>(bars + 32);
     __shared__ int s_seq, s_tile, s_abort, s_tok0, s_qlen, s_ctx;
     __shared__ uint32_t s_tmem;
     const int G = nq / nkv;
