@@ -304,6 +304,34 @@ def test_attention_tcgen05_walks_long_block_tables_in_pieces(d, nq, nkv, block, 
     assert float(err) < 2e-2, float(err)
 
 
+@pytest.mark.parametrize("d,nq,nkv,block,page_list", [(64, 16, 8, 8, 16), (128, 16, 8, 64, None), (128, 32, 8, 16, 32)])
+@pytest.mark.parametrize("window,sinks", [(None, False), (150, False), (None, True)])
+def test_attention_tcgen05_two_row_tiles_a_block(d, nq, nkv, block, page_list, window, sinks):
+    """Enough row tiles for two of them to a block (a pair for every SM): sequences with an odd number of row tiles and with
+    parts of one, ends inside a tile of 128 keys, windows that leave a row tile's first keys out, a ring of page ids of one
+    tile a half; with sinks against the kernel that walks key by key."""
+    seqs = [(0, 1000), (300, 700), (700, 300), (130, 70), (0, 129), (5, 17)]
+    c = _attention_case(d, nq, nkv, block, seqs, window, torch.bfloat16, seed=13)
+    tiles = sum(-(-(ql * (nq // nkv)) // 128) for ql in c["q_lens"])
+    assert tiles * nkv >= 2 * 148
+    out = torch.zeros(c["q"].shape, dtype=torch.bfloat16, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    q, pages, table = dev(c["q"]), dev(c["pages"]), dev(c["table"])
+    sink = 3.0 * torch.randn(nq, device="cuda", generator=torch.Generator("cuda").manual_seed(3)) if sinks else None
+    K().attn_tc(q, nq * d, pages, table, dev(c["cu_q"]), dev(c["ctx_lens"]), len(seqs), tiles, out, nq, nkv, d,
+                1 / math.sqrt(d), window or 0, status, page_list=page_list, sink=sink)
+    want = c["want"]
+    if sinks:
+        ref = torch.empty_like(out)
+        K().paged_attention_simt(q, nq * d, pages, table, dev(c["token_seq"]), dev(c["positions"]), ref, nq, nkv, d,
+                                 1 / math.sqrt(d), window or 0, status, sink=sink)
+        want = ref.cpu().double()
+    torch.cuda.synchronize()
+    assert int(status) == 0
+    # P is rounded to bfloat16 (2^-9) and so is the result: a few times that of the largest output
+    assert float((out.cpu().double() - want).abs().max() / want.abs().max()) < 2e-2
+
+
 def test_attention_tcgen05_context_beyond_one_ring_of_page_ids():
     """The product build at a context of 17 000 tokens in pages of 16: 1 066 page ids a block, more than
     its ring of 1 024 holds.  Only the portion's 200 queries are compared (softmax over keys 0..position
