@@ -1,0 +1,114 @@
+"""The element-wise kernels around the recurrences and the latent attention, in their forms with vector loads and without
+(csrc/ssm.cu, csrc/wkv.cu, csrc/delta_rule.cu, csrc/latent_attention.cu), against the formulas in 64 bits: sequences that end
+around the rows a thread takes (4) and a block's tile (32 and 16), sizes that vectors divide and that they do not, rows that
+start off a 16-byte boundary.
+
+Tolerance: a result is rounded to bfloat16 once (2^-9 of it; twice that is allowed) behind a few dozen 32-bit roundings of
+terms no larger than the largest value (2^-18 of that)."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from firefly_b200.ops import kernels as K
+
+pytestmark = pytest.mark.gpu
+BF, F32, F64 = torch.bfloat16, torch.float32, torch.float64
+LENS = [(1, 2, 3, 4, 5, 31, 32, 33), (63, 1, 64, 65, 7), (4500, 1, 130)]
+
+
+def _rand(*shape, dtype=F32, seed=0):
+    g = torch.Generator("cuda").manual_seed(seed + sum(shape))
+    return torch.randn(*shape, generator=g, device="cuda").to(dtype)
+
+
+def _close(got, want):
+    assert got.dtype == BF
+    err = (got.double() - want).abs()
+    assert bool((err <= 2.0 ** -8 * want.abs() + 2.0 ** -18 * want.abs().max()).all())
+
+
+def _ctx(lens):
+    n = len(lens)
+    cu = torch.tensor([0, *torch.tensor(lens).cumsum(0).tolist()], dtype=torch.int32, device="cuda")
+    seq = torch.repeat_interleave(torch.arange(n), torch.tensor(lens)).to(torch.int32).cuda()
+    return SimpleNamespace(cu_q=cu, token_seq=seq, num_seqs=n, state_slots=torch.arange(n, 0, -1, dtype=torch.int32, device="cuda"),
+                           seq_fresh=(torch.arange(n) % 2).to(torch.int32).cuda())
+
+
+@pytest.mark.parametrize("lens", LENS)
+@pytest.mark.parametrize("channels,col0,taps", [(256, 0, 4), (136, 8, 4), (70, 3, 4), (128, 0, 3), (64, 64, 2)])
+def test_convolution(lens, channels, col0, taps):
+    ctx, T = _ctx(lens), sum(lens)
+    x, w, b = _rand(T, channels + col0 + 5, dtype=BF), _rand(channels, taps), _rand(channels)
+    state = _rand(len(lens) + 1, (taps - 1) * channels)
+    old, out = state.clone(), torch.empty(T, channels, dtype=BF, device="cuda")
+    K.causal_conv_silu(x, col0, channels, w, b, state, 0, ctx, out)
+    at = 0
+    for i, n in enumerate(lens):
+        slot = len(lens) - i
+        front = old[slot].view(taps - 1, channels).double() * (0 if i % 2 else 1)
+        rows = torch.cat([front, x[at:at + n, col0:col0 + channels].double()])
+        want = b.double() + sum(w[:, j].double() * rows[j:j + n] for j in range(taps))
+        _close(out[at:at + n], want * torch.sigmoid(want))
+        assert torch.equal(state[slot].view(taps - 1, channels), rows[-(taps - 1):].float())
+        at += n
+
+
+@pytest.mark.parametrize("width,parts,shift", [(128, 1, 0), (512, 2, 0), (1024, 1, 8), (2048, 8, 0), (4096, 1, 0), (300, 3, 0),
+                                               (1024, 1, 1), (16384, 1, 0)])
+@pytest.mark.parametrize("first", [True, False])
+def test_gated_norm(width, parts, shift, first):
+    T = 37
+    o, g, w = _rand(T, width), _rand(T, width + shift + 3 * (shift % 2), dtype=BF), 1 + 0.1 * _rand(width)
+    y = torch.empty(T, width, dtype=BF, device="cuda")
+    K.gated_rms_norm(o, (g, shift), w, 1e-5, y, parts, first)
+    gd, od = g[:, shift:shift + width].double(), o.double()
+    od = od * gd * torch.sigmoid(gd) if first else od
+    n = od.view(T, parts, -1)
+    n = (n / (n.square().mean(-1, keepdim=True) + 1e-5).sqrt()).reshape(T, width) * w.double()
+    _close(y, n if first else n * torch.sigmoid(gd))
+
+
+@pytest.mark.parametrize("heads,V,shift", [(4, 64, 0), (3, 128, 8), (5, 128, 1), (2, 96, 0), (1, 64, 0)])
+@pytest.mark.parametrize("act", ["sigmoid", "silu"])
+@pytest.mark.parametrize("gate_type", [BF, F32])
+def test_norm_of_heads(heads, V, shift, act, gate_type):
+    T, W = 61, heads * V
+    o, g, w = _rand(T, W), _rand(T, W + shift, dtype=gate_type), 1 + 0.1 * _rand(V)
+    y = torch.empty(T, W, dtype=BF, device="cuda")
+    K.head_norm_gate(o, (g, shift), w, 1e-5, y, heads, V, act)
+    gd, od = g[:, shift:].double(), o.double().view(T, heads, V)
+    n = (od / (od.square().mean(-1, keepdim=True) + 1e-5).sqrt() * w.double()).reshape(T, W)
+    _close(y, n * torch.sigmoid(gd) * (gd if act == "silu" else 1))
+
+
+@pytest.mark.parametrize("lens", LENS)
+@pytest.mark.parametrize("heads,dim", [(4, 64), (3, 128), (5, 24)])
+def test_mix_and_output_of_wkv(lens, heads, dim):
+    ctx, T, W = _ctx(lens), sum(lens), heads * dim
+    x, mu, state = _rand(T, W, dtype=BF), _rand(5, W), _rand(len(lens) + 1, W)
+    mixes = torch.empty(5, T, W, dtype=BF, device="cuda")
+    K.wkv_shift_mix(x, mu, state, 0, ctx, mixes)
+    prev = torch.cat([x[:1].double(), x[:-1].double()])
+    for i in range(len(lens)):
+        prev[int(ctx.cu_q[i])] = state[len(lens) - i].double() * (0 if i % 2 else 1)
+    _close(mixes, x.double() + (prev - x.double()) * mu.double()[:, None])
+    o, g, w = _rand(T, W, seed=1), _rand(T, W, dtype=BF, seed=2), 1 + 0.1 * _rand(W)
+    y = torch.empty(T, W, dtype=BF, device="cuda")
+    K.wkv_out(o, g, w, 1e-5, y, heads, dim)
+    od, gd = o.double().view(T, heads, dim), g.double()
+    n = (od / (od.square().mean(-1, keepdim=True) + 1e-5).sqrt()).reshape(T, W) * w.double()
+    _close(y, n * gd * torch.sigmoid(gd))
+
+
+@pytest.mark.parametrize("T,heads,vdim,shift,per_head", [(33, 4, 128, 0, False), (5, 3, 64, 8, False), (17, 3, 64, 1, False),
+                                                         (9, 5, 20, 0, False), (33, 4, 128, 0, True)])
+def test_gate_of_latent_attention(T, heads, vdim, shift, per_head):
+    n = heads if per_head else heads * vdim
+    val, g = _rand(heads, T, vdim, dtype=BF), _rand(T, n + shift, dtype=BF)[:, shift:]
+    y = torch.empty(T, heads * vdim, dtype=BF, device="cuda")
+    K.latent_gate(val, g, y, heads, vdim, per_head)
+    gate = torch.sigmoid(g.double())
+    gate = gate.repeat_interleave(vdim, 1) if per_head else gate
+    _close(y, val.double().transpose(0, 1).reshape(T, -1) * gate)
