@@ -914,12 +914,16 @@ def _recurrence_scratch_bytes(module: str, entry: str, *sizes: int) -> int:
 
 def _recurrence_scratch(ctx, module: str, entry: str, *sizes: int):
     """Scratch memory for a recurrence that takes a step's prompts a chunk at a time: (pointer, bytes), nothing when the step
-    is none for it or the context has no workspace (the token-by-token kernel runs then)."""
+    is none for it, the context has no workspace or the device has no memory left (the token-by-token kernel runs then)."""
     ws = getattr(ctx, "workspace", None)
     need = _recurrence_scratch_bytes(module, entry, *sizes) if ws is not None else 0
     if need <= 0:
         return c_void_p(0), ctypes.c_longlong(0)
-    return _p(ws.get("scan.records", (-(-need // 4),), torch.float32)), ctypes.c_longlong(need)
+    try:
+        records = ws.get("scan.records", (-(-need // 4),), torch.float32)
+    except torch.OutOfMemoryError:
+        return c_void_p(0), ctypes.c_longlong(0)
+    return _p(records), ctypes.c_longlong(need)
 
 
 def _count_preparing(scratch) -> None:
