@@ -4,7 +4,6 @@
 // A block owns 128 rows of one kv head (row = token * G + head-in-group, so the heads of a
 // group share every key and value it fetches) and walks the visible keys in tiles of 64:
 //   S = Q K^T      tcgen05.mma, Q and K from shared memory (K brought in by TMA, page by page),
-//                  S (128 x 64, float32) in tensor memory;
 //                  S (128 x 64, float32) in tensor memory, two buffers, so that the product for
 //                  the next tile runs while the softmax works on this one;
 //   softmax        four warps, one thread per row: tcgen05.ld of its row of S, mask, running max
@@ -14,7 +13,8 @@
 //                  MMA's N-major operand form), O (128 x D, float32) in tensor memory.
 // One warp starts the TMA copies, a page and panel per lane (K and V have two stages each, freed
 // separately); one warp issues the MMAs, converged, with the issuing lane predicated; two blocks
-// share an SM (at head size 128).
+// share an SM (at head size 128).  Portions with enough row tiles, at head sizes of 64 and 128, take two
+// row tiles a block and tiles of 128 keys instead (attn_tc_pair_kernel below).
 //
 // It replaces, for head sizes that are multiples of 64 and page sizes that divide 64, the
 // mma.sync kernel of attention_mma.cu (which stays for every other size); the reference's
@@ -187,8 +187,9 @@ __device__ __forceinline__ uint32_t exp2_bf16x2(float x0, float x1) {
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(y) : "f"(p1), "f"(p0));        // low half = p0
     return y;
 }
-// Pairs of 32-bit values in one register pair, and the steps of the softmax that work on them: half the
-// instructions of the element-by-element form, which were what the softmax warps spent their time on.
+// Pairs of 32-bit values in one register pair, and the steps of the softmax that work on them: fewer instructions than
+// the element-by-element form (scale, maximum, sum), on which the softmax warps spent their time: attn_tc_kernel 681 -> 640 us
+// for a prompt of 8191 tokens, 60.8 -> 57.4 for 2048 (32 heads on 8 kv heads of 128).
 __device__ __forceinline__ uint64_t pack2(float a, float b) {
     uint64_t r;
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
@@ -656,11 +657,25 @@ attn_tc_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __restri
 }
 
 // ------------------------------------------------------------ two row tiles a block --
+// A block owns two neighbouring row tiles of a kv head and walks the keys in tiles of 128 that both use: while four softmax
+// warps work on the scores of one row tile, the tensor cores form P V and the next Q K^T of the other.  One block fills the
+// SM (all of the tensor memory: S and O of either row tile, P over S; Q and a ring of five K or V tiles in shared memory).
+// What bounded the kernel above was the chain softmax -> P -> P V -> next scores of a block with two blocks an SM, and K and V
+// that every block fetched for itself (a tile's MMAs waited 1100 cycles for them, 26 bytes a cycle and SM from L2); here K and
+// V cross once for 256 rows.  The products of half a tile's keys start when their P is there; the P of a row tile is
+// written while products of the other are running, and a row tile's next scores come behind its P V, so that they also
+// say that O is at rest.  Cycles a tile of 256 x 128: 3700, of which the softmax of a row tile takes 2000 (special-function
+// unit 1024), its products with their hand-over 1600 (1024 at the tensor cores' peak); both chains wait for latencies.
+// Measured (us a launch, 32 heads on 8 kv heads of 128, one prompt; before: the kernel above as it was): 8191 tokens 681 -> 525
+// (1.05 PFLOP/s), 2048 tokens 60.5 -> 54.2.  Tried: two threads a row (16 softmax warps): 548 at 8191 tokens, the exponentials of a
+// row tile then fight for the unit; a fetch of all P before its products start: 532; the MMAs' operand descriptors made
+// anew in 64 bits: 537.
 #define FF_ATC_PAIR (FF_HEAD_DIM <= 128)
 #if FF_ATC_PAIR
-#ifndef FF_PAIR_MIN
-#define FF_PAIR_MIN 296
-#endif
+// From this many row tiles (times kv heads) on, a pair for every SM, row tiles go in pairs.  Below it pairs leave SMs idle: us
+// for one prompt, two tiles a block / one: 1024 tokens (256 tiles) 30.8 / 34.6 and 28.4 / 28.4 at best, 640 tokens (160) 22.4 / 20.6,
+// 384 (96) 18.5 / 14.6.
+constexpr long long PAIR_MIN_TILES = 2 * 148;
 constexpr int PN = 128;                              // keys per tile
 constexpr int PAIR_ROWS = 2 * BM;
 constexpr int PAIR_SLOTS = 5;                        // ring of K and V tiles: K0, V0, K1, V1, ...
@@ -1129,7 +1144,7 @@ FF_EXPORT int ff_attn_tc(const void* q, int q_stride, const void* cache, const i
     std::memcpy(arg.bytes, &map, sizeof(map));
 #if FF_ATC_PAIR
     const long long pairs = (((long long)total_tiles + n_seqs) / 2) * nkv;    // at least ceil(row tiles of a sequence / 2), summed
-    if (num_splits == 1 && !dist_bias && softcap == 0.f && (long long)total_tiles * nkv >= FF_PAIR_MIN && pairs < (1ll << 31)) {
+    if (num_splits == 1 && !dist_bias && softcap == 0.f && (long long)total_tiles * nkv >= PAIR_MIN_TILES && pairs < (1ll << 31)) {
         FF_SMEM_LIMIT(attn_tc_pair_kernel, PAIR_SMEM);
         FF_LAUNCH((attn_tc_pair_kernel), dim3((unsigned)pairs), PAIR_THREADS, PAIR_SMEM, stream, arg, (const bf16*)q, q_stride,
                   block_table, max_blocks, cu_q, ctx_lens, n_seqs, (bf16*)out, out_stride, nq, nkv, block_size, num_blocks,
