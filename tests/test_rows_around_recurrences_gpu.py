@@ -1,5 +1,5 @@
-"""The element-wise kernels around the recurrences and the latent attention, in their forms with vector loads and without
-(csrc/ssm.cu, csrc/wkv.cu, csrc/delta_rule.cu, csrc/latent_attention.cu), against the formulas in 64 bits: sequences that end
+"""The element-wise kernels around the recurrences and the latent attention, and the sum of experts' rows, in their forms with vector loads and without
+(csrc/ssm.cu, csrc/wkv.cu, csrc/delta_rule.cu, csrc/latent_attention.cu, csrc/moe.cu), against the formulas in 64 bits: sequences that end
 around the rows a thread takes (4) and a block's tile (32 and 16), sizes that vectors divide and that they do not, rows that
 start off a 16-byte boundary.
 
@@ -112,3 +112,18 @@ def test_gate_of_latent_attention(T, heads, vdim, shift, per_head):
     gate = torch.sigmoid(g.double())
     gate = gate.repeat_interleave(vdim, 1) if per_head else gate
     _close(y, val.double().transpose(0, 1).reshape(T, -1) * gate)
+
+
+@pytest.mark.parametrize("T,W,top", [(9, 1024, 4), (3, 20, 1), (5, 2500, 8), (7, 1032, 9), (4, 30, 2)])
+@pytest.mark.parametrize("form", ["plain", "shared", "weighted", "written"])
+def test_sum_of_experts_rows(T, W, top, form):
+    rows, wts, res, shared, z = _rand(T * top + 3, W), _rand(T, top), _rand(T, W, seed=1), _rand(T, W, seed=2), _rand(T, seed=3)
+    row_of = torch.randperm(T * top + 3, device="cuda")[:T * top].to(torch.int32)
+    want = (rows.double()[row_of.long()].view(T, top, W) * (1 if form == "weighted" else wts.double()[:, :, None])).sum(1)
+    want = want + (shared.double() * torch.sigmoid(z.double())[:, None] if form != "plain" else 0)
+    want = 0.5 * want + (0 if form == "written" else res.double())
+    got = res.clone()
+    K.moe_combine(got, rows, row_of, None if form == "weighted" else wts, None if form == "plain" else shared, 0.5, top=top,
+                  shared_z=None if form == "plain" else z, overwrite=form == "written")
+    # 32-bit sums of top + 2 terms
+    assert bool(((got.double() - want).abs() <= 2.0 ** -23 * (top + 2) * rows.abs().max() * wts.abs().max().clamp(min=1) * 4).all())
