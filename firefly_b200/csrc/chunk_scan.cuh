@@ -56,22 +56,6 @@ __device__ __forceinline__ void chunk_of_record(const int* cu_q, int n_seqs, int
     }
 }
 
-// The same behind a record whose chunk (or -1) starts at row t0 with `left` rows of its sequence from there on, with the new
-// ones of both: the sequence's next chunk mostly, which needs no look at memory.  False: none.
-__device__ __forceinline__ bool chunk_next_record(const int* cu_q, int n_seqs, int r, int& s, int& chunk, int& t0, int& left) {
-    if (chunk >= 0 && left > CS_C) {
-        ++chunk;
-        t0 += CS_C;
-        left -= CS_C;
-        return true;
-    }
-    chunk_of_record(cu_q, n_seqs, r, s, chunk);
-    if (chunk < 0) return false;
-    t0 = cu_q[s] + chunk * CS_C;
-    left = cu_q[s + 1] - t0;
-    return true;
-}
-
 // ---------------------------------------------------------------------------------- the first kernel's parts --
 // sq, sk, sa: the chunk's q, k and decays in shared memory, [16][NK] 32-bit; rows behind the sequence's end have q = k = 0 and
 // decay 1.  2 NK threads.

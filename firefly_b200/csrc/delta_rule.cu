@@ -280,15 +280,17 @@ __global__ void __launch_bounds__(2 * NK) delta_prepare_kernel(DeltaArgs A, Chun
 #pragma unroll
     for (int i = 0; i < 8; ++i) bias[i] = A.dt_bias[A.decay_per_head ? h : h * NK + col + i];
     const int r0 = blockIdx.x * per_block, r1 = min(n_records, r0 + per_block);
-    int s, chunk = -1, t0 = 0, left = 0;
+    int s, chunk, left = 0;
     uint4 qv, kv;
     float4 d0, d1;
     float braw = 0.f;
     auto fetch = [&](int r) {
-        const bool any = chunk_next_record(cu_q, n_seqs, r, s, chunk, t0, left);
+        chunk_of_record(cu_q, n_seqs, r, s, chunk);
         qv = kv = make_uint4(0, 0, 0, 0);
         d0 = d1 = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (!any) return;
+        if (chunk < 0) return;
+        const int t0 = cu_q[s] + chunk * CS_C;
+        left = cu_q[s + 1] - t0;
         if (row < left) {
             qv = *reinterpret_cast<const uint4*>(qp + (size_t)(t0 + row) * A.q_stride);
             kv = *reinterpret_cast<const uint4*>(kp + (size_t)(t0 + row) * A.k_stride);

@@ -258,14 +258,16 @@ __global__ void __launch_bounds__(2 * NK) wkv_prepare_kernel(const bf16* rkvg, c
     for (int i = 0; i < 8; ++i) w0c[i] = w0[h * NK + col + i];
     if (tid < NK) su[tid] = u[h * NK + tid];
     const int r0 = blockIdx.x * per_block, r1 = min(n_records, r0 + per_block);
-    int s, chunk = -1, t0 = 0, left = 0;
+    int s, chunk, t0 = 0, left = 0;
     uint4 rv, kv;
     float4 d0, d1;
     auto fetch = [&](int r) {
-        const bool any = chunk_next_record(cu_q, n_seqs, r, s, chunk, t0, left);
+        chunk_of_record(cu_q, n_seqs, r, s, chunk);
         rv = kv = make_uint4(0, 0, 0, 0);
         d0 = d1 = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (!any) return;
+        if (chunk < 0) return;
+        t0 = cu_q[s] + chunk * CS_C;
+        left = cu_q[s + 1] - t0;
         if (row < left) {
             const size_t at = (size_t)(t0 + row) * HD;
             rv = *reinterpret_cast<const uint4*>(rp + at);
