@@ -347,7 +347,7 @@ __global__ void moe_combine_kernel(float* __restrict__ residual, const float* ro
 
 // The same sums in the same order, four columns a thread, for up to COMBINE_TOP experts: bound by memory (8192 tokens of 4 rows
 // of 1024 and a shared one: 235 MB), which the form above does not keep busy, as each of its rows' loads waits for an index of its own
-// and moves 4 bytes (53 us; this one COMBINE_US).
+// and moves 4 bytes (53 us; this one 45.5, 5.2 TB/s).
 constexpr int COMBINE_TOP = 8;
 __global__ void __launch_bounds__(256) moe_combine_vec_kernel(float* __restrict__ residual, const float* rows, const int* row_of,
                                                               const float* wts, const float* shared, const float* shared_z,
