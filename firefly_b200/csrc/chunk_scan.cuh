@@ -442,6 +442,13 @@ __global__ void __launch_bounds__(64 * W + CS_LOADERS) chunk_scan_kernel(ChunkSc
                 x[q >> 1][(q & 1) * 2 + 1] = u[q >> 1][(q & 1) * 2 + 1];
                 cm_split3(x[q >> 1][(q & 1) * 2], x[q >> 1][(q & 1) * 2 + 1], va[0][q], va[1][q], va[2][q]);
             }
+            // nor must a write that became one here (a beta that is none, an overflow)
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) odd |= !(fabsf(x[nt][e]) <= 3.4028235e38f);
+            }
+            odd = __any_sync(0xffffffffu, odd);
         }
         if (!odd) cm_mma_parts<DELTA ? 3 : 1, 3>(own, own_low, va, pb);
         else {

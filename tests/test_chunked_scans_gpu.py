@@ -182,3 +182,49 @@ def test_not_finite_values_stay_behind_their_token(kind, bad):
     assert torch.equal(~torch.isfinite(chunked), spoilt)
     assert spoilt[at:, col].all() and not spoilt[:at].any() and not spoilt[:, :col].any()
     assert (chunked[~spoilt] - walked[~spoilt]).norm() <= 2.0 ** -23 * (32 + T) * walked[~spoilt].norm()
+
+
+# what of a token's inputs is spoilt, for every kind of recurrence; "step" is whatever its decay is made of
+INPUTS = [(kind, part) for kind in ("step", "channel", "wkv", "delta") for part in ("q", "k", "v", "step", "beta")
+          if kind == "delta" or part != "beta"]
+
+
+@pytest.mark.parametrize("bad", [math.nan, math.inf, 3e38])
+@pytest.mark.parametrize("at", [37, 40, 95])
+@pytest.mark.parametrize("kind,part", INPUTS)
+def test_spoilt_inputs_stay_behind_their_token(kind, part, at, bad):
+    """A number of any input that is not finite, or so large that sums behind it overflow, leaves the tokens in front of it as the
+    walk token by token does; behind one that is not finite, what the walk leaves finite is finite here (sums next to the
+    largest 32-bit number may overflow in one order and not in another)."""
+    rn = _rand(5)
+    T, N, V = 100, 64, 64
+    x, beta, decay = rn(T, 2 * N + V).to(BF), rn(T, 1).to(BF), 0.8 + 0.1 * torch.rand(T, N, device="cuda")
+    raw = (beta if kind == "step" else rn(T, N)).clone()
+    if kind == "channel":
+        raw = decay
+    if part in "qkv":
+        x[at, {"q": 0, "k": N, "v": 2 * N}[part] + 21] = bad
+    else:
+        (beta if part == "beta" else raw)[at, 0] = bad
+    zeros = lambda *s: torch.zeros(*s, device="cuda")  # noqa: E731
+    out = []
+    for workspace in (Workspace("cuda"), None):
+        ctx = _ctx([T], 1)
+        ctx.workspace = workspace
+        o, state = zeros(T, V), zeros(2, N * V + 8)
+        q, k, v = (x, 0), (x, N), (x, 2 * N)
+        if kind == "step":
+            K.scalar_decay_scan(q, k, v, state, 0, ctx, o, 1, N, V, step=(raw, 0), step_bias=zeros(1), a_log=zeros(1))
+        elif kind == "channel":
+            K.scalar_decay_scan(q, k, v, state, 0, ctx, o, 1, N, V, channel_decay=(raw, 0))
+        elif kind == "wkv":
+            rkvg = torch.stack([x[:, :N], x[:, N:2 * N], x[:, 2 * N:], x[:, :N]]).contiguous()
+            K.wkv_scan(rkvg, raw, zeros(N), zeros(N) + 1, state, N * V, x[:, :8].contiguous(), ctx, o, 1, N)
+        else:
+            K.delta_rule_scan(q, k, v, (beta, 0), (raw, 0), zeros(N), zeros(1), state, 0, ctx, o, 1, N, V)
+        out.append(o)
+    chunked, walked = out
+    assert torch.isfinite(walked[:at]).all() and torch.isfinite(chunked[:at]).all()
+    assert (chunked[:at] - walked[:at]).norm() <= 2.0 ** -23 * (32 + T) * walked[:at].norm()
+    if not math.isfinite(bad):
+        assert not (torch.isfinite(walked) & ~torch.isfinite(chunked)).any()
