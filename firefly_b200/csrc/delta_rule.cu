@@ -319,7 +319,8 @@ __global__ void __launch_bounds__(2 * NK) delta_prepare_kernel(DeltaArgs A, Chun
                 qq += __shfl_xor_sync(0xffffffffu, qq, off);
                 kk += __shfl_xor_sync(0xffffffffu, kk, off);
             }
-            const float fq = A.q_scale / sqrtf(qq + A.unit_eps), fk = 1.0f / sqrtf(kk + A.unit_eps);
+            // rows behind the sequence's end stay zero, also where unit_eps is
+            const float fq = in ? A.q_scale / sqrtf(qq + A.unit_eps) : 0.f, fk = in ? 1.0f / sqrtf(kk + A.unit_eps) : 0.f;
             const float d[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
             if (A.decay_per_head) {
                 const float gd = in ? expf(-rate * dr_softplus(d[0] + bias[0])) : 1.f;

@@ -228,3 +228,20 @@ def test_spoilt_inputs_stay_behind_their_token(kind, part, at, bad):
     assert (chunked[:at] - walked[:at]).norm() <= 2.0 ** -23 * (32 + T) * walked[:at].norm()
     if not math.isfinite(bad):
         assert not (torch.isfinite(walked) & ~torch.isfinite(chunked)).any()
+
+
+@pytest.mark.parametrize("L", [97, 112])
+def test_delta_rule_without_an_epsilon(L):
+    """unit_eps = 0: the rows that fill a sequence's last chunk up are zeros, which have no unit vector."""
+    rn = _rand(9)
+    N = V = 64
+    x, beta, raw = rn(L, 2 * N + V).to(BF), rn(L, 1).to(BF), rn(L, N)
+    state, o = torch.zeros(2, N * V, device="cuda"), torch.zeros(L, V, device="cuda")
+    zeros = lambda *s: torch.zeros(*s, device="cuda")  # noqa: E731
+    K.delta_rule_scan((x, 0), (x, N), (x, 2 * N), (beta, 0), (raw, 0), zeros(N), zeros(1), state, 0, _ctx([L], 1), o, 1, N, V, unit_eps=0.0)
+    q, k = (x[:, i:i + N].double().view(L, 1, N) for i in (0, N))
+    q, k = (y / y.norm(dim=-1, keepdim=True) for y in (q, k))
+    want, S = _walk(q, k, x[:, 2 * N:].double().view(L, 1, V), torch.exp(-F.softplus(raw.double())).view(L, 1, N), torch.sigmoid(beta.double()))
+    tol = 2.0 ** -24 * (32 + L)
+    assert (o.view_as(want).double() - want).norm() <= tol * want.norm()
+    assert (state[1].view(1, V, N).transpose(1, 2).double() - S).norm() <= tol * S.norm()
