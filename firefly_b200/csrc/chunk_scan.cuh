@@ -139,7 +139,7 @@ template <int NK, bool DELTA, bool BEFORE, typename Put>
 __device__ __forceinline__ void chunk_near_pairs(const float* sq, const float* sk, const float* sa, const float* u, Put put) {
     constexpr int L = NK / 8, H = CS_C / 2;
     const int part = threadIdx.x % L, s = threadIdx.x / L, t0 = s & H, ls = s & (H - 1), n = part * 8;
-    float d[8], x[H], y[DELTA ? H : 1];
+    float d[8], x[H], y[DELTA ? H : 1] = {};
     auto row8 = [&](const float* m, int t, float v[8]) {
         *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(m + t * NK + n);
         *reinterpret_cast<float4*>(v + 4) = *reinterpret_cast<const float4*>(m + t * NK + n + 4);

@@ -20,15 +20,10 @@
 namespace ff {
 
 __device__ __forceinline__ float silu_f(float z) { return z / (1.0f + expf(-z)); }
-// 1 / (1 + e^-z) for results that are rounded to 16 bits, without a division's branches: the hardware's reciprocal and one Newton step, right to the last bit or next to it;
-// 0 where e^-z is beyond 8e37.
-__device__ __forceinline__ float sigmoid_f(float z) {
-    const float d = 1.0f + expf(-z);
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-    r = fmaf(r, fmaf(-d, r, 1.0f), r);
-    return d > 8e37f ? 0.f : r;
-}
+// The same for results that are rounded to 16 bits, by CUDA's fast division (2 units in the last place of 32 bits; 0 where e^-z is
+// beyond 2^126, the true result being below 2^-119): 55 us for the convolution of 8192 tokens of 4096 channels, 75 with the division above,
+// 79 with __frcp_rn; 4 of 33 million rounded results differ more than with a true reciprocal.
+__device__ __forceinline__ float silu_fast(float z) { return __fdividef(z, 1.0f + expf(-z)); }
 __device__ __forceinline__ float softplus_f(float z) { return z > 20.f ? z : log1pf(expf(z)); }
 
 // ----------------------------------------------------------------------------- convolution --
@@ -120,7 +115,7 @@ __global__ void __launch_bounds__(128, 4) causal_conv_silu_kernel(const T* in, i
       auto finish = [&](int t, float (&acc)[VEC], const float (&cur)[VEC]) {
 #pragma unroll
         for (int e = 0; e < VEC; ++e) {
-            if (flags & CONV_SILU) acc[e] = sizeof(TO) == 4 ? silu_f(acc[e]) : acc[e] * sigmoid_f(acc[e]);
+            if (flags & CONV_SILU) acc[e] = sizeof(TO) == 4 ? silu_f(acc[e]) : silu_fast(acc[e]);
             if (flags & CONV_ADD_INPUT) acc[e] += cur[e];
         }
         TO* dst = out + (size_t)t * C + c0;

@@ -55,6 +55,30 @@ def test_convolution(lens, channels, col0, taps):
         at += n
 
 
+@pytest.mark.parametrize("wide_input", [False, True])
+def test_silu_of_the_convolution(wide_input):
+    """Every bfloat16 number, and 65536 32-bit ones, through the filter that hands its input on (one weight of 1): SiLU rounded to
+    bfloat16 once (half a unit in the last place) behind an exponential and a division of two 32-bit units each and an addition
+    (2^-20 of it in all), and to 2^-119 where e^-x leaves the range of the fast division."""
+    bits = torch.arange(65536, dtype=torch.int32, device="cuda").to(torch.int16).view(BF)
+    x = bits.view(64, 1024)
+    if wide_input:
+        x = torch.cat([x.float(), torch.linspace(-120, 120, 1024 * 64, device="cuda").view(64, 1024)])
+    T, C = x.shape
+    w = torch.zeros(C, 4, device="cuda")
+    w[:, 3] = 1
+    out, ctx = torch.empty(T, C, dtype=BF, device="cuda"), _ctx([1] * T)       # a token a sequence: no row meets another's zero weight
+    ctx.seq_fresh.fill_(1)
+    K.causal_conv(x, 0, C, w, None, torch.zeros(T + 1, 3 * C, device="cuda"), 0, ctx, out, silu=True)
+    xd, got = x.double(), out.double()
+    want = xd * torch.sigmoid(xd)
+    fine = torch.isfinite(xd)
+    half = torch.ldexp(torch.ones_like(want), torch.frexp(want).exponent - 9)
+    assert bool(((got - want).abs()[fine] <= (half + 2.0 ** -20 * want.abs())[fine] + 2.0 ** -119).all())
+    assert torch.equal(got[xd == float("inf")], xd[xd == float("inf")]) and bool(got[torch.isnan(xd)].isnan().all())
+    assert bool(got[xd == -float("inf")].isnan().all())        # -inf / inf, as the division gives
+
+
 @pytest.mark.parametrize("width,parts,shift", [(128, 1, 0), (512, 2, 0), (1024, 1, 8), (2048, 8, 0), (4096, 1, 0), (300, 3, 0),
                                                (1024, 1, 1), (16384, 1, 0)])
 @pytest.mark.parametrize("first", [True, False])
