@@ -391,6 +391,7 @@ constexpr int SCAN_CHUNK_MIN = 32;
 // their own block; one of 96 10.1 / 18.3).
 constexpr int CHANNEL_CHUNK_MIN = 80;
 constexpr int SC_PP = SC_C + 8;
+constexpr long long SCAN_PREPARE_BLOCKS = 12 * 148;         // blocks of the first kernel that are on the GPU together
 
 struct ScanRecord {
     bf16 P[3][SC_C * SC_PP];
@@ -398,11 +399,14 @@ struct ScanRecord {
 };
 static_assert(sizeof(ScanRecord) % 16 == 0, "a record is copied in 16-byte pieces");
 
-// The first kernel: a block per (chunk, group of heads that share q and k).  Three of its warps multiply q with k once for the
-// group; then four heads at a time, a warp a head sums up the decays and each tile of the product is scaled for each head.
+// The first kernel: a block per (chunk, group of heads that share q and k, share of the group's heads).  Three of its warps multiply q
+// with k once for them; then four heads at a time, a warp a head sums up the decays and each tile of the product is scaled for each
+// head.  Four heads take 4 us whatever else runs, so a group's heads go to as many blocks as still fit the GPU together, each with the
+// product of its own (SCAN_PREPARE_BLOCKS).  Both kernels, us a call, 64 heads of 64 x 64 in one group, all heads of a group in one
+// block / now: one prompt of 64 tokens 64.0 / 18.6, eight of 256 106 / 58.8; 32 heads of 128 x 64: 35.8 / 23.7 and 71.8 / 53.4.
 template <int NK>
 __global__ void __launch_bounds__(128) scalar_decay_prepare_kernel(ScanArgs A, ScanRecord* __restrict__ recs, const int* __restrict__ cu_q,
-                                                                   int n_seqs, int heads) {
+                                                                   int n_seqs, int heads, int heads_a_block) {
     pdl_prologue();
     constexpr int QP = NK + 8;
     __shared__ __align__(16) bf16 sq[SC_C * QP], sk[SC_C * QP];
@@ -411,6 +415,7 @@ __global__ void __launch_bounds__(128) scalar_decay_prepare_kernel(ScanArgs A, S
     chunk_of_record<SC_C>(cu_q, n_seqs, blockIdx.x, s, chunk);
     if (chunk < 0) return;
     const int group = blockIdx.y, row0 = cu_q[s] + chunk * SC_C, n = min(SC_C, cu_q[s + 1] - row0);
+    const int hb0 = blockIdx.z * heads_a_block, hb1 = min(A.heads_per_group, hb0 + heads_a_block);       // heads of the group
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c2 = (lane & 3) * 2;
     const int row_a = (lane & 7) + ((lane >> 3) & 1) * 8, col_a = (lane >> 4) * 8;
     const int row_b = (lane & 7) + (lane >> 4) * 8, col_b = ((lane >> 3) & 1) * 8;
@@ -427,8 +432,8 @@ __global__ void __launch_bounds__(128) scalar_decay_prepare_kernel(ScanArgs A, S
     // P's tiles: rows (tokens) 16 mt.., columns (keys) 16 nh..; keys behind the tokens are not formed
     const int mt = warp >> 1, nh = warp & 1;
     float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-    for (int h0 = 0; h0 < A.heads_per_group; h0 += 4) {
-        if (h0 + warp < A.heads_per_group) {              // the decays of a head, one token a lane
+    for (int h0 = hb0; h0 < hb1; h0 += 4) {
+        if (h0 + warp < hb1) {              // the decays of a head, one token a lane
             const int h = group * A.heads_per_group + h0 + warp;
             ScanRecord* rec = recs + (size_t)blockIdx.x * heads + h;
             const bool in = lane < n;
@@ -462,7 +467,7 @@ __global__ void __launch_bounds__(128) scalar_decay_prepare_kernel(ScanArgs A, S
                 if (lane == 0) rec->end[0] = pw[warp][n];
             }
         }
-        if (h0 == 0) {
+        if (h0 == hb0) {
             cm_copy_wait<0>();
             __syncthreads();
             if (nh <= mt) {
@@ -476,7 +481,7 @@ __global__ void __launch_bounds__(128) scalar_decay_prepare_kernel(ScanArgs A, S
             }
         } else __syncthreads();
         if (nh <= mt) {
-            for (int hw = 0; hw < min(4, A.heads_per_group - h0); ++hw) {
+            for (int hw = 0; hw < min(4, hb1 - h0); ++hw) {
                 const int h = group * A.heads_per_group + h0 + hw;
                 bf16* Pd = recs[(size_t)blockIdx.x * heads + h].P[0];
 #pragma unroll
@@ -1078,8 +1083,10 @@ template <int NK>
 static int scan_chunk_launch(const ScanArgs& A, float* state, long long state_stride, int state_off, const int* cu_q, const int* state_slots,
                              const int* seq_fresh, float* o, int T, int n_seqs, int heads, int V, void* scratch, cudaStream_t stream) {
     ScanRecord* recs = (ScanRecord*)scratch;
-    FF_LAUNCH(scalar_decay_prepare_kernel<NK>, dim3((unsigned)chunk_records<SC_C>(T, n_seqs), heads / A.heads_per_group), 128, 0, stream, A, recs,
-              cu_q, n_seqs, heads);
+    const long long records = chunk_records<SC_C>(T, n_seqs), groups = heads / A.heads_per_group, quads = (A.heads_per_group + 3) / 4;
+    const long long quads_a_block = std::max(1ll, std::min(quads, (records * groups * quads + SCAN_PREPARE_BLOCKS - 1) / SCAN_PREPARE_BLOCKS));
+    FF_LAUNCH(scalar_decay_prepare_kernel<NK>, dim3((unsigned)records, (unsigned)groups, (unsigned)((quads + quads_a_block - 1) / quads_a_block)), 128, 0,
+              stream, A, recs, cu_q, n_seqs, heads, (int)quads_a_block * 4);
 #define FF_SCAN_CHUNK(W)                                                                                                \
     do {                                                                                                                \
         const dim3 grid(n_seqs, heads, (V + 16 * W - 1) / (16 * W));                                                    \

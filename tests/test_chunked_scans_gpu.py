@@ -70,7 +70,9 @@ def _rand(seed):
 
 @pytest.mark.parametrize("lens", LENS)
 @pytest.mark.parametrize("N,V,heads,groups,mode", [(64, 64, 4, 1, "step"), (128, 40, 6, 3, "step"), (128, 128, 2, 2, "constant"),
-                                                   (64, 72, 3, 3, "channel"), (128, 8, 2, 2, "channel")])
+                                                   (64, 72, 3, 3, "channel"), (128, 8, 2, 2, "channel"),
+                                                   # a group's heads in three blocks, the last of them half empty; in two, as many groups fill the GPU
+                                                   (64, 8, 10, 1, "step"), (64, 8, 400, 40, "step")])
 def test_decay_scans(lens, N, V, heads, groups, mode):
     rn = _rand(N + V)
     T, n = sum(lens), len(lens)
