@@ -490,22 +490,26 @@ static int delta_launch(const DeltaArgs& A, float* state, long long state_stride
     return 0;
 }
 
+// `launched`: how many kernels the call put on the stream (1: token by token, 2: by chunks).
 FF_EXPORT int ff_delta_rule_scan(const void* q, int q_stride, int q_off, const void* k, int k_stride, int k_off,
                                  const void* v, int v_stride, int v_off, const void* beta, int beta_stride, int beta_off,
                                  int dtype, const float* a, int a_stride, int a_off, const float* dt_bias,
                                  const float* a_log, int decay_per_head, int heads_per_group, float q_scale, float unit_eps, float* state,
                                  long long state_stride, int state_off, const int* cu_q, const int* state_slots,
                                  const int* seq_fresh, float* o, int T, int n_seqs, int heads, int N, int V,
-                                 void* scratch, long long scratch_bytes, cudaStream_t stream) {
+                                 void* scratch, long long scratch_bytes, int* launched, cudaStream_t stream) {
+    *launched = 0;
     if (T <= 0 || n_seqs <= 0) return 0;
     if (heads_per_group <= 0 || heads % heads_per_group) return FF_ERR_BAD_ARG;
     DeltaArgs A{q, q_stride, q_off, k, k_stride, k_off, v, v_stride, v_off, beta, beta_stride, beta_off,
                 a, a_stride, a_off, dt_bias, a_log, heads_per_group, q_scale, unit_eps, decay_per_head ? 1 : 0};
     const long long need = ff_delta_scratch_bytes(dtype, T, n_seqs, heads, N, V);
     if (need > 0 && scratch && scratch_bytes >= need && delta_layout_in_chunks(A)) {
+        *launched = 2;
         const ChunkScanArgs B{scratch, (const bf16*)v, v_stride, v_off, state, state_stride, state_off, V * N, cu_q, state_slots, seq_fresh, o, heads, V};
         return N == 64 ? delta_chunk_launch<64>(A, B, T, n_seqs, scratch, stream) : delta_chunk_launch<128>(A, B, T, n_seqs, scratch, stream);
     }
+    *launched = 1;
     if (dtype == 0)
         return delta_launch<float>(A, state, state_stride, state_off, cu_q, state_slots, seq_fresh, o, n_seqs, heads, N, V, stream);
     if (dtype == 1)

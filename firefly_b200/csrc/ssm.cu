@@ -1114,11 +1114,12 @@ static int channel_chunk_launch(const ScanArgs& A, const ChunkScanArgs& B, int T
 template <typename T>
 static int scan_launch(const ScanArgs& A, float* state, long long state_stride, int state_off, const int* cu_q,
                        const int* state_slots, const int* seq_fresh, float* o, int T_tot, int n_seqs, int heads, int N, int V,
-                       void* scratch, long long scratch_bytes, cudaStream_t stream) {
+                       void* scratch, long long scratch_bytes, int* launched, cudaStream_t stream) {
     if (!ws_key_size(N) || V <= 0 || V > 256) return FF_ERR_UNSUPPORTED;
     if constexpr (sizeof(T) == 2) {
         const long long need = ff_scan_scratch_bytes(1, A.mode, A.act, T_tot, n_seqs, heads, N, V);
         if (need > 0 && scratch && scratch_bytes >= need && scan_layout_in_chunks(A, heads)) {
+            *launched = 2;
             if (A.mode != 2) {
                 if (N == 64) return scan_chunk_launch<64>(A, state, state_stride, state_off, cu_q, state_slots, seq_fresh, o, T_tot, n_seqs, heads, V, scratch, stream);
                 return scan_chunk_launch<128>(A, state, state_stride, state_off, cu_q, state_slots, seq_fresh, o, T_tot, n_seqs, heads, V, scratch, stream);
@@ -1135,6 +1136,7 @@ static int scan_launch(const ScanArgs& A, float* state, long long state_stride, 
         if (A.mode == 2) FF_SCAN_ONE(NP, true);                                                                         \
         else FF_SCAN_ONE(NP, false);                                                                                    \
     } while (0)
+    *launched = 1;
     switch (ws_key_size(N)) {
         case 16: FF_SCAN(16); break;
         case 32: FF_SCAN(32); break;
@@ -1148,6 +1150,7 @@ static int scan_launch(const ScanArgs& A, float* state, long long state_stride, 
     return 0;
 }
 
+// `launched`: how many kernels the call put on the stream (1: token by token, 2: by chunks).
 FF_EXPORT int ff_scalar_decay_scan(const void* q, int q_stride, int q_off, const void* k, int k_stride, int k_off,
                                    const void* v, int v_stride, int v_off, int dtype, int heads_per_group, int act,
                                    int mode, const float* decay, const void* step, int step_stride, int step_off,
@@ -1155,15 +1158,16 @@ FF_EXPORT int ff_scalar_decay_scan(const void* q, int q_stride, int q_off, const
                                    const float* channel_decay, int cd_stride, int cd_off, float q_scale, float* state,
                                    long long state_stride, int state_off, const int* cu_q, const int* state_slots,
                                    const int* seq_fresh, float* o, int T, int n_seqs, int heads, int N, int V,
-                                   void* scratch, long long scratch_bytes, cudaStream_t stream) {
+                                   void* scratch, long long scratch_bytes, int* launched, cudaStream_t stream) {
+    *launched = 0;
     if (T <= 0 || n_seqs <= 0) return 0;
     if (heads_per_group <= 0 || mode < 0 || mode > 2 || (mode == 2 && !channel_decay)) return FF_ERR_BAD_ARG;
     ScanArgs A{q, q_stride, q_off, k, k_stride, k_off, v, v_stride, v_off, heads_per_group, act, decay,
                step, step_stride, step_off, step_bias, a_log, skip, mode, channel_decay, cd_stride, cd_off, q_scale};
     if (dtype == 0)
-        return scan_launch<float>(A, state, state_stride, state_off, cu_q, state_slots, seq_fresh, o, T, n_seqs, heads, N, V, scratch, scratch_bytes, stream);
+        return scan_launch<float>(A, state, state_stride, state_off, cu_q, state_slots, seq_fresh, o, T, n_seqs, heads, N, V, scratch, scratch_bytes, launched, stream);
     if (dtype == 1)
-        return scan_launch<bf16>(A, state, state_stride, state_off, cu_q, state_slots, seq_fresh, o, T, n_seqs, heads, N, V, scratch, scratch_bytes, stream);
+        return scan_launch<bf16>(A, state, state_stride, state_off, cu_q, state_slots, seq_fresh, o, T, n_seqs, heads, N, V, scratch, scratch_bytes, launched, stream);
     return FF_ERR_BAD_ARG;
 }
 

@@ -443,19 +443,23 @@ static int wkv_chunk_launch(const bf16* rkvg, const float* dlog, const float* w0
     return chunk_scan_launch<D, false>(B, n_seqs, stream);
 }
 
+// `launched`: how many kernels the call put on the stream (1: token by token, 2: by chunks).
 FF_EXPORT int ff_wkv_scan(const void* rkvg, int dtype, const float* dlog, const float* w0, const float* u, float* state,
                           long long state_stride, int prev_off, const void* x, int W, const int* cu_q,
                           const int* state_slots, const int* seq_fresh, float* o, int Ttot, int n_seqs, int heads,
-                          int dim, void* scratch, long long scratch_bytes, cudaStream_t stream) {
+                          int dim, void* scratch, long long scratch_bytes, int* launched, cudaStream_t stream) {
+    *launched = 0;
     if (Ttot <= 0 || n_seqs <= 0) return 0;
     const long long need = ff_wkv_scratch_bytes(dtype, Ttot, n_seqs, heads, dim);
     if (need > 0 && scratch && scratch_bytes >= need && (((uintptr_t)rkvg | (uintptr_t)dlog) & 15) == 0) {
+        *launched = 2;
         const bf16* in = (const bf16*)rkvg;
         const int HD = heads * dim;
         const ChunkScanArgs B{scratch, in + (size_t)2 * Ttot * HD, HD, 0, state, state_stride, 0, dim * dim, cu_q, state_slots, seq_fresh, o, heads, dim};
         if (dim == 64) return wkv_chunk_launch<64>(in, dlog, w0, u, prev_off, (const bf16*)x, W, B, Ttot, n_seqs, scratch, stream);
         return wkv_chunk_launch<128>(in, dlog, w0, u, prev_off, (const bf16*)x, W, B, Ttot, n_seqs, scratch, stream);
     }
+    *launched = 1;
     if (dtype == 0)
         return wkv_scan_launch<float>(rkvg, dlog, w0, u, state, state_stride, prev_off, x, W, cu_q, state_slots,
                                       seq_fresh, o, Ttot, n_seqs, heads, dim, stream);

@@ -926,10 +926,10 @@ def _recurrence_scratch(ctx, module: str, entry: str, *sizes: int):
     return _p(records), ctypes.c_longlong(need)
 
 
-def _count_preparing(scratch) -> None:
+def _count_kernels(launched: c_int) -> None:
+    """``launched``: how many kernels a recurrence's entry put on the stream; the call itself is counted as one."""
     global LAUNCHES
-    if scratch[0].value:
-        LAUNCHES += 1     # the kernel that prepares the chunks
+    LAUNCHES += launched.value - 1
 
 
 def wkv_scan(rkvg, dlog, w0, u, state, prev_off: int, x, ctx, o, heads: int, dim: int) -> None:
@@ -946,11 +946,12 @@ def wkv_scan(rkvg, dlog, w0, u, state, prev_off: int, x, ctx, o, heads: int, dim
     assert w0.dtype == u.dtype == torch.float32 and w0.numel() == HD and u.numel() == HD
     assert state.shape[1] >= prev_off + W and prev_off >= heads * wkv_state_dim(dim) ** 2
     scratch = _recurrence_scratch(ctx, "wkv", "ff_wkv_scratch_bytes", _dt(rkvg), T, ctx.num_seqs, heads, dim)
+    launched = c_int(0)
     _check(_lib("wkv").ff_wkv_scan(_p(rkvg), c_int(_dt(rkvg)), _p(dlog), _p(w0), _p(u), _p(state),
                                   ctypes.c_longlong(state.stride(0)), c_int(prev_off), _p(x), c_int(W), _p(ctx.cu_q),
                                   _p(ctx.state_slots), _p(ctx.seq_fresh), _p(o), c_int(T), c_int(ctx.num_seqs),
-                                  c_int(heads), c_int(dim), *scratch, _stream()), "wkv_scan")
-    _count_preparing(scratch)
+                                  c_int(heads), c_int(dim), *scratch, ctypes.byref(launched), _stream()), "wkv_scan")
+    _count_kernels(launched)
 
 
 def wkv_out(o, gate, norm_w, eps: float, y, heads: int, dim: int) -> None:
@@ -1480,13 +1481,14 @@ def delta_rule_scan(q, k, v, beta, a, dt_bias: torch.Tensor, a_log: torch.Tensor
     assert dt_bias.numel() == (heads if decay_per_head else heads * N)
     assert o.dtype == torch.float32 and o.shape == (T, heads * V) and state.dtype == torch.float32
     scratch = _recurrence_scratch(ctx, "delta_rule", "ff_delta_scratch_bytes", _dt(qm), T, ctx.num_seqs, heads, N, V)
+    launched = c_int(0)
     _check(_lib("delta_rule").ff_delta_rule_scan(
         _p(qm), c_int(qm.stride(0)), c_int(q0), _p(km), c_int(km.stride(0)), c_int(k0), _p(vm), c_int(vm.stride(0)),
         c_int(v0), _p(bm), c_int(bm.stride(0)), c_int(b0), c_int(_dt(qm)), _p(am), c_int(am.stride(0)), c_int(a0),
         _p(dt_bias), _p(a_log), c_int(1 if decay_per_head else 0), c_int(heads_per_group), c_float(q_scale), c_float(unit_eps), _p(state),
         ctypes.c_longlong(state.stride(0)), c_int(state_off), _p(ctx.cu_q), _p(ctx.state_slots), _p(ctx.seq_fresh),
-        _p(o), c_int(T), c_int(ctx.num_seqs), c_int(heads), c_int(N), c_int(V), *scratch, _stream()), "delta_rule_scan")
-    _count_preparing(scratch)
+        _p(o), c_int(T), c_int(ctx.num_seqs), c_int(heads), c_int(N), c_int(V), *scratch, ctypes.byref(launched), _stream()), "delta_rule_scan")
+    _count_kernels(launched)
 
 
 def head_norm_gate(o: torch.Tensor, gate, weight: torch.Tensor, eps: float, y: torch.Tensor, heads: int, V: int,
@@ -1530,14 +1532,15 @@ def scalar_decay_scan(q, k, v, state: torch.Tensor, state_off: int, ctx, o: torc
     if mode == 1:
         assert sm.dtype == qm.dtype and step_bias is not None and a_log is not None
     scratch = _recurrence_scratch(ctx, "ssm", "ff_scan_scratch_bytes", _dt(qm), mode, 1 if silu_inputs else 0, T, ctx.num_seqs, heads, N, V)
+    launched = c_int(0)
     _check(_lib("ssm").ff_scalar_decay_scan(
         _p(qm), c_int(qm.stride(0)), c_int(q0), _p(km), c_int(km.stride(0)), c_int(k0), _p(vm), c_int(vm.stride(0)),
         c_int(v0), c_int(_dt(qm)), c_int(heads_per_group), c_int(1 if silu_inputs else 0), c_int(mode), _p(decay),
         _p(sm), c_int(sm.stride(0) if sm is not None else 0), c_int(s0), _p(step_bias), _p(a_log), _p(skip),
         _p(cm), c_int(cm.stride(0) if cm is not None else 0), c_int(cd0), c_float(q_scale), _p(state),
         ctypes.c_longlong(state.stride(0)), c_int(state_off), _p(ctx.cu_q), _p(ctx.state_slots), _p(ctx.seq_fresh),
-        _p(o), c_int(T), c_int(ctx.num_seqs), c_int(heads), c_int(N), c_int(V), *scratch, _stream()), "scalar_decay_scan")
-    _count_preparing(scratch)
+        _p(o), c_int(T), c_int(ctx.num_seqs), c_int(heads), c_int(N), c_int(V), *scratch, ctypes.byref(launched), _stream()), "scalar_decay_scan")
+    _count_kernels(launched)
 
 
 def gated_rms_norm(o: torch.Tensor, gate, weight: torch.Tensor, eps: float, y: torch.Tensor, parts: int,

@@ -247,3 +247,19 @@ def test_delta_rule_without_an_epsilon(L):
     tol = 2.0 ** -24 * (32 + L)
     assert (o.view_as(want).double() - want).norm() <= tol * want.norm()
     assert (state[1].view(1, V, N).transpose(1, 2).double() - S).norm() <= tol * S.norm()
+
+
+def test_launch_counter_counts_what_ran():
+    """Rows that 16-byte copies do not take are walked token by token, scratch memory or not, and counted as one kernel."""
+    rn = _rand(2)
+    T, N = 100, 64
+    zeros = lambda *s: torch.zeros(*s, device="cuda")  # noqa: E731
+    for shift, kernels in ((0, 2), (1, 1)):
+        x, ctx, o = rn(T, 3 * N + 8).to(BF), _ctx([T], 1), zeros(T, N)
+        q, k, v = ((x, i * N + shift) for i in range(3))
+        for call in (lambda: K.scalar_decay_scan(q, k, v, zeros(2, N * N), 0, ctx, o, 1, N, N, step=(x, 0), step_bias=zeros(1), a_log=zeros(1)),
+                     lambda: K.scalar_decay_scan(q, k, v, zeros(2, N * N), 0, ctx, o, 1, N, N, channel_decay=(zeros(T, N), 0)),
+                     lambda: K.delta_rule_scan(q, k, v, (x, 0), (zeros(T, N), 0), zeros(N), zeros(1), zeros(2, N * N), 0, ctx, o, 1, N, N)):
+            before = K.LAUNCHES
+            call()
+            assert K.LAUNCHES - before == kernels
