@@ -38,6 +38,11 @@ struct ChunkRecord {
 template <int C = CS_C> __host__ __device__ __forceinline__ int chunk_first_record(int t0, int s) { return t0 / C + s; }
 template <int C = CS_C> static inline long long chunk_records(int T, int n_seqs) { return T / C + n_seqs; }
 
+// What 16-byte copies of rows ask for: the low four bits of this, or'ed over the matrices, are zero.
+static inline unsigned row_bits(const void* p, long long stride, long long off, int element) {
+    return (unsigned)((uintptr_t)p | (unsigned long long)(stride * element) | (unsigned long long)(off * element));
+}
+
 // The sequence and chunk of record r (chunk -1: none); all lanes of a warp ask together.
 template <int C = CS_C>
 __device__ __forceinline__ void chunk_of_record(const int* cu_q, int n_seqs, int r, int& s, int& chunk) {

@@ -446,16 +446,16 @@ FF_EXPORT long long ff_delta_state_floats(int heads, int N, int V) {
 // of 32 37.9 / 23.5, of 64 24.9 / 44.2; one of 64 17.4 / 43.7).
 constexpr int DELTA_CHUNK_MIN = 48;
 
-// Bytes of scratch memory that a step of T tokens can use (0: none; without it the token-by-token kernel runs).
-FF_EXPORT long long ff_delta_scratch_bytes(int dtype, int T, int n_seqs, int heads, int N, int V) {
-    if (dtype != 1 || T <= 0 || n_seqs <= 0 || (long long)T < (long long)DELTA_CHUNK_MIN * n_seqs || (N != 64 && N != 128) || V <= 0 || V > 256 || V % 8) return 0;
+// Bytes of scratch memory that a step of T tokens can use (0: none; without it the token-by-token kernel runs).  `bits`: the matrices'
+// addresses, row strides and first columns in bytes, or'ed (row_bits).
+FF_EXPORT long long ff_delta_scratch_bytes(int dtype, int T, int n_seqs, int heads, int N, int V, int bits) {
+    if (dtype != 1 || (bits & 15) || T <= 0 || n_seqs <= 0 || (long long)T < (long long)DELTA_CHUNK_MIN * n_seqs || (N != 64 && N != 128) || V <= 0 || V > 256 || V % 8) return 0;
     return chunk_records(T, n_seqs) * heads * (long long)(N == 64 ? sizeof(ChunkRecord<64, true>) : sizeof(ChunkRecord<128, true>));
 }
 
-static bool delta_layout_in_chunks(const DeltaArgs& A) {
-    auto aligned = [](const void* p, int stride, int off, int per) { return ((uintptr_t)p & 15) == 0 && stride % per == 0 && off % per == 0; };
-    return aligned(A.q, A.q_stride, A.q_off, 8) && aligned(A.k, A.k_stride, A.k_off, 8) && aligned(A.v, A.v_stride, A.v_off, 8) &&
-           (A.decay_per_head || aligned(A.a, A.a_stride, A.a_off, 4));
+static unsigned delta_bits(const DeltaArgs& A) {
+    return row_bits(A.q, A.q_stride, A.q_off, 2) | row_bits(A.k, A.k_stride, A.k_off, 2) | row_bits(A.v, A.v_stride, A.v_off, 2) |
+           (A.decay_per_head ? 0u : row_bits(A.a, A.a_stride, A.a_off, 4));
 }
 
 template <int NK>
@@ -503,8 +503,8 @@ FF_EXPORT int ff_delta_rule_scan(const void* q, int q_stride, int q_off, const v
     if (heads_per_group <= 0 || heads % heads_per_group) return FF_ERR_BAD_ARG;
     DeltaArgs A{q, q_stride, q_off, k, k_stride, k_off, v, v_stride, v_off, beta, beta_stride, beta_off,
                 a, a_stride, a_off, dt_bias, a_log, heads_per_group, q_scale, unit_eps, decay_per_head ? 1 : 0};
-    const long long need = ff_delta_scratch_bytes(dtype, T, n_seqs, heads, N, V);
-    if (need > 0 && scratch && scratch_bytes >= need && delta_layout_in_chunks(A)) {
+    const long long need = ff_delta_scratch_bytes(dtype, T, n_seqs, heads, N, V, (int)delta_bits(A));
+    if (need > 0 && scratch && scratch_bytes >= need) {
         *launched = 2;
         const ChunkScanArgs B{scratch, (const bf16*)v, v_stride, v_off, state, state_stride, state_off, V * N, cu_q, state_slots, seq_fresh, o, heads, V};
         return N == 64 ? delta_chunk_launch<64>(A, B, T, n_seqs, scratch, stream) : delta_chunk_launch<128>(A, B, T, n_seqs, scratch, stream);

@@ -1065,15 +1065,15 @@ static bool scalar_chunk_sizes(int mode, int act, int T, int n_seqs, int N, int 
 static bool channel_chunk_sizes(int mode, int act, int T, int n_seqs, int N, int V) {
     return mode == 2 && !act && (long long)T >= (long long)CHANNEL_CHUNK_MIN * n_seqs && (N == 64 || N == 128) && V % 8 == 0;
 }
-static bool scan_layout_in_chunks(const ScanArgs& A, int heads) {
-    auto aligned = [](const void* p, int stride, int off, int per) { return ((uintptr_t)p & 15) == 0 && stride % per == 0 && off % per == 0; };
-    return heads % A.heads_per_group == 0 && aligned(A.q, A.q_stride, A.q_off, 8) && aligned(A.k, A.k_stride, A.k_off, 8) &&
-           aligned(A.v, A.v_stride, A.v_off, 8) && (A.mode != 2 || aligned(A.channel_decay, A.cd_stride, A.cd_off, 4));
+static unsigned scan_bits(const ScanArgs& A) {
+    return row_bits(A.q, A.q_stride, A.q_off, 2) | row_bits(A.k, A.k_stride, A.k_off, 2) | row_bits(A.v, A.v_stride, A.v_off, 2) |
+           (A.mode == 2 ? row_bits(A.channel_decay, A.cd_stride, A.cd_off, 4) : 0u);
 }
 
-// Bytes of scratch memory that a step of T tokens can use (0: none; without it the token-by-token kernel runs).
-FF_EXPORT long long ff_scan_scratch_bytes(int dtype, int mode, int act, int T, int n_seqs, int heads, int N, int V) {
-    if (dtype != 1 || T <= 0 || n_seqs <= 0 || heads <= 0 || V <= 0 || V > 256) return 0;
+// Bytes of scratch memory that a step of T tokens can use (0: none; without it the token-by-token kernel runs).  `bits`: the matrices'
+// addresses, row strides and first columns in bytes, or'ed (row_bits).
+FF_EXPORT long long ff_scan_scratch_bytes(int dtype, int mode, int act, int T, int n_seqs, int heads, int heads_per_group, int N, int V, int bits) {
+    if (dtype != 1 || T <= 0 || n_seqs <= 0 || heads <= 0 || heads_per_group <= 0 || heads % heads_per_group || V <= 0 || V > 256 || (bits & 15)) return 0;
     if (scalar_chunk_sizes(mode, act, T, n_seqs, N, V)) return chunk_records<SC_C>(T, n_seqs) * heads * (long long)sizeof(ScanRecord);
     if (!channel_chunk_sizes(mode, act, T, n_seqs, N, V)) return 0;
     return chunk_records(T, n_seqs) * heads * (long long)(N == 64 ? sizeof(ChunkRecord<64, false>) : sizeof(ChunkRecord<128, false>));
@@ -1117,8 +1117,8 @@ static int scan_launch(const ScanArgs& A, float* state, long long state_stride, 
                        void* scratch, long long scratch_bytes, int* launched, cudaStream_t stream) {
     if (!ws_key_size(N) || V <= 0 || V > 256) return FF_ERR_UNSUPPORTED;
     if constexpr (sizeof(T) == 2) {
-        const long long need = ff_scan_scratch_bytes(1, A.mode, A.act, T_tot, n_seqs, heads, N, V);
-        if (need > 0 && scratch && scratch_bytes >= need && scan_layout_in_chunks(A, heads)) {
+        const long long need = ff_scan_scratch_bytes(1, A.mode, A.act, T_tot, n_seqs, heads, A.heads_per_group, N, V, (int)scan_bits(A));
+        if (need > 0 && scratch && scratch_bytes >= need) {
             *launched = 2;
             if (A.mode != 2) {
                 if (N == 64) return scan_chunk_launch<64>(A, state, state_stride, state_off, cu_q, state_slots, seq_fresh, o, T_tot, n_seqs, heads, V, scratch, stream);

@@ -427,9 +427,10 @@ FF_EXPORT int ff_wkv_state_dim(int dim) { return dim <= 32 ? 32 : (dim <= 64 ? 6
 // 64 37.5 / 26.6, of 96 30.4 / 38.7; one of 96 12.1 / 21.0).
 constexpr int WKV_CHUNK_MIN = 80;
 
-// Bytes of scratch memory that a step of T tokens can use (0: none; without it the token-by-token kernel runs).
-FF_EXPORT long long ff_wkv_scratch_bytes(int dtype, int T, int n_seqs, int heads, int dim) {
-    if (dtype != 1 || T <= 0 || n_seqs <= 0 || (long long)T < (long long)WKV_CHUNK_MIN * n_seqs || (dim != 64 && dim != 128)) return 0;
+// Bytes of scratch memory that a step of T tokens can use (0: none; without it the token-by-token kernel runs).  `bits`: the addresses of
+// rkvg and dlog, or'ed.
+FF_EXPORT long long ff_wkv_scratch_bytes(int dtype, int T, int n_seqs, int heads, int dim, int bits) {
+    if (dtype != 1 || (bits & 15) || T <= 0 || n_seqs <= 0 || (long long)T < (long long)WKV_CHUNK_MIN * n_seqs || (dim != 64 && dim != 128)) return 0;
     return chunk_records(T, n_seqs) * heads * (long long)(dim == 64 ? sizeof(ChunkRecord<64, false>) : sizeof(ChunkRecord<128, false>));
 }
 
@@ -450,8 +451,8 @@ FF_EXPORT int ff_wkv_scan(const void* rkvg, int dtype, const float* dlog, const 
                           int dim, void* scratch, long long scratch_bytes, int* launched, cudaStream_t stream) {
     *launched = 0;
     if (Ttot <= 0 || n_seqs <= 0) return 0;
-    const long long need = ff_wkv_scratch_bytes(dtype, Ttot, n_seqs, heads, dim);
-    if (need > 0 && scratch && scratch_bytes >= need && (((uintptr_t)rkvg | (uintptr_t)dlog) & 15) == 0) {
+    const long long need = ff_wkv_scratch_bytes(dtype, Ttot, n_seqs, heads, dim, (int)(row_bits(rkvg, 0, 0, 2) | row_bits(dlog, 0, 0, 4)));
+    if (need > 0 && scratch && scratch_bytes >= need) {
         *launched = 2;
         const bf16* in = (const bf16*)rkvg;
         const int HD = heads * dim;

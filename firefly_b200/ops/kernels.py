@@ -912,9 +912,20 @@ def _recurrence_scratch_bytes(module: str, entry: str, *sizes: int) -> int:
     return int(fn(*[c_int(x) for x in sizes]))
 
 
+def _row_bits(*rows) -> int:
+    """The low four bits of (matrix, first column) pairs' addresses, row strides and first columns in bytes, or'ed: 0 where every
+    row can be copied 16 bytes at a time (the twin of `row_bits` in csrc/chunk_scan.cuh)."""
+    bits = 0
+    for m, col in rows:
+        es = m.element_size()
+        bits |= m.data_ptr() | m.stride(-2) * es | col * es
+    return bits & 15
+
+
 def _recurrence_scratch(ctx, module: str, entry: str, *sizes: int):
     """Scratch memory for a recurrence that takes a step's prompts a chunk at a time: (pointer, bytes), nothing when the step
-    is none for it, the context has no workspace or the device has no memory left (the token-by-token kernel runs then)."""
+    is none for it (the entry `entry` of the library says how much it can use), the context has no workspace or the device has no
+    memory left (the token-by-token kernel runs then)."""
     ws = getattr(ctx, "workspace", None)
     need = _recurrence_scratch_bytes(module, entry, *sizes) if ws is not None else 0
     if need <= 0:
@@ -945,7 +956,8 @@ def wkv_scan(rkvg, dlog, w0, u, state, prev_off: int, x, ctx, o, heads: int, dim
     assert o.shape == (T, HD) and o.dtype == torch.float32 and state.dtype == torch.float32
     assert w0.dtype == u.dtype == torch.float32 and w0.numel() == HD and u.numel() == HD
     assert state.shape[1] >= prev_off + W and prev_off >= heads * wkv_state_dim(dim) ** 2
-    scratch = _recurrence_scratch(ctx, "wkv", "ff_wkv_scratch_bytes", _dt(rkvg), T, ctx.num_seqs, heads, dim)
+    scratch = _recurrence_scratch(ctx, "wkv", "ff_wkv_scratch_bytes", _dt(rkvg), T, ctx.num_seqs, heads, dim,
+                                  _row_bits((rkvg, 0), (dlog, 0)))
     launched = c_int(0)
     _check(_lib("wkv").ff_wkv_scan(_p(rkvg), c_int(_dt(rkvg)), _p(dlog), _p(w0), _p(u), _p(state),
                                   ctypes.c_longlong(state.stride(0)), c_int(prev_off), _p(x), c_int(W), _p(ctx.cu_q),
@@ -1480,7 +1492,8 @@ def delta_rule_scan(q, k, v, beta, a, dt_bias: torch.Tensor, a_log: torch.Tensor
     assert dt_bias.dtype == a_log.dtype == torch.float32 and a_log.numel() == heads
     assert dt_bias.numel() == (heads if decay_per_head else heads * N)
     assert o.dtype == torch.float32 and o.shape == (T, heads * V) and state.dtype == torch.float32
-    scratch = _recurrence_scratch(ctx, "delta_rule", "ff_delta_scratch_bytes", _dt(qm), T, ctx.num_seqs, heads, N, V)
+    scratch = _recurrence_scratch(ctx, "delta_rule", "ff_delta_scratch_bytes", _dt(qm), T, ctx.num_seqs, heads, N, V,
+                                  _row_bits((qm, q0), (km, k0), (vm, v0), *(() if decay_per_head else ((am, a0),))))
     launched = c_int(0)
     _check(_lib("delta_rule").ff_delta_rule_scan(
         _p(qm), c_int(qm.stride(0)), c_int(q0), _p(km), c_int(km.stride(0)), c_int(k0), _p(vm), c_int(vm.stride(0)),
@@ -1531,7 +1544,8 @@ def scalar_decay_scan(q, k, v, state: torch.Tensor, state_off: int, ctx, o: torc
     sm, s0 = step if step is not None else (None, 0)
     if mode == 1:
         assert sm.dtype == qm.dtype and step_bias is not None and a_log is not None
-    scratch = _recurrence_scratch(ctx, "ssm", "ff_scan_scratch_bytes", _dt(qm), mode, 1 if silu_inputs else 0, T, ctx.num_seqs, heads, N, V)
+    scratch = _recurrence_scratch(ctx, "ssm", "ff_scan_scratch_bytes", _dt(qm), mode, 1 if silu_inputs else 0, T, ctx.num_seqs, heads,
+                                  heads_per_group, N, V, _row_bits((qm, q0), (km, k0), (vm, v0), *(((cm, cd0),) if mode == 2 else ())))
     launched = c_int(0)
     _check(_lib("ssm").ff_scalar_decay_scan(
         _p(qm), c_int(qm.stride(0)), c_int(q0), _p(km), c_int(km.stride(0)), c_int(k0), _p(vm), c_int(vm.stride(0)),
