@@ -23,6 +23,8 @@ from types import SimpleNamespace
 
 import torch
 
+from .engine.context import Workspace
+
 SIZES = {
     # width, layers, heads of the recurrent mixer (dim 64), attention heads, experts (top 4 of 16, 4 groups keep 2)
     "w1024": dict(width=1024, layers=8, ff=512, shared_ff=1024),
@@ -644,7 +646,7 @@ def papusun_kernel_table(width: int, batch: int, prompt: int, peaks: dict) -> li
             keys_seen = sum(min(win or (1 << 30), i + 1 + ctx_len) for i in range(q)) * n_seqs
             step_ctx = SimpleNamespace(**vars(ctx), ctx_lens=ctx_lens, q_lens=[q] * n_seqs, ctx_lens_host=[ctx_len] * n_seqs,
                                        num_decode_seqs=n_seqs if q == 1 else 0, max_kv_len=q + ctx_len, ranges_by_length=False,
-                                       workspace=_Scratch(dev), captured=False, memo={}, key_share_level=0)
+                                       workspace=Workspace(dev), captured=False, memo={}, key_share_level=0)
             us = _time(lambda: K.paged_attention(q_full, H * ld, lpages, table, step_ctx, latt, H, 1, ld, 192 ** -0.5, win), flush=flush)
             kv_b = (n_seqs * min(win or (1 << 30), q + ctx_len) * ld * 2 if q == 1 else T * ld * 2) + T * 2 * H * ld * 2
             add(f"{name} {label}", us, kv_b, 2 * keys_seen * H * (ld + rank), like=None if not win else "latent attention over every key")
@@ -671,22 +673,6 @@ def papusun_kernel_table(width: int, batch: int, prompt: int, peaks: dict) -> li
         us = _time(lambda: K.add_layer_norm(res, yy, lw, None, 1e-6, out_n, None, 1.0), flush=flush)
         add(f"layer norm with the residual add {label} ({T} rows)", us, T * width * (4 * 3 + 2))
     return rows
-
-
-class _Scratch:
-    """Named scratch buffers for a kernel timed alone (the engine's workspace in small)."""
-
-    def __init__(self, device):
-        self.device, self._bufs = device, {}
-
-    def get(self, tag, shape, dtype):
-        n = 1
-        for s_ in shape:
-            n *= int(s_)
-        buf = self._bufs.get((tag, dtype))
-        if buf is None or buf.numel() < n:
-            buf = self._bufs[(tag, dtype)] = torch.empty(max(n, 1), dtype=dtype, device=self.device)
-        return buf[:n].view(*shape)
 
 
 def papusun_main(args, peaks: dict) -> int:
@@ -752,7 +738,7 @@ def gatutar_kernel_table(width: int, ff: int, batch: int, prompt: int, peaks: di
                               state_slots=torch.arange(1, n_seqs + 1, dtype=torch.int32, device=dev),
                               seq_fresh=torch.zeros(n_seqs, dtype=torch.int32, device=dev),
                               status=torch.zeros(1, dtype=torch.int32, device=dev), ranges_by_length=False, max_kv_len=q + ctx_len,
-                              workspace=_Scratch(dev))
+                              workspace=Workspace(dev))
         ctx.ctx_lens = ctx_lens = torch.full((n_seqs,), ctx_len, dtype=torch.int32, device=dev)
         table = (torch.arange(n_seqs * per, dtype=torch.int32, device=dev) + 1).view(n_seqs, per).contiguous()
         pages = (torch.randn(n_seqs * per + 1, 2, G, block, d, device=dev) * 0.5).to(bf)
@@ -929,7 +915,7 @@ def mumopel_kernel_table(width: int, ff: int, batch: int, prompt: int, peaks: di
         ctx = SimpleNamespace(cu_q=torch.arange(0, T + 1, q, dtype=torch.int32, device=dev), num_seqs=n_seqs,
                               token_seq=torch.arange(T, dtype=torch.int32, device=dev) // q,
                               positions=(torch.arange(T, dtype=torch.int32, device=dev) % q) + ctx_len,
-                              status=torch.zeros(1, dtype=torch.int32, device=dev), workspace=_Scratch(dev))
+                              status=torch.zeros(1, dtype=torch.int32, device=dev), workspace=Workspace(dev))
         ctx_lens = torch.full((n_seqs,), ctx_len, dtype=torch.int32, device=dev)
         table = (torch.arange(n_seqs * per, dtype=torch.int32, device=dev) + 1).view(n_seqs, per).contiguous()
         pages = (torch.randn(n_seqs * per + 1, 2, G, block, d, device=dev) * 0.5).to(bf)
@@ -1018,7 +1004,7 @@ def mumopel_kernel_table(width: int, ff: int, batch: int, prompt: int, peaks: di
         wgu = (torch.randn(2 * inter, width, device=dev) * 0.02).to(bf)
         wdn = (torch.randn(width, inter, device=dev) * 0.02).to(bf)
         da = torch.zeros(T, inter, dtype=bf, device=dev)
-        step = SimpleNamespace(workspace=_Scratch(dev), dtype=bf, status=ctx.status)
+        step = SimpleNamespace(workspace=Workspace(dev), dtype=bf, status=ctx.status)
         us = _time(lambda: linear_swiglu(x, wgu, inter, True, step), flush=flush)
         add(f"dense gate|up product and SwiGLU {label} ({T} rows of {inter})", us, 2 * inter * width * 2 + T * (width + inter) * 2, 4 * T * inter * width)
         us = _time(lambda: linear_into_residual(da, wdn, x0, step, "down"), flush=flush)

@@ -8,7 +8,7 @@ position; that is all the kernels need to find its keys, whatever the cut.
 from __future__ import annotations
 
 from dataclasses import dataclass, field
-from typing import Dict, List, Sequence, Tuple
+from typing import Dict, List, Optional, Sequence, Tuple
 
 import torch
 
@@ -27,6 +27,7 @@ class Workspace:
         self._views: Dict[tuple, torch.Tensor] = {}
         self.frozen = False
         self.version = 0          # counts (re)allocations: graphs that captured an address note it
+        self._refused: Dict[Tuple[str, torch.dtype], int] = {}   # elements that the device had no memory for (`try_get`)
 
     def get(self, tag: str, shape: Sequence[int], dtype: torch.dtype) -> torch.Tensor:
         vkey = (tag, dtype, tuple(shape))
@@ -42,7 +43,7 @@ class Workspace:
             if self.frozen:
                 raise RuntimeError(f"workspace buffer '{tag}' would have to grow to {n} elements "
                                    "while a captured graph uses it")
-            buf = torch.empty(max(n, 1), dtype=dtype, device=self.device)
+            buf = self._allocate(n, dtype)
             self._bufs[key] = buf
             self.version += 1
             self._views.clear()   # views of the buffer that was replaced must not be handed out again
@@ -51,6 +52,31 @@ class Workspace:
         view = buf[:n].view(*shape)
         self._views[vkey] = view
         return view
+
+    def _allocate(self, n: int, dtype: torch.dtype) -> torch.Tensor:
+        return torch.empty(max(n, 1), dtype=dtype, device=self.device)
+
+    def try_get(self, tag: str, shape: Sequence[int], dtype: torch.dtype) -> Optional[torch.Tensor]:
+        """`get` for a buffer that its user can do without: None where it would have to grow and cannot, because the workspace is
+        frozen, a CUDA graph is being captured (its addresses and those of earlier graphs must stay) or the device has no
+        memory.  A size that was refused once is not asked for again, nor a larger one: a refusal makes the allocator give
+        everything back and wait for the device, and the run that sizes the buffers must answer as the capture behind it."""
+        n = 1
+        for s in shape:
+            n *= int(s)
+        key = (tag, dtype)
+        buf = self._bufs.get(key)
+        if buf is None or buf.numel() < n:
+            if self.frozen or n >= self._refused.get(key, n + 1):
+                return None
+            if self.device.type == "cuda" and torch.cuda.is_current_stream_capturing():
+                return None
+            try:
+                return self.get(tag, shape, dtype)
+            except torch.OutOfMemoryError:
+                self._refused[key] = n
+                return None
+        return self.get(tag, shape, dtype)
 
     def get_zeroed(self, tag: str, numel: int, dtype: torch.dtype) -> torch.Tensor:
         """A buffer that is zero when first handed out (and after it grows); users

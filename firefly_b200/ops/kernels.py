@@ -930,9 +930,8 @@ def _recurrence_scratch(ctx, module: str, entry: str, *sizes: int):
     need = _recurrence_scratch_bytes(module, entry, *sizes) if ws is not None else 0
     if need <= 0:
         return c_void_p(0), ctypes.c_longlong(0)
-    try:
-        records = ws.get("scan.records", (-(-need // 4),), torch.float32)
-    except torch.OutOfMemoryError:
+    records = ws.try_get("scan.records", (-(-need // 4),), torch.float32)
+    if records is None:
         return c_void_p(0), ctypes.c_longlong(0)
     return _p(records), ctypes.c_longlong(need)
 
