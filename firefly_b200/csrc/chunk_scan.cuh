@@ -43,9 +43,22 @@ static inline unsigned row_bits(const void* p, long long stride, long long off, 
     return (unsigned)((uintptr_t)p | (unsigned long long)(stride * element) | (unsigned long long)(off * element));
 }
 
+// Which sequences of a step go by chunks: those of at least `chunk_min` tokens, whoever else is in the step, so that a request's numbers
+// do not depend on its company.  `n_long`: how many they are (-1: not known); the other sequences go token by token.
+struct ChunkRoute {
+    bool chunks, walk;                                      // which kernels have anything to do
+    int live;                                               // sequences that go by chunks, for the size of blocks
+    int max_walk;                                           // the token-by-token kernel leaves sequences of this length and longer alone
+    int kernels() const { return 2 * chunks + walk; }
+};
+static inline ChunkRoute chunk_route(bool possible, int n_long, int n_seqs, int chunk_min) {
+    const bool chunks = possible && n_long != 0;
+    return {chunks, !chunks || n_long != n_seqs, n_long > 0 ? n_long : n_seqs, chunks ? chunk_min : 0x7fffffff};
+}
+
 // The sequence and chunk of record r (chunk -1: none); all lanes of a warp ask together.
 template <int C = CS_C>
-__device__ __forceinline__ void chunk_of_record(const int* cu_q, int n_seqs, int r, int& s, int& chunk) {
+__device__ __forceinline__ void chunk_of_record(const int* cu_q, int n_seqs, int r, int min_len, int& s, int& chunk) {
     const int lane = threadIdx.x & 31;
     s = -1;
     for (int s0 = 0; s0 < n_seqs; s0 += 32) {
@@ -57,7 +70,8 @@ __device__ __forceinline__ void chunk_of_record(const int* cu_q, int n_seqs, int
     chunk = -1;
     if (s >= 0) {
         const int i = r - chunk_first_record<C>(cu_q[s], s);
-        if (i * C < cu_q[s + 1] - cu_q[s]) chunk = i;
+        const int len = cu_q[s + 1] - cu_q[s];
+        if (len >= min_len && i * C < len) chunk = i;
     }
 }
 
@@ -246,6 +260,7 @@ struct ChunkScanArgs {
     float* state; long long state_stride; int state_off, head_floats;      // a head's state: [V][NK] floats
     const int* cu_q; const int* state_slots; const int* seq_fresh;
     float* o; int heads, V;                                 // [T, heads * V]
+    int min_len;                                            // shorter sequences are not this kernel's
 };
 
 constexpr int CS_STAGES = 3;
@@ -302,6 +317,7 @@ __global__ void __launch_bounds__(64 * W + CS_LOADERS) chunk_scan_kernel(ChunkSc
     const int s = blockIdx.x, h = blockIdx.y, j0 = blockIdx.z * VB, V = A.V;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t0 = A.cu_q[s], len = A.cu_q[s + 1] - t0, chunks = (len + CS_C - 1) / CS_C;
+    if (len < A.min_len) return;
     if (warp >= 2 * W) {
         // ---- the warps that load
         const int pt = threadIdx.x - 64 * W;
@@ -511,9 +527,9 @@ static inline size_t chunk_even_smem(size_t need, long long blocks) {
 }
 
 template <int NK, int W, bool DELTA>
-static int chunk_scan_one(const ChunkScanArgs& A, int n_seqs, cudaStream_t stream) {
+static int chunk_scan_one(const ChunkScanArgs& A, int n_seqs, int live, cudaStream_t stream) {
     const dim3 grid(n_seqs, A.heads, (A.V + 16 * W - 1) / (16 * W));
-    const size_t smem = chunk_even_smem(sizeof(ChunkScanSmem<NK, W, DELTA>), (long long)grid.x * grid.y * grid.z);
+    const size_t smem = chunk_even_smem(sizeof(ChunkScanSmem<NK, W, DELTA>), (long long)live * grid.y * grid.z);
     FF_SMEM_LIMIT((chunk_scan_kernel<NK, W, DELTA>), 227 * 1024);
     FF_LAUNCH((chunk_scan_kernel<NK, W, DELTA>), grid, 64 * W + CS_LOADERS, smem, stream, A);
     FF_LAUNCH_CHECK();
@@ -522,9 +538,9 @@ static int chunk_scan_one(const ChunkScanArgs& A, int n_seqs, cudaStream_t strea
 
 // Value columns of a block, in sixteens: four warp pairs share a record where that still gives most SMs a block, else two.
 template <int NK, bool DELTA>
-static int chunk_scan_launch(const ChunkScanArgs& A, int n_seqs, cudaStream_t stream) {
-    if ((long long)n_seqs * A.heads * ((A.V + 63) / 64) >= 90) return chunk_scan_one<NK, 4, DELTA>(A, n_seqs, stream);
-    return chunk_scan_one<NK, 2, DELTA>(A, n_seqs, stream);
+static int chunk_scan_launch(const ChunkScanArgs& A, int n_seqs, int live, cudaStream_t stream) {
+    if ((long long)live * A.heads * ((A.V + 63) / 64) >= 90) return chunk_scan_one<NK, 4, DELTA>(A, n_seqs, live, stream);
+    return chunk_scan_one<NK, 2, DELTA>(A, n_seqs, live, stream);
 }
 
 }  // namespace ff

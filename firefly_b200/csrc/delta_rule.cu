@@ -60,7 +60,7 @@ template <typename T, int NP, int PARTS, int VJ>
 __global__ void __launch_bounds__(DR_MAX_THREADS) delta_rule_scan_kernel(
     DeltaArgs A, float* __restrict__ state, size_t state_stride, int state_off, const int* __restrict__ cu_q,
     const int* __restrict__ state_slots, const int* __restrict__ seq_fresh, float* __restrict__ o /*[T, heads*V]*/,
-    int heads, int N, int V, int Vb) {
+    int heads, int N, int V, int Vb, int max_len) {
     pdl_prologue();
     constexpr int KP = NP / PARTS;
     constexpr int CH = NP >= 256 ? DR_CHUNK : 2 * DR_CHUNK;     // tokens staged at a time (shared memory bounds the longest keys)
@@ -74,6 +74,7 @@ __global__ void __launch_bounds__(DR_MAX_THREADS) delta_rule_scan_kernel(
     const int jl = tid / PARTS, part = tid % PARTS;
     const int j0 = blockIdx.z * Vb;                       // the block's first column; the thread's are j0 + jl * VJ + x
     const int t0 = cu_q[s], t1 = cu_q[s + 1];
+    if (t1 - t0 >= max_len) return;                       // such a sequence goes by chunks
     bool live[VJ];
 #pragma unroll
     for (int x = 0; x < VJ; ++x) live[x] = jl * VJ + x < Vb && j0 + jl * VJ + x < V;
@@ -264,7 +265,7 @@ __global__ void __launch_bounds__(DR_MAX_THREADS) delta_rule_scan_kernel(
 // 4 x 2048 tokens, 8 heads of 128 x 128: token by token 1373 us, the two kernels 135 + 216.
 template <int NK>
 __global__ void __launch_bounds__(2 * NK) delta_prepare_kernel(DeltaArgs A, ChunkRecord<NK, true>* __restrict__ recs,
-                                                               const int* __restrict__ cu_q, int n_seqs, int n_records, int per_block, int heads) {
+                                                               const int* __restrict__ cu_q, int n_seqs, int n_records, int per_block, int min_len, int heads) {
     pdl_prologue();
     __shared__ __align__(16) float sq[CS_C * NK], sk[CS_C * NK], sa[CS_C * NK];
     __shared__ __align__(16) ChunkHalves<NK, true> halves;
@@ -285,7 +286,7 @@ __global__ void __launch_bounds__(2 * NK) delta_prepare_kernel(DeltaArgs A, Chun
     float4 d0, d1;
     float braw = 0.f;
     auto fetch = [&](int r) {
-        chunk_of_record(cu_q, n_seqs, r, s, chunk);
+        chunk_of_record(cu_q, n_seqs, r, min_len, s, chunk);
         qv = kv = make_uint4(0, 0, 0, 0);
         d0 = d1 = make_float4(0.f, 0.f, 0.f, 0.f);
         if (chunk < 0) return;
@@ -442,14 +443,18 @@ FF_EXPORT long long ff_delta_state_floats(int heads, int N, int V) {
     return (long long)heads * V * p.NP;
 }
 
-// Tokens a sequence (average of a step) from which chunks are taken (us, chunked / token by token, 8 heads of 128 x 128: eight sequences
-// of 32 37.9 / 23.5, of 64 24.9 / 44.2; one of 64 17.4 / 43.7).
-constexpr int DELTA_CHUNK_MIN = 48;
+// Tokens from which a sequence goes by chunks.  us for n sequences of L tokens, chunks / token by token, 8 heads of 128 x 128:
+//   L     n = 1         4             8             16            32
+//   16    11.9 / 12.4   14.2 / 12.6   16.1 / 12.7   21.0 / 24.3   32.3 / 47.4
+//   24    13.0 / 18.7   16.1 / 19.0   19.1 / 19.0   27.3 / 37.1   50.7 / 73.0
+//   64    17.3 / 43.5   19.7 / 43.7   24.8 / 43.8   45.9 / 86.4   89.8 / 172
+constexpr int DELTA_CHUNK_MIN = 24;
+FF_EXPORT int ff_delta_chunk_min() { return DELTA_CHUNK_MIN; }
 
 // Bytes of scratch memory that a step of T tokens can use (0: none; without it the token-by-token kernel runs).  `bits`: the matrices'
 // addresses, row strides and first columns in bytes, or'ed (row_bits).
 FF_EXPORT long long ff_delta_scratch_bytes(int dtype, int T, int n_seqs, int heads, int N, int V, int bits) {
-    if (dtype != 1 || (bits & 15) || T <= 0 || n_seqs <= 0 || (long long)T < (long long)DELTA_CHUNK_MIN * n_seqs || (N != 64 && N != 128) || V <= 0 || V > 256 || V % 8) return 0;
+    if (dtype != 1 || (bits & 15) || T < DELTA_CHUNK_MIN || n_seqs <= 0 || (N != 64 && N != 128) || V <= 0 || V > 256 || V % 8) return 0;
     return chunk_records(T, n_seqs) * heads * (long long)(N == 64 ? sizeof(ChunkRecord<64, true>) : sizeof(ChunkRecord<128, true>));
 }
 
@@ -459,24 +464,24 @@ static unsigned delta_bits(const DeltaArgs& A) {
 }
 
 template <int NK>
-static int delta_chunk_launch(const DeltaArgs& A, const ChunkScanArgs& B, int T, int n_seqs, void* scratch, cudaStream_t stream) {
+static int delta_chunk_launch(const DeltaArgs& A, const ChunkScanArgs& B, int T, int n_seqs, int live, void* scratch, cudaStream_t stream) {
     const int n_records = (int)chunk_records(T, n_seqs), per_block = chunk_records_a_block((long long)n_records * B.heads);
     FF_LAUNCH(delta_prepare_kernel<NK>, dim3((n_records + per_block - 1) / per_block, B.heads), 2 * NK, 0, stream, A,
-              (ChunkRecord<NK, true>*)scratch, B.cu_q, n_seqs, n_records, per_block, B.heads);
-    return chunk_scan_launch<NK, true>(B, n_seqs, stream);
+              (ChunkRecord<NK, true>*)scratch, B.cu_q, n_seqs, n_records, per_block, B.min_len, B.heads);
+    return chunk_scan_launch<NK, true>(B, n_seqs, live, stream);
 }
 
 template <typename T>
 static int delta_launch(const DeltaArgs& A, float* state, long long state_stride, int state_off, const int* cu_q,
                         const int* state_slots, const int* seq_fresh, float* o, int n_seqs, int heads, int N, int V,
-                        cudaStream_t stream) {
+                        int max_len, cudaStream_t stream) {
     DeltaPlan p;
     if (!delta_plan(N, V, &p)) return FF_ERR_UNSUPPORTED;
     if (p.Vb > 128) return FF_ERR_UNSUPPORTED;
     dim3 grid(n_seqs, heads, p.vsplit);
 #define FF_DELTA(NP, PARTS, VJ)                                                                                    \
     FF_LAUNCH((delta_rule_scan_kernel<T, NP, PARTS, VJ>), grid, p.threads, 0, stream, A, state, (size_t)state_stride, \
-              state_off, cu_q, state_slots, seq_fresh, o, heads, N, V, p.Vb)
+              state_off, cu_q, state_slots, seq_fresh, o, heads, N, V, p.Vb, max_len)
     switch (p.NP) {
         case 16: FF_DELTA(16, 4, 1); break;
         case 32: FF_DELTA(32, 8, 1); break;
@@ -490,31 +495,34 @@ static int delta_launch(const DeltaArgs& A, float* state, long long state_stride
     return 0;
 }
 
-// `launched`: how many kernels the call put on the stream (1: token by token, 2: by chunks).
+// `n_long`: how many of the sequences have ff_delta_chunk_min tokens or more (-1: not known).  `launched`: how many kernels the call put
+// on the stream (1: token by token, 2: by chunks, 3: some sequences so and some so).
 FF_EXPORT int ff_delta_rule_scan(const void* q, int q_stride, int q_off, const void* k, int k_stride, int k_off,
                                  const void* v, int v_stride, int v_off, const void* beta, int beta_stride, int beta_off,
                                  int dtype, const float* a, int a_stride, int a_off, const float* dt_bias,
                                  const float* a_log, int decay_per_head, int heads_per_group, float q_scale, float unit_eps, float* state,
                                  long long state_stride, int state_off, const int* cu_q, const int* state_slots,
                                  const int* seq_fresh, float* o, int T, int n_seqs, int heads, int N, int V,
-                                 void* scratch, long long scratch_bytes, int* launched, cudaStream_t stream) {
+                                 int n_long, void* scratch, long long scratch_bytes, int* launched, cudaStream_t stream) {
     *launched = 0;
     if (T <= 0 || n_seqs <= 0) return 0;
     if (heads_per_group <= 0 || heads % heads_per_group) return FF_ERR_BAD_ARG;
     DeltaArgs A{q, q_stride, q_off, k, k_stride, k_off, v, v_stride, v_off, beta, beta_stride, beta_off,
                 a, a_stride, a_off, dt_bias, a_log, heads_per_group, q_scale, unit_eps, decay_per_head ? 1 : 0};
     const long long need = ff_delta_scratch_bytes(dtype, T, n_seqs, heads, N, V, (int)delta_bits(A));
-    if (need > 0 && scratch && scratch_bytes >= need) {
-        *launched = 2;
-        const ChunkScanArgs B{scratch, (const bf16*)v, v_stride, v_off, state, state_stride, state_off, V * N, cu_q, state_slots, seq_fresh, o, heads, V};
-        return N == 64 ? delta_chunk_launch<64>(A, B, T, n_seqs, scratch, stream) : delta_chunk_launch<128>(A, B, T, n_seqs, scratch, stream);
+    const ChunkRoute R = chunk_route(need > 0 && scratch && scratch_bytes >= need, n_long, n_seqs, DELTA_CHUNK_MIN);
+    *launched = R.kernels();
+    if (R.walk) {
+        int rc = FF_ERR_BAD_ARG;
+        if (dtype == 0)
+            rc = delta_launch<float>(A, state, state_stride, state_off, cu_q, state_slots, seq_fresh, o, n_seqs, heads, N, V, R.max_walk, stream);
+        else if (dtype == 1)
+            rc = delta_launch<bf16>(A, state, state_stride, state_off, cu_q, state_slots, seq_fresh, o, n_seqs, heads, N, V, R.max_walk, stream);
+        if (rc) return rc;
     }
-    *launched = 1;
-    if (dtype == 0)
-        return delta_launch<float>(A, state, state_stride, state_off, cu_q, state_slots, seq_fresh, o, n_seqs, heads, N, V, stream);
-    if (dtype == 1)
-        return delta_launch<bf16>(A, state, state_stride, state_off, cu_q, state_slots, seq_fresh, o, n_seqs, heads, N, V, stream);
-    return FF_ERR_BAD_ARG;
+    if (!R.chunks) return 0;
+    const ChunkScanArgs B{scratch, (const bf16*)v, v_stride, v_off, state, state_stride, state_off, V * N, cu_q, state_slots, seq_fresh, o, heads, V, DELTA_CHUNK_MIN};
+    return N == 64 ? delta_chunk_launch<64>(A, B, T, n_seqs, R.live, scratch, stream) : delta_chunk_launch<128>(A, B, T, n_seqs, R.live, scratch, stream);
 }
 
 // gate_dtype: 32-bit, or the type of y

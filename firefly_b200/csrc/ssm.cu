@@ -249,7 +249,7 @@ template <typename T, int NP, bool CD>
 __global__ void __launch_bounds__(WS_THREADS) scalar_decay_scan_kernel(
     ScanArgs A, float* __restrict__ state, size_t state_stride, int state_off, const int* __restrict__ cu_q,
     const int* __restrict__ state_slots, const int* __restrict__ seq_fresh, float* __restrict__ o /*[T, heads*V]*/,
-    int heads, int N, int V) {
+    int heads, int N, int V, int max_len) {
     pdl_prologue();
     using WS = WideState<NP>;
     constexpr int CH = WS::CH, VB = WS::VB, PQ = CH * NP / WS_THREADS, PV = (CH * VB + WS_THREADS - 1) / WS_THREADS;
@@ -260,6 +260,7 @@ __global__ void __launch_bounds__(WS_THREADS) scalar_decay_scan_kernel(
     const int s = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
     const int j0 = blockIdx.z * VB;
     const int t0 = cu_q[s], t1 = cu_q[s + 1];
+    if (t1 - t0 >= max_len) return;                       // such a sequence goes by chunks
     WS w;
     w.place(tid);
     float* S_g = state + (size_t)state_slots[s] * state_stride + state_off + (size_t)h * V * NP;
@@ -383,13 +384,19 @@ __global__ void __launch_bounds__(WS_THREADS) scalar_decay_scan_kernel(
 // value columns), whose warps hold S^T as the accumulators of mma.sync; the same registers are, split, the left operand of
 // S^T q, so the state goes nowhere between the products.
 // Measured on 4 x 2048 tokens, 32 heads of 128 x 64: token by token with one column a thread 1552 us; the two kernels 33 + 143.
-// From SCAN_CHUNK_MIN tokens a sequence (average of a step) on it is the faster one (us, chunked / token by token wide, 32 heads of
-// 128 x 64: eight sequences of 16 16.1 / 12.7, of 32 16.6 / 22.4, of 64 22.7 / 41.7; one of 32 9.3 / 10.3, of 64 11.4 / 18.3).
 constexpr int SC_C = 32;                                  // tokens a chunk
+// Tokens from which a sequence goes by chunks.  us for n sequences of L tokens, chunks / token by token, 32 heads of 128 x 64 (in one
+// group or in eight the same):
+//   L     n = 1         4             8             16            32
+//   24    9.5 / 7.9     11.6 / 11.6   16.5 / 17.1   25.7 / 26.7   42.9 / 48.8
+//   32    9.7 / 9.9     12.2 / 14.6   16.9 / 21.8   26.1 / 34.4   44.3 / 63.1
+//   64    11.6 / 17.9   14.9 / 26.9   22.4 / 41.1   37.3 / 65.2   63.8 / 121
+// and for a decay per key channel, 16 heads of 64 x 128:
+//   32    7.3 / 7.3     11.7 / 9.9    14.3 / 12.7   19.6 / 17.9   28.6 / 28.6
+//   48    8.3 / 10.1    13.8 / 13.8   16.5 / 17.9   23.5 / 25.5   39.5 / 41.1
+//   64    8.8 / 12.8    14.8 / 17.5   18.3 / 23.3   26.5 / 33.3   47.5 / 53.7
 constexpr int SCAN_CHUNK_MIN = 32;
-// The same for a decay per key channel (us, 16 heads of 64 x 128: eight sequences of 64 34.9 / 23.8, of 96 22.3 / 34.5 with records of
-// their own block; one of 96 10.1 / 18.3).
-constexpr int CHANNEL_CHUNK_MIN = 80;
+constexpr int CHANNEL_CHUNK_MIN = 48;
 constexpr int SC_PP = SC_C + 8;
 constexpr long long SCAN_PREPARE_BLOCKS = 12 * 148;         // blocks of the first kernel that are on the GPU together
 
@@ -406,13 +413,13 @@ static_assert(sizeof(ScanRecord) % 16 == 0, "a record is copied in 16-byte piece
 // block / now: one prompt of 64 tokens 64.0 / 18.6, eight of 256 106 / 58.8; 32 heads of 128 x 64: 35.8 / 23.7 and 71.8 / 53.4.
 template <int NK>
 __global__ void __launch_bounds__(128) scalar_decay_prepare_kernel(ScanArgs A, ScanRecord* __restrict__ recs, const int* __restrict__ cu_q,
-                                                                   int n_seqs, int heads, int heads_a_block) {
+                                                                   int n_seqs, int min_len, int heads, int heads_a_block) {
     pdl_prologue();
     constexpr int QP = NK + 8;
     __shared__ __align__(16) bf16 sq[SC_C * QP], sk[SC_C * QP];
     __shared__ float lh[4][SC_C], ll[4][SC_C], sb[4][SC_C], pw[4][SC_C + 1];
     int s, chunk;
-    chunk_of_record<SC_C>(cu_q, n_seqs, blockIdx.x, s, chunk);
+    chunk_of_record<SC_C>(cu_q, n_seqs, blockIdx.x, min_len, s, chunk);
     if (chunk < 0) return;
     const int group = blockIdx.y, row0 = cu_q[s] + chunk * SC_C, n = min(SC_C, cu_q[s + 1] - row0);
     const int hb0 = blockIdx.z * heads_a_block, hb1 = min(A.heads_per_group, hb0 + heads_a_block);       // heads of the group
@@ -526,7 +533,7 @@ template <int NK, int W>
 __global__ void __launch_bounds__(64 * W + CS_LOADERS) scalar_decay_chunk_kernel(
     ScanArgs A, const ScanRecord* recs_, float* __restrict__ state, size_t state_stride, int state_off, const int* __restrict__ cu_q,
     const int* __restrict__ state_slots, const int* __restrict__ seq_fresh, float* __restrict__ o /*[T, heads*V]*/,
-    int heads, int V) {
+    int heads, int V, int min_len) {
     pdl_prologue();
     using SM = ScanChunkSmem<NK, W>;
     constexpr int QP = SM::QP, VP = SM::VP, PP = SC_PP, NT = NK / 16, VB = 16 * W;
@@ -535,6 +542,7 @@ __global__ void __launch_bounds__(64 * W + CS_LOADERS) scalar_decay_chunk_kernel
     const int s = blockIdx.x, h = blockIdx.y, j0 = blockIdx.z * VB;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t0 = cu_q[s], len = cu_q[s + 1] - t0, chunks = (len + SC_C - 1) / SC_C;
+    if (len < min_len) return;
     if (warp >= 2 * W) {
         // ---- the warps that load
         const int pt = threadIdx.x - 64 * W, group = h / A.heads_per_group;
@@ -743,7 +751,7 @@ __global__ void __launch_bounds__(64 * W + CS_LOADERS) scalar_decay_chunk_kernel
 template <int NK>
 __global__ void __launch_bounds__(2 * NK) channel_decay_prepare_kernel(ScanArgs A, ChunkRecord<NK, false>* __restrict__ recs,
                                                                        const int* __restrict__ cu_q, int n_seqs, int n_records,
-                                                                       int per_block, int heads) {
+                                                                       int per_block, int min_len, int heads) {
     pdl_prologue();
     __shared__ __align__(16) float sq[CS_C * NK], sk[CS_C * NK], sa[CS_C * NK];
     __shared__ __align__(16) ChunkHalves<NK, false> halves;
@@ -757,7 +765,7 @@ __global__ void __launch_bounds__(2 * NK) channel_decay_prepare_kernel(ScanArgs 
     uint4 qv, kv;
     float4 d0, d1;
     auto fetch = [&](int r) {
-        chunk_of_record(cu_q, n_seqs, r, s, chunk);
+        chunk_of_record(cu_q, n_seqs, r, min_len, s, chunk);
         qv = kv = make_uint4(0, 0, 0, 0);
         d0 = d1 = make_float4(1.f, 1.f, 1.f, 1.f);
         if (chunk < 0) return;
@@ -1057,14 +1065,15 @@ FF_EXPORT long long ff_scan_state_floats(int heads, int N, int V) {
     return (long long)heads * V * NP;
 }
 
-// Whether a step's recurrence runs a chunk at a time: bfloat16 prompts, long enough on average, sizes that the tiles take and
-// layouts that 16-byte copies take.  One decay per head and token (its inputs read as they are), or one per key channel.
-static bool scalar_chunk_sizes(int mode, int act, int T, int n_seqs, int N, int V) {
-    return mode != 2 && !act && (long long)T >= (long long)SCAN_CHUNK_MIN * n_seqs && (N == 64 || N == 128) && V % 8 == 0;
+// Whether a step's prompts can go a chunk at a time: bfloat16, sizes that the tiles take and layouts that 16-byte copies take.  One decay
+// per head and token (its inputs read as they are), or one per key channel.
+static bool scalar_chunk_sizes(int mode, int act, int T, int N, int V) {
+    return mode != 2 && !act && T >= SCAN_CHUNK_MIN && (N == 64 || N == 128) && V % 8 == 0;
 }
-static bool channel_chunk_sizes(int mode, int act, int T, int n_seqs, int N, int V) {
-    return mode == 2 && !act && (long long)T >= (long long)CHANNEL_CHUNK_MIN * n_seqs && (N == 64 || N == 128) && V % 8 == 0;
+static bool channel_chunk_sizes(int mode, int act, int T, int N, int V) {
+    return mode == 2 && !act && T >= CHANNEL_CHUNK_MIN && (N == 64 || N == 128) && V % 8 == 0;
 }
+FF_EXPORT int ff_scan_chunk_min(int mode) { return mode == 2 ? CHANNEL_CHUNK_MIN : SCAN_CHUNK_MIN; }
 static unsigned scan_bits(const ScanArgs& A) {
     return row_bits(A.q, A.q_stride, A.q_off, 2) | row_bits(A.k, A.k_stride, A.k_off, 2) | row_bits(A.v, A.v_stride, A.v_off, 2) |
            (A.mode == 2 ? row_bits(A.channel_decay, A.cd_stride, A.cd_off, 4) : 0u);
@@ -1074,29 +1083,29 @@ static unsigned scan_bits(const ScanArgs& A) {
 // addresses, row strides and first columns in bytes, or'ed (row_bits).
 FF_EXPORT long long ff_scan_scratch_bytes(int dtype, int mode, int act, int T, int n_seqs, int heads, int heads_per_group, int N, int V, int bits) {
     if (dtype != 1 || T <= 0 || n_seqs <= 0 || heads <= 0 || heads_per_group <= 0 || heads % heads_per_group || V <= 0 || V > 256 || (bits & 15)) return 0;
-    if (scalar_chunk_sizes(mode, act, T, n_seqs, N, V)) return chunk_records<SC_C>(T, n_seqs) * heads * (long long)sizeof(ScanRecord);
-    if (!channel_chunk_sizes(mode, act, T, n_seqs, N, V)) return 0;
+    if (scalar_chunk_sizes(mode, act, T, N, V)) return chunk_records<SC_C>(T, n_seqs) * heads * (long long)sizeof(ScanRecord);
+    if (!channel_chunk_sizes(mode, act, T, N, V)) return 0;
     return chunk_records(T, n_seqs) * heads * (long long)(N == 64 ? sizeof(ChunkRecord<64, false>) : sizeof(ChunkRecord<128, false>));
 }
 
 template <int NK>
 static int scan_chunk_launch(const ScanArgs& A, float* state, long long state_stride, int state_off, const int* cu_q, const int* state_slots,
-                             const int* seq_fresh, float* o, int T, int n_seqs, int heads, int V, void* scratch, cudaStream_t stream) {
+                             const int* seq_fresh, float* o, int T, int n_seqs, int live, int heads, int V, void* scratch, cudaStream_t stream) {
     ScanRecord* recs = (ScanRecord*)scratch;
     const long long records = chunk_records<SC_C>(T, n_seqs), groups = heads / A.heads_per_group, quads = (A.heads_per_group + 3) / 4;
     const long long quads_a_block = std::max(1ll, std::min(quads, (records * groups * quads + SCAN_PREPARE_BLOCKS - 1) / SCAN_PREPARE_BLOCKS));
     FF_LAUNCH(scalar_decay_prepare_kernel<NK>, dim3((unsigned)records, (unsigned)groups, (unsigned)((quads + quads_a_block - 1) / quads_a_block)), 128, 0,
-              stream, A, recs, cu_q, n_seqs, heads, (int)quads_a_block * 4);
+              stream, A, recs, cu_q, n_seqs, SCAN_CHUNK_MIN, heads, (int)quads_a_block * 4);
 #define FF_SCAN_CHUNK(W)                                                                                                \
     do {                                                                                                                \
         const dim3 grid(n_seqs, heads, (V + 16 * W - 1) / (16 * W));                                                    \
-        const size_t smem = chunk_even_smem(sizeof(ScanChunkSmem<NK, W>), (long long)grid.x * grid.y * grid.z);         \
+        const size_t smem = chunk_even_smem(sizeof(ScanChunkSmem<NK, W>), (long long)live * grid.y * grid.z);           \
         FF_SMEM_LIMIT((scalar_decay_chunk_kernel<NK, W>), 227 * 1024);                                                  \
         FF_LAUNCH((scalar_decay_chunk_kernel<NK, W>), grid, 64 * W + CS_LOADERS, smem, stream,                          \
-                  A, recs, state, (size_t)state_stride, state_off, cu_q, state_slots, seq_fresh, o, heads, V);          \
+                  A, recs, state, (size_t)state_stride, state_off, cu_q, state_slots, seq_fresh, o, heads, V, SCAN_CHUNK_MIN); \
     } while (0)
     // 64 value columns a block if that gives most SMs a block, else 32
-    if ((long long)n_seqs * heads * ((V + 63) / 64) >= 100) FF_SCAN_CHUNK(4);
+    if ((long long)live * heads * ((V + 63) / 64) >= 100) FF_SCAN_CHUNK(4);
     else FF_SCAN_CHUNK(2);
 #undef FF_SCAN_CHUNK
     FF_LAUNCH_CHECK();
@@ -1104,53 +1113,52 @@ static int scan_chunk_launch(const ScanArgs& A, float* state, long long state_st
 }
 
 template <int NK>
-static int channel_chunk_launch(const ScanArgs& A, const ChunkScanArgs& B, int T, int n_seqs, void* scratch, cudaStream_t stream) {
+static int channel_chunk_launch(const ScanArgs& A, const ChunkScanArgs& B, int T, int n_seqs, int live, void* scratch, cudaStream_t stream) {
     const int n_records = (int)chunk_records(T, n_seqs), per_block = chunk_records_a_block((long long)n_records * B.heads);
     FF_LAUNCH(channel_decay_prepare_kernel<NK>, dim3((n_records + per_block - 1) / per_block, B.heads), 2 * NK, 0, stream, A,
-              (ChunkRecord<NK, false>*)scratch, B.cu_q, n_seqs, n_records, per_block, B.heads);
-    return chunk_scan_launch<NK, false>(B, n_seqs, stream);
+              (ChunkRecord<NK, false>*)scratch, B.cu_q, n_seqs, n_records, per_block, B.min_len, B.heads);
+    return chunk_scan_launch<NK, false>(B, n_seqs, live, stream);
 }
 
 template <typename T>
 static int scan_launch(const ScanArgs& A, float* state, long long state_stride, int state_off, const int* cu_q,
                        const int* state_slots, const int* seq_fresh, float* o, int T_tot, int n_seqs, int heads, int N, int V,
-                       void* scratch, long long scratch_bytes, int* launched, cudaStream_t stream) {
+                       int n_long, void* scratch, long long scratch_bytes, int* launched, cudaStream_t stream) {
     if (!ws_key_size(N) || V <= 0 || V > 256) return FF_ERR_UNSUPPORTED;
-    if constexpr (sizeof(T) == 2) {
-        const long long need = ff_scan_scratch_bytes(1, A.mode, A.act, T_tot, n_seqs, heads, A.heads_per_group, N, V, (int)scan_bits(A));
-        if (need > 0 && scratch && scratch_bytes >= need) {
-            *launched = 2;
-            if (A.mode != 2) {
-                if (N == 64) return scan_chunk_launch<64>(A, state, state_stride, state_off, cu_q, state_slots, seq_fresh, o, T_tot, n_seqs, heads, V, scratch, stream);
-                return scan_chunk_launch<128>(A, state, state_stride, state_off, cu_q, state_slots, seq_fresh, o, T_tot, n_seqs, heads, V, scratch, stream);
-            }
-            const ChunkScanArgs B{scratch, (const bf16*)A.v, A.v_stride, A.v_off, state, state_stride, state_off, V * N, cu_q, state_slots, seq_fresh, o, heads, V};
-            return N == 64 ? channel_chunk_launch<64>(A, B, T_tot, n_seqs, scratch, stream) : channel_chunk_launch<128>(A, B, T_tot, n_seqs, scratch, stream);
-        }
-    }
+    const long long need = sizeof(T) == 2 ? ff_scan_scratch_bytes(1, A.mode, A.act, T_tot, n_seqs, heads, A.heads_per_group, N, V, (int)scan_bits(A)) : 0;
+    const ChunkRoute R = chunk_route(need > 0 && scratch && scratch_bytes >= need, n_long, n_seqs, ff_scan_chunk_min(A.mode));
+    *launched = R.kernels();
 #define FF_SCAN_ONE(NP, CD)                                                                                             \
     FF_LAUNCH((scalar_decay_scan_kernel<T, NP, CD>), dim3(n_seqs, heads, (V + WideState<NP>::VB - 1) / WideState<NP>::VB), \
-              WS_THREADS, 0, stream, A, state, (size_t)state_stride, state_off, cu_q, state_slots, seq_fresh, o, heads, N, V)
+              WS_THREADS, 0, stream, A, state, (size_t)state_stride, state_off, cu_q, state_slots, seq_fresh, o, heads, N, V, R.max_walk)
 #define FF_SCAN(NP)                                                                                                     \
     do {                                                                                                                \
         if (A.mode == 2) FF_SCAN_ONE(NP, true);                                                                         \
         else FF_SCAN_ONE(NP, false);                                                                                    \
     } while (0)
-    *launched = 1;
-    switch (ws_key_size(N)) {
-        case 16: FF_SCAN(16); break;
-        case 32: FF_SCAN(32); break;
-        case 64: FF_SCAN(64); break;
-        case 128: FF_SCAN(128); break;
-        default: FF_SCAN(256); break;
+    if (R.walk) {
+        switch (ws_key_size(N)) {
+            case 16: FF_SCAN(16); break;
+            case 32: FF_SCAN(32); break;
+            case 64: FF_SCAN(64); break;
+            case 128: FF_SCAN(128); break;
+            default: FF_SCAN(256); break;
+        }
+        FF_LAUNCH_CHECK();
     }
 #undef FF_SCAN
 #undef FF_SCAN_ONE
-    FF_LAUNCH_CHECK();
-    return 0;
+    if (!R.chunks) return 0;
+    if (A.mode != 2) {
+        if (N == 64) return scan_chunk_launch<64>(A, state, state_stride, state_off, cu_q, state_slots, seq_fresh, o, T_tot, n_seqs, R.live, heads, V, scratch, stream);
+        return scan_chunk_launch<128>(A, state, state_stride, state_off, cu_q, state_slots, seq_fresh, o, T_tot, n_seqs, R.live, heads, V, scratch, stream);
+    }
+    const ChunkScanArgs B{scratch, (const bf16*)A.v, A.v_stride, A.v_off, state, state_stride, state_off, V * N, cu_q, state_slots, seq_fresh, o, heads, V, CHANNEL_CHUNK_MIN};
+    return N == 64 ? channel_chunk_launch<64>(A, B, T_tot, n_seqs, R.live, scratch, stream) : channel_chunk_launch<128>(A, B, T_tot, n_seqs, R.live, scratch, stream);
 }
 
-// `launched`: how many kernels the call put on the stream (1: token by token, 2: by chunks).
+// `n_long`: how many of the sequences have ff_scan_chunk_min tokens or more (-1: not known).  `launched`: how many kernels the call put
+// on the stream (1: token by token, 2: by chunks, 3: some sequences so and some so).
 FF_EXPORT int ff_scalar_decay_scan(const void* q, int q_stride, int q_off, const void* k, int k_stride, int k_off,
                                    const void* v, int v_stride, int v_off, int dtype, int heads_per_group, int act,
                                    int mode, const float* decay, const void* step, int step_stride, int step_off,
@@ -1158,16 +1166,16 @@ FF_EXPORT int ff_scalar_decay_scan(const void* q, int q_stride, int q_off, const
                                    const float* channel_decay, int cd_stride, int cd_off, float q_scale, float* state,
                                    long long state_stride, int state_off, const int* cu_q, const int* state_slots,
                                    const int* seq_fresh, float* o, int T, int n_seqs, int heads, int N, int V,
-                                   void* scratch, long long scratch_bytes, int* launched, cudaStream_t stream) {
+                                   int n_long, void* scratch, long long scratch_bytes, int* launched, cudaStream_t stream) {
     *launched = 0;
     if (T <= 0 || n_seqs <= 0) return 0;
     if (heads_per_group <= 0 || mode < 0 || mode > 2 || (mode == 2 && !channel_decay)) return FF_ERR_BAD_ARG;
     ScanArgs A{q, q_stride, q_off, k, k_stride, k_off, v, v_stride, v_off, heads_per_group, act, decay,
                step, step_stride, step_off, step_bias, a_log, skip, mode, channel_decay, cd_stride, cd_off, q_scale};
     if (dtype == 0)
-        return scan_launch<float>(A, state, state_stride, state_off, cu_q, state_slots, seq_fresh, o, T, n_seqs, heads, N, V, scratch, scratch_bytes, launched, stream);
+        return scan_launch<float>(A, state, state_stride, state_off, cu_q, state_slots, seq_fresh, o, T, n_seqs, heads, N, V, n_long, scratch, scratch_bytes, launched, stream);
     if (dtype == 1)
-        return scan_launch<bf16>(A, state, state_stride, state_off, cu_q, state_slots, seq_fresh, o, T, n_seqs, heads, N, V, scratch, scratch_bytes, launched, stream);
+        return scan_launch<bf16>(A, state, state_stride, state_off, cu_q, state_slots, seq_fresh, o, T, n_seqs, heads, N, V, n_long, scratch, scratch_bytes, launched, stream);
     return FF_ERR_BAD_ARG;
 }
 

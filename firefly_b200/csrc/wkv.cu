@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(WS_THREADS) wkv_scan_kernel(
     const float* __restrict__ w0, const float* __restrict__ u, float* __restrict__ state, size_t state_stride,
     int prev_off, const T* __restrict__ x_, int W, const int* __restrict__ cu_q,
     const int* __restrict__ state_slots, const int* __restrict__ seq_fresh, float* __restrict__ o /*[T,HD]*/,
-    int Ttot, int heads, int dim) {
+    int Ttot, int heads, int dim, int max_len) {
     pdl_prologue();
     using WS = WideState<DIM>;
     constexpr int CH = WS::CH, VB = WS::VB < DIM ? WS::VB : DIM, PQ = CH * DIM / WS_THREADS, PV = CH * VB / WS_THREADS;
@@ -130,6 +130,7 @@ __global__ void __launch_bounds__(WS_THREADS) wkv_scan_kernel(
     __shared__ __align__(16) f32x2 s_v[2][CH][VB];             // each value twice
     const int s = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, j0 = blockIdx.z * VB;
     const int t0 = cu_q[s], t1 = cu_q[s + 1];
+    if (t1 - t0 >= max_len) return;                            // such a sequence goes by chunks
     const int HD = heads * dim;
     float* st = state + (size_t)state_slots[s] * state_stride;
     float* S_g = st + (size_t)h * DIM * DIM;
@@ -244,7 +245,7 @@ __global__ void __launch_bounds__(2 * NK) wkv_prepare_kernel(const bf16* rkvg, c
                                                              const float* __restrict__ u, ChunkRecord<NK, false>* __restrict__ recs,
                                                              float* __restrict__ state, size_t state_stride, int prev_off, const bf16* x, int W,
                                                              const int* __restrict__ cu_q, const int* __restrict__ state_slots, int n_seqs,
-                                                             int n_records, int per_block, int Ttot, int heads) {
+                                                             int n_records, int per_block, int min_len, int Ttot, int heads) {
     pdl_prologue();
     __shared__ __align__(16) float sr[CS_C * NK], sk[CS_C * NK], sw[CS_C * NK], su[NK];
     __shared__ __align__(16) ChunkHalves<NK, false> halves;
@@ -262,7 +263,7 @@ __global__ void __launch_bounds__(2 * NK) wkv_prepare_kernel(const bf16* rkvg, c
     uint4 rv, kv;
     float4 d0, d1;
     auto fetch = [&](int r) {
-        chunk_of_record(cu_q, n_seqs, r, s, chunk);
+        chunk_of_record(cu_q, n_seqs, r, min_len, s, chunk);
         rv = kv = make_uint4(0, 0, 0, 0);
         d0 = d1 = make_float4(0.f, 0.f, 0.f, 0.f);
         if (chunk < 0) return;
@@ -407,10 +408,10 @@ template <typename T>
 static int wkv_scan_launch(const void* rkvg, const float* dlog, const float* w0, const float* u, float* state,
                            long long state_stride, int prev_off, const void* x, int W, const int* cu_q,
                            const int* state_slots, const int* seq_fresh, float* o, int Ttot, int n_seqs, int heads,
-                           int dim, cudaStream_t stream) {
+                           int dim, int max_len, cudaStream_t stream) {
 #define FF_WKV(D)                                                                                                  \
     FF_LAUNCH((wkv_scan_kernel<T, D>), dim3(n_seqs, heads, (dim + min(D, WideState<D>::VB) - 1) / min(D, WideState<D>::VB)), WS_THREADS, 0, stream, \
-              (const T*)rkvg, dlog, w0, u, state, (size_t)state_stride, prev_off, (const T*)x, W, cu_q, state_slots, seq_fresh, o, Ttot, heads, dim)
+              (const T*)rkvg, dlog, w0, u, state, (size_t)state_stride, prev_off, (const T*)x, W, cu_q, state_slots, seq_fresh, o, Ttot, heads, dim, max_len)
     if (dim <= 32) FF_WKV(32);
     else if (dim <= 64) FF_WKV(64);
     else if (dim <= 128) FF_WKV(128);
@@ -423,51 +424,60 @@ static int wkv_scan_launch(const void* rkvg, const float* dlog, const float* w0,
 // the head size the recurrence kernel is instantiated for (its state keeps that many squared floats a head)
 FF_EXPORT int ff_wkv_state_dim(int dim) { return dim <= 32 ? 32 : (dim <= 64 ? 64 : (dim <= 128 ? 128 : -1)); }
 
-// Tokens a sequence (average of a step) from which chunks are taken (us, chunked / token by token, 32 heads of 64: eight sequences of
-// 64 37.5 / 26.6, of 96 30.4 / 38.7; one of 96 12.1 / 21.0).
-constexpr int WKV_CHUNK_MIN = 80;
+// Tokens from which a sequence goes by chunks.  us for n sequences of L tokens, chunks / token by token, 32 heads of 64:
+//   L     n = 1         4             8             16            32
+//   48    9.5 / 10.1    13.4 / 14.9   18.9 / 19.6   32.0 / 26.3   58.7 / 43.2
+//   64    10.9 / 12.8   14.4 / 19.1   22.4 / 25.3   39.4 / 34.3   77.5 / 56.8
+//   256   20.2 / 45.3   38.2 / 70.2   72.3 / 94.4   134 / 130     246 / 217
+// (two of 48: 11.7 / 10.2).  With 512 heads and more in flight the walk keeps the GPU busy by itself and chunks are up to a quarter slower; the rule
+// does not look at that, since it would make a request's numbers depend on how many others there are.
+constexpr int WKV_CHUNK_MIN = 64;
+FF_EXPORT int ff_wkv_chunk_min() { return WKV_CHUNK_MIN; }
 
 // Bytes of scratch memory that a step of T tokens can use (0: none; without it the token-by-token kernel runs).  `bits`: the addresses of
 // rkvg and dlog, or'ed.
 FF_EXPORT long long ff_wkv_scratch_bytes(int dtype, int T, int n_seqs, int heads, int dim, int bits) {
-    if (dtype != 1 || (bits & 15) || T <= 0 || n_seqs <= 0 || (long long)T < (long long)WKV_CHUNK_MIN * n_seqs || (dim != 64 && dim != 128)) return 0;
+    if (dtype != 1 || (bits & 15) || T < WKV_CHUNK_MIN || n_seqs <= 0 || (dim != 64 && dim != 128)) return 0;
     return chunk_records(T, n_seqs) * heads * (long long)(dim == 64 ? sizeof(ChunkRecord<64, false>) : sizeof(ChunkRecord<128, false>));
 }
 
 template <int D>
 static int wkv_chunk_launch(const bf16* rkvg, const float* dlog, const float* w0, const float* u, int prev_off, const bf16* x, int W,
-                            const ChunkScanArgs& B, int Ttot, int n_seqs, void* scratch, cudaStream_t stream) {
+                            const ChunkScanArgs& B, int Ttot, int n_seqs, int live, void* scratch, cudaStream_t stream) {
     const int n_records = (int)chunk_records(Ttot, n_seqs), per_block = chunk_records_a_block((long long)n_records * B.heads);
     FF_LAUNCH(wkv_prepare_kernel<D>, dim3((n_records + per_block - 1) / per_block, B.heads), 2 * D, 0, stream, rkvg, dlog, w0, u,
               (ChunkRecord<D, false>*)scratch, B.state, (size_t)B.state_stride, prev_off, x, W, B.cu_q, B.state_slots, n_seqs, n_records, per_block,
-              Ttot, B.heads);
-    return chunk_scan_launch<D, false>(B, n_seqs, stream);
+              B.min_len, Ttot, B.heads);
+    return chunk_scan_launch<D, false>(B, n_seqs, live, stream);
 }
 
-// `launched`: how many kernels the call put on the stream (1: token by token, 2: by chunks).
+// `n_long`: how many of the sequences have ff_wkv_chunk_min tokens or more (-1: not known).  `launched`: how many kernels the call put
+// on the stream (1: token by token, 2: by chunks, 3: some sequences so and some so).
 FF_EXPORT int ff_wkv_scan(const void* rkvg, int dtype, const float* dlog, const float* w0, const float* u, float* state,
                           long long state_stride, int prev_off, const void* x, int W, const int* cu_q,
                           const int* state_slots, const int* seq_fresh, float* o, int Ttot, int n_seqs, int heads,
-                          int dim, void* scratch, long long scratch_bytes, int* launched, cudaStream_t stream) {
+                          int dim, int n_long, void* scratch, long long scratch_bytes, int* launched, cudaStream_t stream) {
     *launched = 0;
     if (Ttot <= 0 || n_seqs <= 0) return 0;
     const long long need = ff_wkv_scratch_bytes(dtype, Ttot, n_seqs, heads, dim, (int)(row_bits(rkvg, 0, 0, 2) | row_bits(dlog, 0, 0, 4)));
-    if (need > 0 && scratch && scratch_bytes >= need) {
-        *launched = 2;
-        const bf16* in = (const bf16*)rkvg;
-        const int HD = heads * dim;
-        const ChunkScanArgs B{scratch, in + (size_t)2 * Ttot * HD, HD, 0, state, state_stride, 0, dim * dim, cu_q, state_slots, seq_fresh, o, heads, dim};
-        if (dim == 64) return wkv_chunk_launch<64>(in, dlog, w0, u, prev_off, (const bf16*)x, W, B, Ttot, n_seqs, scratch, stream);
-        return wkv_chunk_launch<128>(in, dlog, w0, u, prev_off, (const bf16*)x, W, B, Ttot, n_seqs, scratch, stream);
+    const ChunkRoute R = chunk_route(need > 0 && scratch && scratch_bytes >= need, n_long, n_seqs, WKV_CHUNK_MIN);
+    *launched = R.kernels();
+    if (R.walk) {
+        int rc = FF_ERR_BAD_ARG;
+        if (dtype == 0)
+            rc = wkv_scan_launch<float>(rkvg, dlog, w0, u, state, state_stride, prev_off, x, W, cu_q, state_slots,
+                                        seq_fresh, o, Ttot, n_seqs, heads, dim, R.max_walk, stream);
+        else if (dtype == 1)
+            rc = wkv_scan_launch<bf16>(rkvg, dlog, w0, u, state, state_stride, prev_off, x, W, cu_q, state_slots,
+                                       seq_fresh, o, Ttot, n_seqs, heads, dim, R.max_walk, stream);
+        if (rc) return rc;
     }
-    *launched = 1;
-    if (dtype == 0)
-        return wkv_scan_launch<float>(rkvg, dlog, w0, u, state, state_stride, prev_off, x, W, cu_q, state_slots,
-                                      seq_fresh, o, Ttot, n_seqs, heads, dim, stream);
-    if (dtype == 1)
-        return wkv_scan_launch<bf16>(rkvg, dlog, w0, u, state, state_stride, prev_off, x, W, cu_q, state_slots,
-                                     seq_fresh, o, Ttot, n_seqs, heads, dim, stream);
-    return FF_ERR_BAD_ARG;
+    if (!R.chunks) return 0;
+    const bf16* in = (const bf16*)rkvg;
+    const int HD = heads * dim;
+    const ChunkScanArgs B{scratch, in + (size_t)2 * Ttot * HD, HD, 0, state, state_stride, 0, dim * dim, cu_q, state_slots, seq_fresh, o, heads, dim, WKV_CHUNK_MIN};
+    if (dim == 64) return wkv_chunk_launch<64>(in, dlog, w0, u, prev_off, (const bf16*)x, W, B, Ttot, n_seqs, R.live, scratch, stream);
+    return wkv_chunk_launch<128>(in, dlog, w0, u, prev_off, (const bf16*)x, W, B, Ttot, n_seqs, R.live, scratch, stream);
 }
 
 FF_EXPORT int ff_wkv_out(const float* o, const void* g, int dtype, const float* norm, float eps, void* y, int T,

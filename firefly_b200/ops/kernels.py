@@ -922,18 +922,31 @@ def _row_bits(*rows) -> int:
     return bits & 15
 
 
-def _recurrence_scratch(ctx, module: str, entry: str, *sizes: int):
-    """Scratch memory for a recurrence that takes a step's prompts a chunk at a time: (pointer, bytes), nothing when the step
-    is none for it (the entry `entry` of the library says how much it can use), the context has no workspace or the device has no
-    memory left (the token-by-token kernel runs then)."""
+@functools.lru_cache(maxsize=None)
+def _chunk_min(module: str, entry: str, *kind: int) -> int:
+    return int(getattr(_lib(module), entry)(*[c_int(x) for x in kind]))
+
+
+def _recurrence_scratch(ctx, module: str, entry: str, chunk_min: int, *sizes: int):
+    """What a recurrence needs to know to take long sequences a chunk at a time: (how many have ``chunk_min`` tokens or more, -1 if the
+    context has no host copy of the lengths; scratch memory; its bytes).  No scratch memory when there is no such sequence, when
+    the sizes are none for it (``entry`` of the library says how much it can use), when the context has no workspace or
+    the device no memory left: every sequence is walked token by token then."""
+    lens = getattr(ctx, "q_lens", None)
+    n_long = -1
+    if lens is not None:
+        memo = getattr(ctx, "memo", None)
+        n_long = memo.get(("long_seqs", chunk_min)) if memo is not None else None
+        if n_long is None:
+            n_long = sum(1 for q in lens if q >= chunk_min)
+            if memo is not None:
+                memo[("long_seqs", chunk_min)] = n_long
     ws = getattr(ctx, "workspace", None)
-    need = _recurrence_scratch_bytes(module, entry, *sizes) if ws is not None else 0
-    if need <= 0:
-        return c_void_p(0), ctypes.c_longlong(0)
-    records = ws.try_get("scan.records", (-(-need // 4),), torch.float32)
+    need = _recurrence_scratch_bytes(module, entry, *sizes) if ws is not None and n_long != 0 else 0
+    records = ws.try_get("scan.records", (-(-need // 4),), torch.float32) if need > 0 else None
     if records is None:
-        return c_void_p(0), ctypes.c_longlong(0)
-    return _p(records), ctypes.c_longlong(need)
+        return c_int(n_long), c_void_p(0), ctypes.c_longlong(0)
+    return c_int(n_long), _p(records), ctypes.c_longlong(need)
 
 
 def _count_kernels(launched: c_int) -> None:
@@ -943,7 +956,7 @@ def _count_kernels(launched: c_int) -> None:
 
 
 def wkv_scan(rkvg, dlog, w0, u, state, prev_off: int, x, ctx, o, heads: int, dim: int) -> None:
-    """The recurrence, token by token or (bfloat16 prompts, with ``ctx.workspace`` for scratch memory) a chunk of tokens at a time.  rkvg [4,T,heads*dim] (r, k, v, gate
+    """The recurrence, token by token or (bfloat16 sequences long enough for it, with ``ctx.workspace`` for scratch memory) a chunk of tokens at a time.  rkvg [4,T,heads*dim] (r, k, v, gate
     projections; the gate is not read here), dlog float32 [T,heads*dim] (the decay's inner logarithm without
     its offset w0), state float32 [slots, prev_off + W] with prev_off >= heads * wkv_state_dim(dim)^2 (read unless
     the request is fresh, written back in the kernel's own order, the portion's last row of x saved at prev_off),
@@ -955,7 +968,7 @@ def wkv_scan(rkvg, dlog, w0, u, state, prev_off: int, x, ctx, o, heads: int, dim
     assert o.shape == (T, HD) and o.dtype == torch.float32 and state.dtype == torch.float32
     assert w0.dtype == u.dtype == torch.float32 and w0.numel() == HD and u.numel() == HD
     assert state.shape[1] >= prev_off + W and prev_off >= heads * wkv_state_dim(dim) ** 2
-    scratch = _recurrence_scratch(ctx, "wkv", "ff_wkv_scratch_bytes", _dt(rkvg), T, ctx.num_seqs, heads, dim,
+    scratch = _recurrence_scratch(ctx, "wkv", "ff_wkv_scratch_bytes", _chunk_min("wkv", "ff_wkv_chunk_min"), _dt(rkvg), T, ctx.num_seqs, heads, dim,
                                   _row_bits((rkvg, 0), (dlog, 0)))
     launched = c_int(0)
     _check(_lib("wkv").ff_wkv_scan(_p(rkvg), c_int(_dt(rkvg)), _p(dlog), _p(w0), _p(u), _p(state),
@@ -1476,7 +1489,7 @@ def delta_state_floats(heads: int, N: int, V: int) -> int:
 def delta_rule_scan(q, k, v, beta, a, dt_bias: torch.Tensor, a_log: torch.Tensor, state: torch.Tensor, state_off: int,
                     ctx, o: torch.Tensor, heads: int, N: int, V: int, *, heads_per_group: int = 1, q_scale: float = 1.0,
                     unit_eps: float = 1e-6, decay_per_head: bool = False) -> None:
-    """S = diag(g) S; u = beta (v - S^T k); S += k u^T; o = S^T q per head, token by token or (bfloat16 prompts, with
+    """S = diag(g) S; u = beta (v - S^T k); S += k u^T; o = S^T q per head, token by token or (bfloat16 sequences long enough for it, with
     ``ctx.workspace`` for scratch memory) a chunk of tokens at a time.  ``q``, ``k``, ``v``,
     ``beta``, ``a``: (matrix [T, *], first column); a q/k row holds [groups, N] (made unit vectors here, q also times
     ``q_scale``), a v row [heads, V], a beta row [heads] (its sigmoid is taken here), an ``a`` row float32
@@ -1491,7 +1504,7 @@ def delta_rule_scan(q, k, v, beta, a, dt_bias: torch.Tensor, a_log: torch.Tensor
     assert dt_bias.dtype == a_log.dtype == torch.float32 and a_log.numel() == heads
     assert dt_bias.numel() == (heads if decay_per_head else heads * N)
     assert o.dtype == torch.float32 and o.shape == (T, heads * V) and state.dtype == torch.float32
-    scratch = _recurrence_scratch(ctx, "delta_rule", "ff_delta_scratch_bytes", _dt(qm), T, ctx.num_seqs, heads, N, V,
+    scratch = _recurrence_scratch(ctx, "delta_rule", "ff_delta_scratch_bytes", _chunk_min("delta_rule", "ff_delta_chunk_min"), _dt(qm), T, ctx.num_seqs, heads, N, V,
                                   _row_bits((qm, q0), (km, k0), (vm, v0), *(() if decay_per_head else ((am, a0),))))
     launched = c_int(0)
     _check(_lib("delta_rule").ff_delta_rule_scan(
@@ -1522,8 +1535,8 @@ def head_norm_gate(o: torch.Tensor, gate, weight: torch.Tensor, eps: float, y: t
 def scalar_decay_scan(q, k, v, state: torch.Tensor, state_off: int, ctx, o: torch.Tensor, heads: int, N: int, V: int, *,
                       heads_per_group: int = 1, silu_inputs: bool = False, decay: Optional[torch.Tensor] = None,
                       step=None, step_bias=None, a_log=None, skip=None, channel_decay=None, q_scale: float = 1.0) -> None:
-    """S = a S + b k v^T, o = S^T q (+ skip * v) per head, token by token or (bfloat16 prompts, with ``ctx.workspace`` for scratch
-    memory) a chunk of tokens at a time.
+    """S = a S + b k v^T, o = S^T q (+ skip * v) per head, token by token or (bfloat16 sequences long enough for it, with
+    ``ctx.workspace`` for scratch memory) a chunk of tokens at a time.
     ``q``, ``k``, ``v``: (matrix [T, *], first column); a q/k row holds [groups, N], a v row [heads, V].
     Either ``decay`` float32 [heads] (a constant, b = 1), ``channel_decay`` = (float32 matrix, first column) whose rows
     hold [heads, N] decays (S = diag(a) S + k v^T), or ``step`` = (matrix, first column) with ``step_bias``,
@@ -1543,7 +1556,7 @@ def scalar_decay_scan(q, k, v, state: torch.Tensor, state_off: int, ctx, o: torc
     sm, s0 = step if step is not None else (None, 0)
     if mode == 1:
         assert sm.dtype == qm.dtype and step_bias is not None and a_log is not None
-    scratch = _recurrence_scratch(ctx, "ssm", "ff_scan_scratch_bytes", _dt(qm), mode, 1 if silu_inputs else 0, T, ctx.num_seqs, heads,
+    scratch = _recurrence_scratch(ctx, "ssm", "ff_scan_scratch_bytes", _chunk_min("ssm", "ff_scan_chunk_min", mode), _dt(qm), mode, 1 if silu_inputs else 0, T, ctx.num_seqs, heads,
                                   heads_per_group, N, V, _row_bits((qm, q0), (km, k0), (vm, v0), *(((cm, cd0),) if mode == 2 else ())))
     launched = c_int(0)
     _check(_lib("ssm").ff_scalar_decay_scan(

@@ -17,13 +17,14 @@ from firefly_b200.ops import kernels as K
 
 pytestmark = pytest.mark.gpu
 BF = torch.bfloat16
-LENS = [(15, 16, 17, 400), (31, 32, 33, 330), (1, 260), (112, 128, 144)]
+# ends around chunks of 16 and 32; around the shortest length that goes by chunks, 24 to 64; all of them by chunks
+LENS = [(15, 16, 17, 400), (31, 32, 33, 330), (1, 260), (112, 128, 144), (23, 24, 25, 47, 48, 49, 63, 64, 65)]
 
 
 def _ctx(lens, fresh):
     n = len(lens)
     cu = torch.tensor([0, *torch.tensor(lens).cumsum(0).tolist()], dtype=torch.int32, device="cuda")
-    return SimpleNamespace(cu_q=cu, num_seqs=n, state_slots=torch.arange(n, 0, -1, dtype=torch.int32, device="cuda"),
+    return SimpleNamespace(cu_q=cu, num_seqs=n, q_lens=list(lens), state_slots=torch.arange(n, 0, -1, dtype=torch.int32, device="cuda"),
                            seq_fresh=torch.full((n,), fresh, dtype=torch.int32, device="cuda"), workspace=Workspace("cuda"))
 
 
@@ -46,13 +47,13 @@ def _walk(q, k, v, decay, beta=None, bonus=None, S=None):
     return o, S
 
 
-def _check(call, inputs, lens, heads, V, T, bonus=None):
+def _check(call, inputs, lens, heads, V, T, chunk_min, bonus=None):
     """A step of prompts on fresh slots, then one of single tokens behind them, against `_walk`."""
     n, tol = len(lens), 2.0 ** -24 * (32 + max(lens))
     o, o1 = torch.empty(T, heads * V, device="cuda"), torch.empty(n, heads * V, device="cuda")
     before = K.LAUNCHES
     call(0, T, _ctx(lens, 1), o)
-    assert K.LAUNCHES == before + 2                        # the chunks' two kernels ran
+    assert K.LAUNCHES - before == 2 * (max(lens) >= chunk_min) + (min(lens) < chunk_min)      # two kernels for chunks, one that walks
     call(T, T + n, _ctx([1] * n, 0), o1)                   # token by token, from the state that the chunks left
     at = 0
     for i, L in enumerate(lens):
@@ -105,7 +106,7 @@ def test_decay_scans(lens, N, V, heads, groups, mode):
         if mode == "constant":
             return q, k, v, const.double()[None, :, None].expand_as(k)
         return q * 0.125, k, v, alpha[a:b].view(b - a, heads, N)
-    _check(call, inputs, lens, heads, V, T)
+    _check(call, inputs, lens, heads, V, T, K._lib("ssm").ff_scan_chunk_min(2 if mode == "channel" else 0))
 
 
 @pytest.mark.parametrize("lens", LENS)
@@ -125,7 +126,7 @@ def test_wkv_scan(lens, dim, heads):
     def inputs(a, b):
         r = (rkvg[:, a:b] if a < T else rkvg1[:, a - T:b - T]).reshape(4, b - a, heads, dim)
         return r[0], r[1], r[2], torch.exp(-torch.exp(dlog[a:b].double() + w0.double())).view(b - a, heads, dim)
-    _check(call, inputs, lens, heads, dim, T, bonus=u.view(heads, dim))
+    _check(call, inputs, lens, heads, dim, T, K._lib("wkv").ff_wkv_chunk_min(), bonus=u.view(heads, dim))
 
 
 @pytest.mark.parametrize("lens", LENS)
@@ -151,7 +152,7 @@ def test_delta_rule_scan(lens, N, V, heads, per_group, per_head):
         s = F.softplus(a_raw[a:b].double() + bias.double(), threshold=1e9).view(b - a, heads, -1).expand(b - a, heads, N)
         return (q * N ** -0.5, k, xx[:, 2 * G * N:].view(b - a, heads, V), torch.exp(-torch.exp(a_log.double())[None, :, None] * s),
                 torch.sigmoid(beta[a:b].double()))
-    _check(call, inputs, lens, heads, V, T)
+    _check(call, inputs, lens, heads, V, T, K._lib("delta_rule").ff_delta_chunk_min())
 
 
 @pytest.mark.parametrize("bad", [math.nan, math.inf])
@@ -264,3 +265,39 @@ def test_rows_off_a_boundary_are_walked_without_scratch_memory():
             call()
             assert K.LAUNCHES - before == kernels and (ctx.workspace.bytes() > 0) == (kernels == 2)
             ctx.workspace = Workspace("cuda")
+
+
+@pytest.mark.parametrize("kind", ["step", "channel", "wkv", "delta"])
+@pytest.mark.parametrize("lens", [[1] * 24 + [256, 200], [30, 20, 500, 70, 1], [64] * 40])
+@pytest.mark.parametrize("known", [True, False])
+def test_company_changes_nothing(kind, lens, known):
+    """A sequence's outputs and state are bit for bit those of the sequence alone in a step, beside single tokens or beside prompts,
+    whether the host knows the lengths or not."""
+    rn = _rand(7)
+    H, N, V, T = 4, 64, 64, sum(lens)
+    x, beta, raw = rn(T, (2 * N + V) * H).to(BF), rn(T, H).to(BF), rn(T, H * N)
+    alpha, one, many = torch.sigmoid(4 * raw), rn(H), rn(H * N)
+    start = rn(len(lens) + 1, H * V * N + 8)
+
+    def step(a, b, step_lens, state):
+        ctx, o = _ctx(step_lens, 0), torch.zeros(b - a, H * V, device="cuda")
+        if not known:
+            del ctx.q_lens
+        q, k, v = ((x[a:b], i * H * N) for i in range(3))
+        if kind == "step":
+            K.scalar_decay_scan(q, k, v, state, 0, ctx, o, H, N, V, step=(beta[a:b], 0), step_bias=one, a_log=one, skip=one)
+        elif kind == "channel":
+            K.scalar_decay_scan(q, k, v, state, 0, ctx, o, H, N, V, channel_decay=(alpha[a:b], 0))
+        elif kind == "wkv":
+            rkvg = torch.stack([x[a:b, i * H * N:(i + 1) * H * N] for i in (0, 1, 2, 0)]).contiguous()
+            K.wkv_scan(rkvg, raw[a:b], many, many, state, H * N * N, x[a:b, :8].contiguous(), ctx, o, H, N)
+        else:
+            K.delta_rule_scan(q, k, v, (beta[a:b], 0), (raw[a:b], 0), many, one, state, 0, ctx, o, H, N, V)
+        return o
+
+    together = start.clone()
+    o, at = step(0, T, lens, together), 0
+    for i, L in enumerate(lens):
+        alone = start[len(lens) - i - 1:len(lens) - i + 1].clone()       # the sequence's slot is the second of two
+        assert torch.equal(step(at, at + L, [L], alone), o[at:at + L]) and torch.equal(alone[1], together[len(lens) - i])
+        at += L

@@ -25,7 +25,7 @@ class _Small(Workspace):
 
 def _scratch(ws, monkeypatch, numbers):
     monkeypatch.setattr(K, "_recurrence_scratch_bytes", lambda *a: 4 * numbers)
-    p, size = K._recurrence_scratch(SimpleNamespace(workspace=ws), "ssm", "ff_scan_scratch_bytes")
+    _, p, size = K._recurrence_scratch(SimpleNamespace(workspace=ws), "ssm", "ff_scan_scratch_bytes", 32)
     assert (p.value is None) == (size.value == 0)
     return size.value // 4
 
@@ -61,3 +61,15 @@ def test_a_frozen_workspace_answers_none(monkeypatch):
     ws.frozen = True
     assert _scratch(ws, monkeypatch, 60) == 0 and _scratch(ws, monkeypatch, 50) == 50 and _scratch(ws, monkeypatch, 40) == 40
     assert ws.asked == [50]
+
+
+def test_no_long_sequence_no_scratch_memory(monkeypatch):
+    """What goes by chunks is counted from the host's copy of the lengths, once a step; a step without such a sequence asks for nothing."""
+    monkeypatch.setattr(K, "_recurrence_scratch_bytes", lambda *a: 40)
+    for lens, n_long in (([1, 1, 31], 0), ([1, 32, 500], 2), (None, -1)):
+        ws = _Small(100)
+        ctx = SimpleNamespace(workspace=ws, q_lens=lens, memo={})
+        for _ in range(2):
+            n, p, size = K._recurrence_scratch(ctx, "ssm", "ff_scan_scratch_bytes", 32)
+            assert n.value == n_long and size.value == (0 if n_long == 0 else 40) and len(ws.asked) == (n_long != 0)
+            assert lens is None or ctx.memo[("long_seqs", 32)] == n_long
