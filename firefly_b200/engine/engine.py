@@ -193,9 +193,16 @@ class Engine:
         """Bytes to leave for the scratch memory of the largest step and the library's own: activations
         of ``max_num_batched_tokens`` tokens (about 64 bytes per token and hidden unit covers the
         residual, the projections and a feed-forward four times as wide), logits of every request in
-        32-bit twice (eager and captured), and half a gigabyte for the matrix library's workspaces."""
+        32-bit twice (eager and captured), what the recurrences keep of a step's chunks (for the longest step, and once more for the
+        longest one that is captured, which has a workspace of its own), and half a gigabyte for the matrix library's workspaces."""
         spec = self.model.spec
-        return (opts.max_num_batched_tokens * spec.hidden_size * 64
+        tokens, n = opts.max_num_batched_tokens, opts.max_batch_size_limit
+        recurrences = getattr(self.model, "step_scratch_bytes", lambda *_: 0)
+        records = recurrences(tokens, n)
+        if opts.use_cuda_graphs and opts.capture_repeating_steps:
+            from .graphs import DecodeGraphs
+            records += recurrences(min(tokens, DecodeGraphs.SHAPE_MAX_TOKENS), n)
+        return (tokens * spec.hidden_size * 64 + records
                 + 2 * opts.max_batch_size_limit * spec.vocab_size * 4 + (512 << 20))
 
     # ---- the reference's interface ----------------------------------------------

@@ -13,7 +13,7 @@ import torch
 from ..cache.spec import filter_slot, sub_slot
 from ..config.base import ModelSpec
 from ..parts import Runtime, build_part, part_class
-from ..parts.base import declared, host_synchronous
+from ..parts.base import declared, host_synchronous, step_scratch_bytes
 from ..weights.loader import WeightSpec
 
 
@@ -101,6 +101,10 @@ class DecoderModel:
                     raise ValueError(f"layer {layer} reads cache slot {slot}, whose shape "
                                      f"{whole.get(slot)} is not what it needs ({want})")
         return out
+
+    def step_scratch_bytes(self, tokens: int, sequences: int) -> int:
+        """Scratch memory beyond activations that a step of so many tokens and sequences takes (`Part.step_scratch_bytes`)."""
+        return max((step_scratch_bytes(b, tokens, sequences) for b in self.blocks), default=0)
 
     # -- run ------------------------------------------------------------------
     def forward(self, ctx) -> torch.Tensor:

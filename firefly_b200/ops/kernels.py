@@ -949,6 +949,11 @@ def _recurrence_scratch(ctx, module: str, entry: str, chunk_min: int, *sizes: in
     return c_int(n_long), _p(records), ctypes.c_longlong(need)
 
 
+def wkv_scratch_bytes(dtype: torch.dtype, tokens: int, sequences: int, heads: int, dim: int) -> int:
+    """Scratch memory that `wkv_scan` takes for a step that has a sequence long enough for chunks."""
+    return _recurrence_scratch_bytes("wkv", "ff_wkv_scratch_bytes", _DT[dtype], tokens, sequences, heads, dim, 0)
+
+
 def _count_kernels(launched: c_int) -> None:
     """``launched``: how many kernels a recurrence's entry put on the stream; the call itself is counted as one."""
     global LAUNCHES
@@ -1355,6 +1360,14 @@ def scan_state_floats(heads: int, N: int, V: int) -> int:
     return heads * V * scan_key_size(N, V)
 
 
+def scan_scratch_bytes(dtype: torch.dtype, tokens: int, sequences: int, heads: int, heads_per_group: int, N: int, V: int, *,
+                       channel_decay: bool) -> int:
+    """Scratch memory that `scalar_decay_scan` (inputs read as they are; ``channel_decay``: a decay per key channel) takes for a step that
+    has a sequence long enough for chunks."""
+    return _recurrence_scratch_bytes("ssm", "ff_scan_scratch_bytes", _DT[dtype], 2 if channel_decay else 1, 0, tokens, sequences, heads,
+                                     heads_per_group, N, V, 0)
+
+
 def scan_state_floats_of_kernel(heads: int, N: int, V: int) -> int:
     fn = _lib("ssm").ff_scan_state_floats
     fn.restype = ctypes.c_longlong
@@ -1474,6 +1487,11 @@ def delta_state_floats_plan(heads: int, N: int, V: int) -> int:
     if not (0 < N <= 256 and 0 < V <= 256):
         raise KernelError(f"delta rule: key size {N} / value size {V} not supported (up to 256 each)")
     return heads * V * scan_key_size(N, V)
+
+
+def delta_scratch_bytes(dtype: torch.dtype, tokens: int, sequences: int, heads: int, N: int, V: int) -> int:
+    """Scratch memory that `delta_rule_scan` takes for a step that has a sequence long enough for chunks."""
+    return _recurrence_scratch_bytes("delta_rule", "ff_delta_scratch_bytes", _DT[dtype], tokens, sequences, heads, N, V, 0)
 
 
 def delta_state_floats(heads: int, N: int, V: int) -> int:

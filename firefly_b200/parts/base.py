@@ -129,6 +129,14 @@ def host_synchronous(part) -> bool:
     return any(host_synchronous(p) for p in inner()) if callable(inner) else False
 
 
+def step_scratch_bytes(part, tokens: int, sequences: int) -> int:
+    """The most that `Part.step_scratch_bytes` gives for ``part`` and the parts it holds: they run one behind the other on one buffer."""
+    own = getattr(part, "step_scratch_bytes", None)
+    inner = getattr(part, "parts", None)
+    return max([int(own(tokens, sequences)) if callable(own) else 0]
+               + [step_scratch_bytes(p, tokens, sequences) for p in (inner() if callable(inner) else ())])
+
+
 @dataclass
 class Runtime:
     """The surroundings a part may use: where it runs and in which type."""
@@ -180,6 +188,11 @@ class Part:
         hands it to ``bind`` under its name; a part must still be able to bind from the plain
         sources (tensors made by hand)."""
         return []
+
+    def step_scratch_bytes(self, tokens: int, sequences: int) -> int:
+        """Scratch memory beyond activations that a step of so many tokens and sequences takes if it is there (a recurrence's records
+        of chunks, `scan.records`); the engine leaves room for it when it sizes the cache."""
+        return 0
 
     def bind(self, tensors: Mapping[str, torch.Tensor]) -> None:
         pass

@@ -78,6 +78,9 @@ class ChannelDeltaMixer(Part):
     def cache_spec(self):
         return StateSpec((self.state_floats + (self.taps - 1) * self.C,), torch.float32)
 
+    def step_scratch_bytes(self, tokens: int, sequences: int) -> int:
+        return K.delta_scratch_bytes(self.rt.dtype, tokens, sequences, self.H, self.D, self.V)
+
     def _wide(self):
         n = self.name
         return [(n("q"), self.GD), (n("k"), self.GD), (n("v"), self.HV), (n("b"), self.H)]

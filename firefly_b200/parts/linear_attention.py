@@ -126,6 +126,9 @@ class GatedLinearAttention(Part):
     def cache_spec(self):
         return StateSpec((self.state_floats,), torch.float32)
 
+    def step_scratch_bytes(self, tokens: int, sequences: int) -> int:
+        return K.scan_scratch_bytes(self.rt.dtype, tokens, sequences, self.heads, 1, self.dim, self.vdim, channel_decay=True)
+
     def _sources(self):
         n = self.name
         return [(n("q"), self.kq), (n("k"), self.kq), (n("v"), self.kv), (n("g"), self.kv), (n("a1"), self.rank)]

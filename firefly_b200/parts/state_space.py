@@ -57,6 +57,9 @@ class StateSpaceMixer(Part):
     def cache_spec(self):
         return StateSpec((self.scan_floats + (self.taps - 1) * self.channels,), torch.float32)
 
+    def step_scratch_bytes(self, tokens: int, sequences: int) -> int:
+        return K.scan_scratch_bytes(self.rt.dtype, tokens, sequences, self.heads, self.heads // self.groups, self.N, self.vdim, channel_decay=False)
+
     def weight_specs(self) -> List[WeightSpec]:
         n = self.name
         return [WeightSpec(n("in"), (self.proj_width, self.hidden)),

@@ -54,6 +54,9 @@ class WKVMixer(Part):
     def cache_spec(self):
         return StateSpec((self.prev_off + self.hidden,), torch.float32)
 
+    def step_scratch_bytes(self, tokens: int, sequences: int) -> int:
+        return K.wkv_scratch_bytes(self.rt.dtype, tokens, sequences, self.heads, self.dim)
+
     def weight_specs(self) -> List[WeightSpec]:
         n, W, hd = self.name, self.hidden, self.hd
         out = [WeightSpec(n(f"mu.{s}"), (W,), init="norm", as_float32=True) for s in "rkvgw"]

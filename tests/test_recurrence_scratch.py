@@ -1,12 +1,18 @@
 """The scratch memory that the recurrences over prompts can do without (`Workspace.try_get`, `ops/kernels.py: _recurrence_scratch`):
-what happens where the device refuses it, in a run that sizes the buffers and in the capture behind it."""
+what happens where the device refuses it, in a run that sizes the buffers and in the capture behind it, and that the engine leaves
+room for it."""
 from types import SimpleNamespace
 
 import pytest
 import torch
 
+from firefly_b200.config.base import PartSpec
 from firefly_b200.engine.context import Workspace
+from firefly_b200.engine.engine import Engine, EngineOptions
+from firefly_b200.engine.graphs import DecodeGraphs
+from firefly_b200.models.decoder import DecoderModel
 from firefly_b200.ops import kernels as K
+from firefly_b200.parts.base import Runtime, build_part
 
 
 class _Small(Workspace):
@@ -73,3 +79,51 @@ def test_no_long_sequence_no_scratch_memory(monkeypatch):
             n, p, size = K._recurrence_scratch(ctx, "ssm", "ff_scan_scratch_bytes", 32)
             assert n.value == n_long and size.value == (0 if n_long == 0 else 40) and len(ws.asked) == (n_long != 0)
             assert lens is None or ctx.memo[("long_seqs", 32)] == n_long
+
+
+class _Holder:
+    def __init__(self, *parts):
+        self._parts = parts
+
+    def parts(self):
+        return list(self._parts)
+
+
+def test_the_engine_leaves_room_for_the_records():
+    """The largest of a model's parts counts, wherever it stands, for the longest step and for the longest captured one."""
+    mixer = lambda scale: SimpleNamespace(step_scratch_bytes=lambda tokens, n: scale * (tokens + n))  # noqa: E731
+    model = SimpleNamespace(blocks=[_Holder(object(), mixer(3)), _Holder(_Holder(mixer(7)), mixer(5)), object()],
+                            spec=SimpleNamespace(hidden_size=16, vocab_size=100))
+    model.step_scratch_bytes = lambda tokens, n: DecoderModel.step_scratch_bytes(model, tokens, n)
+    plain = SimpleNamespace(spec=model.spec)
+    opts = EngineOptions(max_num_batched_tokens=8000, max_batch_size_limit=10)
+    estimate = lambda m, o: Engine._scratch_estimate(SimpleNamespace(model=m), o)  # noqa: E731
+    assert estimate(model, opts) - estimate(plain, opts) == 7 * 8010 + 7 * (DecodeGraphs.SHAPE_MAX_TOKENS + 10)
+    opts.use_cuda_graphs = False
+    assert estimate(model, opts) - estimate(plain, opts) == 7 * 8010
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["wkv", "state_space", "channel_delta", "gated_linear_attention", "linear_attention"])
+def test_a_mixer_says_what_its_recurrence_takes(kind):
+    H, N, lens = 4, 64, [300, 1, 70]
+    T, n, bf = sum(lens), len(lens), torch.bfloat16
+    params = dict(hidden_size=256, eps=1e-6, heads=H, dim=N)
+    params.update({"wkv": dict(decay_rank=8), "state_space": dict(vdim=N, state=N, conv=4), "linear_attention": dict(decay=[0.9] * H),
+                   "gated_linear_attention": dict(decay_rank=8, tau=16.0), "channel_delta": dict(kv_heads=H, vdim=N, conv=4)}[kind])
+    part = build_part("mixer", PartSpec(kind, params), Runtime(torch.device("cuda"), bf))
+    x = torch.randn(T, 4 * H * N, device="cuda").to(bf)
+    f = lambda *s: torch.randn(*s, device="cuda")  # noqa: E731
+    cu = torch.tensor([0, 300, 301, 371], dtype=torch.int32, device="cuda")
+    ctx = SimpleNamespace(cu_q=cu, num_seqs=n, q_lens=lens, workspace=Workspace("cuda"), memo={},
+                          state_slots=torch.arange(1, n + 1, dtype=torch.int32, device="cuda"), seq_fresh=torch.ones(n, dtype=torch.int32, device="cuda"))
+    state, o, q, k, v = f(n + 1, H * N * N + 256), f(T, H * N), (x, 0), (x, H * N), (x, 2 * H * N)
+    if kind == "wkv":
+        K.wkv_scan(x.view(T, 4, H * N).transpose(0, 1).contiguous(), f(T, H * N), f(H * N), f(H * N), state, H * N * N, x[:, :256].contiguous(), ctx, o, H, N)
+    elif kind == "channel_delta":
+        K.delta_rule_scan(q, k, v, (x, 0), (f(T, H * N), 0), f(H * N), f(H), state, 0, ctx, o, H, N, N)
+    else:
+        kw = {"state_space": dict(step=(x, 0), step_bias=f(H), a_log=f(H), heads_per_group=H), "linear_attention": dict(decay=f(H), silu_inputs=True),
+              "gated_linear_attention": dict(channel_decay=(torch.rand(T, H * N, device="cuda"), 0))}[kind]
+        K.scalar_decay_scan(q, k, v, state, 0, ctx, o, H, N, N, **kw)
+    assert part.step_scratch_bytes(T, n) == ctx.workspace.bytes() and (ctx.workspace.bytes() > 0) == (kind != "linear_attention")
