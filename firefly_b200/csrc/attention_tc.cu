@@ -13,7 +13,7 @@
 //                  MMA's N-major operand form), O (128 x D, float32) in tensor memory.
 // One warp starts the TMA copies, a page and panel per lane (K and V have two stages each, freed
 // separately); one warp issues the MMAs, converged, with the issuing lane predicated; two blocks
-// share an SM (at head size 128).  Portions with enough row tiles, at head sizes of 64 and 128, take two
+// share an SM (at head size 128).  Portions with enough row tiles and keys, at head sizes of 64 and 128, take two
 // row tiles a block and tiles of 128 keys instead (attn_tc_pair_kernel below).
 //
 // It replaces, for head sizes that are multiples of 64 and page sizes that divide 64, the
@@ -672,10 +672,6 @@ attn_tc_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __restri
 // anew in 64 bits: 537.
 #define FF_ATC_PAIR (FF_HEAD_DIM <= 128)
 #if FF_ATC_PAIR
-// From this many row tiles (times kv heads) on, a pair for every SM, row tiles go in pairs.  Below it pairs leave SMs idle: us
-// for one prompt, two tiles a block / one: 1024 tokens (256 tiles) 30.8 / 34.6 and 28.4 / 28.4 at best, 640 tokens (160) 22.4 / 20.6,
-// 384 (96) 18.5 / 14.6.
-constexpr long long PAIR_MIN_TILES = 2 * 148;
 constexpr int PN = 128;                              // keys per tile
 constexpr int PAIR_ROWS = 2 * BM;
 constexpr int PAIR_SLOTS = 5;                        // ring of K and V tiles: K0, V0, K1, V1, ...
@@ -1122,11 +1118,13 @@ FF_EXPORT int ff_attn_tc_block_m() { return BM; }
 // results in part_o (float [tokens * nq * num_splits * D]) and part_ml (float [tokens * nq * num_splits * 2]),
 // indexed by the token's row in q/out; a second kernel joins them for the n_tokens rows from tok_base on
 // (the rows of the sequences given here).
+// two_tiles: two row tiles a block where that kernel takes the call (heads of 64 and 128, one share, neither bias nor cap), as the caller
+// finds it faster.
 FF_EXPORT int ff_attn_tc(const void* q, int q_stride, const void* cache, const int* block_table, int max_blocks,
                          const int* cu_q, const int* ctx_lens, int n_seqs, int total_tiles, void* out,
                          int out_stride, int nq, int nkv, int block_size, int num_blocks, float scale, int window,
                          int* status, int num_splits, float* part_o, float* part_ml, int tok_base, int n_tokens,
-                         const float* dist_bias, int bias_len, float softcap, const float* sink, cudaStream_t stream) {
+                         const float* dist_bias, int bias_len, float softcap, const float* sink, int two_tiles, cudaStream_t stream) {
     if (n_seqs <= 0 || total_tiles <= 0) return 0;
     if (nkv <= 0 || nq % nkv || (dist_bias && (window <= 0 || bias_len < window))) return FF_ERR_BAD_ARG;
     if (num_splits < 1 || (num_splits > 1 && (!part_o || !part_ml || n_tokens <= 0 || tok_base < 0))) return FF_ERR_BAD_ARG;
@@ -1144,7 +1142,7 @@ FF_EXPORT int ff_attn_tc(const void* q, int q_stride, const void* cache, const i
     std::memcpy(arg.bytes, &map, sizeof(map));
 #if FF_ATC_PAIR
     const long long pairs = (((long long)total_tiles + n_seqs) / 2) * nkv;    // at least ceil(row tiles of a sequence / 2), summed
-    if (num_splits == 1 && !dist_bias && softcap == 0.f && (long long)total_tiles * nkv >= PAIR_MIN_TILES && pairs < (1ll << 31)) {
+    if (two_tiles && num_splits == 1 && !dist_bias && softcap == 0.f && pairs < (1ll << 31)) {
         FF_SMEM_LIMIT(attn_tc_pair_kernel, PAIR_SMEM);
         FF_LAUNCH((attn_tc_pair_kernel), dim3((unsigned)pairs), PAIR_THREADS, PAIR_SMEM, stream, arg, (const bf16*)q, q_stride,
                   block_table, max_blocks, cu_q, ctx_lens, n_seqs, (bf16*)out, out_stride, nq, nkv, block_size, num_blocks,

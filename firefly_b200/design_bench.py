@@ -152,7 +152,7 @@ def kernel_table(width: int, ff: int, batch: int, prompt: int, peaks: dict) -> l
     hd = heads * dim
     for label, n_seqs, q in (("prefill", batch, prompt), ("decode", batch * 8, 1)):
         T = n_seqs * q
-        ctx = SimpleNamespace(cu_q=torch.arange(0, T + 1, q, dtype=torch.int32, device=dev), num_seqs=n_seqs,
+        ctx = SimpleNamespace(cu_q=torch.arange(0, T + 1, q, dtype=torch.int32, device=dev), num_seqs=n_seqs, q_lens=[q] * n_seqs, workspace=Workspace(dev),
                               state_slots=torch.arange(1, n_seqs + 1, dtype=torch.int32, device=dev),
                               seq_fresh=torch.zeros(n_seqs, dtype=torch.int32, device=dev))
         state = torch.zeros(n_seqs + 1, hd * dim + width, dtype=torch.float32, device=dev)
@@ -222,7 +222,7 @@ def pepolorn_kernel_table(width: int, ff: int, batch: int, prompt: int, peaks: d
     P_ = 2 * inner + 2 * G * N + heads
     for label, n_seqs, q in (("prefill", batch, prompt), ("decode", batch * 8, 1)):
         T = n_seqs * q
-        ctx = SimpleNamespace(cu_q=torch.arange(0, T + 1, q, dtype=torch.int32, device=dev), num_seqs=n_seqs,
+        ctx = SimpleNamespace(cu_q=torch.arange(0, T + 1, q, dtype=torch.int32, device=dev), num_seqs=n_seqs, q_lens=[q] * n_seqs, workspace=Workspace(dev),
                               token_seq=torch.arange(T, dtype=torch.int32, device=dev) // q,
                               positions=(torch.arange(T, dtype=torch.int32, device=dev) % q) + (0 if q > 1 else 2048),
                               state_slots=torch.arange(1, n_seqs + 1, dtype=torch.int32, device=dev),
@@ -372,7 +372,7 @@ def kefisun_kernel_table(width: int, batch: int, prompt: int, peaks: dict) -> li
     for label, n_seqs, q, ctx_len in (("prefill", batch, prompt, 0), ("decode", batch * 8, 1, prompt)):
         T = n_seqs * q
         per = -(-(q + ctx_len) // block)
-        ctx = SimpleNamespace(cu_q=torch.arange(0, T + 1, q, dtype=torch.int32, device=dev), num_seqs=n_seqs,
+        ctx = SimpleNamespace(cu_q=torch.arange(0, T + 1, q, dtype=torch.int32, device=dev), num_seqs=n_seqs, q_lens=[q] * n_seqs, workspace=Workspace(dev),
                               token_seq=torch.arange(T, dtype=torch.int32, device=dev) // q,
                               positions=(torch.arange(T, dtype=torch.int32, device=dev) % q) + ctx_len,
                               state_slots=torch.arange(1, n_seqs + 1, dtype=torch.int32, device=dev),
@@ -426,7 +426,7 @@ def kefisun_kernel_table(width: int, batch: int, prompt: int, peaks: dict) -> li
             for name, bt in (("attention tcgen05, window and bias", bias), ("attention tcgen05, window", None)):
                 try:
                     us = _time(lambda: K.attn_tc(qo, H * d, pages, table, ctx.cu_q, ctx_lens, n_seqs, tiles, att, H, G, d, d ** -0.5, window,
-                                                 ctx.status, **({"dist_bias": bt} if bt is not None else {})), flush=flush)
+                                                 ctx.status, two_tiles=K.attn_tc_two_tiles([q] * n_seqs, [0] * n_seqs, H // G, G, window), **({"dist_bias": bt} if bt is not None else {})), flush=flush)
                     add(f"{name} {label}", us, kv_bytes, flops, like=None if bt is None else "attention tcgen05, window")
                 except TypeError:
                     pass
@@ -568,7 +568,7 @@ def papusun_kernel_table(width: int, batch: int, prompt: int, peaks: dict) -> li
     for label, n_seqs, q, ctx_len in (("prefill", batch, prompt, 0), ("decode", batch * 8, 1, prompt)):
         T = n_seqs * q
         per = -(-(q + ctx_len) // block)
-        ctx = SimpleNamespace(cu_q=torch.arange(0, T + 1, q, dtype=torch.int32, device=dev), num_seqs=n_seqs,
+        ctx = SimpleNamespace(cu_q=torch.arange(0, T + 1, q, dtype=torch.int32, device=dev), num_seqs=n_seqs, q_lens=[q] * n_seqs, workspace=Workspace(dev),
                               token_seq=torch.arange(T, dtype=torch.int32, device=dev) // q,
                               positions=(torch.arange(T, dtype=torch.int32, device=dev) % q) + ctx_len,
                               state_slots=torch.arange(1, n_seqs + 1, dtype=torch.int32, device=dev),
@@ -594,7 +594,7 @@ def papusun_kernel_table(width: int, batch: int, prompt: int, peaks: dict) -> li
             tiles = n_seqs * -(-(q * (H // G)) // 128)
             for name, cap in (("attention tcgen05, every key, capped scores", 50.0), ("attention tcgen05, every key", 0.0)):
                 us = _time(lambda: K.attn_tc(qkv, C, pages, table, ctx.cu_q, ctx_lens, n_seqs, tiles, att, H, G, d, d ** -0.5, 0,
-                                             ctx.status, softcap=cap), flush=flush)
+                                             ctx.status, two_tiles=K.attn_tc_two_tiles([q] * n_seqs, [0] * n_seqs, H // G, G, 0), softcap=cap), flush=flush)
                 add(f"{name} {label}", us, kv_bytes, flops, like="attention tcgen05, every key" if cap else None)
         else:
             keys = ctx_len + 1
@@ -644,9 +644,9 @@ def papusun_kernel_table(width: int, batch: int, prompt: int, peaks: dict) -> li
         latt = torch.empty(T, H * ld, dtype=bf, device=dev)
         for name, win in (("latent attention inside a window", window), ("latent attention over every key", 0)):
             keys_seen = sum(min(win or (1 << 30), i + 1 + ctx_len) for i in range(q)) * n_seqs
-            step_ctx = SimpleNamespace(**vars(ctx), ctx_lens=ctx_lens, q_lens=[q] * n_seqs, ctx_lens_host=[ctx_len] * n_seqs,
+            step_ctx = SimpleNamespace(**{**vars(ctx), "workspace": Workspace(dev)}, ctx_lens=ctx_lens, ctx_lens_host=[ctx_len] * n_seqs,
                                        num_decode_seqs=n_seqs if q == 1 else 0, max_kv_len=q + ctx_len, ranges_by_length=False,
-                                       workspace=Workspace(dev), captured=False, memo={}, key_share_level=0)
+                                       captured=False, memo={}, key_share_level=0)
             us = _time(lambda: K.paged_attention(q_full, H * ld, lpages, table, step_ctx, latt, H, 1, ld, 192 ** -0.5, win), flush=flush)
             kv_b = (n_seqs * min(win or (1 << 30), q + ctx_len) * ld * 2 if q == 1 else T * ld * 2) + T * 2 * H * ld * 2
             add(f"{name} {label}", us, kv_b, 2 * keys_seen * H * (ld + rank), like=None if not win else "latent attention over every key")
@@ -732,7 +732,7 @@ def gatutar_kernel_table(width: int, ff: int, batch: int, prompt: int, peaks: di
     for label, n_seqs, q, ctx_len in (("prefill", batch, prompt, 0), ("decode", batch * 8, 1, prompt)):
         T = n_seqs * q
         per = -(-(q + ctx_len) // block)
-        ctx = SimpleNamespace(cu_q=torch.arange(0, T + 1, q, dtype=torch.int32, device=dev), num_seqs=n_seqs,
+        ctx = SimpleNamespace(cu_q=torch.arange(0, T + 1, q, dtype=torch.int32, device=dev), num_seqs=n_seqs, q_lens=[q] * n_seqs,
                               token_seq=torch.arange(T, dtype=torch.int32, device=dev) // q,
                               positions=(torch.arange(T, dtype=torch.int32, device=dev) % q) + ctx_len,
                               state_slots=torch.arange(1, n_seqs + 1, dtype=torch.int32, device=dev),
@@ -764,7 +764,7 @@ def gatutar_kernel_table(width: int, ff: int, batch: int, prompt: int, peaks: di
             tiles = n_seqs * -(-(q * (H // G)) // 128)
             for name, sink in (("attention tcgen05 with a sink", True), ("attention tcgen05", False)):
                 us = _time(lambda: K.attn_tc(qkv, C, pages, table, ctx.cu_q, ctx_lens, n_seqs, tiles, att, H, G, d, d ** -0.5, 0,
-                                             ctx.status, sink=sink), flush=flush)
+                                             ctx.status, two_tiles=K.attn_tc_two_tiles([q] * n_seqs, [0] * n_seqs, H // G, G, 0), sink=sink), flush=flush)
                 add(f"{name} {label}", us, T * (2 * H + 2 * G) * d * 2, flops, like="attention tcgen05" if sink else None)
         else:
             keys = ctx_len + 1
@@ -912,7 +912,7 @@ def mumopel_kernel_table(width: int, ff: int, batch: int, prompt: int, peaks: di
     for label, n_seqs, q, ctx_len in (("prefill", batch, prompt, 0), ("decode", batch * 8, 1, prompt)):
         T = n_seqs * q
         per = -(-(q + ctx_len) // block)
-        ctx = SimpleNamespace(cu_q=torch.arange(0, T + 1, q, dtype=torch.int32, device=dev), num_seqs=n_seqs,
+        ctx = SimpleNamespace(cu_q=torch.arange(0, T + 1, q, dtype=torch.int32, device=dev), num_seqs=n_seqs, q_lens=[q] * n_seqs,
                               token_seq=torch.arange(T, dtype=torch.int32, device=dev) // q,
                               positions=(torch.arange(T, dtype=torch.int32, device=dev) % q) + ctx_len,
                               status=torch.zeros(1, dtype=torch.int32, device=dev), workspace=Workspace(dev))
@@ -938,11 +938,11 @@ def mumopel_kernel_table(width: int, ff: int, batch: int, prompt: int, peaks: di
             tiles = n_seqs * -(-(q * (H // G)) // 128)
             for name, sink, mask in (("attention tcgen05, sinks, chunks", sinks, -MUMOPEL_CHUNK), ("attention tcgen05", None, 0)):
                 us = _time(lambda: K.attn_tc(qkv, C, pages, table, ctx.cu_q, ctx_lens, n_seqs, tiles, att, H, G, d, d ** -0.5, mask,
-                                             ctx.status, sink=sink), flush=flush)
+                                             ctx.status, two_tiles=K.attn_tc_two_tiles([q] * n_seqs, [0] * n_seqs, H // G, G, mask), sink=sink), flush=flush)
                 add(f"{name} {label}", us, T * (2 * H + 2 * G) * d * 2, flops, like="attention tcgen05" if mask else None)
             small = 256                                                          # chunks that bind: what is outside is not walked
             us = _time(lambda: K.attn_tc(qkv, C, pages, table, ctx.cu_q, ctx_lens, n_seqs, tiles, att, H, G, d, d ** -0.5, -small,
-                                         ctx.status, sink=sinks), flush=flush)
+                                         ctx.status, two_tiles=K.attn_tc_two_tiles([q] * n_seqs, [0] * n_seqs, H // G, G, -small), sink=sinks), flush=flush)
             add(f"attention tcgen05, sinks, chunks of {small} {label}", us, T * (2 * H + 2 * G) * d * 2,
                 4 * n_seqs * (-(-q // small)) * (small * (small + 1) // 2) * H * d, like="attention tcgen05")
         else:

@@ -10,7 +10,7 @@ from __future__ import annotations
 import ctypes
 import functools
 from ctypes import c_float, c_int, c_size_t, c_void_p
-from typing import Optional, Union
+from typing import Optional, Sequence, Union
 
 import torch
 
@@ -619,12 +619,14 @@ def tc_attention_supported(dtype: torch.dtype, d: int, block_size: int, max_kv_l
 
 def attn_tc(q, q_stride, pages, table, cu_q, ctx_lens, n_seqs, total_tiles, out, nq, nkv, d, scale, window,
             status, page_list: Optional[int] = None, shares=None, dist_bias: Optional[torch.Tensor] = None,
-            softcap: float = 0.0, sink: Sink = None) -> None:
+            softcap: float = 0.0, sink: Sink = None, two_tiles: bool = False) -> None:
     """tcgen05 flash attention over the paged cache (bfloat16); total_tiles counts row tiles of 128.
     ``shares`` = (count, part_o, part_ml, first row, rows): every row tile's keys are shared out over
     ``count`` blocks and a second kernel joins their partial results (for prompts so short that their
     row tiles alone would leave most SMs idle); the scratch tensors are float32 with at least
-    (first row + rows) * nq * count * d and ... * 2 elements.  ``dist_bias``, ``sink``: as for `paged_attention_simt`."""
+    (first row + rows) * nq * count * d and ... * 2 elements.  ``dist_bias``, ``sink``: as for `paged_attention_simt`.
+    ``two_tiles``: two row tiles a block (`attn_tc_two_tiles`), where the kernel for that takes the call: heads of 64 and 128, no
+    shares, neither bias nor cap."""
     _need_cuda(pages, table, cu_q, ctx_lens, out, status, dist_bias)
     num_blocks, planes, _, block_size, _ = pages.shape
     count, part_o, part_ml, row0, rows = shares if shares is not None else (1, None, None, 0, 0)
@@ -637,7 +639,7 @@ def attn_tc(q, q_stride, pages, table, cu_q, ctx_lens, n_seqs, total_tiles, out,
         c_int(n_seqs), c_int(total_tiles), _p(out), c_int(out.shape[1]), c_int(nq), c_int(nkv),
         c_int(block_size), c_int(num_blocks), c_float(scale), c_int(window), _p(status), c_int(count), _p(part_o),
         _p(part_ml), c_int(row0), c_int(rows), *_bias_args(dist_bias, nq, window), c_float(softcap),
-        _sink_arg(sink, nq), _stream()), "attn_tc")
+        _sink_arg(sink, nq), c_int(1 if two_tiles else 0), _stream()), "attn_tc")
     if count > 1:
         global LAUNCHES
         LAUNCHES += 1     # the kernel that joins the shares
@@ -655,6 +657,26 @@ def attn_tc_shares(total_tiles: int, nkv: int, max_key_tiles: int) -> int:
     if not USE_TC_SHARES or units * 4 >= places * 3 or max_key_tiles < 8:
         return 1
     return max(1, min(8, places // units, max_key_tiles // 4))
+
+
+def attn_tc_two_tiles(q_lens: Sequence[int], ctx_lens: Sequence[int], G: int, nkv: int, window: int = 0) -> bool:
+    """Whether blocks of two row tiles take a step's portions faster than blocks of one: with a pair for every SM at least, and by the
+    two kernels' measured times a block.  With k tiles of 64 keys a row tile walks on average, two blocks of one row tile on an
+    SM take 3 + k and a block of two 5 + 0.8 k (it has the SM for itself, so nothing covers its start and its end, and a
+    sequence's odd row tile leaves half of it idle).  Against 197 measured steps (heads of 128, G = 4; one to 128 sequences of 1 to 8191
+    tokens behind 0 to 2000) the choice loses 6 % at most and 0.1 % on average.  us, one row tile a block / two: one prompt of 2048
+    56.5 / 53.1, of 8191 636 / 564, four of 512 34.3 / 36.5, 64 of 16 19.1 / 40.0, 64 of 64 46 / 62 and behind 2000 tokens 240 / 220."""
+    one = two = pairs = 0.0
+    for q, c in zip(q_lens, ctx_lens):
+        tiles = -(-q * G // 128)
+        keys = c + q / 2
+        if window:
+            keys = min(keys, abs(window) + 64 // G)
+        k = keys / 64 + 0.5
+        pairs += (tiles + 1) // 2
+        one += tiles / 2 * (3 + k)
+        two += (tiles + 1) // 2 * (5 + 0.8 * k)
+    return pairs * nkv >= sm_count() and two < one
 
 
 def decode_splits(n_seqs: int, nkv: int, max_kv_len: int) -> int:
@@ -794,17 +816,22 @@ def paged_attention(q: torch.Tensor, q_stride: int, pages: torch.Tensor, table: 
                 if window:                       # a row tile's tokens and the keys in front of the first of them
                     key_tiles = min(key_tiles, (abs(window) + 128 // G) // 64 + 2)
                 count = attn_tc_shares(tiles, nkv, key_tiles)
-                plan = (tiles, count, sum(ctx.q_lens[:n_dec]), sum(ctx.q_lens[n_dec:]))
+                lens, before = ctx.q_lens[n_dec:], ctx.ctx_lens_host[n_dec:]
+                if ctx.captured:                 # at least what the level says of the longest portion and its context
+                    before = [max(0, 256 * getattr(ctx, "key_share_level", 0) - ql) for ql in lens]
+                two_tiles = count == 1 and attn_tc_two_tiles(lens, before, G, nkv, window)
+                plan = (tiles, count, two_tiles, sum(ctx.q_lens[:n_dec]), sum(lens))
                 if memo is not None:
                     memo[("attn_tc_plan", G, nkv, n_dec, ctx.captured, window)] = plan
-            tiles, count, row0, rows = plan
+            tiles, count, two_tiles, row0, rows = plan
             shares = None
             if count > 1:
                 cells = (row0 + rows) * nq * count
                 shares = (count, ctx.workspace.get("attn.tc_part_o", (cells * d,), torch.float32),
                           ctx.workspace.get("attn.tc_part_ml", (cells * 2,), torch.float32), row0, rows)
             attn_tc(q, q_stride, pages, table_t, cu_q_t, ctx_lens_t, n - n_dec, tiles,
-                    out, nq, nkv, d, scale, window, ctx.status, shares=shares, dist_bias=dist_bias, softcap=softcap, sink=sink)
+                    out, nq, nkv, d, scale, window, ctx.status, shares=shares, dist_bias=dist_bias, softcap=softcap, sink=sink,
+                    two_tiles=two_tiles)
         else:
             tiles = sum(-(-(ql * G) // 64) for ql in ctx.q_lens[n_dec:])
             attn_tiled(q, q_stride, pages, table_t, cu_q_t, ctx_lens_t, n - n_dec,
