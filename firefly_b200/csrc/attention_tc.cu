@@ -483,9 +483,12 @@ attn_tc_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __restri
                 w[e] = exp2_scaled(s[2 * e], s[2 * e + 1], scale2, neg_m2);
                 add_pair(w[e], sum4[(e & 1) * 2], sum4[(e & 1) * 2 + 1]);
             }
-            // Tensor memory is written only between products: the last P V must be complete before P
-            // of this tile is stored (stores issued while it was still running gave wrong sums, although
-            // they go to other columns), and before O is rescaled.  It was issued a whole tile ago.
+            // The last P V must be complete before O is rescaled.  It was issued a whole tile ago.  Every warp waits for
+            // it at every tile, whether it rescales or not: the barrier tells its phases apart by one bit, and a warp
+            // that left one out would take the P V before for the one it waits for (at the end: O read a product too early,
+            // which is what gave wrong sums when the wait stood only in front of a rescale).  P itself may be stored while that
+            // product runs, as it lies in the other buffer: with the wait kept in front of rescales and of the last tile, 300 runs
+            // each of four shapes had the bits of this form.
             if (j > 0) {
                 ok = mb_wait(sa(&bars[B_PV_DONE]), (j - 1) & 1, status, abort_flag);
                 ok = __all_sync(0xffffffffu, ok);
@@ -663,8 +666,8 @@ attn_tc_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __restri
 // What bounded the kernel above was the chain softmax -> P -> P V -> next scores of a block with two blocks an SM, and K and V
 // that every block fetched for itself (a tile's MMAs waited 1100 cycles for them, 26 bytes a cycle and SM from L2); here K and
 // V cross once for 256 rows.  The products of half a tile's keys start when their P is there; the P of a row tile is
-// written while products of the other are running, and a row tile's next scores come behind its P V, so that they also
-// say that O is at rest.  Cycles a tile of 256 x 128: 3700, of which the softmax of a row tile takes 2000 (special-function
+// written while products of the other are running (and its second half while those of its first are: other columns), and a row
+// tile's next scores come behind its P V, so that they also say that O is at rest; every warp waits for every one of them.  Cycles a tile of 256 x 128: 3700, of which the softmax of a row tile takes 2000 (special-function
 // unit 1024), its products with their hand-over 1600 (1024 at the tensor cores' peak); both chains wait for latencies.
 // Measured (us a launch, 32 heads on 8 kv heads of 128, one prompt; before: the kernel above as it was): 8191 tokens 681 -> 525
 // (1.05 PFLOP/s), 2048 tokens 60.5 -> 54.2.  Tried: two threads a row (16 softmax warps): 548 at 8191 tokens, the exponentials of a
