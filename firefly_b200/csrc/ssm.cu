@@ -240,7 +240,7 @@ struct ScanArgs {
 // One block per (sequence, head, VB value columns), token by token (scan_wide.cuh).  A chunk's q, k, v and decays are staged in
 // 32-bit in one of two buffers; the next chunk's are asked for before the current one is walked and staged behind it, so
 // a chunk has one barrier.  CD: mode 2, a decay per key channel (staged beside q and k).
-// This is the kernel for steps of few tokens, for 32-bit inputs, for inputs that pass SiLU (both factors of every product
+// This is the kernel for steps of few tokens, for 32-bit inputs, for constant decays, for inputs that pass SiLU (both factors of every product
 // would have to be split, and on sums that lean to one side, as those of SiLU's do, the tensor cores' cut-off leaves 8e-7 where
 // this one leaves 1e-7) and for sizes that the chunked ones do not take.  Against one column a thread: 758 -> 279 us
 // for three sequences of 1501, 1000 and 700 tokens with 16 heads of 64 x 128, 1256 -> 745 us for 4 x 2048 tokens, SiLU, 8 heads
@@ -369,7 +369,7 @@ __global__ void __launch_bounds__(WS_THREADS) scalar_decay_scan_kernel(
 }
 
 // ------------------------------------------------------------------- the recurrence, a chunk of tokens at a time --
-// Modes 0 and 1 over prompts, bfloat16 inputs that are read as they are.  With L_t the sum of the logarithms of the decays up
+// Mode 1 over prompts, bfloat16 inputs that are read as they are.  With L_t the sum of the logarithms of the decays up
 // to token t of a chunk and S the state in front of it:
 //
 //   P_ts = (q_t . k_s) exp(L_t - L_s) b_s   for s <= t
@@ -417,7 +417,7 @@ __global__ void __launch_bounds__(128) scalar_decay_prepare_kernel(ScanArgs A, S
     pdl_prologue();
     constexpr int QP = NK + 8;
     __shared__ __align__(16) bf16 sq[SC_C * QP], sk[SC_C * QP];
-    __shared__ float lh[4][SC_C], ll[4][SC_C], sb[4][SC_C], pw[4][SC_C + 1];
+    __shared__ float lh[4][SC_C], ll[4][SC_C], sb[4][SC_C];
     int s, chunk;
     chunk_of_record<SC_C>(cu_q, n_seqs, blockIdx.x, min_len, s, chunk);
     if (chunk < 0) return;
@@ -440,39 +440,27 @@ __global__ void __launch_bounds__(128) scalar_decay_prepare_kernel(ScanArgs A, S
     const int mt = warp >> 1, nh = warp & 1;
     float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
     for (int h0 = hb0; h0 < hb1; h0 += 4) {
-        if (h0 + warp < hb1) {              // the decays of a head, one token a lane
+        if (h0 + warp < hb1) {                            // the decays of a head, one token a lane
             const int h = group * A.heads_per_group + h0 + warp;
             ScanRecord* rec = recs + (size_t)blockIdx.x * heads + h;
             const bool in = lane < n;
-            if (A.mode == 1) {
-                const float rate = expf(A.a_log[h]);
-                const float dt = in ? softplus_f(to_float(stepp[(size_t)(row0 + lane) * A.step_stride + h]) + A.step_bias[h]) : 0.f;
-                // at most e^-200 a token: 0 in 32 bits, and the sums stay exact enough to be subtracted from one another
-                double L = in ? (double)(-rate * dt < -200.f ? -200.f : -rate * dt) : 0.0;
+            const float rate = expf(A.a_log[h]);
+            const float dt = in ? softplus_f(to_float(stepp[(size_t)(row0 + lane) * A.step_stride + h]) + A.step_bias[h]) : 0.f;
+            // at most e^-200 a token: 0 in 32 bits, and the sums stay exact enough to be subtracted from one another
+            double L = in ? (double)(-rate * dt < -200.f ? -200.f : -rate * dt) : 0.0;
 #pragma unroll
-                for (int off = 1; off < 32; off <<= 1) {
-                    const double up = __shfl_up_sync(0xffffffffu, L, off);
-                    if (lane >= off) L += up;
-                }
-                const double Lend = __shfl_sync(0xffffffffu, L, 31);
-                const float hi = (float)L;
-                lh[warp][lane] = hi;
-                ll[warp][lane] = (float)(L - (double)hi);
-                sb[warp][lane] = dt;
-                rec->e[lane] = expf(hi) * A.q_scale;
-                rec->w[lane] = dt * expf((float)(Lend - L));
-                if (lane == 0) rec->end[0] = expf((float)Lend);
-            } else {                                      // powers of the constant decay, for any sign and zero
-                const double a = (double)A.decay[h];
-                double p = 1.0;
-                for (int r = 0; r < lane; ++r) p *= a;
-                pw[warp][lane] = (float)p;
-                if (lane == 31) pw[warp][32] = (float)(p * a);
-                __syncwarp();
-                rec->e[lane] = pw[warp][lane + 1] * A.q_scale;
-                rec->w[lane] = in ? pw[warp][n - 1 - lane] : 0.f;
-                if (lane == 0) rec->end[0] = pw[warp][n];
+            for (int off = 1; off < 32; off <<= 1) {
+                const double up = __shfl_up_sync(0xffffffffu, L, off);
+                if (lane >= off) L += up;
             }
+            const double Lend = __shfl_sync(0xffffffffu, L, 31);
+            const float hi = (float)L;
+            lh[warp][lane] = hi;
+            ll[warp][lane] = (float)(L - (double)hi);
+            sb[warp][lane] = dt;
+            rec->e[lane] = expf(hi) * A.q_scale;
+            rec->w[lane] = dt * expf((float)(Lend - L));
+            if (lane == 0) rec->end[0] = expf((float)Lend);
         }
         if (h0 == hb0) {
             cm_copy_wait<0>();
@@ -501,7 +489,7 @@ __global__ void __launch_bounds__(128) scalar_decay_prepare_kernel(ScanArgs A, S
                         for (int e = 0; e < 2; ++e) {
                             const int us = u + e;
                             float d = 0.f;
-                            if (us <= t) d = A.mode == 0 ? pw[hw][t - us] : expf((lh[hw][t] - lh[hw][us]) + (ll[hw][t] - ll[hw][us])) * sb[hw][us];
+                            if (us <= t) d = expf((lh[hw][t] - lh[hw][us]) + (ll[hw][t] - ll[hw][us])) * sb[hw][us];
                             // a key behind the token counts nothing, whatever its product is
                             x[e] = us <= t ? acc[nt][r * 2 + e] * (d * A.q_scale) : 0.f;
                         }
@@ -605,7 +593,7 @@ __global__ void __launch_bounds__(64 * W + CS_LOADERS) scalar_decay_chunk_kernel
     const int ld = heads * V, t_own = half * 16 + c2;
     float* op = o + (size_t)(t0 + t_own) * ld + (size_t)h * V + jr[0];
     const bool all_cols = j0 + VB <= V;
-    const float skip = (A.mode == 1 && A.skip) ? A.skip[h] : 0.f;
+    const float skip = A.skip ? A.skip[h] : 0.f;
     for (int i = 0; i < chunks; ++i) {
         __syncthreads();
         const typename SM::Stage& st = sm.stage[i % 3];
@@ -1068,7 +1056,7 @@ FF_EXPORT long long ff_scan_state_floats(int heads, int N, int V) {
 // Whether a step's prompts can go a chunk at a time: bfloat16, sizes that the tiles take and layouts that 16-byte copies take.  One decay
 // per head and token (its inputs read as they are), or one per key channel.
 static bool scalar_chunk_sizes(int mode, int act, int T, int N, int V) {
-    return mode != 2 && !act && T >= SCAN_CHUNK_MIN && (N == 64 || N == 128) && V % 8 == 0;
+    return mode == 1 && !act && T >= SCAN_CHUNK_MIN && (N == 64 || N == 128) && V % 8 == 0;
 }
 static bool channel_chunk_sizes(int mode, int act, int T, int N, int V) {
     return mode == 2 && !act && T >= CHANNEL_CHUNK_MIN && (N == 64 || N == 128) && V % 8 == 0;
@@ -1149,7 +1137,7 @@ static int scan_launch(const ScanArgs& A, float* state, long long state_stride, 
 #undef FF_SCAN
 #undef FF_SCAN_ONE
     if (!R.chunks) return 0;
-    if (A.mode != 2) {
+    if (A.mode == 1) {
         if (N == 64) return scan_chunk_launch<64>(A, state, state_stride, state_off, cu_q, state_slots, seq_fresh, o, T_tot, n_seqs, R.live, heads, V, scratch, stream);
         return scan_chunk_launch<128>(A, state, state_stride, state_off, cu_q, state_slots, seq_fresh, o, T_tot, n_seqs, R.live, heads, V, scratch, stream);
     }

@@ -106,7 +106,7 @@ def test_decay_scans(lens, N, V, heads, groups, mode):
         if mode == "constant":
             return q, k, v, const.double()[None, :, None].expand_as(k)
         return q * 0.125, k, v, alpha[a:b].view(b - a, heads, N)
-    _check(call, inputs, lens, heads, V, T, K._lib("ssm").ff_scan_chunk_min(2 if mode == "channel" else 0))
+    _check(call, inputs, lens, heads, V, T, 1 << 30 if mode == "constant" else K._lib("ssm").ff_scan_chunk_min(2 if mode == "channel" else 1))
 
 
 @pytest.mark.parametrize("lens", LENS)
