@@ -138,6 +138,44 @@ def test_gate_of_latent_attention(T, heads, vdim, shift, per_head):
     _close(y, val.double().transpose(0, 1).reshape(T, -1) * gate)
 
 
+@pytest.mark.parametrize("H,dim,rot,rank,planes,shift", [(3, 16, 64, 200, 1, 0), (8, 128, 64, 512, 1, 8), (2, 24, 8, 8, 1, 0), (5, 16, 48, 264, 1, 0),
+                                                         (3, 16, 64, 200, 2, 0), (2, 16, 72, 64, 1, 0), (2, 16, 64, 520, 1, 0), (3, 16, 64, 200, 1, 1)])
+@pytest.mark.parametrize("interleaved", [False, True])
+@pytest.mark.parametrize("writes", [True, False])
+def test_rows_of_latent_attention(H, dim, rot, rank, planes, shift, interleaved, writes):
+    """Query and cache rows in the form with a warp a token and in the other (two planes, rotations of more than 64, ranks above 512, rows
+    off a 16-byte boundary): ranks that fill no whole round of a warp, a page outside the pool, a layer that writes no rows."""
+    T, d, block, blocks = 37, rank + rot, 8, 7
+    q, dkv, q_abs = _rand(T, H * (dim + rot), dtype=BF), _rand(T, d + shift, dtype=BF, seed=1)[:, shift:], _rand(H, T, rank, dtype=BF, seed=2)
+    w, freq = 1 + 0.1 * _rand(rank), 10000.0 ** (-torch.arange(rot // 2, dtype=F64, device="cuda") * 2 / rot)
+    table = torch.tensor([[3, 1, 6], [2, blocks, 5]], dtype=torch.int32, device="cuda")      # the second sequence's second page is none
+    ctx = SimpleNamespace(positions=torch.cat([torch.arange(2, 22), torch.arange(17)]).to(torch.int32).cuda(),
+                          token_seq=torch.tensor([0] * 20 + [1] * 17, dtype=torch.int32, device="cuda"), status=torch.zeros(1, dtype=torch.int32, device="cuda"))
+    pages, q_full = torch.full((blocks, planes, 1, block, d), 7.0, dtype=BF, device="cuda"), torch.empty(T, H * d, dtype=BF, device="cuda")
+    K.latent_finish(q, dkv if writes else None, q_abs, w, 1e-6, freq, ctx, table, pages, q_full, H, dim, rot, rank, interleaved=interleaved)
+    ang = ctx.positions.double()[:, None] * freq
+
+    def turned(x):                                        # [T, n, rot]
+        a, b = (x[..., 0::2], x[..., 1::2]) if interleaved else (x[..., :rot // 2], x[..., rot // 2:])
+        cs, sn = torch.cos(ang)[:, None], torch.sin(ang)[:, None]
+        a, b = a * cs - b * sn, b * cs + a * sn
+        return torch.stack([a, b], -1).flatten(-2) if interleaved else torch.cat([a, b], -1)
+    qd = q.double().view(T, H, dim + rot)[..., dim:]
+    _close(q_full.view(T, H, d), torch.cat([q_abs.double().transpose(0, 1), turned(qd)], -1))
+    page = table[ctx.token_seq.long(), ctx.positions.long() // block].long()
+    ok = page < blocks
+    assert int(ctx.status) == (2 if writes else 0) and int(ok.sum()) == T - 8
+    want = torch.full(pages.shape, 7.0, dtype=F64, device="cuda")
+    if writes:
+        x = dkv.double()
+        c = x[:, :rank] / (x[:, :rank].square().mean(-1, keepdim=True) + 1e-6).sqrt() * w.double()
+        at = (page[ok], 0, 0, ctx.positions.long()[ok] % block)
+        want[at] = torch.cat([c, turned(x[:, None, rank:])[:, 0]], -1)[ok]
+        if planes == 2:
+            want[(page[ok], 1, 0, at[3])] = torch.cat([c, torch.zeros(T, rot, dtype=F64, device="cuda")], -1)[ok]
+    _close(pages, want)
+
+
 @pytest.mark.parametrize("T,W,top", [(9, 1024, 4), (3, 20, 1), (5, 2500, 8), (7, 1032, 9), (4, 30, 2)])
 @pytest.mark.parametrize("form", ["plain", "shared", "weighted", "written"])
 def test_sum_of_experts_rows(T, W, top, form):
