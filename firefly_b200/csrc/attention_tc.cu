@@ -62,7 +62,16 @@ constexpr int ATC_THREADS = 192;        // warps 0-3 softmax, warp 4 loads, warp
 constexpr int MAX_PAGE_LIST = FF_ATC_PAGE_LIST;
 static_assert(MAX_PAGE_LIST >= 16 && MAX_PAGE_LIST % 16 == 0, "two halves of whole tiles (up to 8 pages each)");
 constexpr float LOG2E = 1.4426950408889634f;
-constexpr unsigned long long WAIT_LIMIT_CYCLES = 2000000000ull;
+#ifndef FF_ATC_WAIT_LIMIT_CYCLES
+#define FF_ATC_WAIT_LIMIT_CYCLES 2000000000ull       // about a second
+#endif
+constexpr unsigned long long WAIT_LIMIT_CYCLES = FF_ATC_WAIT_LIMIT_CYCLES;
+// (a test build never starts the copies of one tile of keys, so that the waits for it run out)
+#ifdef FF_ATC_TEST_DROP_TILE
+#define FF_ATC_LOADS(tile, kv) ((kv) != 0 || (tile) != FF_ATC_TEST_DROP_TILE)
+#else
+#define FF_ATC_LOADS(tile, kv) true
+#endif
 
 constexpr int Q_BYTES = BM * D * 2;
 constexpr int KV_TILE_BYTES = BN * D * 2;            // one K or V tile
@@ -107,6 +116,12 @@ __device__ __forceinline__ bool mb_wait(uint32_t bar, uint32_t parity, int* stat
         }
     }
     return true;
+}
+// a load warp that gives up: the copies still on their way to `bar` land (or this limit passes) before the block's memory goes away
+__device__ __forceinline__ void mb_let_land(uint32_t bar, uint32_t parity) {
+    const unsigned long long start = clock64();
+    while (!mb_try(bar, parity))
+        if (clock64() - start > WAIT_LIMIT_CYCLES) break;
 }
 __device__ __forceinline__ void tma_2d(uint32_t dst, const void* map, int x, int y, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -573,6 +588,7 @@ attn_tc_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __restri
         bool ok = n_tiles == 0 || mb_wait(sa(&bars[B_PAGES_READY]), 0, status, abort_flag);
         ok = __all_sync(0xffffffffu, ok);
         const int p = lane / PANELS, h = lane % PANELS;                  // this lane's page and panel of a tile
+        int issued[2] = {0, 0};                                          // tiles of K and of V asked for
         auto load_tile = [&](int j, int kv) -> bool {
             const int s = j % KV_STAGES;
             if (kv == 0 && j >= 2 * tiles_per_half && j % tiles_per_half == 0) {
@@ -588,7 +604,8 @@ attn_tc_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __restri
             const uint32_t bar = sa(&bars[(kv ? B_V_FULL : B_K_FULL) + s]);
             if (lane == 0) mb_expect_tx(bar, (uint32_t)(__popc(boxes) * block_size * 128));
             __syncwarp();
-            if (page >= 0) {
+            issued[kv] = j + 1;
+            if (page >= 0 && FF_ATC_LOADS(j, kv)) {
                 unsigned char* st = (kv ? Vs : Ks) + (size_t)s * KV_TILE_BYTES;
                 const int y = ((page * FF_KV_PLANES + kv * (FF_KV_PLANES - 1)) * nkv + kh) * block_size;
                 tma_2d(sa(st + h * (BN * 128) + p * block_size * 128), &kv_map, h * 64, y, bar);
@@ -599,6 +616,11 @@ attn_tc_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __restri
         for (int j = 0; j < n_tiles && ok; ++j) {
             if (j + 1 < n_tiles) ok = load_tile(j + 1, 0);
             if (ok) ok = load_tile(j, 1);
+        }
+        if (*abort_flag) {
+            for (int kv = 0; kv < 2; ++kv)
+                for (int j = max(0, issued[kv] - KV_STAGES); j < issued[kv]; ++j)
+                    mb_let_land(sa(&bars[(kv ? B_V_FULL : B_K_FULL) + j % KV_STAGES]), (j / KV_STAGES) & 1);
         }
     } else if (warp == 5) {
         // ------------------------------------------------ MMAs -----------------
@@ -905,6 +927,7 @@ attn_tc_pair_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __r
         bool ok = n_tiles == 0 || mb_wait(sa(&bars[PB_PAGES]), 0, status, abort_flag);
         ok = __all_sync(0xffffffffu, ok);
         const int p = lane / PANELS, h = lane % PANELS;                  // this lane's page and panel of a tile
+        int issued = 0;                                                  // tiles of K and V asked for
         for (int c = 0; c < 2 * n_tiles && ok; ++c) {
             const int j = c >> 1, kv = c & 1, slot = c % PAIR_SLOTS;
             if (kv == 0 && j >= 2 * tph && j % tph == 0) {
@@ -933,10 +956,15 @@ attn_tc_pair_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __r
             const uint32_t bar = sa(&bars[PB_FULL + slot]);
             if (lane == 0) mb_expect_tx(bar, (uint32_t)(__popc(boxes) * block_size * 128));
             __syncwarp();
-            if (page >= 0) {
+            issued = c + 1;
+            if (page >= 0 && FF_ATC_LOADS(j, kv)) {
                 const int y = ((page * FF_KV_PLANES + kv * (FF_KV_PLANES - 1)) * nkv + kh) * block_size;
                 tma_2d(sa(st + h * (PN * 128) + p * block_size * 128), &kv_map, h * 64, y, bar);
             }
+        }
+        if (*abort_flag) {
+            for (int c = max(0, issued - PAIR_SLOTS); c < issued; ++c)
+                mb_let_land(sa(&bars[PB_FULL + c % PAIR_SLOTS]), (c / PAIR_SLOTS) & 1);
         }
     } else {
         // Everything the products are addressed by is the same in all lanes and is added up from 32-bit bases: with

@@ -362,6 +362,28 @@ def test_attention_tcgen05_two_row_tiles_over_pages_of_one_plane(d, nq, block):
     assert int(status) == 0 and _rows_error(out.cpu(), ref.cpu(), d) < 2.0 ** -7
 
 
+@pytest.mark.parametrize("two_tiles", [False, True])
+def test_attention_tcgen05_a_wait_that_runs_out_ends_the_kernel_with_a_status(two_tiles, monkeypatch):
+    """A test build in which the copies of one tile of keys are never started and waits give up after a few milliseconds: the kernel
+    returns, says that a wait ran out, stores nothing of the rows that needed the tile, and the next ordinary launch is right."""
+    from firefly_b200.ops.build import load_module
+    d, nq, nkv, block, seqs = 128, 8, 2, 16, [(0, 400)]
+    c = _attention_case(d, nq, nkv, block, seqs, None, torch.bfloat16, seed=13)
+    args = [dev(c["q"]), nq * d, dev(c["pages"]), dev(c["table"]), dev(c["cu_q"]), dev(c["ctx_lens"]), 1, 13]
+    lib = load_module("attention_tc.cu", {"FF_HEAD_DIM": d, "FF_ATC_TEST_DROP_TILE": 1, "FF_ATC_WAIT_LIMIT_CYCLES": "8000000ull"})
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = torch.full(c["q"].shape, 7.0, dtype=torch.bfloat16, device="cuda")
+    with monkeypatch.context() as m:
+        m.setattr(K(), "_attn_tc_lib", lambda *a: lib)
+        K().attn_tc(*args, out, nq, nkv, d, 1 / math.sqrt(d), 0, status, two_tiles=two_tiles)
+    torch.cuda.synchronize()                                   # the kernel came back
+    assert int(status) == 107
+    assert bool((out[256:] == 7.0).all())                      # these rows see the tile that never came
+    status.zero_()
+    K().attn_tc(*args, out, nq, nkv, d, 1 / math.sqrt(d), 0, status, two_tiles=two_tiles)
+    assert int(status) == 0 and _rows_error(out.cpu(), c["want"], d) < 2.0 ** -7
+
+
 def test_attention_tcgen05_context_beyond_one_ring_of_page_ids():
     """The product build at a context of 17 000 tokens in pages of 16: 1 066 page ids a block, more than
     its ring of 1 024 holds.  Only the portion's 200 queries are compared (softmax over keys 0..position
