@@ -939,7 +939,7 @@ def _recurrence_scratch_bytes(module: str, entry: str, *sizes: int) -> int:
     return int(fn(*[c_int(x) for x in sizes]))
 
 
-def _row_bits(*rows) -> int:
+def _row_bits(rows) -> int:
     """The low four bits of (matrix, first column) pairs' addresses, row strides and first columns in bytes, or'ed: 0 where every
     row can be copied 16 bytes at a time (the twin of `row_bits` in csrc/chunk_scan.cuh)."""
     bits = 0
@@ -954,10 +954,10 @@ def _chunk_min(module: str, entry: str, *kind: int) -> int:
     return int(getattr(_lib(module), entry)(*[c_int(x) for x in kind]))
 
 
-def _recurrence_scratch(ctx, module: str, entry: str, chunk_min: int, *sizes: int):
+def _recurrence_scratch(ctx, module: str, entry: str, chunk_min: int, rows, *sizes: int):
     """What a recurrence needs to know to take long sequences a chunk at a time: (how many have ``chunk_min`` tokens or more, -1 if the
     context has no host copy of the lengths; scratch memory; its bytes).  No scratch memory when there is no such sequence, when
-    the sizes are none for it (``entry`` of the library says how much it can use), when the context has no workspace or
+    the sizes or the layout of ``rows`` (`_row_bits`) are none for it (``entry`` of the library says how much it can use), when the context has no workspace or
     the device no memory left: every sequence is walked token by token then."""
     lens = getattr(ctx, "q_lens", None)
     n_long = -1
@@ -969,7 +969,7 @@ def _recurrence_scratch(ctx, module: str, entry: str, chunk_min: int, *sizes: in
             if memo is not None:
                 memo[("long_seqs", chunk_min)] = n_long
     ws = getattr(ctx, "workspace", None)
-    need = _recurrence_scratch_bytes(module, entry, *sizes) if ws is not None and n_long != 0 else 0
+    need = _recurrence_scratch_bytes(module, entry, *sizes, _row_bits(rows)) if ws is not None and n_long != 0 else 0
     records = ws.try_get("scan.records", (-(-need // 4),), torch.float32) if need > 0 else None
     if records is None:
         return c_int(n_long), c_void_p(0), ctypes.c_longlong(0)
@@ -1000,8 +1000,8 @@ def wkv_scan(rkvg, dlog, w0, u, state, prev_off: int, x, ctx, o, heads: int, dim
     assert o.shape == (T, HD) and o.dtype == torch.float32 and state.dtype == torch.float32
     assert w0.dtype == u.dtype == torch.float32 and w0.numel() == HD and u.numel() == HD
     assert state.shape[1] >= prev_off + W and prev_off >= heads * wkv_state_dim(dim) ** 2
-    scratch = _recurrence_scratch(ctx, "wkv", "ff_wkv_scratch_bytes", _chunk_min("wkv", "ff_wkv_chunk_min"), _dt(rkvg), T, ctx.num_seqs, heads, dim,
-                                  _row_bits((rkvg, 0), (dlog, 0)))
+    scratch = _recurrence_scratch(ctx, "wkv", "ff_wkv_scratch_bytes", _chunk_min("wkv", "ff_wkv_chunk_min"), ((rkvg, 0), (dlog, 0)),
+                                  _dt(rkvg), T, ctx.num_seqs, heads, dim)
     launched = c_int(0)
     _check(_lib("wkv").ff_wkv_scan(_p(rkvg), c_int(_dt(rkvg)), _p(dlog), _p(w0), _p(u), _p(state),
                                   ctypes.c_longlong(state.stride(0)), c_int(prev_off), _p(x), c_int(W), _p(ctx.cu_q),
@@ -1549,8 +1549,8 @@ def delta_rule_scan(q, k, v, beta, a, dt_bias: torch.Tensor, a_log: torch.Tensor
     assert dt_bias.dtype == a_log.dtype == torch.float32 and a_log.numel() == heads
     assert dt_bias.numel() == (heads if decay_per_head else heads * N)
     assert o.dtype == torch.float32 and o.shape == (T, heads * V) and state.dtype == torch.float32
-    scratch = _recurrence_scratch(ctx, "delta_rule", "ff_delta_scratch_bytes", _chunk_min("delta_rule", "ff_delta_chunk_min"), _dt(qm), T, ctx.num_seqs, heads, N, V,
-                                  _row_bits((qm, q0), (km, k0), (vm, v0), *(() if decay_per_head else ((am, a0),))))
+    scratch = _recurrence_scratch(ctx, "delta_rule", "ff_delta_scratch_bytes", _chunk_min("delta_rule", "ff_delta_chunk_min"),
+                                  (q, k, v) if decay_per_head else (q, k, v, a), _dt(qm), T, ctx.num_seqs, heads, N, V)
     launched = c_int(0)
     _check(_lib("delta_rule").ff_delta_rule_scan(
         _p(qm), c_int(qm.stride(0)), c_int(q0), _p(km), c_int(km.stride(0)), c_int(k0), _p(vm), c_int(vm.stride(0)),
@@ -1601,8 +1601,9 @@ def scalar_decay_scan(q, k, v, state: torch.Tensor, state_off: int, ctx, o: torc
     sm, s0 = step if step is not None else (None, 0)
     if mode == 1:
         assert sm.dtype == qm.dtype and step_bias is not None and a_log is not None
-    scratch = _recurrence_scratch(ctx, "ssm", "ff_scan_scratch_bytes", _chunk_min("ssm", "ff_scan_chunk_min", mode), _dt(qm), mode, 1 if silu_inputs else 0, T, ctx.num_seqs, heads,
-                                  heads_per_group, N, V, _row_bits((qm, q0), (km, k0), (vm, v0), *(((cm, cd0),) if mode == 2 else ())))
+    scratch = _recurrence_scratch(ctx, "ssm", "ff_scan_scratch_bytes", _chunk_min("ssm", "ff_scan_chunk_min", mode),
+                                  (q, k, v, channel_decay) if mode == 2 else (q, k, v), _dt(qm), mode, 1 if silu_inputs else 0, T,
+                                  ctx.num_seqs, heads, heads_per_group, N, V)
     launched = c_int(0)
     _check(_lib("ssm").ff_scalar_decay_scan(
         _p(qm), c_int(qm.stride(0)), c_int(q0), _p(km), c_int(km.stride(0)), c_int(k0), _p(vm), c_int(vm.stride(0)),

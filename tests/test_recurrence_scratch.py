@@ -31,7 +31,7 @@ class _Small(Workspace):
 
 def _scratch(ws, monkeypatch, numbers):
     monkeypatch.setattr(K, "_recurrence_scratch_bytes", lambda *a: 4 * numbers)
-    _, p, size = K._recurrence_scratch(SimpleNamespace(workspace=ws), "ssm", "ff_scan_scratch_bytes", 32)
+    _, p, size = K._recurrence_scratch(SimpleNamespace(workspace=ws), "ssm", "ff_scan_scratch_bytes", 32, ())
     assert (p.value is None) == (size.value == 0)
     return size.value // 4
 
@@ -76,7 +76,7 @@ def test_no_long_sequence_no_scratch_memory(monkeypatch):
         ws = _Small(100)
         ctx = SimpleNamespace(workspace=ws, q_lens=lens, memo={})
         for _ in range(2):
-            n, p, size = K._recurrence_scratch(ctx, "ssm", "ff_scan_scratch_bytes", 32)
+            n, p, size = K._recurrence_scratch(ctx, "ssm", "ff_scan_scratch_bytes", 32, ())
             assert n.value == n_long and size.value == (0 if n_long == 0 else 40) and len(ws.asked) == (n_long != 0)
             assert lens is None or ctx.memo[("long_seqs", 32)] == n_long
 
