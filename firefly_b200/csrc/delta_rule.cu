@@ -56,7 +56,8 @@ static inline bool delta_plan(int N, int V, DeltaPlan* p) {
     return true;
 }
 
-template <typename T, int NP, int PARTS, int VJ>
+// SOME: sequences of max_len tokens and more go by chunks (else every sequence is this kernel's).
+template <typename T, int NP, int PARTS, int VJ, bool SOME>
 __global__ void __launch_bounds__(DR_MAX_THREADS) delta_rule_scan_kernel(
     DeltaArgs A, float* __restrict__ state, size_t state_stride, int state_off, const int* __restrict__ cu_q,
     const int* __restrict__ state_slots, const int* __restrict__ seq_fresh, float* __restrict__ o /*[T, heads*V]*/,
@@ -73,8 +74,9 @@ __global__ void __launch_bounds__(DR_MAX_THREADS) delta_rule_scan_kernel(
     const int lane = tid & 31, warp = tid >> 5, nwarps = nthr >> 5;
     const int jl = tid / PARTS, part = tid % PARTS;
     const int j0 = blockIdx.z * Vb;                       // the block's first column; the thread's are j0 + jl * VJ + x
-    const int t0 = cu_q[s], t1 = cu_q[s + 1];
-    if (t1 - t0 >= max_len) return;                       // such a sequence goes by chunks
+    const int t0 = cu_q[s], t1s = cu_q[s + 1];
+    const bool mine = !SOME || t1s - t0 < max_len;                 // a sequence that goes by chunks is empty here (as in ssm.cu)
+    const int t1 = mine ? t1s : t0;
     bool live[VJ];
 #pragma unroll
     for (int x = 0; x < VJ; ++x) live[x] = jl * VJ + x < Vb && j0 + jl * VJ + x < V;
@@ -252,7 +254,7 @@ __global__ void __launch_bounds__(DR_MAX_THREADS) delta_rule_scan_kernel(
 #pragma unroll
         for (int i = 0; i < KP; i += 4) {
             float* p = S_g + (size_t)(j0 + jl * VJ + x) * NP + i * PARTS + part * 4;
-            if (!live[x]) continue;
+            if (!live[x] || !mine) continue;
             if (vec) *reinterpret_cast<float4*>(p) = make_float4(S[x][i], S[x][i + 1], S[x][i + 2], S[x][i + 3]);
             else { p[0] = S[x][i]; p[1] = S[x][i + 1]; p[2] = S[x][i + 2]; p[3] = S[x][i + 3]; }
         }
@@ -479,9 +481,15 @@ static int delta_launch(const DeltaArgs& A, float* state, long long state_stride
     if (!delta_plan(N, V, &p)) return FF_ERR_UNSUPPORTED;
     if (p.Vb > 128) return FF_ERR_UNSUPPORTED;
     dim3 grid(n_seqs, heads, p.vsplit);
-#define FF_DELTA(NP, PARTS, VJ)                                                                                    \
-    FF_LAUNCH((delta_rule_scan_kernel<T, NP, PARTS, VJ>), grid, p.threads, 0, stream, A, state, (size_t)state_stride, \
+#define FF_DELTA_ONE(NP, PARTS, VJ, SOME)                                                                          \
+    FF_LAUNCH((delta_rule_scan_kernel<T, NP, PARTS, VJ, SOME>), grid, p.threads, 0, stream, A, state, (size_t)state_stride, \
               state_off, cu_q, state_slots, seq_fresh, o, heads, N, V, p.Vb, max_len)
+#define FF_DELTA(NP, PARTS, VJ)                                                                                    \
+    do {                                                                                                           \
+        constexpr bool SOME = sizeof(T) == 2 && (NP == 64 || NP == 128);        /* no other size goes by chunks */  \
+        if (SOME && max_len != 0x7fffffff) FF_DELTA_ONE(NP, PARTS, VJ, SOME);                                      \
+        else FF_DELTA_ONE(NP, PARTS, VJ, false);                                                                   \
+    } while (0)
     switch (p.NP) {
         case 16: FF_DELTA(16, 4, 1); break;
         case 32: FF_DELTA(32, 8, 1); break;
@@ -491,6 +499,7 @@ static int delta_launch(const DeltaArgs& A, float* state, long long state_stride
         default: return FF_ERR_UNSUPPORTED;
     }
 #undef FF_DELTA
+#undef FF_DELTA_ONE
     FF_LAUNCH_CHECK();
     return 0;
 }

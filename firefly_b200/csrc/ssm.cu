@@ -245,7 +245,8 @@ struct ScanArgs {
 // this one leaves 1e-7) and for sizes that the chunked ones do not take.  Against one column a thread: 758 -> 279 us
 // for three sequences of 1501, 1000 and 700 tokens with 16 heads of 64 x 128, 1256 -> 745 us for 4 x 2048 tokens, SiLU, 8 heads
 // of 128 x 128.
-template <typename T, int NP, bool CD>
+// SOME: sequences of max_len tokens and more go by chunks (else every sequence is this kernel's).
+template <typename T, int NP, bool CD, bool SOME>
 __global__ void __launch_bounds__(WS_THREADS) scalar_decay_scan_kernel(
     ScanArgs A, float* __restrict__ state, size_t state_stride, int state_off, const int* __restrict__ cu_q,
     const int* __restrict__ state_slots, const int* __restrict__ seq_fresh, float* __restrict__ o /*[T, heads*V]*/,
@@ -259,8 +260,11 @@ __global__ void __launch_bounds__(WS_THREADS) scalar_decay_scan_kernel(
     __shared__ float s_a[2][CH], s_d[2][CH];
     const int s = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
     const int j0 = blockIdx.z * VB;
-    const int t0 = cu_q[s], t1 = cu_q[s + 1];
-    if (t1 - t0 >= max_len) return;                       // such a sequence goes by chunks
+    const int t0 = cu_q[s], t1s = cu_q[s + 1];
+    // a sequence that goes by chunks is empty here: a return would put the lengths' way from memory in front of the state's (3.2 -> 3.4 us
+    // for eight single tokens of 16 heads of 64 x 128)
+    const bool mine = !SOME || t1s - t0 < max_len;
+    const int t1 = mine ? t1s : t0;
     WS w;
     w.place(tid);
     float* S_g = state + (size_t)state_slots[s] * state_stride + state_off + (size_t)h * V * NP;
@@ -365,7 +369,7 @@ __global__ void __launch_bounds__(WS_THREADS) scalar_decay_scan_kernel(
         if (c0 + CH < t1) stage(b ^ 1, min(CH, t1 - c0 - CH));
         __syncthreads();
     }
-    w.store(S_g, j0, V);
+    if (mine) w.store(S_g, j0, V);
 }
 
 // ------------------------------------------------------------------- the recurrence, a chunk of tokens at a time --
@@ -1116,13 +1120,17 @@ static int scan_launch(const ScanArgs& A, float* state, long long state_stride, 
     const long long need = sizeof(T) == 2 ? ff_scan_scratch_bytes(1, A.mode, A.act, T_tot, n_seqs, heads, A.heads_per_group, N, V, (int)scan_bits(A)) : 0;
     const ChunkRoute R = chunk_route(need > 0 && scratch && scratch_bytes >= need, n_long, n_seqs, ff_scan_chunk_min(A.mode));
     *launched = R.kernels();
-#define FF_SCAN_ONE(NP, CD)                                                                                             \
-    FF_LAUNCH((scalar_decay_scan_kernel<T, NP, CD>), dim3(n_seqs, heads, (V + WideState<NP>::VB - 1) / WideState<NP>::VB), \
+#define FF_SCAN_ONE(NP, CD, SOME)                                                                                       \
+    FF_LAUNCH((scalar_decay_scan_kernel<T, NP, CD, SOME>), dim3(n_seqs, heads, (V + WideState<NP>::VB - 1) / WideState<NP>::VB), \
               WS_THREADS, 0, stream, A, state, (size_t)state_stride, state_off, cu_q, state_slots, seq_fresh, o, heads, N, V, R.max_walk)
 #define FF_SCAN(NP)                                                                                                     \
     do {                                                                                                                \
-        if (A.mode == 2) FF_SCAN_ONE(NP, true);                                                                         \
-        else FF_SCAN_ONE(NP, false);                                                                                    \
+        if (sizeof(T) == 2 && (NP == 64 || NP == 128) && R.chunks) {                                                    \
+            constexpr bool SOME = sizeof(T) == 2 && (NP == 64 || NP == 128);    /* no other size goes by chunks */       \
+            if (A.mode == 2) FF_SCAN_ONE(NP, true, SOME);                                                               \
+            else FF_SCAN_ONE(NP, false, SOME);                                                                          \
+        } else if (A.mode == 2) FF_SCAN_ONE(NP, true, false);                                                           \
+        else FF_SCAN_ONE(NP, false, false);                                                                             \
     } while (0)
     if (R.walk) {
         switch (ws_key_size(N)) {

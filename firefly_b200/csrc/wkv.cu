@@ -129,8 +129,9 @@ __global__ void __launch_bounds__(WS_THREADS) wkv_scan_kernel(
     __shared__ __align__(16) float s_r[2][CH][DIM], s_k[2][CH][DIM], s_w[2][CH][DIM];
     __shared__ __align__(16) f32x2 s_v[2][CH][VB];             // each value twice
     const int s = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, j0 = blockIdx.z * VB;
-    const int t0 = cu_q[s], t1 = cu_q[s + 1];
-    if (t1 - t0 >= max_len) return;                            // such a sequence goes by chunks
+    const int t0 = cu_q[s], t1s = cu_q[s + 1];
+    const bool mine = t1s - t0 < max_len;                      // a sequence that goes by chunks is empty here (as in ssm.cu)
+    const int t1 = mine ? t1s : t0;
     const int HD = heads * dim;
     float* st = state + (size_t)state_slots[s] * state_stride;
     float* S_g = st + (size_t)h * DIM * DIM;
@@ -230,7 +231,7 @@ __global__ void __launch_bounds__(WS_THREADS) wkv_scan_kernel(
         if (c0 + CH < t1) stage(b ^ 1);
         __syncthreads();
     }
-    w.store(S_g, j0, holds ? dim : 0);
+    if (mine) w.store(S_g, j0, holds ? dim : 0);
     // the sequence's last input row, for the first token of its next step
     if (h == 0 && blockIdx.z == 0 && t1 > t0) {
         const T* last = pdl_fresh(x_) + (size_t)(t1 - 1) * W;
