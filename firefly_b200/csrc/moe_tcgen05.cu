@@ -165,8 +165,13 @@ moe_grouped_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
                 if constexpr (KIND == MOE_GATEUP) {
                     float u[16];
                     tc_ld16(acc + BC / 2 + c0, u);
+                    if (a.act == 1) {                                  // one branch for all: a branch a value would keep them from overlapping
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) v[i] = clamped_glu_fast(v[i] * wr, u[i] * wr, a.limit, a.act);
+                        for (int i = 0; i < 16; ++i) v[i] = clamped_glu_fast(v[i] * wr, u[i] * wr, a.limit, 1);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) v[i] = clamped_glu_fast(v[i] * wr, u[i] * wr, a.limit, 0);
+                    }
                 } else if constexpr (KIND == MOE_UP) {
 #pragma unroll
                     for (int i = 0; i < 16; ++i) v[i] = relu2(v[i] * wr);
@@ -224,31 +229,363 @@ static int grouped_launch(const CUtensorMap& ma, const CUtensorMap& mb0, const C
     return 0;
 }
 
+// ------------------------------------------------------------------------------ pairs of SMs that stay --
+// The same products where they fill the GPU: one pair of blocks (tcgen05 cta_group::2) per pair of SMs walks over tiles of 256
+// rows of one expert x 256 matrix rows (8192 tokens, 4 of 16 experts of 512 x 1024: gate|up 120.7 -> 77.1 us with the gather, down 77.8 -> 47.9;
+// the one-block kernel with its activation behind one branch 99.6).  What bounded the kernel above at these sizes: an SM's own 128 x 256 tile reads 96 bytes
+// from L2 for every clock that its MMAs take, two stages of 48 KB are all that two blocks an SM have room for, a TMA gather of
+// four rows keeps the copy engine for 60 clocks and more, twice what the MMAs of its rows take, and a thread's 16-byte stores of its own row
+// reach the L2 as half sectors.  Here each block of a pair loads its 128 rows and half of the matrix rows (64 bytes a clock), six
+// stages ahead, from rows that moe_gather_kernel has put side by side; two accumulators in tensor memory let a tile's epilogue run
+// under the next tile's main loop; and a warp's 32 rows leave through shared memory, 128 bytes of each at a time, as TMA stores.
+// (Rows picked by cp.async and a proxy fence for every stage took 1.2 us a stage where the MMAs take 0.3.)
+constexpr int GP_EPI = 8;                                              // epilogue warps: two for every 32 rows, each half of the columns
+constexpr int GP_THREADS = 64 + 32 * GP_EPI;
+constexpr int GP_ROWS = 256, GP_BC = 256, GP_STAGES = 6, GP_STAGE_BYTES = 2 * GM * BK * 2, GP_BOX = 32 * 128, GP_STAGING = GP_EPI * GP_BOX;
+constexpr size_t GP_SMEM = (size_t)GP_STAGES * GP_STAGE_BYTES + GP_STAGING + 1024 /* alignment slack */ + 256 /* barriers */;
+
+// The tiles of 256 rows, expert after expert; every role of a block walks the list by itself.
+struct GroupWalk {
+    const int* seg;
+    int E, e, base, lo, hi;
+    __device__ __forceinline__ void begin(const int* s, int experts) { seg = s; E = experts; e = 0; base = 0; lo = s[0]; hi = s[1]; }
+    __device__ __forceinline__ bool find(int m) {                      // m never decreases; false: behind the last tile
+        for (;;) {
+            const int n = (hi - lo + GP_ROWS - 1) / GP_ROWS;
+            if (m < base + n) return true;
+            base += n;
+            if (++e >= E) return false;
+            lo = hi;
+            hi = seg[e + 1];
+        }
+    }
+    __device__ __forceinline__ int row0(int m) const { return lo + (m - base) * GP_ROWS; }
+};
+
+// Loads, MMA and completion over the pair (as in gemm_pair.cu): a load is counted on the barrier of the pair's first block.
+__device__ __forceinline__ void gp_load_2d(bool issue, uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+                 "@q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}"
+                 ::"r"(dst), "l"(map), "r"(bar & 0xFEFFFFFFu), "r"(x), "r"(y), "r"((uint32_t)issue) : "memory");
+}
+__device__ __forceinline__ void gp_store_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(map), "r"(src), "r"(x), "r"(y) : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void gp_mma(bool issue, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+                 "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                 ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"((uint32_t)issue) : "memory");
+}
+__device__ __forceinline__ void gp_commit(bool issue, uint32_t bar) {   // arrives in both blocks
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
+                 "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+                 ::"r"(bar), "h"((uint16_t)3), "r"((uint32_t)issue) : "memory");
+}
+__device__ __forceinline__ void gp_arrive_leader(uint32_t bar) {
+    uint32_t peer;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(peer) : "r"(bar));
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(peer) : "memory");
+}
+__device__ __forceinline__ uint32_t pack_bf16(float x, float y) {
+    __nv_bfloat162 p = __floats2bfloat162_rn(x, y);
+    return *reinterpret_cast<uint32_t*>(&p);
+}
+
+template <int KIND>
+__global__ void __launch_bounds__(GP_THREADS)
+moe_grouped_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b0,
+                        const __grid_constant__ CUtensorMap map_b1, const __grid_constant__ CUtensorMap map_out, const GroupedArgs a, const int E) {
+    constexpr int COLS = KIND == MOE_GATEUP ? GP_BC / 2 : GP_BC;       // output columns of a tile
+    constexpr int BOX_COLS = KIND == MOE_DOWN ? 32 : 64;               // of 128 bytes of an output row
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* tiles = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    unsigned char* staging = tiles + (size_t)GP_STAGES * GP_STAGE_BYTES;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(staging + GP_STAGING);
+    // [0..S) full (the first block's), [S..2S) empty, [2S..2S+2) accumulator ready, [2S+2..2S+4) accumulator free (the first block's)
+    constexpr int FULL = 0, EMPTY = GP_STAGES, READY = 2 * GP_STAGES, FREE = READY + 2;
+    __shared__ uint32_t s_tmem_base;
+    __shared__ int s_abort;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const bool issue = lane == 0;
+    const int half = blockIdx.x & 1;                                   // the cluster is (2, 1, 1)
+    const int pairs = gridDim.x >> 1, NT = (a.N + COLS - 1) / COLS;
+    const int n_iters = (a.K + BK - 1) / BK;
+
+    if (threadIdx.x == 0) {
+        s_abort = 0;
+        for (int i = 0; i < FREE; ++i) mbar_init(smem_addr(&bars[i]), 1);
+        for (int i = FREE; i < FREE + 2; ++i) mbar_init(smem_addr(&bars[i]), 2 * GP_EPI);  // the epilogue warps of both blocks
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
+                     ::"r"(smem_addr(&s_tmem_base)), "r"((uint32_t)(2 * GP_BC)) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();                                                // the other block's barriers are there
+    tc_fence_after();
+    const uint32_t tmem_base = s_tmem_base;
+    volatile int* abort_flag = &s_abort;
+    grid_launch_dependents();
+    // the plan and the rows come from the kernels in front
+    grid_dependency_wait();
+    GroupWalk walk;
+    walk.begin(pdl_fresh(a.seg), E);
+
+    if (warp == 0) {
+        // ------------------------------------------------ producer: TMA loads --
+        const CUtensorMap* mb = KIND == MOE_GATEUP && half ? &map_b1 : &map_b0;
+        int g = 0;                                                     // stages asked for
+        bool ok = true;
+        for (int i = blockIdx.x >> 1; ok; i += pairs) {
+            const int m = i / NT, n0 = (i - m * NT) * COLS;
+            if (!walk.find(m)) break;
+            const int row0 = walk.row0(m) + half * GM;
+            const int y = walk.e * a.N + n0 + (KIND == MOE_GATEUP ? 0 : half * GM);
+            for (int it = 0; it < n_iters; ++it, ++g) {
+                const int s = g % GP_STAGES;
+                if (g >= GP_STAGES &&
+                    !__all_sync(0xffffffffu, mbar_wait(smem_addr(&bars[EMPTY + s]), ((g / GP_STAGES) & 1) ^ 1, a.status, abort_flag, 111))) {
+                    ok = false;
+                    break;
+                }
+                const uint32_t full = smem_addr(&bars[FULL + s]), sa = smem_addr(tiles + (size_t)s * GP_STAGE_BYTES);
+                if (half == 0) mbar_expect_tx(issue, full, 2 * GP_STAGE_BYTES);            // both blocks' bytes
+                __syncwarp();
+                gp_load_2d(issue, sa, &map_a, it * BK, row0, full);
+                gp_load_2d(issue, sa + GM * BK * 2, mb, it * BK, y, full);
+            }
+        }
+        // the last stages' releases, which come from the first block's MMAs, have arrived before this block goes
+        for (int it = max(0, g - GP_STAGES); ok && it < g; ++it)
+            ok = __all_sync(0xffffffffu, mbar_wait(smem_addr(&bars[EMPTY + it % GP_STAGES]), (it / GP_STAGES) & 1, a.status, abort_flag, 111));
+        if (half == 0 && *abort_flag) {
+            // let the copies that are still in flight land before the blocks' memory goes away
+            const unsigned long long start = clock64();
+            for (int it = max(0, g - GP_STAGES); it < g; ++it) {
+                while (!mbar_try_wait(smem_addr(&bars[FULL + it % GP_STAGES]), (it / GP_STAGES) & 1))
+                    if (clock64() - start > WAIT_LIMIT_CYCLES) break;
+            }
+        }
+    } else if (warp == 1) {
+        // ------------------------------------------------ MMA issuer: the first block's ----------
+        if (half == 0) {
+            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(GP_BC >> 3) << 17) | ((uint32_t)(GP_ROWS >> 4) << 24);
+            int g = 0, t = 0;
+            bool ok = true;
+            for (int i = blockIdx.x >> 1; ok; i += pairs, ++t) {
+                if (!walk.find(i / NT)) break;
+                const int buf = t & 1;
+                if (t >= 2 && !__all_sync(0xffffffffu, mbar_wait(smem_addr(&bars[FREE + buf]), ((t >> 1) & 1) ^ 1, a.status, abort_flag, 112))) break;
+                tc_fence_after();
+                for (int it = 0; it < n_iters; ++it, ++g) {
+                    const int s = g % GP_STAGES;
+                    ok = __all_sync(0xffffffffu, mbar_wait(smem_addr(&bars[FULL + s]), (g / GP_STAGES) & 1, a.status, abort_flag, 112));
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t sa = smem_addr(tiles + (size_t)s * GP_STAGE_BYTES), sb = sa + GM * BK * 2;
+#pragma unroll
+                    for (int k = 0; k < BK / UMMA_K; ++k)
+                        gp_mma(issue, tmem_base + buf * GP_BC, smem_desc_sw128(sa + k * UMMA_K * 2), smem_desc_sw128(sb + k * UMMA_K * 2), idesc,
+                               (it > 0 || k > 0) ? 1u : 0u);
+                    gp_commit(issue, smem_addr(&bars[EMPTY + s]));     // the stage is free in both blocks
+                    __syncwarp();
+                }
+                if (ok) gp_commit(issue, smem_addr(&bars[READY + buf]));
+            }
+        }
+    } else {
+        // ------------------------------------------------ epilogue: one accumulator row a thread --
+        const int quad = warp & 3, part = (warp - 2) >> 2;             // this warp's 32 lanes of tensor memory, and which half of the columns
+        unsigned char* box = staging + (warp - 2) * GP_BOX;            // 32 rows x 128 bytes on their way out; the other warp's fills meanwhile
+        const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
+        // 16 bytes of this thread's row, where the 128-byte swizzle has them (eight rows' pieces lie in different banks)
+        auto stage16 = [&](int chunk, uint4 v) {
+            *reinterpret_cast<uint4*>(box + lane * 128 + ((chunk ^ (lane & 7)) << 4)) = v;
+        };
+        // the box has to be free: the store that took it last has read it
+        auto box_free = [&]() {
+            if (issue) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            __syncwarp();
+        };
+        // the warp's box goes to rows row0 .., columns c ..; where the expert ends among the rows (or a wait ran out) row by row
+        auto leave = [&](int row0, int rows, int c) {
+            if (rows >= 32) {
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (issue) gp_store_2d(&map_out, smem_addr(box), c, row0);
+            } else {
+                __syncwarp();
+                const int w_row = lane >> 3, w_chunk = lane & 7, col = c + w_chunk * (BOX_COLS / 8);      // eight lanes a row's 128 bytes
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const int r = j * 4 + w_row;
+                    const uint4 v = *reinterpret_cast<const uint4*>(box + r * 128 + ((w_chunk ^ (r & 7)) << 4));
+                    if (r < rows && col < a.N) {
+                        const size_t at = (size_t)(row0 + r) * a.N + col;
+                        if constexpr (KIND == MOE_DOWN) *reinterpret_cast<uint4*>((float*)a.out + at) = v;
+                        else *reinterpret_cast<uint4*>((bf16*)a.out + at) = v;
+                    }
+                }
+                __syncwarp();
+            }
+        };
+        int t = 0;
+        for (int i = blockIdx.x >> 1;; i += pairs, ++t) {
+            const int m = i / NT, n0 = (i - m * NT) * COLS, buf = t & 1;
+            if (!walk.find(m)) break;
+            const int row0 = walk.row0(m) + half * GM + quad * 32;
+            const int rows = walk.hi - row0;                           // of this warp: <= 0 where the expert ends in front of it
+            const float wr = KIND != MOE_DOWN && a.row_w && lane < rows ? pdl_fresh(a.row_w)[row0 + lane] : 1.0f;
+            if (!__all_sync(0xffffffffu, mbar_wait(smem_addr(&bars[READY + buf]), (t >> 1) & 1, a.status, abort_flag, 113))) break;
+            tc_fence_after();
+            const uint32_t acc = lane_base + buf * GP_BC;
+            if (rows > 0) {
+                const int cols = min(COLS, a.N - n0);
+#pragma unroll 1
+                for (int c0 = part * (COLS / 2); c0 < min(cols, (part + 1) * (COLS / 2)); c0 += BOX_COLS) {
+                    if constexpr (KIND == MOE_DOWN) {
+                        float v[32];
+                        tc_ld32(acc + c0, v);
+                        box_free();
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            stage16(j, make_uint4(__float_as_uint(v[4 * j]), __float_as_uint(v[4 * j + 1]), __float_as_uint(v[4 * j + 2]), __float_as_uint(v[4 * j + 3])));
+                    } else {
+                        box_free();
+#pragma unroll
+                        for (int c1 = 0; c1 < BOX_COLS; c1 += 32) {
+                            float v[32];
+                            tc_ld32(acc + c0 + c1, v);
+                            if constexpr (KIND == MOE_GATEUP) {
+                                float u[32];
+                                tc_ld32(acc + GP_BC / 2 + c0 + c1, u);
+                                // one branch for all: a branch a value would keep them from overlapping
+                                if (a.act == 1) {
+#pragma unroll
+                                    for (int x = 0; x < 32; ++x) v[x] = clamped_glu_fast(v[x] * wr, u[x] * wr, a.limit, 1);
+                                } else {
+#pragma unroll
+                                    for (int x = 0; x < 32; ++x) v[x] = clamped_glu_fast(v[x] * wr, u[x] * wr, a.limit, 0);
+                                }
+                            } else {
+#pragma unroll
+                                for (int x = 0; x < 32; ++x) v[x] = relu2(v[x] * wr);
+                            }
+#pragma unroll
+                            for (int j = 0; j < 4; ++j)
+                                stage16((c1 >> 3) + j, make_uint4(pack_bf16(v[8 * j], v[8 * j + 1]), pack_bf16(v[8 * j + 2], v[8 * j + 3]),
+                                                                  pack_bf16(v[8 * j + 4], v[8 * j + 5]), pack_bf16(v[8 * j + 6], v[8 * j + 7])));
+                        }
+                    }
+                    leave(row0, rows, n0 + c0);
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (issue) gp_arrive_leader(smem_addr(&bars[FREE + buf]));
+        }
+        if (issue) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");       // the stores have left this block's memory and are there
+    }
+    // the pair's tensor memory is freed together, and its first block's barriers serve both
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();
+    if (warp == 1) {
+        __syncwarp();
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)(2 * GP_BC)) : "memory");
+    }
+}
+
+template <int KIND>
+static int grouped_pair_launch(const CUtensorMap& ma, const CUtensorMap& mb0, const CUtensorMap& mb1, const CUtensorMap& mo, const GroupedArgs& a,
+                               int E, int max_tiles, cudaStream_t stream) {
+    constexpr int COLS = KIND == MOE_GATEUP ? GP_BC / 2 : GP_BC;
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return (int)e;
+    FF_SMEM_LIMIT(moe_grouped_pair_kernel<KIND>, GP_SMEM);
+    const long long items = (long long)max_tiles * ((a.N + COLS - 1) / COLS);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * (unsigned)(items < sms / 2 ? items : sms / 2));
+    cfg.blockDim = dim3(GP_THREADS);
+    cfg.dynamicSmemBytes = GP_SMEM;
+    cfg.stream = stream;
+    cudaLaunchAttribute attrs[2];
+    attrs[0].id = cudaLaunchAttributeClusterDimension;
+    attrs[0].val.clusterDim.x = 2;
+    attrs[0].val.clusterDim.y = attrs[0].val.clusterDim.z = 1;
+    attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attrs;
+    cfg.numAttrs = g_ff_pdl ? 2 : 1;
+    return (int)cudaLaunchKernelEx(&cfg, moe_grouped_pair_kernel<KIND>, ma, mb0, mb1, mo, a, E);
+}
+
+// The tokens' rows in the order of the plan, a warp a row of `pieces` 16-byte pieces.
+__global__ void __launch_bounds__(256) moe_gather_kernel(const uint4* x, const int* src_tok, const int* n_rows /* the plan's: seg[E] */, uint4* rows,
+                                                         int room, int pieces) {
+    pdl_prologue();
+    const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (r >= min(room, *pdl_fresh(n_rows))) return;
+    const uint4* from = pdl_fresh(x) + (size_t)pdl_fresh(src_tok)[r] * pieces;
+    uint4* to = rows + (size_t)r * pieces;
+    for (int i = lane; i < pieces; i += 128) {
+        uint4 v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (i + 32 * j < pieces) v[j] = from[i + 32 * j];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (i + 32 * j < pieces) to[i + 32 * j] = v[j];
+    }
+}
+
 }  // namespace ff
 
 using namespace ff;
 
 // a: bfloat16 [a_rows, K] (kind MOE_DOWN: the sorted rows themselves; else the tokens' rows, picked by src_tok).
 // b0, b1: bfloat16 [E, N, K].  The plan's row tiles have 128 rows.  wide: 256 weight rows a block instead of 128.
+// n_rows: of `out`, at least the plan's.  gathered (may be null): room for as many rows of K values; with it pairs of SMs multiply 256 rows with 256 weight rows at a time (N a
+// multiple of 8; kind MOE_DOWN: any pointer but null, nothing is gathered).  launched: kernels put on the stream.
 FF_EXPORT int ff_moe_grouped_tc(const void* a, int a_rows, const int* src_tok, const void* b0, const void* b1, int E, int kind,
                                 const int* seg, const int* tile_expert, const int* tile_row0, const int* n_tiles,
                                 const float* row_w, void* out, int max_tiles, int N, int K, float limit, int act, int wide,
-                                int* status, cudaStream_t stream) {
+                                void* gathered, int n_rows, int* status, int* launched, cudaStream_t stream) {
+    *launched = 0;
     if (max_tiles <= 0) return 0;
     if (kind < MOE_DOWN || kind > MOE_UP || (kind == MOE_GATEUP && !b1) || !status || a_rows <= 0 || E <= 0 || N <= 0 || K <= 0 || K % 8)
         return FF_ERR_BAD_ARG;
-    if ((((uintptr_t)a | (uintptr_t)b0 | (uintptr_t)b1 | (uintptr_t)out) & 15) != 0 || (long long)E * N >= (1ll << 31) || max_tiles > 65535)
+    if ((((uintptr_t)a | (uintptr_t)b0 | (uintptr_t)b1 | (uintptr_t)out | (uintptr_t)gathered) & 15) != 0 || (long long)E * N >= (1ll << 31) || max_tiles > 65535)
         return FF_ERR_BAD_ARG;
-    const int bc = wide ? 256 : 128, box = kind == MOE_GATEUP ? bc / 2 : bc;
-    CUtensorMap ma, mb0, mb1;
-    int rc = make_map(a, a_rows, K, kind == MOE_DOWN ? GM : 1, &ma);       // a gather's box is one row high
+    if (gathered && (N % 8 || n_rows <= 0)) return FF_ERR_BAD_ARG;
+    const bool down = kind == MOE_DOWN;
+    if (gathered && !down) {
+        FF_LAUNCH(moe_gather_kernel, (n_rows + 7) / 8, 256, 0, stream, (const uint4*)a, src_tok, seg + E, (uint4*)gathered, n_rows, K / 8);
+        FF_LAUNCH_CHECK();
+        ++*launched;
+        a = gathered;
+        a_rows = n_rows;
+    }
+    const int bc = wide ? 256 : 128, box = gathered ? GM : kind == MOE_GATEUP ? bc / 2 : bc;
+    CUtensorMap ma, mb0, mb1, mo;
+    int rc = make_map(a, a_rows, K, down || gathered ? GM : 1, &ma);       // a gather's box is one row high
     if (rc) return rc;
     rc = make_map(b0, E * N, K, box, &mb0);
     if (rc) return rc;
     mb1 = mb0;
     if (kind == MOE_GATEUP && (rc = make_map(b1, E * N, K, box, &mb1))) return rc;
+    if (gathered && (rc = make_map(out, n_rows, N, 32, &mo, down ? 4 : 2))) return rc;
     GroupedArgs g{src_tok, seg, tile_expert, tile_row0, n_tiles, row_w, out, N, K, limit, act, status};
-#define FF_GROUPED(KIND) return wide ? grouped_launch<KIND, 256>(ma, mb0, mb1, g, max_tiles, stream) \
+    ++*launched;
+#define FF_GROUPED(KIND) return gathered ? grouped_pair_launch<KIND>(ma, mb0, mb1, mo, g, E, max_tiles, stream) \
+                              : wide ? grouped_launch<KIND, 256>(ma, mb0, mb1, g, max_tiles, stream) \
                                      : grouped_launch<KIND, 128>(ma, mb0, mb1, g, max_tiles, stream)
     if (kind == MOE_GATEUP) FF_GROUPED(MOE_GATEUP);
     if (kind == MOE_UP) FF_GROUPED(MOE_UP);

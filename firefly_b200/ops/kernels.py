@@ -1068,6 +1068,11 @@ def latent_gate(val, g, y, heads: int, vdim: int, per_head: bool = False) -> Non
 # --------------------------------------------------------------------------- #
 # routed experts (csrc/moe.cu)
 MOE_WIDE_BLOCKS_PER_SM = 1.5   # tiles of 256 weight rows a block as soon as they come to this many blocks an SM, else of 128
+# Pairs of SMs from this many rows an expert on.  us for the first (gate|up, with its gather) and second product, one block / pairs:
+# 16 experts of 512 x 1024: 75 rows an expert 18.9 + 13.7 / 18.5 + 13.5, 150 24.3 + 13.6 / 18.4 + 13.9, 2048 99.6 + 77.8 / 77.1 + 47.9;
+# 32 experts: 75 19.7 + 12.0 / 26.1 + 15.4, 150 27.6 + 20.2 / 27.1 + 16.9; 16 of 1024 x 2048: 75 34.6 + 13.0 / 37.5 + 19.6, 150
+# 48.9 + 26.8 / 41.5 + 21.4, 2048 324 + 207 / 241 + 123.
+MOE_PAIR_ROWS = 128
 MOE_FORCE_PLAIN = False     # tests flip this to hold the tensor-core grouped product against the plain one
 
 
@@ -1086,6 +1091,11 @@ ROUTE_SOFTMAX, ROUTE_SIGMOID, ROUTE_CHOSEN_SOFTMAX = 0, 1, 2   # how router logi
 GROUP_BY_BEST, GROUP_BY_TWO_BEST = 0, 1        # a group's score: its largest choice score, or the sum of its two largest
 GLU_CLAMPED_SWISH, GLU_SILU = 0, 1             # an expert's activation (gated experts)
 MOE_DOWN, MOE_GATE_UP, MOE_UP = 0, 1, 2        # the grouped products: second one, first one of gated / ungated experts
+
+
+def moe_on_pairs(rows: int, E: int, N: int) -> bool:
+    """True if a grouped product runs on pairs of SMs (256 rows x 256 matrix rows a tile)."""
+    return rows >= MOE_PAIR_ROWS * E and N % 8 == 0
 
 
 def moe_route(z, ids, wts, groups: int, keep: int, *, score: int = ROUTE_SOFTMAX, correction=None,
@@ -1131,14 +1141,15 @@ def moe_plan(ids, E: int, seg, row_of, src_tok, tile_expert, tile_row0, n_tiles,
 
 def moe_grouped(a, src_tok, b0, b1, plan, out, limit: float = 0.0, tensor_cores: bool = False,
                 act: int = GLU_CLAMPED_SWISH, kind: Optional[int] = None, row_w=None,
-                status: Optional[torch.Tensor] = None) -> None:
+                status: Optional[torch.Tensor] = None, gathered: Optional[torch.Tensor] = None) -> None:
     """Grouped product over the experts' stacked matrices.  With ``b1`` (gate|up): rows of ``a`` [T,K] gathered
     by src_tok, b0/b1 [E,N,K], out[row] = g * sigmoid(1.702 g) * (u + 1) with the clamps of ``limit``
     (``act`` GLU_CLAMPED_SWISH) or silu(g) * u (GLU_SILU), in a's type.  Without: a [rows,K] in place, out float32 [rows,N];
     or, with ``kind`` MOE_UP (experts without a gate), gathered rows and out[row] = relu(u)^2 in a's type.  ``row_w`` float32
     [rows] (first products): a row's products are multiplied by it in front of the activation.  ``plan`` = (seg, tile_expert, tile_row0, n_tiles,
     max_tiles), made with the same ``tensor_cores``: a tensor-core kernel (bfloat16, K % 8 == 0) or the plain one.
-    The tensor-core kernel (tcgen05) needs ``status`` (int32 [1]: where a wait that runs out is told)."""
+    The tensor-core kernel (tcgen05) needs ``status`` (int32 [1]: where a wait that runs out is told).  ``gathered`` [rows, K]: scratch for
+    a first product's rows side by side, without which it does not go to pairs of SMs (`moe_on_pairs`)."""
     seg, tile_expert, tile_row0, n_tiles, max_tiles = plan
     _need_cuda(a, src_tok, b0, b1, out, row_w)
     if kind is None:
@@ -1153,10 +1164,19 @@ def moe_grouped(a, src_tok, b0, b1, plan, out, limit: float = 0.0, tensor_cores:
         if status is None:
             raise KernelError("moe_grouped: the tensor-core kernel needs a status word")
         cols = 128 if kind == MOE_GATE_UP else 256
-        _check(_lib("moe_tcgen05").ff_moe_grouped_tc(
+        rows = out.shape[0]
+        pairs = moe_on_pairs(rows, E, N) and (kind == MOE_DOWN or gathered is not None)
+        if pairs and kind != MOE_DOWN:
+            _need_cuda(gathered)
+            assert gathered.dtype == a.dtype and gathered.shape == (rows, Kd)
+        launched = c_int()
+        code = _lib("moe_tcgen05").ff_moe_grouped_tc(
             _p(a), c_int(a.shape[0]), _p(src_tok), _p(b0), _p(b1), c_int(E), c_int(kind), _p(seg), _p(tile_expert), _p(tile_row0),
             _p(n_tiles), _p(row_w), _p(out), c_int(max_tiles), c_int(N), c_int(Kd), c_float(limit), c_int(act),
-            c_int(1 if max_tiles * -(-N // cols) >= MOE_WIDE_BLOCKS_PER_SM * sm_count() else 0), _p(status), _stream()), "moe_grouped_tc")
+            c_int(1 if max_tiles * -(-N // cols) >= MOE_WIDE_BLOCKS_PER_SM * sm_count() else 0),
+            _p((a if kind == MOE_DOWN else gathered) if pairs else None), c_int(rows), _p(status), ctypes.byref(launched), _stream())
+        _check(code, "moe_grouped_tc")
+        _count_kernels(launched)
         return
     _check(_lib("moe").ff_moe_grouped(_p(a), _p(src_tok), _p(b0), _p(b1), c_int(_dt(a)), c_int(kind),
                                      _p(seg), _p(tile_expert), _p(tile_row0), _p(n_tiles), _p(row_w), _p(out), c_int(max_tiles),

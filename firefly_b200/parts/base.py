@@ -190,8 +190,8 @@ class Part:
         return []
 
     def step_scratch_bytes(self, tokens: int, sequences: int) -> int:
-        """Scratch memory beyond activations that a step of so many tokens and sequences takes if it is there (a recurrence's records
-        of chunks, `scan.records`); the engine leaves room for it when it sizes the cache."""
+        """Scratch memory beyond activations that a step of so many tokens and sequences takes if it is there (`scan.records`: a recurrence's
+        records of chunks, the rows of routed experts); the engine leaves room for it when it sizes the cache."""
         return 0
 
     def bind(self, tensors: Mapping[str, torch.Tensor]) -> None:

@@ -152,6 +152,14 @@ class GroupedExperts(Part):
                 else self._matrix(tensors[self.name("shared.up")])
             self.w_sh_down = self._matrix(tensors[self.name("shared.down")])
 
+    def _gathered_bytes(self, rows: int, dtype: torch.dtype) -> int:
+        """Scratch that the first product uses for its rows side by side (0: it picks them one by one)."""
+        on_pairs = K.moe_on_tensor_cores(dtype, (self.hidden, self.ff)) and K.moe_on_pairs(rows, self.E, self.ff)
+        return rows * self.hidden * 2 if on_pairs else 0
+
+    def step_scratch_bytes(self, tokens: int, sequences: int) -> int:
+        return self._gathered_bytes(tokens * self.top, self.rt.dtype)
+
     def forward(self, x, ctx, accumulate_into=None, residual_scale: float = 1.0, as_rows: bool = False):
         T, ws, W, top = x.shape[0], ctx.workspace, self.hidden, self.top
         dt = self.w_up.dtype
@@ -177,10 +185,15 @@ class GroupedExperts(Part):
         K.moe_plan(ids, self.E, seg, row_of, src_tok, tile_e, tile_r, n_tiles, tc, wts if self.weight_on_input else None, row_w)
         plan = (seg, tile_e, tile_r, n_tiles, max_tiles)
         act = ws.get("moe.act", (rows, self.ff), dt)
+        need = self._gathered_bytes(rows, dt)
+        gathered = ws.try_get("scan.records", (need // 4,), torch.float32) if need else None
+        if gathered is not None:
+            gathered = gathered.view(dt).view(rows, W)
         if self.gated:
-            K.moe_grouped(x, src_tok, self.w_gate, self.w_up, plan, act, self.limit, tc, self.activation, row_w=row_w, status=ctx.status)
+            K.moe_grouped(x, src_tok, self.w_gate, self.w_up, plan, act, self.limit, tc, self.activation, row_w=row_w, status=ctx.status,
+                          gathered=gathered)
         else:
-            K.moe_grouped(x, src_tok, self.w_up, None, plan, act, 0.0, tc, kind=K.MOE_UP, row_w=row_w, status=ctx.status)
+            K.moe_grouped(x, src_tok, self.w_up, None, plan, act, 0.0, tc, kind=K.MOE_UP, row_w=row_w, status=ctx.status, gathered=gathered)
         outs = ws.get("moe.rows", (rows, W), torch.float32)
         K.moe_grouped(act, src_tok, self.w_down, None, plan, outs, 0.0, tc, status=ctx.status)
         shared = None

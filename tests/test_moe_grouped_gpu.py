@@ -103,6 +103,41 @@ def test_rows_do_not_depend_on_what_shares_their_tile(monkeypatch):
     assert all(torch.equal(first, v) for v in got.values())
 
 
+@pytest.mark.parametrize("skew", [False, True])
+@pytest.mark.parametrize("shape", SHAPES + [(2500, 4, 2, 320, 264), (1200, 40, 4, 64, 512)])
+def test_pairs_of_sms_give_the_bits_of_single_blocks(shape, skew, monkeypatch):
+    """Tiles of 256 rows over two SMs: every kind, experts of no, few and many rows, more tiles than pairs and fewer; the results
+    are those of the one-block kernel, which the test above holds against 64 bits."""
+    from firefly_b200.ops import kernels as K
+    T, E, top, W, F = shape
+    if skew and top > (E + 1) // 2:
+        pytest.skip("not enough experts for the skewed choice")
+    x, ids, gate, up, down, wts = (t.cuda() for t in _case(T, E, top, W, F, T + E, skew))
+    n = T * top
+    tiles = K.moe_max_tiles(n, E, True)
+    i32 = dict(dtype=torch.int32, device="cuda")
+    seg, row_of, src, te, tr, nt = (torch.empty(k, **i32) for k in (E + 1, n, n, tiles, tiles, 1))
+    row_w, status = torch.empty(n, device="cuda"), torch.zeros(1, **i32)
+    K.moe_plan(ids, E, seg, row_of, src, te, tr, nt, True, wts, row_w)
+    act_rows = torch.randn(n, F, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).cuda()
+    got = {}
+    for pairs in (0, 1 << 30):
+        monkeypatch.setattr(K, "MOE_PAIR_ROWS", pairs)
+        outs = []
+        for kind, act, weighted in (("gate_up", 0, False), ("gate_up", 1, True), ("up", 0, True), ("down", 0, False)):
+            first = kind != "down"
+            out = torch.full((n, F if first else W), float("nan"), dtype=torch.bfloat16 if first else torch.float32, device="cuda")
+            b0, b1 = {"gate_up": (gate, up), "up": (up, None), "down": (down, None)}[kind]
+            room = torch.full((n, W), float("nan"), dtype=torch.bfloat16, device="cuda")
+            K.moe_grouped(x if first else act_rows, src, b0, b1, (seg, te, tr, nt, tiles), out, 0.8, True, act=act,
+                          kind=K.MOE_UP if kind == "up" else None, row_w=row_w if weighted else None, status=status, gathered=room)
+            outs.append(out)
+        got[pairs] = outs
+    assert int(status[0]) == 0
+    for a, b in zip(*got.values()):
+        assert not torch.isnan(a).any() and torch.equal(a, b)
+
+
 @pytest.mark.parametrize("T,E,top", [(1, 3, 1), (5, 4, 4), (700, 11, 3), (1024, 16, 4), (1025, 16, 4), (3000, 300, 2), (16384, 16, 4), (2111, 5, 2)])
 @pytest.mark.parametrize("tc", [True, False])
 def test_the_plan_sorts_every_choice_by_expert(T, E, top, tc):
