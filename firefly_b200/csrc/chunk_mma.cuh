@@ -9,6 +9,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "scan_wide.cuh"
 
 namespace ff {
 
@@ -28,6 +29,25 @@ __device__ __forceinline__ void cm_mma(float c[4], const uint32_t a[4], const ui
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
+// c += x and the columns of c times a pair, two columns an instruction: the warps of a walk have an instruction every second clock and
+// no more, so what is not a product counts too
+__device__ __forceinline__ void cm_add(float c[4], const float x[4]) {
+#pragma unroll
+    for (int e = 0; e < 4; e += 2) {
+        const f32x2 r = f2_add(f2_pack(c[e], c[e + 1]), f2_pack(x[e], x[e + 1]));
+        c[e] = f2_low(r);
+        c[e + 1] = f2_high(r);
+    }
+}
+__device__ __forceinline__ void cm_scale(float c[4], f32x2 by) {
+#pragma unroll
+    for (int e = 0; e < 4; e += 2) {
+        const f32x2 r = f2_mul(f2_pack(c[e], c[e + 1]), by);
+        c[e] = f2_low(r);
+        c[e + 1] = f2_high(r);
+    }
+}
+
 // c + small += A B with A held in NA parts and B in NB (1: bfloat16 as it is, 3: split).  The tensor core cuts its sums off
 // instead of rounding them, always toward zero, and a chain of products on one accumulator adds that up.  So the products of
 // the leading parts, which are 16 bits long and lose next to nothing among themselves, start from zero every time and are
@@ -43,7 +63,7 @@ __device__ __forceinline__ void cm_mma_parts(float c[4], float small[4], const u
         for (int j = NB - 1; j >= 0; --j)
             if (i + j == 1 || i + j == 2) cm_mma(small, a[i], b[j]);
     }
-    c[0] += t[0]; c[1] += t[1]; c[2] += t[2]; c[3] += t[3];
+    cm_add(c, t);
 }
 // The same for two neighbouring tiles of eight columns, their right operand as ldmatrix gives it: r[part] = two registers of the
 // first tile, two of the second.
@@ -55,7 +75,6 @@ __device__ __forceinline__ void cm_mma_rows(float c[2][4], float small[2][4], co
     cm_mma_parts<NA, NB>(c[0], small[0], a, b0);
     cm_mma_parts<NA, NB>(c[1], small[1], a, b1);
 }
-__device__ __forceinline__ void cm_add(float c[4], const float x[4]) { c[0] += x[0]; c[1] += x[1]; c[2] += x[2]; c[3] += x[3]; }
 
 __device__ __forceinline__ uint32_t cm_pack(float lo, float hi) {      // (lo in the low half)
     uint32_t r;
@@ -67,13 +86,12 @@ __device__ __forceinline__ float cm_hi(uint32_t p) { return __uint_as_float(p & 
 
 // (x, y) as three packed pairs of bfloat16
 __device__ __forceinline__ void cm_split3(float x, float y, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
+    const f32x2 minus = f2_pack(-1.f, -1.f);
     p0 = cm_pack(x, y);
-    x -= cm_lo(p0);
-    y -= cm_hi(p0);
-    p1 = cm_pack(x, y);
-    x -= cm_lo(p1);
-    y -= cm_hi(p1);
-    p2 = cm_pack(x, y);
+    f32x2 rest = f2_fma(f2_pack(cm_lo(p0), cm_hi(p0)), minus, f2_pack(x, y));
+    p1 = cm_pack(f2_low(rest), f2_high(rest));
+    rest = f2_fma(f2_pack(cm_lo(p1), cm_hi(p1)), minus, rest);
+    p2 = cm_pack(f2_low(rest), f2_high(rest));
 }
 
 // is one of the two bfloat16 numbers of `p` an infinity or not a number?

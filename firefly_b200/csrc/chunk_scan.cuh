@@ -15,22 +15,29 @@
 
 #include "chunk_mma.cuh"
 
+#include <type_traits>
+
 namespace ff {
 
 constexpr int CS_C = 16;                                    // tokens a chunk
-// Records a block of the first kernel forms, one behind the other (the next one's inputs are on their way while it forms one): up
-// to four while that leaves every SM eight blocks, else one, so that short steps do not leave SMs idle.
-static inline int chunk_records_a_block(long long records_and_heads) { return records_and_heads >= 4 * 8 * 148 ? 4 : 1; }
-
+// A record: rows side by side, so that whole sectors are written (with the pitch that shared memory wants,
+// which made rows straddle them, the first kernels took 67 us instead of 46, 40 instead of 31 and 102 instead of 82).
 template <int NK, bool DELTA>
 struct ChunkRecord {
-    static constexpr int QP = NK + 8, PP = CS_C + 8;        // row pitches: 16-byte pieces of eight rows lie in different banks
-    bf16 qe[3][CS_C * QP];                                  // q E (the decays in front of the token for a read-out in front of the write)
-    bf16 kf[3][CS_C * QP];                                  // k F
-    bf16 P[3][CS_C * PP];
+    bf16 qe[3][CS_C * NK];                                  // q E (the decays in front of the token for a read-out in front of the write)
+    bf16 kf[3][CS_C * NK];                                  // k F
+    bf16 P[3][CS_C * CS_C];
     float G[NK];
-    bf16 ke[DELTA ? 3 : 1][DELTA ? CS_C * QP : 8];          // k E
-    bf16 TB[DELTA ? 3 : 1][DELTA ? CS_C * PP : 8];          // T diag(beta)
+    bf16 ke[DELTA ? 3 : 1][DELTA ? CS_C * NK : 8];          // k E
+    bf16 TB[DELTA ? 3 : 1][DELTA ? CS_C * CS_C : 8];        // T diag(beta)
+};
+// The same as the walk has it in shared memory.
+template <int NK, bool DELTA>
+struct ChunkRows {
+    static constexpr int QP = NK + 8, PP = CS_C + 8;        // row pitches: 16-byte pieces of eight rows lie in different banks
+    bf16 qe[3][CS_C * QP], kf[3][CS_C * QP], P[3][CS_C * PP];
+    float G[NK];
+    bf16 ke[DELTA ? 3 : 1][DELTA ? CS_C * QP : 8], TB[DELTA ? 3 : 1][DELTA ? CS_C * PP : 8];
 };
 
 // With chunks of C tokens, a sequence that starts at token t0 of the step and is number s has its records from here on; at
@@ -56,201 +63,203 @@ static inline ChunkRoute chunk_route(bool possible, int n_long, int n_seqs, int 
     return {chunks, !chunks || n_long != n_seqs, n_long > 0 ? n_long : n_seqs, chunks ? chunk_min : 0x7fffffff};
 }
 
-// The sequence and chunk of record r (chunk -1: none); all lanes of a warp ask together.
+// The sequence and chunk of record r (chunk -1: none), the chunk's first token and how many the sequence has from there on; all lanes of
+// a warp ask together, and the sequence's borders come from the lanes that have read them.
 template <int C = CS_C>
-__device__ __forceinline__ void chunk_of_record(const int* cu_q, int n_seqs, int r, int min_len, int& s, int& chunk) {
+__device__ __forceinline__ void chunk_of_record(const int* cu_q, int n_seqs, int r, int min_len, int& s, int& chunk, int& row0, int& left) {
     const int lane = threadIdx.x & 31;
+    int begin = 0, end = 0;
     s = -1;
     for (int s0 = 0; s0 < n_seqs; s0 += 32) {
-        const bool mine = s0 + lane < n_seqs && chunk_first_record<C>(cu_q[s0 + lane], s0 + lane) <= r;
-        const unsigned m = __ballot_sync(0xffffffffu, mine);
-        if (m) s = s0 + 31 - __clz(m);
+        const int i = min(s0 + lane, n_seqs - 1), at = cu_q[i], next = cu_q[i + 1];
+        const unsigned m = __ballot_sync(0xffffffffu, s0 + lane < n_seqs && chunk_first_record<C>(at, s0 + lane) <= r);
+        if (m) {
+            const int l = 31 - __clz(m);
+            s = s0 + l;
+            begin = __shfl_sync(0xffffffffu, at, l);
+            end = __shfl_sync(0xffffffffu, next, l);
+        }
         if (m != 0xffffffffu) break;
     }
     chunk = -1;
+    row0 = left = 0;
     if (s >= 0) {
-        const int i = r - chunk_first_record<C>(cu_q[s], s);
-        const int len = cu_q[s + 1] - cu_q[s];
-        if (len >= min_len && i * C < len) chunk = i;
+        const int i = r - chunk_first_record<C>(begin, s);
+        if (end - begin >= min_len && i * C < end - begin) {
+            chunk = i;
+            row0 = begin + i * C;
+            left = end - row0;
+        }
     }
 }
 
 // ---------------------------------------------------------------------------------- the first kernel's parts --
-// sq, sk, sa: the chunk's q, k and decays in shared memory, [16][NK] 32-bit; rows behind the sequence's end have q = k = 0 and
-// decay 1.  2 NK threads.
+// A warp forms 64 key channels of a record, two a lane, all sixteen tokens: NK / 64 warps a record, CF_WARPS warps a block.  Token
+// after token in registers: d_s, k of an earlier token times the decays since, is all that P needs of it, and k F in the end; a row
+// of P is the lanes' shares of q_t d_s, joined by shuffles that halve the sums a lane still adds up.
+// Formed out of rows in shared memory with a thread a token and eight channels, the same rows were read once for every token in front:
+// 90 % of the shared-memory pipe.  What bounds it now are some 2400 instructions a warp (delta rule: 5900, the decays' logarithms
+// and exponentials among them) and the 16 to 20 warps an SM that their registers leave to hide waits with.
+// us, before / now: wkv, 4900 tokens of 32 heads of 64 74.4 / 46, channel decays, 3000 tokens of 16 heads of 64 46.1 / 31, delta rule, 8192 tokens of 8
+// heads of 128 136 / 82.  (The delta rule with its rows in registers, as the other two have them, took a tenth longer; the other two with
+// theirs in shared memory are no faster and keep the second kernel's blocks off the SMs until they end: 12 us longer for wkv.)
+constexpr int CF_WARPS = 4;
+template <int NK> constexpr int cf_warps_a_record() { return NK / 64; }
+template <int NK> constexpr int cf_records() { return CF_WARPS / cf_warps_a_record<NK>(); }
+template <int NK> static inline dim3 cf_grid(int n_records, int heads) { return dim3((unsigned)((n_records + cf_records<NK>() - 1) / cf_records<NK>()), (unsigned)heads); }
 
-// A thread's eight neighbouring elements of a chunk: row tid / (NK / 8), columns 8 (tid % (NK / 8)) ..
-__device__ __forceinline__ void chunk_unpack(const uint4& v, float x[8]) {
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) { x[2 * i] = cm_lo(w[i]); x[2 * i + 1] = cm_hi(w[i]); }
-}
-__device__ __forceinline__ void chunk_stage8(float* to, const float x[8]) {
-    *reinterpret_cast<float4*>(to) = make_float4(x[0], x[1], x[2], x[3]);
-    *reinterpret_cast<float4*>(to + 4) = make_float4(x[4], x[5], x[6], x[7]);
-}
-
-// The chunk's two halves of eight tokens, each row scaled to the border between them: a pair of tokens on either side of it
-// needs no more than the product of these rows.
 template <int NK, bool DELTA>
-struct ChunkHalves {
-    static constexpr int HP = NK + 4;                       // row pitch: 16-byte pieces of eight rows lie in different banks
-    float q[CS_C / 2][HP], k[CS_C / 2][HP];                 // tokens 8..: q times the decays of 8 ..; tokens ..7: k times the ones behind it up to 7
-    float k_late[DELTA ? CS_C / 2 : 1][DELTA ? HP : 4];     // tokens 8..: k as q
+struct ChunkForm {                                          // of one record
+    static constexpr int PITCH = CS_C + 4;
+    struct Rows { uint32_t q[DELTA ? CS_C : 1][32], k[DELTA ? CS_C : 1][32]; float2 a[DELTA ? CS_C : 1][32]; };       // a warp's 64 channels, two a lane
+    Rows rows[DELTA ? cf_warps_a_record<NK>() : 1];
+    float P[cf_warps_a_record<NK>()][CS_C][PITCH];          // each warp's share of q_t d_s, s <= t
+    float M[DELTA ? cf_warps_a_record<NK>() : 1][DELTA ? CS_C : 1][PITCH];         // and of k_t d_s, s < t; then T diag(beta)
+    float sums[DELTA ? cf_warps_a_record<NK>() : 1][32];    // of q^2 and k^2 of the tokens
+    float2 unit[DELTA ? CS_C : 1];                          // what q and k are multiplied by
+    float beta[DELTA ? CS_C : 1];
 };
-
-// q E, k F, k E and G, and the halves.  Thread (pair of channels, side, half of the tokens).  BEFORE: E without the token's own decay.
-template <int NK, bool DELTA, bool BEFORE>
-__device__ __forceinline__ void chunk_scaled_rows(ChunkRecord<NK, DELTA>* rec, ChunkHalves<NK, DELTA>& hs, const float* sq, const float* sk, const float* sa) {
-    using R = ChunkRecord<NK, DELTA>;
-    constexpr int H = CS_C / 2, PW = R::QP / 2, PART = CS_C * PW;
-    const int n = 2 * (threadIdx.x % (NK / 2)), side = threadIdx.x / (NK / 2) & 1, half = threadIdx.x / NK;
-    auto decay = [&](int t) { return *reinterpret_cast<const float2*>(sa + t * NK + n); };
-    auto put = [&](bf16* to, int t, float x, float y) {
-        uint32_t* dst = reinterpret_cast<uint32_t*>(to) + t * PW + n / 2;
-        cm_split3(x, y, dst[0], dst[PART], dst[2 * PART]);
-    };
-    float2 base = make_float2(1.f, 1.f), e = base;          // the decays of the half that lies between, and those within the own half
-    if (side == 0) {                                        // products from the chunk's start
-        if (half) {
-#pragma unroll
-            for (int t = 0; t < H; ++t) { const float2 a = decay(t); base.x *= a.x; base.y *= a.y; }
-        }
-#pragma unroll
-        for (int i = 0; i < H; ++i) {
-            const int t = half * H + i;
-            const float2 a = decay(t), q = *reinterpret_cast<const float2*>(sq + t * NK + n);
-            const float2 out = e;
-            e.x *= a.x;
-            e.y *= a.y;
-            const float2 r = BEFORE ? make_float2(q.x * out.x, q.y * out.y) : make_float2(q.x * e.x, q.y * e.y);
-            put(rec->qe[0], t, r.x * base.x, r.y * base.y);
-            if (half) *reinterpret_cast<float2*>(&hs.q[i][n]) = r;
-            if constexpr (DELTA) {
-                const float2 k = *reinterpret_cast<const float2*>(sk + t * NK + n);
-                put(rec->ke[0], t, k.x * e.x * base.x, k.y * e.y * base.y);
-                if (half) *reinterpret_cast<float2*>(&hs.k_late[i][n]) = make_float2(k.x * e.x, k.y * e.y);
-            }
-        }
-        if (half) *reinterpret_cast<float2*>(&rec->G[n]) = make_float2(e.x * base.x, e.y * base.y);
-    } else {                                                // products to the chunk's end
-        if (!half) {
-#pragma unroll
-            for (int t = CS_C - 1; t >= H; --t) { const float2 a = decay(t); base.x *= a.x; base.y *= a.y; }
-        }
-#pragma unroll
-        for (int i = H - 1; i >= 0; --i) {
-            const int t = half * H + i;
-            const float2 a = decay(t), k = *reinterpret_cast<const float2*>(sk + t * NK + n);
-            const float2 r = make_float2(k.x * e.x, k.y * e.y);
-            put(rec->kf[0], t, r.x * base.x, r.y * base.y);
-            if (!half) *reinterpret_cast<float2*>(&hs.k[i][n]) = r;
-            e.x *= a.x;
-            e.y *= a.y;
-        }
-    }
+// all warps of the thread's record
+template <int NK> __device__ __forceinline__ void cf_sync() {
+    if constexpr (NK == 64) __syncwarp();
+    else cm_barrier(1 + threadIdx.x / (NK / 2), NK / 2);
 }
 
-// Pairs of tokens of one half: sum_n q_t[n] k_s[n] prod(decays of s+1 .. t) for s <= t (BEFORE: .. t-1, and sum_n q_t[n] k_s[n] u[n]
-// for s = t), zero else; with DELTA also the same of k_t.  Thread (s, eight channels) walks the half's tokens; the channels'
-// shares are joined over NK / 8 neighbouring threads, which ends with one token each: put(t, s, of q, of k).
-template <int NK, bool DELTA, bool BEFORE, typename Put>
-__device__ __forceinline__ void chunk_near_pairs(const float* sq, const float* sk, const float* sa, const float* u, Put put) {
-    constexpr int L = NK / 8, H = CS_C / 2;
-    const int part = threadIdx.x % L, s = threadIdx.x / L, t0 = s & H, ls = s & (H - 1), n = part * 8;
-    float d[8], x[H], y[DELTA ? H : 1] = {};
-    auto row8 = [&](const float* m, int t, float v[8]) {
-        *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(m + t * NK + n);
-        *reinterpret_cast<float4*>(v + 4) = *reinterpret_cast<const float4*>(m + t * NK + n + 4);
-    };
-    row8(sk, s, d);
+__device__ __forceinline__ f32x2 cf_pair(uint32_t p) { return f2_pack(cm_lo(p), cm_hi(p)); }
+
+// Asks for a warp's rows of q and k (bfloat16) and, with DECAYS, of what the decays are made of (32-bit): the `left` first of sixteen
+// tokens, zeros behind them.  q, k, a: the warp's first channel of the chunk's first token; rows on 16 bytes.
+template <bool DECAYS, typename Rows>
+__device__ __forceinline__ void cf_fetch(Rows& to, const bf16* q, size_t q_stride, const bf16* k, size_t k_stride, const float* a, size_t a_stride, int left) {
+    const int lane = threadIdx.x & 31;
 #pragma unroll
-    for (int i = 0; i < H; ++i) {
-        float q[8], a[8], k[8], p0 = 0.f, p1 = 0.f, r0 = 0.f, r1 = 0.f;
-        row8(sq, t0 + i, q);
-        row8(sa, t0 + i, a);
-        if constexpr (DELTA) row8(sk, t0 + i, k);
-#pragma unroll
-        for (int c = 0; c < 8; c += 2) {
-            if (!BEFORE) { d[c] *= i > ls ? a[c] : 1.f; d[c + 1] *= i > ls ? a[c + 1] : 1.f; }
-            if constexpr (BEFORE) {
-                p0 += q[c] * (i == ls ? d[c] * u[n + c] : d[c]);
-                p1 += q[c + 1] * (i == ls ? d[c + 1] * u[n + c + 1] : d[c + 1]);
-            } else {
-                p0 += q[c] * d[c];
-                p1 += q[c + 1] * d[c + 1];
-            }
-            if constexpr (DELTA) { r0 += k[c] * d[c]; r1 += k[c + 1] * d[c + 1]; }
-            if (BEFORE) { d[c] *= i > ls ? a[c] : 1.f; d[c + 1] *= i > ls ? a[c + 1] : 1.f; }
-        }
-        x[i] = i >= ls ? p0 + p1 : 0.f;
-        if constexpr (DELTA) y[i] = r0 + r1;
+    for (int i = 0; i < 4; ++i) {
+        const int t = i * 4 + (lane >> 3), c = lane & 7;
+        const bool in = t < left;
+        cm_copy16(&to.q[t][c * 4], q + (in ? t * q_stride + c * 8 : 0), in);
+        cm_copy16(&to.k[t][c * 4], k + (in ? t * k_stride + c * 8 : 0), in);
     }
-    int t = t0, off = 1;
+    if (DECAYS) {
 #pragma unroll
-    for (int m = H / 2; m >= 1; m >>= 1) {                  // every step halves the tokens a thread still adds up
-        const bool up = part & off;
+        for (int i = 0; i < 8; ++i) {
+            const int t = i * 2 + (lane >> 4), c = lane & 15;
+            const bool in = t < left;
+            cm_copy16(&to.a[t][c * 2], a + (in ? t * a_stride + c * 4 : 0), in);
+        }
+    }
+    cm_copy_commit();
+    cm_copy_wait<0>();
+    __syncwarp();
+}
+
+// v[0 .. V) summed over groups of LANES lanes; a lane keeps the sum cf_kept<V>(lane).
+template <int V, int LANES>
+__device__ __forceinline__ float cf_join(float (&v)[CS_C]) {
+    const int lane = threadIdx.x & 31;
+    int off = 1;
+#pragma unroll
+    for (int m = V / 2; m >= 1; m >>= 1) {
+        const bool up = lane & off;
 #pragma unroll
         for (int i = 0; i < m; ++i) {
-            const float away = up ? x[i] : x[i + m];
-            x[i] = (up ? x[i + m] : x[i]) + __shfl_xor_sync(0xffffffffu, away, off);
-            if constexpr (DELTA) {
-                const float away_y = up ? y[i] : y[i + m];
-                y[i] = (up ? y[i + m] : y[i]) + __shfl_xor_sync(0xffffffffu, away_y, off);
-            }
+            const float away = up ? v[i] : v[i + m];
+            v[i] = (up ? v[i + m] : v[i]) + __shfl_xor_sync(0xffffffffu, away, off);
         }
-        if (up) t += m;
         off <<= 1;
     }
 #pragma unroll
-    for (; off < L; off <<= 1) {
-        x[0] += __shfl_xor_sync(0xffffffffu, x[0], off);
-        if constexpr (DELTA) y[0] += __shfl_xor_sync(0xffffffffu, y[0], off);
-    }
-    if (part < H) put(t, s, x[0], DELTA ? y[0] : 0.f);
+    for (; off < LANES; off <<= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
+    return v[0];
+}
+template <int V> __device__ __forceinline__ int cf_kept(int lane) {
+    int i = 0, m = V / 2;
+#pragma unroll
+    for (int off = 1; off < V; off <<= 1, m >>= 1) i += (lane & off) ? m : 0;
+    return i;
 }
 
-// Pairs across the border: token 8 + i and token s, a thread 32 channels of one pair.
-template <int NK, bool DELTA, typename Put>
-__device__ __forceinline__ void chunk_far_pairs(const ChunkHalves<NK, DELTA>& hs, Put put) {
-    constexpr int L = NK / 32, H = CS_C / 2;
-    const int part = threadIdx.x % L, s = threadIdx.x / L % H, i = threadIdx.x / (L * H);
-    float p0 = 0.f, p1 = 0.f, r0 = 0.f, r1 = 0.f;
+// The lane's two channels (of the warp's 64) of q E, k E, k F and G into the record, and the shares of P (and M) into sh.  token(t): q, k
+// and the decays of the lane's channels.  BEFORE: the read-out sees the state in front of the token's own decay and write, and its
+// own write by u.
+template <int NK, bool DELTA, bool BEFORE, typename Token>
+__device__ __forceinline__ void chunk_form(ChunkRecord<NK, DELTA>* rec, ChunkForm<NK, DELTA>& sh, int warp, f32x2 u, Token token) {
+    constexpr int PW = NK / 2, PART = CS_C * PW;
+    const int lane = threadIdx.x & 31, col = warp * 32 + lane;
+    auto put = [&](bf16* to, int t, f32x2 v) {
+        uint32_t* dst = reinterpret_cast<uint32_t*>(to) + t * PW + col;
+        cm_split3(f2_low(v), f2_high(v), dst[0], dst[PART], dst[2 * PART]);
+    };
+    f32x2 d[CS_C], E = f2_pack(1.f, 1.f), q, k, a, q_next, k_next, a_next;
+    token(0, q_next, k_next, a_next);
 #pragma unroll
-    for (int c = 0; c < 32; c += 4) {
-        const int n = c * L + part * 4;                     // neighbouring threads read neighbouring pieces
-        const float4 k = *reinterpret_cast<const float4*>(&hs.k[s][n]), q = *reinterpret_cast<const float4*>(&hs.q[i][n]);
-        p0 += q.x * k.x + q.y * k.y;
-        p1 += q.z * k.z + q.w * k.w;
+    for (int t = 0; t < CS_C; ++t) {
+        q = q_next;
+        k = k_next;
+        a = a_next;
+        if (t + 1 < CS_C) token(t + 1, q_next, k_next, a_next);        // in front of the writes of sums below, which the compiler must not pass
+        if (!BEFORE) {
+            E = f2_mul(E, a);
+#pragma unroll
+            for (int s = 0; s < t; ++s) d[s] = f2_mul(d[s], a);
+            d[t] = k;
+        }
+        put(rec->qe[0], t, f2_mul(q, E));
+        if constexpr (DELTA) put(rec->ke[0], t, f2_mul(k, E));
+        float x[CS_C], y[CS_C];
+#pragma unroll
+        for (int s = 0; s < CS_C; ++s) {
+            x[s] = s < t || (!BEFORE && s == t) ? f2_sum(f2_mul(q, d[s])) : 0.f;
+            if constexpr (DELTA) y[s] = s < t ? f2_sum(f2_mul(k, d[s])) : 0.f;
+        }
+        if constexpr (BEFORE) x[t] = f2_sum(f2_mul(f2_mul(q, u), k));
+        if constexpr (DELTA) {                              // half of the lanes go on with the sums of q, half with those of k
+            const bool other = lane & 16;
+#pragma unroll
+            for (int s = 0; s <= t; ++s) {
+                const float away = other ? x[s] : y[s];
+                x[s] = (other ? y[s] : x[s]) + __shfl_xor_sync(0xffffffffu, away, 16);
+            }
+        }
+        constexpr int L = DELTA ? 16 : 32;
+        float sum;
+        int at;
+        if (t == 0) { sum = cf_join<1, L>(x); at = cf_kept<1>(lane); }
+        else if (t < 2) { sum = cf_join<2, L>(x); at = cf_kept<2>(lane); }
+        else if (t < 4) { sum = cf_join<4, L>(x); at = cf_kept<4>(lane); }
+        else if (t < 8) { sum = cf_join<8, L>(x); at = cf_kept<8>(lane); }
+        else { sum = cf_join<16, L>(x); at = cf_kept<16>(lane); }
         if constexpr (DELTA) {
-            const float4 kl = *reinterpret_cast<const float4*>(&hs.k_late[i][n]);
-            r0 += kl.x * k.x + kl.y * k.y;
-            r1 += kl.z * k.z + kl.w * k.w;
+            if (lane & 16) sh.M[warp][t][at] = sum;
+            else sh.P[warp][t][at] = sum;
+        } else sh.P[warp][t][at] = sum;
+        if constexpr (BEFORE) {
+            E = f2_mul(E, a);
+#pragma unroll
+            for (int s = 0; s < t; ++s) d[s] = f2_mul(d[s], a);
+            d[t] = k;
         }
     }
-    float x = p0 + p1, y = r0 + r1;
 #pragma unroll
-    for (int off = 1; off < L; off <<= 1) {
-        x += __shfl_xor_sync(0xffffffffu, x, off);
-        if constexpr (DELTA) y += __shfl_xor_sync(0xffffffffu, y, off);
-    }
-    if (part == 0) put(H + i, s, x, y);
+    for (int t = 0; t < CS_C; ++t) put(rec->kf[0], t, d[t]);
+    *reinterpret_cast<float2*>(&rec->G[2 * col]) = make_float2(f2_low(E), f2_high(E));
 }
 
-// one number of a [16][16] matrix of a record, split
-__device__ __forceinline__ void chunk_put(bf16* to, int t, int s, float x) {
-    uint32_t p0, p1, p2;
-    cm_split3(x, 0.f, p0, p1, p2);
-    constexpr int pitch = CS_C + 8, part = CS_C * pitch;
-    const int at = t * pitch + s;
-    reinterpret_cast<uint16_t*>(to)[at] = (uint16_t)p0;
-    reinterpret_cast<uint16_t*>(to)[at + part] = (uint16_t)p1;
-    reinterpret_cast<uint16_t*>(to)[at + 2 * part] = (uint16_t)p2;
-}
-// the same of a pair across the border, with the zero on the other side of the diagonal
-__device__ __forceinline__ void chunk_put_far(bf16* to, int t, int s, float x) {
-    chunk_put(to, t, s, x);
-    chunk_put(to, t - CS_C / 2, s + CS_C / 2, 0.f);
+// A lower triangle of 16 x 16 (the sum of N shares) into its place in a record, split, with zeros above the diagonal; the record's threads.
+template <int NK, int N, int PITCH>
+__device__ __forceinline__ void chunk_emit(bf16* to, const float (*m)[CS_C][PITCH]) {
+    constexpr int PW = CS_C / 2, PART = CS_C * PW, THREADS = NK / 2;
+#pragma unroll
+    for (int i = 0; i < CS_C * CS_C / 2 / THREADS; ++i) {
+        const int idx = threadIdx.x % THREADS + i * THREADS, t = idx / (CS_C / 2), s = idx % (CS_C / 2) * 2;
+        float2 x = *reinterpret_cast<const float2*>(&m[0][t][s]);
+        if constexpr (N == 2) {
+            const float2 y = *reinterpret_cast<const float2*>(&m[1][t][s]);
+            x.x += y.x;
+            x.y += y.y;
+        }
+        uint32_t* dst = reinterpret_cast<uint32_t*>(to) + t * PW + s / 2;
+        cm_split3(s <= t ? x.x : 0.f, s + 1 <= t ? x.y : 0.f, dst[0], dst[PART], dst[2 * PART]);
+    }
 }
 
 // ---------------------------------------------------------------------------------- the second kernel --
@@ -293,7 +302,7 @@ __device__ __forceinline__ void chunk_lower(float (*tmp)[CS_C + 1], const float 
 
 template <int NK, int W, bool DELTA>
 struct ChunkScanSmem {
-    struct Stage { ChunkRecord<NK, DELTA> rec; bf16 v[CS_C * (16 * W + 8)]; };
+    struct Stage { ChunkRows<NK, DELTA> rec; bf16 v[CS_C * (16 * W + 8)]; };
     Stage stage[CS_STAGES];
     float xch[2][2 * W][DELTA ? 12 : 4][32];
     float slow[2 * W][16][CS_C + 1];
@@ -304,14 +313,19 @@ struct ChunkScanSmem {
 // products.  The two exchange their shares of S^T (q E) and S^T (k E); what follows of the read-out each does for eight of the
 // tokens.  Two more warps bring in records and values by 16-byte copies, two chunks ahead; one barrier a chunk.
 // (With all keys in one warp, which also did its own loads, a chunk took half as long again: 135 against 90 us for three
-// sequences of 1501, 1000 and 700 tokens with 16 heads of 64 x 128, 384 against 232 us for the delta rule on 4 x 2048 tokens.)
+// sequences of 1501, 1000 and 700 tokens with 16 heads of 64 x 128, 384 against 232 us for the delta rule on 4 x 2048 tokens.  With a
+// quarter of the keys in a warp and twice the warps: 139 against 107 and 242 against 216.  With the read-out of a chunk ended behind
+// the next one's barrier, so that only G S + (k F)^T v runs from chunk to chunk: 112 against 107, and as long for scalar decays.  What bounds a
+// chunk is neither that chain nor the tensor cores (half of their time) nor the copies (a stage more or two: the same) but two warps a
+// scheduler, which wait for their own instructions half of the time.)
 template <int NK, int W, bool DELTA>
 __global__ void __launch_bounds__(64 * W + CS_LOADERS) chunk_scan_kernel(ChunkScanArgs A) {
     pdl_prologue();
-    using R = ChunkRecord<NK, DELTA>;
+    using R = ChunkRows<NK, DELTA>;
+    using Record = ChunkRecord<NK, DELTA>;
     using SM = ChunkScanSmem<NK, W, DELTA>;
     constexpr int QP = R::QP, PP = R::PP, VB = 16 * W, VP = VB + 8, NT = NK / 16;
-    static_assert(sizeof(R) % 16 == 0, "a record is copied in 16-byte pieces");
+    static_assert(sizeof(Record) % 16 == 0 && sizeof(R) % 16 == 0, "a record is copied in 16-byte pieces");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SM& sm = *reinterpret_cast<SM*>(smem_raw);
     const int s = blockIdx.x, h = blockIdx.y, j0 = blockIdx.z * VB, V = A.V;
@@ -321,15 +335,28 @@ __global__ void __launch_bounds__(64 * W + CS_LOADERS) chunk_scan_kernel(ChunkSc
     if (warp >= 2 * W) {
         // ---- the warps that load
         const int pt = threadIdx.x - 64 * W;
-        const unsigned char* src = reinterpret_cast<const unsigned char*>(pdl_fresh((const R*)A.records) + (size_t)chunk_first_record(t0, s) * A.heads + h);
+        const Record* recs = pdl_fresh((const Record*)A.records) + (size_t)chunk_first_record(t0, s) * A.heads + h;
+        // rows of N pieces of 16 bytes, which lie `pitch` numbers apart in shared memory
+        auto copy_rows = [&](auto n, bf16* to, int pitch, const bf16* from, int rows) {
+            constexpr int N = decltype(n)::value;
+#pragma unroll 8
+            for (int p = pt; p < rows * N; p += CS_LOADERS) cm_copy16(to + p / N * pitch + p % N * 8, from + p * 8, true);
+        };
+        using Row = std::integral_constant<int, NK / 8>;
+        using Pair = std::integral_constant<int, CS_C / 8>;
         const bf16* vp = pdl_fresh(A.v) + A.v_off + (size_t)h * V + j0;
         auto load = [&](int i) {
             if (i < chunks) {
                 typename SM::Stage& st = sm.stage[i % CS_STAGES];
-                unsigned char* dst = reinterpret_cast<unsigned char*>(&st.rec);
-                const unsigned char* from = src + (size_t)i * A.heads * sizeof(R);
-#pragma unroll 8
-                for (int p = pt; p < (int)(sizeof(R) / 16); p += CS_LOADERS) cm_copy16(dst + p * 16, from + p * 16, true);
+                const Record* from = recs + (size_t)i * A.heads;
+                copy_rows(Row(), st.rec.qe[0], QP, from->qe[0], 3 * CS_C);
+                copy_rows(Row(), st.rec.kf[0], QP, from->kf[0], 3 * CS_C);
+                copy_rows(Pair(), st.rec.P[0], PP, from->P[0], 3 * CS_C);
+                if (pt < NK / 4) cm_copy16(st.rec.G + pt * 4, from->G + pt * 4, true);
+                if constexpr (DELTA) {
+                    copy_rows(Row(), st.rec.ke[0], QP, from->ke[0], 3 * CS_C);
+                    copy_rows(Pair(), st.rec.TB[0], PP, from->TB[0], 3 * CS_C);
+                }
                 for (int p = pt; p < CS_C * (VB / 8); p += CS_LOADERS) {
                     const int r = p / (VB / 8), c = p % (VB / 8) * 8;
                     const bool in = i * CS_C + r < len && j0 + c < V;
@@ -399,11 +426,14 @@ __global__ void __launch_bounds__(64 * W + CS_LOADERS) chunk_scan_kernel(ChunkSc
             float (*mine)[32] = sm.xch[i & 1][warp];
             const float (*theirs)[32] = sm.xch[i & 1][other];
 #pragma unroll
+            for (int nt = 0; nt < 2; ++nt) {
+                cm_add(acc[nt], low[nt]);
+                if constexpr (DELTA) cm_add(pred[nt], plow[nt]);
+            }
+#pragma unroll
             for (int e = 0; e < 4; ++e) {
-                mine[e][lane] = half ? acc[0][e] + low[0][e] : acc[1][e] + low[1][e];
+                mine[e][lane] = half ? acc[0][e] : acc[1][e];
                 if constexpr (DELTA) {
-                    pred[0][e] += plow[0][e];
-                    pred[1][e] += plow[1][e];
                     mine[4 + e][lane] = pred[0][e];
                     mine[8 + e][lane] = pred[1][e];
                 }
@@ -411,7 +441,7 @@ __global__ void __launch_bounds__(64 * W + CS_LOADERS) chunk_scan_kernel(ChunkSc
             cm_barrier(1 + tile, 64);
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                own[e] = (half ? acc[1][e] + low[1][e] : acc[0][e] + low[0][e]) + theirs[e][lane];
+                own[e] = (half ? acc[1][e] : acc[0][e]) + theirs[e][lane];
                 own_low[e] = 0.f;
                 if constexpr (DELTA) {
                     pred[0][e] += theirs[4 + e][lane];
@@ -497,9 +527,9 @@ __global__ void __launch_bounds__(64 * W + CS_LOADERS) chunk_scan_kernel(ChunkSc
             float sl[2][4];
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) {
-                const float2 G2 = *reinterpret_cast<const float2*>(&rec.G[k0 + m * 16 + nt * 8 + c2]);
+                cm_scale(S[2 * m + nt], *reinterpret_cast<const f32x2*>(&rec.G[k0 + m * 16 + nt * 8 + c2]));
 #pragma unroll
-                for (int e = 0; e < 4; ++e) { S[2 * m + nt][e] *= (e & 1) ? G2.y : G2.x; sl[nt][e] = 0.f; }
+                for (int e = 0; e < 4; ++e) sl[nt][e] = 0.f;
             }
             cm_mma_rows(&S[2 * m], sl, va, r);
             cm_add(S[2 * m], sl[0]);

@@ -84,6 +84,26 @@ static inline int set_smem_limit_once(K* kernel, size_t bytes, bool* flags) {
         if (_rc) return _rc;                                                        \
     } while (0)
 
+// A kernel whose blocks on an SM are bounded by static shared memory asks for the largest share of the SM's memory, once per device.
+template <typename K>
+static inline int set_all_shared_once(K* kernel, bool* flags) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return (int)e;
+    if (dev < 0 || dev >= kMaxDevices) return FF_ERR_UNSUPPORTED;
+    if (flags[dev]) return 0;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) return (int)e;
+    flags[dev] = true;
+    return 0;
+}
+#define FF_ALL_SHARED(kernel)                                                       \
+    do {                                                                            \
+        static bool _set[ff::kMaxDevices];                                          \
+        int _rc = ff::set_all_shared_once(kernel, _set);                            \
+        if (_rc) return _rc;                                                        \
+    } while (0)
+
 #define FF_LAUNCH(kernel, grid, block, smem, stream, ...)                                              \
     do {                                                                                               \
         int _rc = ff::launch_kernel(kernel, dim3(grid), dim3(block), (size_t)(smem), stream, __VA_ARGS__); \

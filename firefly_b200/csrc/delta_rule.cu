@@ -261,115 +261,103 @@ __global__ void __launch_bounds__(DR_MAX_THREADS) delta_rule_scan_kernel(
     }
 }
 
-// Prompts in bfloat16, sixteen tokens at a time (chunk_scan.cuh): the first kernel, a block per (a few records, head).  It makes
-// q and k unit vectors, forms the decays, the products of pairs of tokens, and the inverse of the unit lower triangle by
-// forward substitution, a column a thread.
-// 4 x 2048 tokens, 8 heads of 128 x 128: token by token 1373 us, the two kernels 135 + 216.
+// Prompts in bfloat16, sixteen tokens at a time (chunk_scan.cuh): the first kernel, a block per (CF_WARPS warps of records, head).  It
+// makes q and k unit vectors, forms the decays, the products of pairs of tokens, and the inverse of the unit lower triangle by
+// forward substitution, a column a lane.
 template <int NK>
-__global__ void __launch_bounds__(2 * NK) delta_prepare_kernel(DeltaArgs A, ChunkRecord<NK, true>* __restrict__ recs,
-                                                               const int* __restrict__ cu_q, int n_seqs, int n_records, int per_block, int min_len, int heads) {
+__global__ void __launch_bounds__(32 * CF_WARPS, 5) delta_prepare_kernel(DeltaArgs A, ChunkRecord<NK, true>* __restrict__ recs,
+                                                                      const int* __restrict__ cu_q, int n_seqs, int n_records, int min_len, int heads) {
     pdl_prologue();
-    __shared__ __align__(16) float sq[CS_C * NK], sk[CS_C * NK], sa[CS_C * NK];
-    __shared__ __align__(16) ChunkHalves<NK, true> halves;
-    __shared__ float sM[CS_C][CS_C + 1], s_beta[CS_C];
-    const int h = blockIdx.y, group = h / A.heads_per_group, tid = threadIdx.x;
-    const int row = tid / (NK / 8), col = tid % (NK / 8) * 8;
-    const bf16* qp = pdl_fresh((const bf16*)A.q) + A.q_off + (size_t)group * NK + col;
-    const bf16* kp = pdl_fresh((const bf16*)A.k) + A.k_off + (size_t)group * NK + col;
-    const bf16* bp = pdl_fresh((const bf16*)A.beta) + A.beta_off + h;
-    const float* ap = pdl_fresh(A.a) + A.a_off + (A.decay_per_head ? (size_t)h : (size_t)h * NK + col);
+    __shared__ __align__(16) ChunkForm<NK, true> form[cf_records<NK>()];
+    constexpr int WR = cf_warps_a_record<NK>();
+    const int h = blockIdx.y, group = h / A.heads_per_group, lane = threadIdx.x & 31, warp = threadIdx.x / 32 % WR, c0 = warp * 64, c = c0 + 2 * lane;
+    const int r = blockIdx.x * cf_records<NK>() + threadIdx.x / (32 * WR);
+    if (r >= n_records) return;
+    int s, chunk, t0, left;
+    chunk_of_record(cu_q, n_seqs, r, min_len, s, chunk, t0, left);
+    if (chunk < 0) return;
+    ChunkForm<NK, true>& sh = form[threadIdx.x / (32 * WR)];
+    const bf16* qp = pdl_fresh((const bf16*)A.q) + A.q_off + (size_t)group * NK + c0 + (size_t)t0 * A.q_stride;
+    const bf16* kp = pdl_fresh((const bf16*)A.k) + A.k_off + (size_t)group * NK + c0 + (size_t)t0 * A.k_stride;
+    const float* ap = pdl_fresh(A.a) + A.a_off + (size_t)t0 * A.a_stride + (A.decay_per_head ? h : h * NK + c0);
     const float rate = expf(A.a_log[h]);
-    float bias[8];
+    auto& rows = sh.rows[warp];
+    if (A.decay_per_head) {                                 // a lane a token, the same for every channel
+        cf_fetch<false>(rows, qp, A.q_stride, kp, A.k_stride, ap, A.a_stride, left);
+        float g = 1.f;
+        if (lane < CS_C && lane < left) g = expf(-rate * dr_softplus(ap[(size_t)lane * A.a_stride] + A.dt_bias[h]));
 #pragma unroll
-    for (int i = 0; i < 8; ++i) bias[i] = A.dt_bias[A.decay_per_head ? h : h * NK + col + i];
-    const int r0 = blockIdx.x * per_block, r1 = min(n_records, r0 + per_block);
-    int s, chunk, left = 0;
-    uint4 qv, kv;
-    float4 d0, d1;
-    float braw = 0.f;
-    auto fetch = [&](int r) {
-        chunk_of_record(cu_q, n_seqs, r, min_len, s, chunk);
-        qv = kv = make_uint4(0, 0, 0, 0);
-        d0 = d1 = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (chunk < 0) return;
-        const int t0 = cu_q[s] + chunk * CS_C;
-        left = cu_q[s + 1] - t0;
-        if (row < left) {
-            qv = *reinterpret_cast<const uint4*>(qp + (size_t)(t0 + row) * A.q_stride);
-            kv = *reinterpret_cast<const uint4*>(kp + (size_t)(t0 + row) * A.k_stride);
-            const float* a = ap + (size_t)(t0 + row) * A.a_stride;
-            if (A.decay_per_head) d0.x = *a;
-            else {
-                d0 = *reinterpret_cast<const float4*>(a);
-                d1 = *reinterpret_cast<const float4*>(a + 4);
-            }
-            if (col == 0) braw = to_float(bp[(size_t)(t0 + row) * A.beta_stride]);
+        for (int t = 0; t < CS_C; ++t) {
+            const float a = __shfl_sync(0xffffffffu, g, t);
+            rows.a[t][lane] = make_float2(a, a);
         }
-    };
-    fetch(r0);
-    for (int r = r0; r < r1; ++r) {
-        const bool any = chunk >= 0, in = row < left;
-        ChunkRecord<NK, true>* rec = recs + (size_t)r * heads + h;
-        if (any) {
-            float xq[8], xk[8], xa[8];
-            chunk_unpack(qv, xq);
-            chunk_unpack(kv, xk);
-            float qq = 0.f, kk = 0.f;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) { qq += xq[i] * xq[i]; kk += xk[i] * xk[i]; }
-#pragma unroll
-            for (int off = 1; off < NK / 8; off <<= 1) {
-                qq += __shfl_xor_sync(0xffffffffu, qq, off);
-                kk += __shfl_xor_sync(0xffffffffu, kk, off);
-            }
-            // rows behind the sequence's end stay zero, also where unit_eps is
-            const float fq = in ? A.q_scale / sqrtf(qq + A.unit_eps) : 0.f, fk = in ? 1.0f / sqrtf(kk + A.unit_eps) : 0.f;
-            const float d[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
-            if (A.decay_per_head) {
-                const float gd = in ? expf(-rate * dr_softplus(d[0] + bias[0])) : 1.f;
-#pragma unroll
-                for (int i = 0; i < 8; ++i) xa[i] = gd;
-            } else {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) xa[i] = in ? expf(-rate * dr_softplus(d[i] + bias[i])) : 1.f;
-            }
-#pragma unroll
-            for (int i = 0; i < 8; ++i) { xq[i] *= fq; xk[i] *= fk; }
-            chunk_stage8(sq + row * NK + col, xq);
-            chunk_stage8(sk + row * NK + col, xk);
-            chunk_stage8(sa + row * NK + col, xa);
-            if (col == 0) s_beta[row] = in ? 1.0f / (1.0f + expf(-braw)) : 0.f;
+    } else {
+        cf_fetch<true>(rows, qp, A.q_stride, kp, A.k_stride, ap, A.a_stride, left);
+        const float bx = A.dt_bias[h * NK + c], by = A.dt_bias[h * NK + c + 1];
+#pragma unroll 2
+        for (int t = 0; t < CS_C; ++t) {
+            float2& a = rows.a[t][lane];
+            a = t < left ? make_float2(expf(-rate * dr_softplus(a.x + bx)), expf(-rate * dr_softplus(a.y + by))) : make_float2(1.f, 1.f);
         }
-        __syncthreads();
-        if (r + 1 < r1) fetch(r + 1);
-        if (any) {
-            chunk_scaled_rows<NK, true, false>(rec, halves, sq, sk, sa);
-            chunk_near_pairs<NK, true, false>(sq, sk, sa, nullptr, [&](int t, int u, float x, float y) {
-                chunk_put(rec->P[0], t, u, x);
-                sM[t][u] = s_beta[t] * y;
-            });
-        }
-        __syncthreads();
-        if (any) {
-            chunk_far_pairs<NK, true>(halves, [&](int t, int u, float x, float y) {
-                chunk_put_far(rec->P[0], t, u, x);
-                sM[t][u] = s_beta[t] * y;
-            });
-        }
-        __syncthreads();
-        if (any && tid < CS_C) {
-            float x[CS_C];
-#pragma unroll
-            for (int t = 0; t < CS_C; ++t) {
-                float y = t == tid ? s_beta[t] : 0.f;
-#pragma unroll
-                for (int u = 0; u < t; ++u) y -= sM[t][u] * x[u];
-                x[t] = y;
-                chunk_put(rec->TB[0], t, tid, y);
-            }
-        }
-        __syncthreads();
     }
+    if (warp == 0 && lane < CS_C) {
+        const bf16* bp = pdl_fresh((const bf16*)A.beta) + A.beta_off + h;
+        sh.beta[lane] = lane < left ? 1.0f / (1.0f + expf(-to_float(bp[(size_t)(t0 + lane) * A.beta_stride]))) : 0.f;
+    }
+    // the tokens' lengths: 32 sums over the record's channels, a lane each (q's 16, then k's)
+    {
+        float x[CS_C];
+        const bool other = lane & 16;
+#pragma unroll
+        for (int t = 0; t < CS_C; ++t) {
+            const uint32_t qv = rows.q[t][lane], kv = rows.k[t][lane];
+            const float q0 = cm_lo(qv), q1 = cm_hi(qv), k0 = cm_lo(kv), k1 = cm_hi(kv);
+            const float qq = q0 * q0 + q1 * q1, kk = k0 * k0 + k1 * k1, away = other ? qq : kk;
+            x[t] = (other ? kk : qq) + __shfl_xor_sync(0xffffffffu, away, 16);
+        }
+        const float mine = cf_join<16, 16>(x);
+        sh.sums[warp][(lane & 16) + cf_kept<16>(lane)] = mine;
+        cf_sync<NK>();
+        if (warp == 0) {
+            float sum = sh.sums[0][lane];
+            if constexpr (WR == 2) sum += sh.sums[1][lane];
+            // rows behind the sequence's end stay zero, also where unit_eps is
+            const float f = (lane & 15) < left ? ((lane & 16) ? 1.0f : A.q_scale) / sqrtf(sum + A.unit_eps) : 0.f;
+            reinterpret_cast<float*>(sh.unit)[(lane & 15) * 2 + (lane >> 4)] = f;
+        }
+        cf_sync<NK>();
+    }
+    ChunkRecord<NK, true>* rec = recs + (size_t)r * heads + h;
+    chunk_form<NK, true, false>(rec, sh, warp, 0ull, [&](int t, f32x2& q, f32x2& k, f32x2& a) {
+        const float2 f = sh.unit[t];
+        q = f2_mul(cf_pair(rows.q[t][lane]), f2_pack(f.x, f.x));
+        k = f2_mul(cf_pair(rows.k[t][lane]), f2_pack(f.y, f.y));
+        a = *reinterpret_cast<const f32x2*>(&rows.a[t][lane]);
+    });
+    cf_sync<NK>();
+    chunk_emit<NK, WR>(rec->P[0], sh.P);
+    if (warp == 0) {
+        float x[CS_C];
+#pragma unroll
+        for (int t = 0; t < CS_C; ++t) {
+            const float b = sh.beta[t];
+            float y = t == lane ? b : 0.f;
+#pragma unroll
+            for (int u = 0; u < t; ++u) {
+                float m = sh.M[0][t][u];
+                if constexpr (WR == 2) m += sh.M[1][t][u];
+                y -= b * m * x[u];
+            }
+            x[t] = y;
+        }
+        __syncwarp();                                       // everything has been read
+        if (lane < CS_C) {
+#pragma unroll
+            for (int t = 0; t < CS_C; ++t) sh.M[0][t][lane] = x[t];
+        }
+    }
+    cf_sync<NK>();
+    chunk_emit<NK, 1>(rec->TB[0], sh.M);
 }
 
 // y[t, h*V + i] = o[t, h*V + i] / sqrt(mean_i o[t, h, :]^2 + eps) * w[i] * act(gate[t, gate_off + h*V + i]):
@@ -467,9 +455,10 @@ static unsigned delta_bits(const DeltaArgs& A) {
 
 template <int NK>
 static int delta_chunk_launch(const DeltaArgs& A, const ChunkScanArgs& B, int T, int n_seqs, int live, void* scratch, cudaStream_t stream) {
-    const int n_records = (int)chunk_records(T, n_seqs), per_block = chunk_records_a_block((long long)n_records * B.heads);
-    FF_LAUNCH(delta_prepare_kernel<NK>, dim3((n_records + per_block - 1) / per_block, B.heads), 2 * NK, 0, stream, A,
-              (ChunkRecord<NK, true>*)scratch, B.cu_q, n_seqs, n_records, per_block, B.min_len, B.heads);
+    const int n_records = (int)chunk_records(T, n_seqs);
+    FF_ALL_SHARED(delta_prepare_kernel<NK>);
+    FF_LAUNCH(delta_prepare_kernel<NK>, cf_grid<NK>(n_records, B.heads), 32 * CF_WARPS, 0, stream, A, (ChunkRecord<NK, true>*)scratch, B.cu_q,
+              n_seqs, n_records, B.min_len, B.heads);
     return chunk_scan_launch<NK, true>(B, n_seqs, live, stream);
 }
 

@@ -21,6 +21,11 @@ __device__ __forceinline__ f32x2 f2_fma(f32x2 a, f32x2 b, f32x2 c) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     return d;
 }
+__device__ __forceinline__ f32x2 f2_add(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
 __device__ __forceinline__ f32x2 f2_mul(f32x2 a, f32x2 b) {
     f32x2 d;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
@@ -32,6 +37,7 @@ __device__ __forceinline__ f32x2 f2_pack(float lo, float hi) {
     return d;
 }
 __device__ __forceinline__ float f2_low(f32x2 a) { return __uint_as_float((unsigned)a); }
+__device__ __forceinline__ float f2_high(f32x2 a) { return __uint_as_float((unsigned)(a >> 32)); }
 __device__ __forceinline__ float f2_sum(f32x2 a) {
     float lo, hi;
     asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a));

@@ -422,10 +422,10 @@ __global__ void __launch_bounds__(128) scalar_decay_prepare_kernel(ScanArgs A, S
     constexpr int QP = NK + 8;
     __shared__ __align__(16) bf16 sq[SC_C * QP], sk[SC_C * QP];
     __shared__ float lh[4][SC_C], ll[4][SC_C], sb[4][SC_C];
-    int s, chunk;
-    chunk_of_record<SC_C>(cu_q, n_seqs, blockIdx.x, min_len, s, chunk);
+    int s, chunk, row0, left;
+    chunk_of_record<SC_C>(cu_q, n_seqs, blockIdx.x, min_len, s, chunk, row0, left);
     if (chunk < 0) return;
-    const int group = blockIdx.y, row0 = cu_q[s] + chunk * SC_C, n = min(SC_C, cu_q[s + 1] - row0);
+    const int group = blockIdx.y, n = min(SC_C, left);
     const int hb0 = blockIdx.z * heads_a_block, hb1 = min(A.heads_per_group, hb0 + heads_a_block);       // heads of the group
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c2 = (lane & 3) * 2;
     const int row_a = (lane & 7) + ((lane >> 3) & 1) * 8, col_a = (lane >> 4) * 8;
@@ -627,19 +627,21 @@ __global__ void __launch_bounds__(64 * W + CS_LOADERS) scalar_decay_chunk_kernel
             float (*mine)[32] = sm.xch[i & 1][warp];
             const float (*theirs)[32] = sm.xch[i & 1][other];
 #pragma unroll
+            for (int nt = 0; nt < 4; ++nt) cm_add(acc[nt], low[nt]);
+#pragma unroll
             for (int nt = 0; nt < 2; ++nt) {
 #pragma unroll
-                for (int e = 0; e < 4; ++e) mine[nt * 4 + e][lane] = half ? acc[nt][e] + low[nt][e] : acc[2 + nt][e] + low[2 + nt][e];
+                for (int e = 0; e < 4; ++e) mine[nt * 4 + e][lane] = half ? acc[nt][e] : acc[2 + nt][e];
             }
             cm_barrier(1 + tile, 64);
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) {
-                const float2 e2 = *reinterpret_cast<const float2*>(&st.rec.e[nt * 8 + t_own]);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    own[nt][e] = ((half ? acc[2 + nt][e] + low[2 + nt][e] : acc[nt][e] + low[nt][e]) + theirs[nt * 4 + e][lane]) * ((e & 1) ? e2.y : e2.x);
+                    own[nt][e] = (half ? acc[2 + nt][e] : acc[nt][e]) + theirs[nt * 4 + e][lane];
                     own_low[nt][e] = 0.f;
                 }
+                cm_scale(own[nt], *reinterpret_cast<const f32x2*>(&st.rec.e[nt * 8 + t_own]));
             }
         }
         // the chunk's values, V^T: 16 value columns x 32 tokens
@@ -717,8 +719,9 @@ __global__ void __launch_bounds__(64 * W + CS_LOADERS) scalar_decay_chunk_kernel
             float sl[2][4];
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) {
+                cm_scale(S[2 * m + nt], f2_pack(end, end));
 #pragma unroll
-                for (int e = 0; e < 4; ++e) { S[2 * m + nt][e] *= end; sl[nt][e] = 0.f; }
+                for (int e = 0; e < 4; ++e) sl[nt][e] = 0.f;
             }
 #pragma unroll
             for (int b = 0; b < 2; ++b) {
@@ -738,62 +741,43 @@ __global__ void __launch_bounds__(64 * W + CS_LOADERS) scalar_decay_chunk_kernel
     }
 }
 
-// Mode 2 over bfloat16 prompts: sixteen tokens at a time (chunk_scan.cuh).  This is the first kernel: a block per (a few records,
-// head).
+// Mode 2 over bfloat16 prompts: sixteen tokens at a time (chunk_scan.cuh).  This is the first kernel: a block per (CF_WARPS warps of
+// records, head).
 template <int NK>
-__global__ void __launch_bounds__(2 * NK) channel_decay_prepare_kernel(ScanArgs A, ChunkRecord<NK, false>* __restrict__ recs,
-                                                                       const int* __restrict__ cu_q, int n_seqs, int n_records,
-                                                                       int per_block, int min_len, int heads) {
+__global__ void __launch_bounds__(32 * CF_WARPS) channel_decay_prepare_kernel(ScanArgs A, ChunkRecord<NK, false>* __restrict__ recs,
+                                                                              const int* __restrict__ cu_q, int n_seqs, int n_records, int min_len,
+                                                                              int heads) {
     pdl_prologue();
-    __shared__ __align__(16) float sq[CS_C * NK], sk[CS_C * NK], sa[CS_C * NK];
-    __shared__ __align__(16) ChunkHalves<NK, false> halves;
-    const int h = blockIdx.y, group = h / A.heads_per_group, tid = threadIdx.x;
-    const int row = tid / (NK / 8), col = tid % (NK / 8) * 8;
-    const bf16* qp = pdl_fresh((const bf16*)A.q) + A.q_off + (size_t)group * NK + col;
-    const bf16* kp = pdl_fresh((const bf16*)A.k) + A.k_off + (size_t)group * NK + col;
-    const float* cdp = pdl_fresh(A.channel_decay) + A.cd_off + (size_t)h * NK + col;
-    const int r0 = blockIdx.x * per_block, r1 = min(n_records, r0 + per_block);
-    int s, chunk, left = 0;
-    uint4 qv, kv;
-    float4 d0, d1;
-    auto fetch = [&](int r) {
-        chunk_of_record(cu_q, n_seqs, r, min_len, s, chunk);
-        qv = kv = make_uint4(0, 0, 0, 0);
-        d0 = d1 = make_float4(1.f, 1.f, 1.f, 1.f);
-        if (chunk < 0) return;
-        const int t0 = cu_q[s] + chunk * CS_C;
-        left = cu_q[s + 1] - t0;
-        if (row < left) {
-            qv = *reinterpret_cast<const uint4*>(qp + (size_t)(t0 + row) * A.q_stride);
-            kv = *reinterpret_cast<const uint4*>(kp + (size_t)(t0 + row) * A.k_stride);
-            d0 = *reinterpret_cast<const float4*>(cdp + (size_t)(t0 + row) * A.cd_stride);
-            d1 = *reinterpret_cast<const float4*>(cdp + (size_t)(t0 + row) * A.cd_stride + 4);
-        }
-    };
-    fetch(r0);
-    for (int r = r0; r < r1; ++r) {
-        const bool any = chunk >= 0;
-        if (any) {
-            float xq[8], xk[8];
-            chunk_unpack(qv, xq);
-            chunk_unpack(kv, xk);
-            const float xa[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
+    __shared__ __align__(16) ChunkForm<NK, false> form[cf_records<NK>()];
+    constexpr int WR = cf_warps_a_record<NK>();
+    const int h = blockIdx.y, group = h / A.heads_per_group, warp = threadIdx.x / 32 % WR, c = warp * 64 + 2 * (threadIdx.x & 31);
+    const int r = blockIdx.x * cf_records<NK>() + threadIdx.x / (32 * WR);
+    if (r >= n_records) return;
+    int s, chunk, t0, left;
+    chunk_of_record(cu_q, n_seqs, r, min_len, s, chunk, t0, left);
+    if (chunk < 0) return;
+    const bf16* qp = pdl_fresh((const bf16*)A.q) + A.q_off + (size_t)group * NK + c + (size_t)t0 * A.q_stride;
+    const bf16* kp = pdl_fresh((const bf16*)A.k) + A.k_off + (size_t)group * NK + c + (size_t)t0 * A.k_stride;
+    const float* ap = pdl_fresh(A.channel_decay) + A.cd_off + (size_t)h * NK + c + (size_t)t0 * A.cd_stride;
+    uint32_t qv[CS_C], kv[CS_C];
+    float2 av[CS_C];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) xq[i] *= A.q_scale;
-            chunk_stage8(sq + row * NK + col, xq);
-            chunk_stage8(sk + row * NK + col, xk);
-            chunk_stage8(sa + row * NK + col, xa);
-        }
-        __syncthreads();
-        if (r + 1 < r1) fetch(r + 1);
-        ChunkRecord<NK, false>* rec = recs + (size_t)r * heads + h;
-        if (any) {
-            chunk_scaled_rows<NK, false, false>(rec, halves, sq, sk, sa);
-            chunk_near_pairs<NK, false, false>(sq, sk, sa, nullptr, [&](int t, int u, float x, float) { chunk_put(rec->P[0], t, u, x); });
-        }
-        __syncthreads();
-        if (any) chunk_far_pairs<NK, false>(halves, [&](int t, int u, float x, float) { chunk_put_far(rec->P[0], t, u, x); });
+    for (int t = 0; t < CS_C; ++t) {
+        const bool in = t < left;
+        qv[t] = in ? *reinterpret_cast<const uint32_t*>(qp + (size_t)t * A.q_stride) : 0u;
+        kv[t] = in ? *reinterpret_cast<const uint32_t*>(kp + (size_t)t * A.k_stride) : 0u;
+        av[t] = in ? *reinterpret_cast<const float2*>(ap + (size_t)t * A.cd_stride) : make_float2(1.f, 1.f);
     }
+    ChunkForm<NK, false>& sh = form[threadIdx.x / (32 * WR)];
+    ChunkRecord<NK, false>* rec = recs + (size_t)r * heads + h;
+    const f32x2 scale = f2_pack(A.q_scale, A.q_scale);
+    chunk_form<NK, false, false>(rec, sh, warp, 0ull, [&](int t, f32x2& q, f32x2& k, f32x2& a) {
+        q = f2_mul(cf_pair(qv[t]), scale);
+        k = cf_pair(kv[t]);
+        a = f2_pack(av[t].x, av[t].y);
+    });
+    cf_sync<NK>();
+    chunk_emit<NK, WR>(rec->P[0], sh.P);
 }
 
 // ------------------------------------------------------------------- decays from a low-rank projection --
@@ -1106,9 +1090,9 @@ static int scan_chunk_launch(const ScanArgs& A, float* state, long long state_st
 
 template <int NK>
 static int channel_chunk_launch(const ScanArgs& A, const ChunkScanArgs& B, int T, int n_seqs, int live, void* scratch, cudaStream_t stream) {
-    const int n_records = (int)chunk_records(T, n_seqs), per_block = chunk_records_a_block((long long)n_records * B.heads);
-    FF_LAUNCH(channel_decay_prepare_kernel<NK>, dim3((n_records + per_block - 1) / per_block, B.heads), 2 * NK, 0, stream, A,
-              (ChunkRecord<NK, false>*)scratch, B.cu_q, n_seqs, n_records, per_block, B.min_len, B.heads);
+    const int n_records = (int)chunk_records(T, n_seqs);
+    FF_LAUNCH(channel_decay_prepare_kernel<NK>, cf_grid<NK>(n_records, B.heads), 32 * CF_WARPS, 0, stream, A, (ChunkRecord<NK, false>*)scratch, B.cu_q,
+              n_seqs, n_records, B.min_len, B.heads);
     return chunk_scan_launch<NK, false>(B, n_seqs, live, stream);
 }
 

@@ -239,75 +239,51 @@ __global__ void __launch_bounds__(WS_THREADS) wkv_scan_kernel(
     }
 }
 
-// Prompts in bfloat16, sixteen tokens at a time (chunk_scan.cuh): the first kernel, a block per (a few records, head).  The
-// read-out sees the state in front of the token's own decay and write; the bonus term is the diagonal of P.
+// Prompts in bfloat16, sixteen tokens at a time (chunk_scan.cuh): the first kernel, a block per (CF_WARPS warps of records, head).
+// The read-out sees the state in front of the token's own decay and write; the bonus term is the diagonal of P.
 template <int NK>
-__global__ void __launch_bounds__(2 * NK) wkv_prepare_kernel(const bf16* rkvg, const float* dlog, const float* __restrict__ w0,
-                                                             const float* __restrict__ u, ChunkRecord<NK, false>* __restrict__ recs,
-                                                             float* __restrict__ state, size_t state_stride, int prev_off, const bf16* x, int W,
-                                                             const int* __restrict__ cu_q, const int* __restrict__ state_slots, int n_seqs,
-                                                             int n_records, int per_block, int min_len, int Ttot, int heads) {
+__global__ void __launch_bounds__(32 * CF_WARPS) wkv_prepare_kernel(const bf16* rkvg, const float* dlog, const float* __restrict__ w0,
+                                                                    const float* __restrict__ u, ChunkRecord<NK, false>* __restrict__ recs,
+                                                                    float* __restrict__ state, size_t state_stride, int prev_off, const bf16* x, int W,
+                                                                    const int* __restrict__ cu_q, const int* __restrict__ state_slots, int n_seqs,
+                                                                    int n_records, int min_len, int Ttot, int heads) {
     pdl_prologue();
-    __shared__ __align__(16) float sr[CS_C * NK], sk[CS_C * NK], sw[CS_C * NK], su[NK];
-    __shared__ __align__(16) ChunkHalves<NK, false> halves;
-    const int h = blockIdx.y, HD = heads * NK, tid = threadIdx.x;
-    const int row = tid / (NK / 8), col = tid % (NK / 8) * 8;
-    const bf16* rp = pdl_fresh(rkvg) + h * NK + col;
+    __shared__ __align__(16) ChunkForm<NK, false> form[cf_records<NK>()];
+    constexpr int WR = cf_warps_a_record<NK>();
+    const int h = blockIdx.y, HD = heads * NK, lane = threadIdx.x & 31, warp = threadIdx.x / 32 % WR;
+    const int r = blockIdx.x * cf_records<NK>() + threadIdx.x / (32 * WR);
+    if (r >= n_records) return;
+    int s, chunk, t0, left;
+    chunk_of_record(cu_q, n_seqs, r, min_len, s, chunk, t0, left);
+    if (chunk < 0) return;
+    const int c = h * NK + warp * 64 + 2 * lane;
+    const bf16* rp = pdl_fresh(rkvg) + (size_t)t0 * HD + c;
     const bf16* kp = rp + (size_t)Ttot * HD;
-    const float* dp = pdl_fresh(dlog) + h * NK + col;
-    float w0c[8];
+    const float* dp = pdl_fresh(dlog) + (size_t)t0 * HD + c;
+    uint32_t rv[CS_C], kv[CS_C];
+    float2 dv[CS_C];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) w0c[i] = w0[h * NK + col + i];
-    if (tid < NK) su[tid] = u[h * NK + tid];
-    const int r0 = blockIdx.x * per_block, r1 = min(n_records, r0 + per_block);
-    int s, chunk, t0 = 0, left = 0;
-    uint4 rv, kv;
-    float4 d0, d1;
-    auto fetch = [&](int r) {
-        chunk_of_record(cu_q, n_seqs, r, min_len, s, chunk);
-        rv = kv = make_uint4(0, 0, 0, 0);
-        d0 = d1 = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (chunk < 0) return;
-        t0 = cu_q[s] + chunk * CS_C;
-        left = cu_q[s + 1] - t0;
-        if (row < left) {
-            const size_t at = (size_t)(t0 + row) * HD;
-            rv = *reinterpret_cast<const uint4*>(rp + at);
-            kv = *reinterpret_cast<const uint4*>(kp + at);
-            d0 = *reinterpret_cast<const float4*>(dp + at);
-            d1 = *reinterpret_cast<const float4*>(dp + at + 4);
-        }
-    };
-    fetch(r0);
-    for (int r = r0; r < r1; ++r) {
-        const bool any = chunk >= 0, in = row < left;
-        if (any) {
-            float xr[8], xk[8], xw[8];
-            chunk_unpack(rv, xr);
-            chunk_unpack(kv, xk);
-            const float d[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
-#pragma unroll
-            for (int i = 0; i < 8; ++i) xw[i] = in ? expf(-expf(d[i] + w0c[i])) : 1.f;
-            chunk_stage8(sr + row * NK + col, xr);
-            chunk_stage8(sk + row * NK + col, xk);
-            chunk_stage8(sw + row * NK + col, xw);
-        }
-        __syncthreads();
-        const int seq = s, first_row = t0, rows = left;
-        if (r + 1 < r1) fetch(r + 1);
-        ChunkRecord<NK, false>* rec = recs + (size_t)r * heads + h;
-        if (any) {
-            chunk_scaled_rows<NK, false, true>(rec, halves, sr, sk, sw);
-            chunk_near_pairs<NK, false, true>(sr, sk, sw, su, [&](int t, int i, float y, float) { chunk_put(rec->P[0], t, i, y); });
-            // the sequence's last input row, for the first token of its next step
-            if (h == 0 && rows <= CS_C) {
-                const bf16* last = pdl_fresh(x) + (size_t)(first_row + rows - 1) * W;
-                float* prev = state + (size_t)state_slots[seq] * state_stride + prev_off;
-                for (int i = tid; i < W; i += 2 * NK) prev[i] = to_float(last[i]);
-            }
-        }
-        __syncthreads();
-        if (any) chunk_far_pairs<NK, false>(halves, [&](int t, int i, float y, float) { chunk_put_far(rec->P[0], t, i, y); });
+    for (int t = 0; t < CS_C; ++t) {
+        const bool in = t < left;
+        rv[t] = in ? *reinterpret_cast<const uint32_t*>(rp + (size_t)t * HD) : 0u;
+        kv[t] = in ? *reinterpret_cast<const uint32_t*>(kp + (size_t)t * HD) : 0u;
+        dv[t] = in ? *reinterpret_cast<const float2*>(dp + (size_t)t * HD) : make_float2(0.f, 0.f);
+    }
+    const float w0x = w0[c], w0y = w0[c + 1];
+    ChunkForm<NK, false>& sh = form[threadIdx.x / (32 * WR)];
+    ChunkRecord<NK, false>* rec = recs + (size_t)r * heads + h;
+    chunk_form<NK, false, true>(rec, sh, warp, f2_pack(u[c], u[c + 1]), [&](int t, f32x2& q, f32x2& k, f32x2& a) {
+        q = cf_pair(rv[t]);
+        k = cf_pair(kv[t]);
+        a = t < left ? f2_pack(expf(-expf(dv[t].x + w0x)), expf(-expf(dv[t].y + w0y))) : f2_pack(1.f, 1.f);
+    });
+    cf_sync<NK>();
+    chunk_emit<NK, WR>(rec->P[0], sh.P);
+    // the sequence's last input row, for the first token of its next step
+    if (h == 0 && left <= CS_C) {
+        const bf16* last = pdl_fresh(x) + (size_t)(t0 + left - 1) * W;
+        float* prev = state + (size_t)state_slots[s] * state_stride + prev_off;
+        for (int i = threadIdx.x % (32 * WR); i < W; i += 32 * WR) prev[i] = to_float(last[i]);
     }
 }
 
@@ -445,9 +421,9 @@ FF_EXPORT long long ff_wkv_scratch_bytes(int dtype, int T, int n_seqs, int heads
 template <int D>
 static int wkv_chunk_launch(const bf16* rkvg, const float* dlog, const float* w0, const float* u, int prev_off, const bf16* x, int W,
                             const ChunkScanArgs& B, int Ttot, int n_seqs, int live, void* scratch, cudaStream_t stream) {
-    const int n_records = (int)chunk_records(Ttot, n_seqs), per_block = chunk_records_a_block((long long)n_records * B.heads);
-    FF_LAUNCH(wkv_prepare_kernel<D>, dim3((n_records + per_block - 1) / per_block, B.heads), 2 * D, 0, stream, rkvg, dlog, w0, u,
-              (ChunkRecord<D, false>*)scratch, B.state, (size_t)B.state_stride, prev_off, x, W, B.cu_q, B.state_slots, n_seqs, n_records, per_block,
+    const int n_records = (int)chunk_records(Ttot, n_seqs);
+    FF_LAUNCH(wkv_prepare_kernel<D>, cf_grid<D>(n_records, B.heads), 32 * CF_WARPS, 0, stream, rkvg, dlog, w0, u,
+              (ChunkRecord<D, false>*)scratch, B.state, (size_t)B.state_stride, prev_off, x, W, B.cu_q, B.state_slots, n_seqs, n_records,
               B.min_len, Ttot, B.heads);
     return chunk_scan_launch<D, false>(B, n_seqs, live, stream);
 }
