@@ -20,10 +20,6 @@
 namespace ff {
 
 __device__ __forceinline__ float silu_f(float z) { return z / (1.0f + expf(-z)); }
-// The same for results that are rounded to 16 bits, by CUDA's fast division (2 units in the last place of 32 bits; 0 where e^-z is
-// beyond 2^126, the true result being below 2^-119): 55 us for the convolution of 8192 tokens of 4096 channels, 75 with the division above,
-// 79 with __frcp_rn; 4 of 33 million rounded results differ more than with a true reciprocal.
-__device__ __forceinline__ float silu_fast(float z) { return __fdividef(z, 1.0f + expf(-z)); }
 __device__ __forceinline__ float softplus_f(float z) { return z > 20.f ? z : log1pf(expf(z)); }
 
 // ----------------------------------------------------------------------------- convolution --
@@ -42,7 +38,7 @@ constexpr int CONV_AHEAD = 4;
 // TAPS > 0: the number of taps is known when the kernel is built (the window stays in registers); 0: any number
 // up to CONV_MAX_TAPS.
 template <typename T, typename TO, int VEC, int TAPS>
-__global__ void __launch_bounds__(128, 4) causal_conv_silu_kernel(const T* in, int in_stride, int in_off,
+__global__ void __launch_bounds__(128, VEC > 1 ? 6 : 4) causal_conv_silu_kernel(const T* in, int in_stride, int in_off,
                                         const float* __restrict__ w /*[C,taps]*/, const float* __restrict__ bias,
                                         const float* state, size_t state_stride, int conv_off,
                                         const int* __restrict__ token_seq, const int* __restrict__ cu_q,
@@ -70,15 +66,12 @@ __global__ void __launch_bounds__(128, 4) causal_conv_silu_kernel(const T* in, i
             for (int j = 0; j < MT; ++j) wt[j][e] = j < taps ? w[(size_t)(c0 + e) * taps + j] : 0.f;
         }
     }
-    auto load_row = [&](int tt, float* dst) {           // the inputs of token tt (a row of this step)
-        const T* src = in + (size_t)tt * in_stride + in_off + c0;
-        if constexpr (VEC == 1) dst[0] = to_float(src[0]);
-        else {
-            const uint4 raw = *reinterpret_cast<const uint4*>(src);
-            const T* v = reinterpret_cast<const T*>(&raw);
+    struct alignas(VEC * sizeof(T)) Raw { T v[VEC]; };
+    auto ask = [&](int tt) { return *reinterpret_cast<const Raw*>(in + (size_t)tt * in_stride + in_off + c0); };      // the inputs of token tt (a row of this step)
+    auto load_row = [&](int tt, float* dst) {
+        const Raw raw = ask(tt);
 #pragma unroll
-            for (int e = 0; e < VEC; ++e) dst[e] = to_float(v[e]);
-        }
+        for (int e = 0; e < VEC; ++e) dst[e] = to_float(raw.v[e]);
     };
     // the window in front of token t of sequence s: rows of this step where they exist, else the saved rows
     auto fill_window = [&](int t, int s) {
@@ -98,25 +91,38 @@ __global__ void __launch_bounds__(128, 4) causal_conv_silu_kernel(const T* in, i
             }
         }
     };
-    // The rows and sequences of CONV_AHEAD tokens are asked for together: with one at a time the walk waits for memory at every
-    // token.  With a channel's four weights in one load and no division in the SiLU: 118 -> 55 us on 8192 tokens of 4096
-    // channels, whose bytes take 21; what is left is instructions, a dozen for every two bytes in and out.
+    // The rows and sequences of CONV_AHEAD tokens are asked for together, while the CONV_AHEAD in front of them are worked on: with one at
+    // a time the walk waits for memory at every token.  Four channels a thread leave an SM the warps that hide the rest.  8192 tokens
+    // of 4096 channels, whose bytes take 21 us: a token at a time 118, four at a time with nothing asked for ahead and eight channels a thread 50, now 42 (48 of these 50 with the SiLU as it was).
     int s_prev = -1;
     float rows[CONV_AHEAD][VEC];
-    int seqs[CONV_AHEAD];
+    Raw next[CONV_AHEAD];
+    int seqs[CONV_AHEAD], next_seqs[CONV_AHEAD];
+    auto ask_ahead = [&](int t) {
+#pragma unroll
+        for (int a = 0; a < CONV_AHEAD; ++a)
+            if (t + a < tile1) {
+                next_seqs[a] = token_seq[t + a];
+                next[a] = ask(t + a);
+            }
+    };
+    ask_ahead(tile0);
     for (int tb = tile0; tb < tile1; tb += CONV_AHEAD) {
 #pragma unroll
       for (int a = 0; a < CONV_AHEAD; ++a) {
-        if (tb + a < tile1) {
-          seqs[a] = token_seq[tb + a];
-          load_row(tb + a, rows[a]);
-        }
-      }
-      auto finish = [&](int t, float (&acc)[VEC], const float (&cur)[VEC]) {
+        seqs[a] = next_seqs[a];
 #pragma unroll
-        for (int e = 0; e < VEC; ++e) {
-            if (flags & CONV_SILU) acc[e] = sizeof(TO) == 4 ? silu_f(acc[e]) : silu_fast(acc[e]);
-            if (flags & CONV_ADD_INPUT) acc[e] += cur[e];
+        for (int e = 0; e < VEC; ++e) rows[a][e] = to_float(next[a].v[e]);
+      }
+      ask_ahead(tb + CONV_AHEAD);
+      auto finish = [&](int t, float (&acc)[VEC], const float (&cur)[VEC]) {
+        if (flags & CONV_SILU) {
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) acc[e] = silu_for<TO>(acc[e]);
+        }
+        if (flags & CONV_ADD_INPUT) {
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) acc[e] += cur[e];
         }
         TO* dst = out + (size_t)t * C + c0;
         if constexpr (VEC == 1) dst[0] = from_float<TO>(acc[0]);
@@ -139,8 +145,15 @@ __global__ void __launch_bounds__(128, 4) causal_conv_silu_kernel(const T* in, i
 #pragma unroll
             for (int j = 0; j < MT; ++j) {
               const int from = a - (MT - 1) + j;            // row of this batch, or (negative) of the window
+              const float (&x)[VEC] = from >= 0 ? rows[from >= 0 ? from : 0] : win[from < 0 ? MT - 1 + from : 0];
+              if constexpr (VEC % 2 == 0) {                 // two channels an instruction
 #pragma unroll
-              for (int e = 0; e < VEC; ++e) acc[e] += wt[j][e] * (from >= 0 ? rows[from >= 0 ? from : 0][e] : win[from < 0 ? MT - 1 + from : 0][e]);
+                for (int e = 0; e < VEC; e += 2) {
+                  const f32x2 r = f2_fma(f2_pack(wt[j][e], wt[j][e + 1]), f2_pack(x[e], x[e + 1]), f2_pack(acc[e], acc[e + 1]));
+                  acc[e] = f2_low(r);
+                  acc[e + 1] = f2_high(r);
+                }
+              } else acc[0] += wt[j][0] * x[0];
             }
             finish(tb + a, acc, rows[a]);
           }
@@ -860,7 +873,7 @@ __global__ void gated_rms_norm_kernel(const float* o, const T* z, int z_stride, 
     float ss = 0.f;
     for (int i = threadIdx.x; i < per; i += blockDim.x) {
         float v = orow[i];
-        if (order == 0) v *= silu_f(to_float(zrow[i]));
+        if (order == 0) v *= silu_for<T>(to_float(zrow[i]));
         ss += v * v;
     }
     ss = block_sum(ss, scratch);
@@ -869,8 +882,8 @@ __global__ void gated_rms_norm_kernel(const float* o, const T* z, int z_stride, 
     for (int i = threadIdx.x; i < per; i += blockDim.x) {
         const float zv = to_float(zrow[i]);
         float v = orow[i];
-        if (order == 0) v = v * silu_f(zv) * inv * w[g * per + i];
-        else v = v * inv * w[g * per + i] / (1.0f + expf(-zv));
+        if (order == 0) v = v * silu_for<T>(zv) * inv * w[g * per + i];
+        else v = v * inv * w[g * per + i] * sigmoid_for<T>(zv);
         yrow[i] = from_float<T>(v);
     }
 }
@@ -907,10 +920,10 @@ __global__ void __launch_bounds__(256) gated_rms_norm_vec_kernel(const float* o,
     for (int m = 0; m < MAXV; ++m) {
         if ((m * TP + lane) * 4 < per) {
             if (order == 0) {
-                ov[m].x *= silu_f(to_float(zv[m].v[0]));
-                ov[m].y *= silu_f(to_float(zv[m].v[1]));
-                ov[m].z *= silu_f(to_float(zv[m].v[2]));
-                ov[m].w *= silu_f(to_float(zv[m].v[3]));
+                ov[m].x *= silu_for<T>(to_float(zv[m].v[0]));
+                ov[m].y *= silu_for<T>(to_float(zv[m].v[1]));
+                ov[m].z *= silu_for<T>(to_float(zv[m].v[2]));
+                ov[m].w *= silu_for<T>(to_float(zv[m].v[3]));
             }
             ss += (ov[m].x * ov[m].x + ov[m].y * ov[m].y) + (ov[m].z * ov[m].z + ov[m].w * ov[m].w);
         }
@@ -936,7 +949,7 @@ __global__ void __launch_bounds__(256) gated_rms_norm_vec_kernel(const float* o,
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const float r = v[e] * inv * wv[e];
-                out.v[e] = from_float<T>(order == 0 ? r : r / (1.0f + expf(-to_float(zv[m].v[e]))));
+                out.v[e] = from_float<T>(order == 0 ? r : r * sigmoid_for<T>(to_float(zv[m].v[e])));
             }
             *reinterpret_cast<Four*>(yrow + i) = out;
         }
@@ -952,10 +965,10 @@ static int conv_launch(const void* in, int in_stride, int in_off, const float* w
                        long long state_stride, int conv_off, const int* token_seq, const int* cu_q, const int* state_slots,
                        const int* seq_fresh, void* out, int T_, int n_seqs, int C, int taps, int flags,
                        cudaStream_t stream) {
-    constexpr int V = 16 / (int)sizeof(T);
+    constexpr int V = 16 / (int)sizeof(T), PER = 4;
     const bool vec = taps >= 2 && taps <= 4 && C % V == 0 && in_off % V == 0 && in_stride % V == 0 &&
                      (((uintptr_t)in | (uintptr_t)out | (uintptr_t)w) & 15) == 0;
-    const int per = vec ? V : 1;
+    const int per = vec ? PER : 1;
     const int lanes = (C + per - 1) / per;
     const int threads = lanes >= 128 ? 128 : ((lanes + 31) / 32) * 32;
     // a thread's weights are read once for its tile of tokens; few tokens get small tiles, so that they still fill the GPU
@@ -967,9 +980,9 @@ static int conv_launch(const void* in, int in_stride, int in_off, const float* w
               tile, flags)
     if (vec) {
         switch (taps) {
-            case 2: FF_CONV(V, 2); break;
-            case 3: FF_CONV(V, 3); break;
-            case 4: FF_CONV(V, 4); break;
+            case 2: FF_CONV(PER, 2); break;
+            case 3: FF_CONV(PER, 3); break;
+            case 4: FF_CONV(PER, 4); break;
             default: return FF_ERR_BAD_ARG;      // not reached: `vec` holds only for 2 to 4 taps
         }
     } else {
