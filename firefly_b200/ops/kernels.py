@@ -81,6 +81,7 @@ _MODULES = {
     "layer_norm": ("layer_norm.cu", None),
     "wkv": ("wkv.cu", None),
     "latent_attention": ("latent_attention.cu", None),
+    "gemm_few": ("gemm_few.cu", None),
     "moe": ("moe.cu", None),
     "moe_tcgen05": ("moe_tcgen05.cu", None),
     "ssm": ("ssm.cu", None),
@@ -417,6 +418,55 @@ def gemm_tc(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, epilogue: 
         _p(x), _p(weight), _p(out), c_int(out.stride(0)), c_int(T), c_int(N), c_int(Kd), c_int(epilogue),
         c_int(want_splits), c_int(1 if USE_PDL else 0), _p(xw), _p(xw_w), _p(ssq_out), _p(ssq_in),
         c_int(parts), c_int(dim), c_float(eps), _p(status), _stream()), "gemm_tc")
+
+
+USE_GEMM_FEW = True        # tests flip this to compare with `gemm_tc`
+
+
+@functools.lru_cache(maxsize=4096)
+def _gemm_few_takes(T: int, N: int, Kd: int) -> bool:
+    return bool(_lib("gemm_few").ff_gemm_few_usable(c_int(T), c_int(N), c_int(Kd)))
+
+
+def gemm_few_usable(T: int, N: int, Kd: int) -> bool:
+    """True if the product of a few tokens with a small matrix (csrc/gemm_few.cu) takes this size."""
+    return USE_GEMM_FEW and _gemm_few_takes(T, N, Kd)
+
+
+@functools.lru_cache(maxsize=None)
+def gemm_few_rows() -> int:
+    """Matrix rows that a row of that product's sums of squares stands for."""
+    return int(_lib("gemm_few").ff_gemm_few_rows())
+
+
+def gemm_few(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, epilogue: int, *, norm_out: Optional[tuple] = None,
+             norm_in: Optional[tuple] = None) -> None:
+    """`gemm_tc` for at most eight tokens and a short K in steps of 32 (`gemm_few_usable`); ``norm_out``'s sums of squares are
+    [ceil(N / gemm_few_rows()), T]."""
+    _need_cuda(x, weight, out)
+    assert x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16
+    T, Kd = x.shape
+    N = weight.shape[0]
+    assert weight.shape[1] == Kd
+    assert out.dtype == (torch.bfloat16 if epilogue in (EPI_BF16, EPI_SWIGLU, EPI_RELU2) else torch.float32)
+    assert out.shape[0] == T and out.shape[1] == (N // 2 if epilogue == EPI_SWIGLU else N)
+    xw = xw_w = ssq_out = ssq_in = None
+    parts = dim = 0
+    eps = 0.0
+    if norm_out is not None:
+        xw, xw_w, ssq_out = norm_out
+        _need_cuda(xw, xw_w, ssq_out)
+        assert epilogue == EPI_RESIDUAL_ADD and xw.dtype == torch.bfloat16 and xw.shape == (T, N)
+        assert xw_w.dtype == torch.float32 and xw_w.numel() == N
+        assert ssq_out.dtype == torch.float32 and ssq_out.numel() >= -(-N // gemm_few_rows()) * T
+    if norm_in is not None:
+        ssq_in, dim, eps = norm_in
+        _need_cuda(ssq_in)
+        assert ssq_in.dtype == torch.float32 and ssq_in.dim() == 2 and ssq_in.shape[1] == T
+        parts = ssq_in.shape[0]
+    _check(_lib("gemm_few").ff_gemm_few(
+        _p(x), _p(weight), _p(out), c_int(out.stride(0)), c_int(T), c_int(N), c_int(Kd), c_int(epilogue), _p(xw), _p(xw_w), _p(ssq_out),
+        _p(ssq_in), c_int(parts), c_int(dim), c_float(eps), _stream()), "gemm_few")
 
 
 def gemm_pair_plan(T: int, N: int, K: int, want_ranges: int):

@@ -72,7 +72,9 @@ def _tc(x, weight, out, epilogue, ctx, norm_out=None) -> None:
     if isinstance(x, FoldedNorm):
         kw["norm_in"] = (x.ssq, x.norm.size, x.norm.eps)
         x = x.xw
-    if x.shape[0] > K.GEMM_TC_MAX_TOKENS:
+    if K.gemm_few_usable(x.shape[0], N, Kd):
+        K.gemm_few(x, weight, out, epilogue, norm_out=norm_out, **kw)
+    elif x.shape[0] > K.GEMM_TC_MAX_TOKENS:
         K.gemm_pair(x, weight, out, epilogue, _pair_ranges(x.shape[0], N, Kd), ctx.status, norm_out=norm_out, **kw)
     else:
         K.gemm_tc(x, weight, out, epilogue, _splits(N, Kd), ctx.status, norm_out=norm_out, **kw)
@@ -116,7 +118,9 @@ def linear_into_residual(x: torch.Tensor, weight: torch.Tensor, residual: Option
         if then_norm is not None and K.FOLD_NORM and getattr(then_norm, "foldable", False) \
                 and then_norm.size == weight.shape[0]:
             from .norm import FoldedNorm
-            xw, nw, ssq = then_norm.fold_buffers(x.shape[0], ctx)
+            few = K.gemm_few_usable(x.shape[0], *weight.shape)     # its sums of squares stand for fewer rows than the others' tiles
+            xw, nw, ssq = then_norm.fold_buffers(x.shape[0], ctx, K.gemm_few_rows()) if few \
+                else then_norm.fold_buffers(x.shape[0], ctx)
             _tc(x, weight, residual, K.EPI_RESIDUAL_ADD, ctx, norm_out=(xw, nw, ssq))
             return FoldedNorm(then_norm, residual, xw, ssq, ctx)
         _tc(x, weight, residual, K.EPI_RESIDUAL_ADD, ctx)

@@ -107,10 +107,10 @@ class RMSNorm(Part):
                         eps_next=following.eps if following is not None else 0.0, out=out)
         return out
 
-    def fold_buffers(self, T: int, ctx):
+    def fold_buffers(self, T: int, ctx, tile: int = 128):
         """(xw [T, size] bfloat16, norm weight, ssq [tiles, T] float32) for a product that folds this
-        norm into its residual-adding epilogue."""
-        tiles = -(-self.size // 128)
+        norm into its residual-adding epilogue, in tiles of ``tile`` columns."""
+        tiles = -(-self.size // tile)
         xw = ctx.workspace.get(self.fold_tag + ".xw", (T, self.size), torch.bfloat16)
         ssq = ctx.workspace.get(self.fold_tag + ".ssq", (tiles, T), torch.float32)
         return xw, self.weight, ssq
