@@ -10,24 +10,6 @@
 namespace ff {
 
 // ---------------------------------------------------------------- embedding --
-template <typename TT>
-__global__ void embedding_kernel(const int* __restrict__ ids, const TT* __restrict__ table,
-                                 float* __restrict__ out, int H, int V, float scale, int* __restrict__ status) {
-    pdl_prologue();
-    const int t = blockIdx.x;
-    int id = ids[t];
-    if (id < 0 || id >= V) {  // never read outside the table; report it
-        if (threadIdx.x == 0) atomicExch(status, 1);
-        id = 0;
-    }
-    const TT* src = table + (size_t)id * H;
-    float* dst = out + (size_t)t * H;
-    for (int i = threadIdx.x; i < H; i += blockDim.x) dst[i] = to_float(src[i]) * scale;
-}
-
-// ------------------------------------------------------ residual add + norm --
-// residual[src,:] (+= delta[src,:]);  out[r,:] = v * rsqrt(mean(v^2)+eps) * w
-// src = row_idx ? row_idx[r] : r.  With row_idx the residual is not written back.
 // four consecutive elements of either type
 __device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ float4 load4(const bf16* p) {
@@ -45,6 +27,45 @@ __device__ __forceinline__ void store4(bf16* p, float4 v) {
     *reinterpret_cast<uint2*>(p) = raw;
 }
 
+// VEC elements a thread and step, 16 bytes of the table's row where sizes and addresses allow: with one element at a time a row of 4096
+// was a chain of sixteen rounds of 2-byte loads, 13.4 us for 8 tokens and 20 us for 2048 (floor 7.7).
+template <typename TT, int VEC>
+__global__ void embedding_kernel(const int* __restrict__ ids, const TT* __restrict__ table,
+                                 float* __restrict__ out, int H, int V, float scale, int* __restrict__ status) {
+    pdl_prologue();
+    const int t = blockIdx.x;
+    int id = pdl_fresh(ids)[t];
+    if (id < 0 || id >= V) {  // never read outside the table; report it
+        if (threadIdx.x == 0) atomicExch(status, 1);
+        id = 0;
+    }
+    const TT* src = table + (size_t)id * H;
+    float* dst = out + (size_t)t * H;
+    if constexpr (VEC == 1) {
+        for (int i = threadIdx.x; i < H; i += blockDim.x) dst[i] = to_float(src[i]) * scale;
+    } else {
+        for (int i = threadIdx.x * VEC; i < H; i += blockDim.x * VEC) {
+            float4 v[VEC / 4];
+            if constexpr (sizeof(TT) == 2) {
+                const uint4 raw = *reinterpret_cast<const uint4*>(src + i);
+                const uint32_t p[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+                    v[j] = make_float4(__uint_as_float(p[2 * j] << 16), __uint_as_float(p[2 * j] & 0xffff0000u),
+                                       __uint_as_float(p[2 * j + 1] << 16), __uint_as_float(p[2 * j + 1] & 0xffff0000u));
+            } else {
+                v[0] = load4(src + i);
+            }
+#pragma unroll
+            for (int j = 0; j < VEC / 4; ++j)
+                store4(dst + i + 4 * j, make_float4(v[j].x * scale, v[j].y * scale, v[j].z * scale, v[j].w * scale));
+        }
+    }
+}
+
+// ------------------------------------------------------ residual add + norm --
+// residual[src,:] (+= delta[src,:]);  out[r,:] = v * rsqrt(mean(v^2)+eps) * w
+// src = row_idx ? row_idx[r] : r.  With row_idx the residual is not written back.
 // VEC = 4: four elements a thread and step (needs H % 4 == 0); VEC = 1: any H.
 template <typename TD, typename TO, int VEC>
 __global__ void add_rms_norm_kernel(float* __restrict__ residual, const TD* __restrict__ delta,
@@ -224,13 +245,21 @@ FF_EXPORT int ff_scatter_int(int* buf, const int* upd, int cap, int len, cudaStr
 FF_EXPORT int ff_embedding(const int* ids, const void* table, int table_dtype, float* out, int T,
                            int H, int V, float scale, int* status, cudaStream_t stream) {
     if (T <= 0) return 0;
-    int threads = H >= 1024 ? 256 : (H >= 256 ? 128 : 64);
-    if (table_dtype == 0)
-        FF_LAUNCH((embedding_kernel<float>), T, threads, 0, stream, ids, (const float*)table, out, H, V, scale, status);
-    else if (table_dtype == 1)
-        FF_LAUNCH((embedding_kernel<bf16>), T, threads, 0, stream, ids, (const bf16*)table, out, H, V, scale, status);
-    else
-        return FF_ERR_BAD_ARG;
+    if (table_dtype != 0 && table_dtype != 1) return FF_ERR_BAD_ARG;
+    const int vec = table_dtype == 1 ? 8 : 4;
+    if (H % vec == 0 && (((uintptr_t)table | (uintptr_t)out) & 15) == 0) {
+        const int threads = min(512, max(32, (H / vec + 31) / 32 * 32));
+        if (table_dtype == 0)
+            FF_LAUNCH((embedding_kernel<float, 4>), T, threads, 0, stream, ids, (const float*)table, out, H, V, scale, status);
+        else
+            FF_LAUNCH((embedding_kernel<bf16, 8>), T, threads, 0, stream, ids, (const bf16*)table, out, H, V, scale, status);
+    } else {
+        const int threads = H >= 1024 ? 256 : (H >= 256 ? 128 : 64);
+        if (table_dtype == 0)
+            FF_LAUNCH((embedding_kernel<float, 1>), T, threads, 0, stream, ids, (const float*)table, out, H, V, scale, status);
+        else
+            FF_LAUNCH((embedding_kernel<bf16, 1>), T, threads, 0, stream, ids, (const bf16*)table, out, H, V, scale, status);
+    }
     FF_LAUNCH_CHECK();
     return 0;
 }
