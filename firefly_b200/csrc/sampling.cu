@@ -54,11 +54,12 @@ __device__ __forceinline__ void block_best(float& best, int& best_i, float* s_va
 }
 
 // grid (rows, chunks).  With one chunk the token is written at once; else each block leaves
-// its chunk's best in scratch memory for sample_final_kernel.
+// its chunk's best in scratch memory for sample_final_kernel.  `status` (may be null): this word, as the kernels in
+// front left it, is written behind the last token, so that one copy to the host brings both (a second one costs 6 us).
 __global__ void sample_kernel(const float* __restrict__ logits, int V, size_t row_stride,
                               const float* __restrict__ temperature, const long long* __restrict__ seeds,
                               const long long* __restrict__ counters, int* __restrict__ out,
-                              float* __restrict__ part_val, int* __restrict__ part_idx) {
+                              float* __restrict__ part_val, int* __restrict__ part_idx, const int* __restrict__ status) {
     __shared__ float s_val[32];
     __shared__ int s_idx[32];
     pdl_prologue();      // the logits come from the kernel in front
@@ -75,13 +76,16 @@ __global__ void sample_kernel(const float* __restrict__ logits, int V, size_t ro
     scan_range(row, c * per, min(V, (c + 1) * per), greedy, inv_t, seed, ctr, best, best_i);
     block_best(best, best_i, s_val, s_idx);
     if (threadIdx.x == 0) {
-        if (chunks == 1) out[r] = best_i == 0x7fffffff ? 0 : best_i;
+        if (chunks == 1) {
+            out[r] = best_i == 0x7fffffff ? 0 : best_i;
+            if (status && r == 0) out[gridDim.x] = *pdl_fresh(status);
+        }
         else { part_val[r * chunks + c] = best; part_idx[r * chunks + c] = best_i; }
     }
 }
 
 __global__ void sample_final_kernel(const float* __restrict__ part_val, const int* __restrict__ part_idx,
-                                    int chunks, int* __restrict__ out) {
+                                    int chunks, int* __restrict__ out, const int* __restrict__ status) {
     __shared__ float s_val[32];
     __shared__ int s_idx[32];
     pdl_prologue();      // the chunks' results come from sample_kernel
@@ -90,7 +94,10 @@ __global__ void sample_final_kernel(const float* __restrict__ part_val, const in
     int best_i = 0x7fffffff;
     for (int c = threadIdx.x; c < chunks; c += blockDim.x) better(best, best_i, part_val[r * chunks + c], part_idx[r * chunks + c]);
     block_best(best, best_i, s_val, s_idx);
-    if (threadIdx.x == 0) out[r] = best_i == 0x7fffffff ? 0 : best_i;
+    if (threadIdx.x == 0) {
+        out[r] = best_i == 0x7fffffff ? 0 : best_i;
+        if (status && r == 0) out[gridDim.x] = *pdl_fresh(status);
+    }
 }
 
 }  // namespace ff
@@ -101,13 +108,14 @@ using namespace ff;
 // that many blocks and needs scratch memory of rows*chunks floats and ints.
 FF_EXPORT int ff_sample(const float* logits, int rows, int V, size_t row_stride,
                         const float* temperature, const long long* seeds, const long long* counters,
-                        int* out, int chunks, float* part_val, int* part_idx, cudaStream_t stream) {
+                        int* out, int chunks, float* part_val, int* part_idx, const int* status,
+                        cudaStream_t stream) {
     if (rows <= 0) return 0;
     if (V <= 0 || chunks < 1 || chunks > 1024) return FF_ERR_BAD_ARG;
     if (chunks > 1 && (!part_val || !part_idx)) return FF_ERR_BAD_ARG;
     FF_LAUNCH((sample_kernel), dim3(rows, chunks), SAMPLE_THREADS, 0, stream, logits, V, row_stride, temperature,
-              seeds, counters, out, part_val, part_idx);
+              seeds, counters, out, part_val, part_idx, status);
     if (chunks > 1)
-        FF_LAUNCH((sample_final_kernel), rows, 32, 0, stream, (const float*)part_val, (const int*)part_idx, chunks, out);
+        FF_LAUNCH((sample_final_kernel), rows, 32, 0, stream, (const float*)part_val, (const int*)part_idx, chunks, out, status);
     return 0;
 }

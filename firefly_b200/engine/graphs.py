@@ -41,14 +41,37 @@ from .runner import MetaLayout, ModelRunner, StepEntry, StepError
 
 class _Bucket:
     __slots__ = ("size", "layout", "meta_host", "meta_stage", "meta_dev", "graph", "logits", "tokens", "h_tokens",
-                 "events", "launches", "lanes", "turn", "by_length", "samp_stage", "samp_dev", "samp_greedy", "h_status",
-                 "changes", "full_upload", "q_lens", "rows", "starts", "stage_events")
+                 "events", "launches", "lanes", "turn", "by_length", "samp_stage", "samp_dev", "samp_greedy",
+                 "changes", "full_upload", "q_lens", "rows", "starts", "stage_events", "host", "stages", "heads")
+
+    def set_buffers(self, layout: MetaLayout, sampled: int, device) -> None:
+        """Metadata and result buffers, two of everything the host touches while a replay may still be using the
+        other, and the views of them that every step asks for again."""
+        self.layout = layout
+        self.meta_host = torch.zeros(layout.size, dtype=torch.int32).pin_memory()
+        self.meta_stage = [torch.zeros(layout.size, dtype=torch.int32).pin_memory() for _ in range(2)]
+        self.meta_dev = torch.zeros(layout.size, dtype=torch.int32, device=device)
+        self.host, self.stages = self.meta_host.numpy(), [t.numpy() for t in self.meta_stage]
+        self.heads = (self.meta_dev[:layout.head_size], [t[:layout.head_size] for t in self.meta_stage])
+        # one more element than rows are sampled: the device's status word, which the sampler puts behind the tokens
+        self.tokens = torch.zeros(sampled + 1, dtype=torch.int32, device=device)
+        self.h_tokens = [torch.zeros(sampled + 1, dtype=torch.int32).pin_memory() for _ in range(2)]
+
+    def upload(self, k: int, full: bool) -> int:
+        """Put the metadata (its head, or all of it) on its way to the device; how many integers that are."""
+        upto = self.layout.size if full else self.layout.head_size
+        self.stages[k][:upto] = self.host[:upto]
+        if full:
+            self.meta_dev.copy_(self.meta_stage[k], non_blocking=True)
+        else:
+            self.heads[0].copy_(self.heads[1][k], non_blocking=True)
+        return upto
 
 
 class LaunchedStep:
     """A replay that has been put on the stream: its tokens arrive in ``h_tokens`` once
     ``event`` has passed."""
-    __slots__ = ("bucket", "n", "h_tokens", "event", "logits", "h_status", "status_code")
+    __slots__ = ("bucket", "n", "h_tokens", "event", "logits", "status_code")
 
 
 class _Capture:
@@ -114,7 +137,7 @@ class DecodeGraphs:
         page.  Every write into a block table is also noted in ``b.changes`` (offset, values), from
         which the step's update list is made."""
         r, lay = self.runner, b.layout
-        h = b.meta_host.numpy()
+        h = b.host
         n = len(entries)
         if b.lanes is None:
             # constant parts, and every lane as padding: a dummy token at position 0 in the scratch page
@@ -146,23 +169,28 @@ class DecodeGraphs:
                 for off, w in zip(lay.tables, lay.widths):
                     put(off + i * w, [SCRATCH_PAGE])        # position 0 reads and writes the first entry only
                 b.lanes[i] = None
+        if not n:
+            return
+        # what changes in every step goes in array by array (64 lanes one by one cost 46 us in front of the replay)
+        toks = [int(e.tokens[0]) for e in entries]
+        if min(toks) < 0 or max(toks) >= r.vocab_size:
+            raise ValueError(f"token id {next(t for t in toks if not 0 <= t < r.vocab_size)} outside the vocabulary")
+        held = [e.cache.num_tokens for e in entries]
+        if max(held) + 1 > r.max_model_len:
+            raise ValueError(f"request {entries[held.index(max(held))].cache.request_id!r} exceeds max_model_len")
+        h[lay.token_ids: lay.token_ids + n] = toks
+        h[lay.positions: lay.positions + n] = held
+        h[lay.ctx_lens: lay.ctx_lens + n] = held
+        h[lay.seq_fresh: lay.seq_fresh + n] = [e.cache.fresh for e in entries]
         for i, e in enumerate(entries):
             rc = e.cache
-            cl = rc.num_tokens
-            tok = int(e.tokens[0])
-            if not (0 <= tok < r.vocab_size):
-                raise ValueError(f"token id {tok} outside the vocabulary")
-            if cl + 1 > r.max_model_len:
-                raise ValueError(f"request {rc.request_id!r} exceeds max_model_len")
-            h[lay.token_ids + i] = tok
-            h[lay.positions + i] = cl
-            h[lay.ctx_lens + i] = cl
-            h[lay.seq_fresh + i] = 1 if rc.fresh else 0
+            lens = [len(t) for t in rc.tables]
             old = b.lanes[i]
             same = old is not None and old[0] == rc.serial
+            if same and old[1] == lens and old[2] == rc.first_live:
+                continue
             if not same:
                 h[lay.state_slots + i] = rc.state_slot
-            lens = []
             for g, table in enumerate(rc.tables):
                 row = lay.tables[g] + i * lay.widths[g]
                 if same and old[2][g] == rc.first_live[g] and old[1][g] <= len(table):
@@ -172,14 +200,13 @@ class DecodeGraphs:
                     # entries behind the request's pages are never read (a key's page index is below its
                     # count of pages), so what an earlier request left there may stay
                     put(row, list(table))
-                lens.append(len(table))
             b.lanes[i] = (rc.serial, lens, list(rc.first_live))
 
     def _write_updates(self, b: _Bucket) -> bool:
         """The step's table changes as (index, value) pairs in the buffer's update list.  False if
         they do not fit: then the whole buffer has to be uploaded."""
         lay = b.layout
-        h = b.meta_host.numpy()
+        h = b.host
         count = sum(len(v) for _, v in b.changes)
         fits = count <= lay.update_cap and not b.full_upload
         if fits:
@@ -198,20 +225,13 @@ class DecodeGraphs:
         r = self.runner
         b = _Bucket()
         b.size = size
-        b.layout = MetaLayout(size, size, size, r.max_blocks, update_cap=max(64, 4 * size))
+        b.set_buffers(MetaLayout(size, size, size, r.max_blocks, update_cap=max(64, 4 * size)), size, r.device)
         b.changes, b.full_upload = [], True
-        b.meta_host = torch.zeros(b.layout.size, dtype=torch.int32).pin_memory()
-        # two of everything the host touches while a replay may still be using the other
-        b.meta_stage = [torch.zeros(b.layout.size, dtype=torch.int32).pin_memory() for _ in range(2)]
-        b.meta_dev = torch.zeros(b.layout.size, dtype=torch.int32, device=r.device)
-        b.tokens = torch.zeros(size, dtype=torch.int32, device=r.device)
         # per lane: seed (int64), counter (int64), temperature (float32), in this order so that the
         # 64-bit values are aligned whatever the size; all zero = every lane greedy
         b.samp_stage = [torch.zeros(5 * size, dtype=torch.int32).pin_memory() for _ in range(2)]
         b.samp_dev = torch.zeros(5 * size, dtype=torch.int32, device=r.device)
         b.samp_greedy = True
-        b.h_tokens = [torch.zeros(size, dtype=torch.int32).pin_memory() for _ in range(2)]
-        b.h_status = [torch.zeros(1, dtype=torch.int32).pin_memory() for _ in range(2)]
         b.events = [torch.cuda.Event() for _ in range(2)]
         b.turn = 0
         b.lanes = None
@@ -270,7 +290,7 @@ class DecodeGraphs:
     def _sample(self, b: _Bucket, logits: torch.Tensor) -> None:
         d, n = b.samp_dev, b.size
         K.sample(logits, b.tokens, d[4 * n:].view(torch.float32), d[:2 * n].view(torch.int64),
-                 d[2 * n: 4 * n].view(torch.int64))
+                 d[2 * n: 4 * n].view(torch.int64), status=self.runner.status)
 
     def _upload_sampling(self, b: _Bucket, k: int, sampling) -> None:
         """Per-lane (temperature, seed, counter) for the next replay; nothing is copied while
@@ -303,13 +323,10 @@ class DecodeGraphs:
         k = b.turn
         b.turn ^= 1
         self._upload_sampling(b, k, sampling)
-        stage = b.meta_stage[k]
         # the head (tokens, positions, lengths, the update list) always; the tables only when more of
         # them changed than the list holds
-        upto = b.layout.head_size if self._write_updates(b) else b.layout.size
+        upto = b.upload(k, full=not self._write_updates(b))
         self.full_uploads += upto == b.layout.size
-        stage[:upto].copy_(b.meta_host[:upto])
-        b.meta_dev[:upto].copy_(stage[:upto], non_blocking=True)
         self.h2d_bytes += 4 * upto
         if tokens_from_last_replay:
             lay = b.layout
@@ -323,12 +340,10 @@ class DecodeGraphs:
         self.kernel_launches += launches
         step = LaunchedStep()
         step.bucket, step.n, step.logits = b, n, logits[:n]
-        step.h_tokens, step.event, step.h_status, step.status_code = None, None, None, 0
+        step.h_tokens, step.event, step.status_code = None, None, 0
         if want_tokens:
             step.h_tokens = b.h_tokens[k]
-            step.h_tokens[:n].copy_(b.tokens[:n], non_blocking=True)
-            step.h_status = b.h_status[k]              # the status word rides behind the tokens
-            step.h_status.copy_(self.runner.status, non_blocking=True)
+            step.h_tokens.copy_(b.tokens, non_blocking=True)      # the status word rides behind the tokens
             step.event = b.events[k]
             step.event.record()
         for e in entries:
@@ -392,22 +407,17 @@ class DecodeGraphs:
         n, T, nr = len(q_lens), sum(q_lens), len(rows)
         b = _Bucket()
         b.size, b.q_lens, b.rows = n, list(q_lens), list(rows)
-        b.layout = lay = MetaLayout(T, n, max(nr, 1), r.max_blocks, update_cap=max(64, 4 * n))
+        lay = MetaLayout(T, n, max(nr, 1), r.max_blocks, update_cap=max(64, 4 * n))
+        b.set_buffers(lay, nr, r.device)
         b.changes, b.full_upload = [], True
-        b.meta_host = torch.zeros(lay.size, dtype=torch.int32).pin_memory()
-        b.meta_stage = [torch.zeros(lay.size, dtype=torch.int32).pin_memory() for _ in range(2)]
         b.stage_events = [None, None]
-        b.meta_dev = torch.zeros(lay.size, dtype=torch.int32, device=r.device)
-        b.tokens = torch.zeros(max(nr, 1), dtype=torch.int32, device=r.device)
         b.samp_stage = [torch.zeros(5 * max(nr, 1), dtype=torch.int32).pin_memory() for _ in range(2)]
         b.samp_dev = torch.zeros(5 * max(nr, 1), dtype=torch.int32, device=r.device)
         b.samp_greedy = True
-        b.h_tokens = [torch.zeros(max(nr, 1), dtype=torch.int32).pin_memory() for _ in range(2)]
-        b.h_status = [torch.zeros(1, dtype=torch.int32).pin_memory() for _ in range(2)]
         b.events = [torch.cuda.Event() for _ in range(2)]
         b.turn, b.by_length = 0, None
         b.lanes = [None] * n
-        h = b.meta_host.numpy()
+        h = b.host
         b.starts = []
         pos = 0
         for i, ql in enumerate(q_lens):
@@ -455,12 +465,12 @@ class DecodeGraphs:
 
     def _sample_rows(self, b: _Bucket, logits: torch.Tensor, nr: int) -> None:
         d = b.samp_dev
-        K.sample(logits, b.tokens[:nr], d[4 * nr:].view(torch.float32), d[:2 * nr].view(torch.int64),
-                 d[2 * nr: 4 * nr].view(torch.int64))
+        K.sample(logits, b.tokens, d[4 * nr:].view(torch.float32), d[:2 * nr].view(torch.int64),
+                 d[2 * nr: 4 * nr].view(torch.int64), status=self.runner.status)
 
     def _fill_shape(self, b: _Bucket, entries: Sequence[StepEntry]) -> None:
         r, lay = self.runner, b.layout
-        h = b.meta_host.numpy()
+        h = b.host
 
         def put(off, values):
             h[off: off + len(values)] = values
@@ -518,11 +528,8 @@ class DecodeGraphs:
             size_was, b.size = b.size, nr          # the sampling buffer has one lane per wanted row
             self._upload_sampling(b, k, sampling)
             b.size = size_was
-        stage = b.meta_stage[k]
-        upto = b.layout.head_size if self._write_updates(b) else b.layout.size
+        upto = b.upload(k, full=not self._write_updates(b))
         self.full_uploads += upto == b.layout.size
-        stage[:upto].copy_(b.meta_host[:upto])
-        b.meta_dev[:upto].copy_(stage[:upto], non_blocking=True)
         b.stage_events[k].record()
         self.h2d_bytes += 4 * upto
         b.graph.replay()
@@ -533,11 +540,11 @@ class DecodeGraphs:
         self.runner.steps_run += 1
         if not nr:
             return None, 0
-        b.h_tokens[k][:nr].copy_(b.tokens[:nr], non_blocking=True)
-        b.h_status[k].copy_(self.runner.status, non_blocking=True)
+        b.h_tokens[k].copy_(b.tokens, non_blocking=True)
         b.events[k].record()
         b.events[k].synchronize()
-        return b.h_tokens[k][:nr].tolist(), int(b.h_status[k][0])
+        *tokens, status = b.h_tokens[k].tolist()
+        return tokens, status
 
     @staticmethod
     def collect(step: LaunchedStep) -> Optional[List[int]]:
@@ -545,8 +552,9 @@ class DecodeGraphs:
         if step.event is None:
             return None
         step.event.synchronize()
-        step.status_code = int(step.h_status[0])
-        return step.h_tokens[:step.n].tolist()
+        got = step.h_tokens.tolist()
+        step.status_code = got[-1]
+        return got[:step.n]
 
     def run(self, entries: Sequence[StepEntry], want_tokens: bool = True, sampling=None
             ) -> Tuple[torch.Tensor, Optional[List[int]]]:

@@ -290,18 +290,21 @@ _sample_scratch = {}
 
 
 def sample(logits: torch.Tensor, out: torch.Tensor, temperature: Optional[torch.Tensor] = None,
-           seeds: Optional[torch.Tensor] = None, counters: Optional[torch.Tensor] = None) -> None:
+           seeds: Optional[torch.Tensor] = None, counters: Optional[torch.Tensor] = None,
+           status: Optional[torch.Tensor] = None) -> None:
     """out[r] = arg-max of logits[r] (lowest index on ties), or, where
     temperature[r] > 0, a draw from softmax(logits[r] / temperature[r]) with the
-    random numbers of (seeds[r], counters[r]).
+    random numbers of (seeds[r], counters[r]).  ``status``: out has one more element, into
+    which this word is copied.
 
     The one wrapper that keeps memory of its own: the partial results of rows split over several
     blocks live in a scratch pair per device that grows when more rows come.  It never grows while
     the stream is being captured (an error then: the run before the capture sizes it)."""
     global LAUNCHES
-    _need_cuda(logits, out, temperature, seeds, counters)
+    _need_cuda(logits, out, temperature, seeds, counters, status)
     assert logits.dtype == torch.float32 and out.dtype == torch.int32 and logits.dim() == 2
     rows, V = logits.shape
+    assert status is None or (status.dtype == torch.int32 and out.dim() == 1 and out.numel() > rows)
     if temperature is not None:
         assert temperature.dtype == torch.float32 and seeds.dtype == torch.int64 \
             and counters.dtype == torch.int64
@@ -321,7 +324,7 @@ def sample(logits: torch.Tensor, out: torch.Tensor, temperature: Optional[torch.
         pv, pi = buf
     _check(_lib("sampling").ff_sample(_p(logits), c_int(rows), c_int(V), c_size_t(logits.stride(0)),
                                      _p(temperature), _p(seeds), _p(counters), _p(out), c_int(chunks),
-                                     _p(pv), _p(pi), _stream()), "sample")
+                                     _p(pv), _p(pi), _p(status), _stream()), "sample")
     if chunks > 1:
         LAUNCHES += 1
 

@@ -1,4 +1,4 @@
-"""The first kernel of a step: rows out of the embedding."""
+"""The first and the last kernel of a step: rows out of the embedding, and the sampled tokens with the status word behind them."""
 import pytest
 import torch
 
@@ -19,3 +19,12 @@ def test_embedding_rows_by_16_bytes_and_one_by_one(H, shift, dtype):
     ids[3] = -1
     K.embedding(ids, table, out, status)
     assert int(status) == 1
+
+
+@pytest.mark.parametrize("rows,V", [(1, 300), (5, 300), (1, 151936), (64, 32768)])
+def test_status_word_behind_the_tokens(rows, V):
+    from firefly_b200.ops import kernels as K
+    logits = torch.randn(rows, V, device="cuda")
+    out, status = torch.full((rows + 2,), -7, dtype=torch.int32, device="cuda"), torch.full((1,), 42, dtype=torch.int32, device="cuda")
+    K.sample(logits, out, status=status)
+    assert out[:rows].tolist() == logits.argmax(-1).tolist() and out[rows:].tolist() == [42, -7]
