@@ -410,6 +410,8 @@ struct DecodeHeads {
     float temp_coef;           // heads finished here: q also times 1 + temp_coef ln(floor((pos + 1) / temp_every) + 1)
     int temp_every;            // (0: no such factor; it needs q_norm_w)
     int value_is_key;          // heads finished here: the row is q heads | k heads and the raw key is the value
+    int beside;                // the kernel in front is the same step's attention over prompts (attention_tc.cu): nothing here
+                               // depends on it, and it lets this one start only when what both read is there
 };
 constexpr int HC = D / 64;     // elements of each half of a head that a lane holds (heads finished in a warp)
 
@@ -621,7 +623,7 @@ attn_decode_body(const bf16* __restrict__ q, int q_stride, const bf16* __restric
         for (int c = G * CHUNKS + threadIdx.x; c < 16 * CHUNKS; c += NTHREADS)
             *reinterpret_cast<uint4*>(Qs + (c / CHUNKS) * KSTR + (c % CHUNKS) * 8) = make_uint4(0, 0, 0, 0);
     }
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (HEADS || !hd.beside) asm volatile("griddepcontrol.wait;" ::: "memory");
     if constexpr (UNITS) {
         if (split == 0 && kh == 0 && threadIdx.x == 0) un.seq_ranges[seq] = ranges;
     }
@@ -790,8 +792,9 @@ attn_decode_kernel(const bf16* __restrict__ q, int q_stride, const bf16* __restr
                    float* __restrict__ part_o, float* __restrict__ part_ml, int nq, int nkv,
                    int block_size, int num_blocks, float scale_log2, int window, int num_splits,
                    const float* __restrict__ dist_bias, int bias_len, float softcap_log2, const float* __restrict__ sink,
-                   int* __restrict__ status) {
+                   int beside, int* __restrict__ status) {
     DecodeHeads hd{};
+    hd.beside = beside;
     hd.sink = sink;
     hd.status = status;           // may be null: a missing page is then not reported
     hd.dist_bias = dist_bias;
@@ -800,6 +803,7 @@ attn_decode_kernel(const bf16* __restrict__ q, int q_stride, const bf16* __restr
     attn_decode_body<false, false, false>(q, q_stride, cache, block_table, max_blocks, cu_q, ctx_lens, out, out_stride,
                                    part_o, part_ml, nq, nkv, block_size, num_blocks, scale_log2, window, num_splits,
                                    hd, DecodeUnits{});
+    if (beside) asm volatile("griddepcontrol.wait;" ::: "memory");      // this kernel's end says that the one in front has ended too
 }
 template <bool XHEADS>
 __global__ void __launch_bounds__(NTHREADS)
@@ -827,6 +831,7 @@ attn_decode_units_kernel(const bf16* __restrict__ q, int q_stride, const bf16* _
         attn_decode_body<HEADS, true, XHEADS>(q, q_stride, cache, block_table, max_blocks, cu_q, ctx_lens, out, out_stride,
                                       part_o, part_ml, nq, nkv, block_size, num_blocks, scale_log2, window, 0, hd,
                                       un);
+    if (hd.beside) asm volatile("griddepcontrol.wait;" ::: "memory");   // as above
 }
 
 // out[token of seq, head, :] = sum_s w_s o_s / sum_s w_s l_s,  w_s = 2^(m_s - max m).
@@ -1019,19 +1024,19 @@ FF_EXPORT int ff_attn_decode(const void* q, int q_stride, const void* cache, con
                              int max_blocks, const int* cu_q, const int* ctx_lens, int n_seqs, void* out,
                              int out_stride, float* part_o, float* part_ml, int nq, int nkv,
                              int block_size, int num_blocks, float scale, int window, int num_splits,
-                             const float* dist_bias, int bias_len, float softcap, const float* sink, int* status,
-                             cudaStream_t stream) {
+                             const float* dist_bias, int bias_len, float softcap, const float* sink, int parts, int beside,
+                             int* status, cudaStream_t stream) {
     if (n_seqs <= 0) return 0;
     if (nkv <= 0 || nq % nkv || num_splits < 1 || (dist_bias && (window <= 0 || bias_len < window))) return FF_ERR_BAD_ARG;
     if (nq / nkv > 16) return FF_ERR_UNSUPPORTED;
     FF_SMEM_LIMIT(attn_decode_kernel, DECODE_SMEM);
     dim3 grid(n_seqs, nkv, num_splits);
-    FF_LAUNCH((attn_decode_kernel), grid, NTHREADS, DECODE_SMEM, stream, 
+    if (parts & 1) FF_LAUNCH((attn_decode_kernel), grid, NTHREADS, DECODE_SMEM, stream, 
         (const bf16*)q, q_stride, (const bf16*)cache, block_table, max_blocks, cu_q, ctx_lens, (bf16*)out,
         out_stride, part_o, part_ml, nq, nkv, block_size, num_blocks, scale * LOG2E, window, num_splits, dist_bias,
-        bias_len, softcap * LOG2E, sink, status);
+        bias_len, softcap * LOG2E, sink, beside, status);
     FF_LAUNCH_CHECK();
-    if (num_splits > 1) {
+    if (num_splits > 1 && (parts & 2)) {
         dim3 cgrid(n_seqs, nq);
         if (num_splits > 8)
             FF_LAUNCH((attn_combine_many_kernel), cgrid, COMBINE_THREADS, 0, stream, part_o, part_ml, cu_q, (bf16*)out,
@@ -1064,7 +1069,7 @@ FF_EXPORT int ff_attn_decode_heads(const void* qkv, int row_width, void* cache, 
     FF_SMEM_LIMIT(attn_decode_heads_kernel<false>, DECODE_SMEM);
     FF_SMEM_LIMIT(attn_decode_heads_kernel<true>, DECODE_SMEM);
     DecodeHeads hd{q_norm_w, k_norm_w, eps, cos_sin, max_positions, (bf16*)cache, status, nullptr, 0, 0.f, sink, temp_coef,
-                   temp_every, value_is_key};
+                   temp_every, value_is_key, 0};
     dim3 grid(n_seqs, nkv, num_splits);
     if (sink || temp_every > 0 || value_is_key)
         FF_LAUNCH((attn_decode_heads_kernel<true>), grid, NTHREADS, DECODE_SMEM, stream,
@@ -1100,7 +1105,8 @@ FF_EXPORT int ff_attn_decode_units(const void* q, int q_stride, void* cache, con
                                    int max_ranges, int finish_heads, const float* q_norm_w,
                                    const float* k_norm_w, float eps, const float* cos_sin, int max_positions,
                                    const float* dist_bias, int bias_len, float softcap, const float* sink, float temp_coef,
-                                   int temp_every, int value_is_key, int* status, cudaStream_t stream) {
+                                   int temp_every, int value_is_key, int parts, int beside, int* status, cudaStream_t stream) {
+    if (finish_heads && beside) return FF_ERR_BAD_ARG;
     if (finish_heads && temp_every > 0 && !q_norm_w) return FF_ERR_BAD_ARG;
     if (FF_KV_PLANES != 2 && finish_heads) return FF_ERR_UNSUPPORTED;
     if (n_seqs <= 0) return 0;
@@ -1116,10 +1122,11 @@ FF_EXPORT int ff_attn_decode_units(const void* q, int q_stride, void* cache, con
     FF_SMEM_LIMIT((attn_decode_units_kernel<true, false>), DECODE_SMEM);
     FF_SMEM_LIMIT((attn_decode_units_kernel<false, false>), DECODE_SMEM);
     DecodeHeads hd{q_norm_w, k_norm_w, eps, cos_sin, max_positions, (bf16*)cache, status, dist_bias, bias_len,
-                   softcap * LOG2E, sink, temp_coef, temp_every, value_is_key};
+                   softcap * LOG2E, sink, temp_coef, temp_every, value_is_key, beside};
     DecodeUnits un{n_seqs, max_ranges, seq_ranges, units};
     dim3 grid(nkv, units);
-    if (finish_heads && (sink || temp_every > 0 || value_is_key))
+    if (!(parts & 1)) {}
+    else if (finish_heads && (sink || temp_every > 0 || value_is_key))
         FF_LAUNCH((attn_decode_units_kernel<true, true>), grid, NTHREADS, DECODE_SMEM, stream,
             (const bf16*)q, q_stride, (const bf16*)cache, block_table, max_blocks, cu_q, ctx_lens, (bf16*)out,
             out_stride, part_o, part_ml, nq, nkv, block_size, num_blocks, scale * LOG2E, window, hd, un);
@@ -1132,7 +1139,7 @@ FF_EXPORT int ff_attn_decode_units(const void* q, int q_stride, void* cache, con
             (const bf16*)q, q_stride, (const bf16*)cache, block_table, max_blocks, cu_q, ctx_lens, (bf16*)out,
             out_stride, part_o, part_ml, nq, nkv, block_size, num_blocks, scale * LOG2E, window, hd, un);
     FF_LAUNCH_CHECK();
-    if (units > n_seqs && max_ranges > 1) {
+    if (units > n_seqs && max_ranges > 1 && (parts & 2)) {
         dim3 cgrid(n_seqs, nq);
         // a sequence gets at most this many ranges: many of them take the form that spreads them over warps
         const int most = max_ranges < units - n_seqs + 1 ? max_ranges : units - n_seqs + 1;

@@ -291,7 +291,6 @@ attn_tc_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __restri
     // of the tile's keys and leaves an unnormalised result with its (reference max, sum) for the join
     // kernel.  For prompts so short that their row tiles would leave most SMs idle while each block
     // walks a long chain of key tiles alone.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* Qs = base;                                        // [PANELS][128][128 B]
@@ -321,7 +320,10 @@ attn_tc_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __restri
                      ::"r"(sa(&s_tmem)), "r"((uint32_t)TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    // The next kernel may start once every block is behind this wait (and here, so that it may count on what the kernels in front
+    // wrote without a wait of its own: the decode attention beside this one, attention_mma.cu).
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // Row tiles are handed out last first, for all kv heads before the next tile: in a prompt the
     // late tiles see the most keys, and the long blocks should not be the ones that start last.
     const int vtile = (int)(units / (unsigned)nkv) - 1 - (int)(unit / (unsigned)nkv);
@@ -1149,13 +1151,14 @@ FF_EXPORT int ff_attn_tc_block_m() { return BM; }
 // results in part_o (float [tokens * nq * num_splits * D]) and part_ml (float [tokens * nq * num_splits * 2]),
 // indexed by the token's row in q/out; a second kernel joins them for the n_tokens rows from tok_base on
 // (the rows of the sequences given here).
+// parts: 1 the attention itself, 2 the kernel that joins the shares, 3 both (a caller may put another kernel between them).
 // two_tiles: two row tiles a block where that kernel takes the call (heads of 64 and 128, one share, neither bias nor cap), as the caller
 // finds it faster.
 FF_EXPORT int ff_attn_tc(const void* q, int q_stride, const void* cache, const int* block_table, int max_blocks,
                          const int* cu_q, const int* ctx_lens, int n_seqs, int total_tiles, void* out,
                          int out_stride, int nq, int nkv, int block_size, int num_blocks, float scale, int window,
                          int* status, int num_splits, float* part_o, float* part_ml, int tok_base, int n_tokens,
-                         const float* dist_bias, int bias_len, float softcap, const float* sink, int two_tiles, cudaStream_t stream) {
+                         const float* dist_bias, int bias_len, float softcap, const float* sink, int two_tiles, int parts, cudaStream_t stream) {
     if (n_seqs <= 0 || total_tiles <= 0) return 0;
     if (nkv <= 0 || nq % nkv || (dist_bias && (window <= 0 || bias_len < window))) return FF_ERR_BAD_ARG;
     if (num_splits < 1 || (num_splits > 1 && (!part_o || !part_ml || n_tokens <= 0 || tok_base < 0))) return FF_ERR_BAD_ARG;
@@ -1174,6 +1177,7 @@ FF_EXPORT int ff_attn_tc(const void* q, int q_stride, const void* cache, const i
 #if FF_ATC_PAIR
     const long long pairs = (((long long)total_tiles + n_seqs) / 2) * nkv;    // at least ceil(row tiles of a sequence / 2), summed
     if (two_tiles && num_splits == 1 && !dist_bias && softcap == 0.f && pairs < (1ll << 31)) {
+        if (!(parts & 1)) return 0;
         FF_SMEM_LIMIT(attn_tc_pair_kernel, PAIR_SMEM);
         FF_LAUNCH((attn_tc_pair_kernel), dim3((unsigned)pairs), PAIR_THREADS, PAIR_SMEM, stream, arg, (const bf16*)q, q_stride,
                   block_table, max_blocks, cu_q, ctx_lens, n_seqs, (bf16*)out, out_stride, nq, nkv, block_size, num_blocks,
@@ -1182,10 +1186,10 @@ FF_EXPORT int ff_attn_tc(const void* q, int q_stride, const void* cache, const i
     }
 #endif
     if ((long long)total_tiles * nkv * num_splits >= (1ll << 31)) return FF_ERR_UNSUPPORTED;
-    FF_LAUNCH((attn_tc_kernel), dim3((unsigned)(total_tiles * nkv * num_splits)), ATC_THREADS, ATC_SMEM, stream, arg,
+    if (parts & 1) FF_LAUNCH((attn_tc_kernel), dim3((unsigned)(total_tiles * nkv * num_splits)), ATC_THREADS, ATC_SMEM, stream, arg,
               (const bf16*)q, q_stride, block_table, max_blocks, cu_q, ctx_lens, n_seqs, (bf16*)out, out_stride, nq, nkv,
               block_size, num_blocks, scale * LOG2E, window, status, num_splits, part_o, part_ml, dist_bias, bias_len, softcap * LOG2E, sink);
-    if (num_splits > 1) {
+    if (num_splits > 1 && (parts & 2)) {
         const int n_pairs = n_tokens * nq, per_block = JOIN_THREADS / (D / 4);
         FF_LAUNCH((attn_tc_join_kernel), dim3((unsigned)((n_pairs + per_block - 1) / per_block)), JOIN_THREADS, 0, stream,
                   (const float*)part_o, (const float*)part_ml, (bf16*)out, out_stride, nq, num_splits, tok_base, n_pairs);

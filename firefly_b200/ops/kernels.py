@@ -586,20 +586,25 @@ def attn_tiled(q, q_stride, pages, table, cu_q, ctx_lens, n_seqs, total_tiles, o
         c_float(softcap), _sink_arg(sink, nq), _p(status), _stream()), "attn_tiled")
 
 
+BOTH_PARTS, ATTENTION_PART, JOIN_PART = 3, 1, 2     # of an attention whose keys are shared out over blocks
+
+
 def attn_decode(q, q_stride, pages, table, cu_q, ctx_lens, n_seqs, out, part_o, part_ml, nq, nkv, d,
                 scale, window, num_splits, status: Optional[torch.Tensor] = None,
-                dist_bias: Optional[torch.Tensor] = None, softcap: float = 0.0, sink: Sink = None) -> None:
+                dist_bias: Optional[torch.Tensor] = None, softcap: float = 0.0, sink: Sink = None,
+                parts: int = BOTH_PARTS, beside: bool = False) -> None:
     """Split-KV tensor-core attention when every sequence has one token (bfloat16).  ``status``,
-    ``dist_bias`` and ``sink`` as for `attn_tiled`."""
+    ``dist_bias`` and ``sink`` as for `attn_tiled`; ``parts``, ``beside``: as `paged_attention` uses them."""
     _need_cuda(pages, table, cu_q, ctx_lens, out, part_o, part_ml, status, dist_bias)
     num_blocks, planes, _, block_size, _ = pages.shape
     _check(_attn_lib(d, planes).ff_attn_decode(
         _p(q), c_int(q_stride), _p(pages), _p(table), c_int(table.shape[1]), _p(cu_q), _p(ctx_lens),
         c_int(n_seqs), _p(out), c_int(out.shape[1]), _p(part_o), _p(part_ml), c_int(nq), c_int(nkv),
         c_int(block_size), c_int(num_blocks), c_float(scale), c_int(window), c_int(num_splits),
-        *_bias_args(dist_bias, nq, window), c_float(softcap), _sink_arg(sink, nq), _p(status), _stream()), "attn_decode")
+        *_bias_args(dist_bias, nq, window), c_float(softcap), _sink_arg(sink, nq), c_int(parts), c_int(1 if beside else 0),
+        _p(status), _stream()), "attn_decode")
     global LAUNCHES
-    if num_splits > 1:
+    if num_splits > 1 and parts == BOTH_PARTS:
         LAUNCHES += 1     # the kernel that joins the splits
 
 
@@ -672,14 +677,14 @@ def tc_attention_supported(dtype: torch.dtype, d: int, block_size: int, max_kv_l
 
 def attn_tc(q, q_stride, pages, table, cu_q, ctx_lens, n_seqs, total_tiles, out, nq, nkv, d, scale, window,
             status, page_list: Optional[int] = None, shares=None, dist_bias: Optional[torch.Tensor] = None,
-            softcap: float = 0.0, sink: Sink = None, two_tiles: bool = False) -> None:
+            softcap: float = 0.0, sink: Sink = None, two_tiles: bool = False, parts: int = BOTH_PARTS) -> None:
     """tcgen05 flash attention over the paged cache (bfloat16); total_tiles counts row tiles of 128.
     ``shares`` = (count, part_o, part_ml, first row, rows): every row tile's keys are shared out over
     ``count`` blocks and a second kernel joins their partial results (for prompts so short that their
     row tiles alone would leave most SMs idle); the scratch tensors are float32 with at least
     (first row + rows) * nq * count * d and ... * 2 elements.  ``dist_bias``, ``sink``: as for `paged_attention_simt`.
     ``two_tiles``: two row tiles a block (`attn_tc_two_tiles`), where the kernel for that takes the call: heads of 64 and 128, no
-    shares, neither bias nor cap."""
+    shares, neither bias nor cap.  ``parts``: the attention, the join of its shares or both."""
     _need_cuda(pages, table, cu_q, ctx_lens, out, status, dist_bias)
     num_blocks, planes, _, block_size, _ = pages.shape
     count, part_o, part_ml, row0, rows = shares if shares is not None else (1, None, None, 0, 0)
@@ -692,8 +697,8 @@ def attn_tc(q, q_stride, pages, table, cu_q, ctx_lens, n_seqs, total_tiles, out,
         c_int(n_seqs), c_int(total_tiles), _p(out), c_int(out.shape[1]), c_int(nq), c_int(nkv),
         c_int(block_size), c_int(num_blocks), c_float(scale), c_int(window), _p(status), c_int(count), _p(part_o),
         _p(part_ml), c_int(row0), c_int(rows), *_bias_args(dist_bias, nq, window), c_float(softcap),
-        _sink_arg(sink, nq), c_int(1 if two_tiles else 0), _stream()), "attn_tc")
-    if count > 1:
+        _sink_arg(sink, nq), c_int(1 if two_tiles else 0), c_int(parts), _stream()), "attn_tc")
+    if count > 1 and parts == BOTH_PARTS:
         global LAUNCHES
         LAUNCHES += 1     # the kernel that joins the shares
 
@@ -796,7 +801,7 @@ def _decode_scratch(ws, n: int, nq: int, nkv: int, d: int, splits: int):
 def attn_decode_units(q, q_stride, pages, table, cu_q, ctx_lens, n_seqs, out, part_o, part_ml, seq_ranges,
                       nq, nkv, d, scale, window, units, max_ranges, heads=None, status=None,
                       dist_bias: Optional[torch.Tensor] = None, softcap: float = 0.0, sink: Sink = None, q_temp=None,
-                      value_is_key: bool = False) -> None:
+                      value_is_key: bool = False, parts: int = BOTH_PARTS, beside: bool = False) -> None:
     """Split-KV decode attention with `units` blocks per kv head shared out among the sequences
     in proportion to their lengths.  ``heads = (q_norm_w, k_norm_w, eps, cos_sin)``: q is the raw
     q|k|v projection and the kernel finishes the heads itself (``q_temp``, ``value_is_key``: as for
@@ -812,11 +817,11 @@ def attn_decode_units(q, q_stride, pages, table, cu_q, ctx_lens, n_seqs, out, pa
         c_int(nkv), c_int(block_size), c_int(num_blocks), c_float(scale), c_int(window), c_int(units),
         c_int(max_ranges), c_int(1 if heads is not None else 0), _p(qw), _p(kw), c_float(eps), _p(cos_sin),
         c_int(cos_sin.shape[0] if cos_sin is not None else 0), *_bias_args(dist_bias, nq, window), c_float(softcap),
-        _sink_arg(sink, nq), *_temp_args(q_temp), c_int(1 if value_is_key else 0), _p(status), _stream()),
-        "attn_decode_units")
+        _sink_arg(sink, nq), *_temp_args(q_temp), c_int(1 if value_is_key else 0), c_int(parts), c_int(1 if beside else 0),
+        _p(status), _stream()), "attn_decode_units")
     global LAUNCHES, BY_LENGTH_CALLS
-    BY_LENGTH_CALLS += 1
-    if units > n_seqs and max_ranges > 1:
+    BY_LENGTH_CALLS += parts != JOIN_PART
+    if units > n_seqs and max_ranges > 1 and parts == BOTH_PARTS:
         LAUNCHES += 1     # the kernel that joins the ranges
 
 
@@ -836,19 +841,25 @@ def paged_attention(q: torch.Tensor, q_stride: int, pages: torch.Tensor, table: 
     G = nq // nkv
     n = ctx.num_seqs
     n_dec = ctx.num_decode_seqs if G <= 16 else 0      # these come first in the step's arrays
+    tc = n_dec < n and USE_TC_ATTENTION and tc_attention_supported(q.dtype, d, pages.shape[3], ctx.max_kv_len)
+
     if n_dec:
         # one-token sequences: split-KV kernel
         # a window or a chunk bounds the keys a query walks, however long its sequence is
         splits = decode_splits(n_dec, nkv, min(ctx.max_kv_len, abs(window)) if window else ctx.max_kv_len)
         units = decode_units(n_dec, nkv, d, ctx.ranges_by_length)
         part_o, part_ml, seq_ranges = _decode_scratch(ctx.workspace, n_dec, nq, nkv, d, splits)
+
+    def single_tokens(parts: int, beside: bool = False) -> None:
         if units:
             attn_decode_units(q, q_stride, pages, table, ctx.cu_q, ctx.ctx_lens, n_dec, out, part_o, part_ml,
                               seq_ranges, nq, nkv, d, scale, window, units, DECODE_MAX_RANGES, status=ctx.status,
-                              dist_bias=dist_bias, softcap=softcap, sink=sink)
-        else:
+                              dist_bias=dist_bias, softcap=softcap, sink=sink, parts=parts, beside=beside)
+        elif parts != JOIN_PART or splits > 1:
             attn_decode(q, q_stride, pages, table, ctx.cu_q, ctx.ctx_lens, n_dec, out, part_o, part_ml, nq, nkv,
-                        d, scale, window, splits, ctx.status, dist_bias, softcap, sink)
+                        d, scale, window, splits, ctx.status, dist_bias, softcap, sink, parts=parts, beside=beside)
+    if n_dec and not tc:
+        single_tokens(BOTH_PARTS)
     if n_dec < n:
         # portions of prompts: tiled kernel over the remaining sequences (token offsets in cu_q are absolute)
         # every layer of a step asks the same of the step's arrays: worked out once and kept with the step
@@ -859,7 +870,7 @@ def paged_attention(q: torch.Tensor, q_stride: int, pages: torch.Tensor, table: 
             if memo is not None:
                 memo[("attn_tail", id(table), n_dec)] = tail
         table_t, cu_q_t, ctx_lens_t = tail
-        if USE_TC_ATTENTION and tc_attention_supported(q.dtype, d, pages.shape[3], ctx.max_kv_len):
+        if tc:
             plan = memo.get(("attn_tc_plan", G, nkv, n_dec, ctx.captured, window)) if memo is not None else None
             if plan is None:
                 tiles = sum(-(-(ql * G) // 128) for ql in ctx.q_lens[n_dec:])
@@ -882,9 +893,20 @@ def paged_attention(q: torch.Tensor, q_stride: int, pages: torch.Tensor, table: 
                 cells = (row0 + rows) * nq * count
                 shares = (count, ctx.workspace.get("attn.tc_part_o", (cells * d,), torch.float32),
                           ctx.workspace.get("attn.tc_part_ml", (cells * 2,), torch.float32), row0, rows)
-            attn_tc(q, q_stride, pages, table_t, cu_q_t, ctx_lens_t, n - n_dec, tiles,
-                    out, nq, nkv, d, scale, window, ctx.status, shares=shares, dist_bias=dist_bias, softcap=softcap, sink=sink,
-                    two_tiles=two_tiles)
+            def portions(parts: int) -> None:
+                attn_tc(q, q_stride, pages, table_t, cu_q_t, ctx_lens_t, n - n_dec, tiles, out, nq, nkv, d, scale, window, ctx.status,
+                        shares=shares, dist_bias=dist_bias, softcap=softcap, sink=sink, two_tiles=two_tiles, parts=parts)
+            if not n_dec:
+                portions(BOTH_PARTS)
+            else:
+                # The two attentions need nothing of one another: the single tokens' blocks run in the places that the portions' leave
+                # and need not wait for their end (one after the other they took 69 us a layer for 2 x 256 + 24 tokens, now 63, and 66 for 2048 + 1, now 60),
+                # and the kernels that join partial results come behind both.
+                portions(ATTENTION_PART)
+                single_tokens(ATTENTION_PART, beside=True)
+                if count > 1:
+                    portions(JOIN_PART)
+                single_tokens(JOIN_PART)
         else:
             tiles = sum(-(-(ql * G) // 64) for ql in ctx.q_lens[n_dec:])
             attn_tiled(q, q_stride, pages, table_t, cu_q_t, ctx_lens_t, n - n_dec,
