@@ -739,13 +739,15 @@ def attn_tc_two_tiles(q_lens: Sequence[int], ctx_lens: Sequence[int], G: int, nk
 
 def decode_splits(n_seqs: int, nkv: int, max_kv_len: int) -> int:
     """Ranges of keys per (sequence, kv head).  Three blocks of the decode kernel fit an SM: few
-    sequences get as many ranges as fill those places once (at most 20), many sequences three.
+    sequences get as many ranges as fill those places once (2 to 20), many sequences three.
     Measured on the 8B shape at context 2100 (ms per step, ranges): batch 1 3.29 (24), 4 3.51 (13),
     8 3.70 (6) against 3.83 (8), 16 4.18 (3) against 4.39 (8), 32 5.43 (3) against 5.70 (8),
-    64 8.08 (3) against 8.34 (8)."""
+    64 8.08 (3) against 8.34 (8).  Two ranges where they fit the places once and three do not: 24 sequences of 2000 tokens, the kernel and
+    its join, 70 us against 81."""
     tiles = max(1, -(-max_kv_len // 64))
     places = 3 * sm_count()
-    want = max(3, min(places // max(1, n_seqs * nkv), 20))
+    once = places // max(1, n_seqs * nkv)
+    want = min(once, 20) if once >= 2 else 3
     return max(1, min(want, tiles, 64))
 
 
