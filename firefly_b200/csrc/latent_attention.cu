@@ -108,7 +108,8 @@ __global__ void latent_finish_kernel(
 
 // The same in bfloat16 with one plane, kv_rank and rot_dim in steps of 8, the whole of rot_dim rotated in at most 32 pairs and
 // everything on 16 bytes: a warp a token, pair i of every head on lane i, rows of q_abs 16 bytes a lane, no barrier.  A block a
-// token spends its time waiting: 77 -> 32 us on 13800 tokens of 8 heads of 192 + 64, whose bytes take 19.
+// token spends its time waiting: 77 -> 27 us on 13800 tokens of 8 heads of 192 + 64, whose bytes take 19.
+constexpr int LF_HEADS = 8, LF_PIECES = 6;
 __global__ void __launch_bounds__(256) latent_finish_warp_kernel(
     const bf16* q_src, int q_stride, const bf16* dkv_src, int dkv_stride, const bf16* q_abs, const float* __restrict__ c_norm_w, float eps,
     const double* __restrict__ freq, const int* __restrict__ positions, const int* __restrict__ token_seq, const int* __restrict__ block_table,
@@ -123,13 +124,40 @@ __global__ void __launch_bounds__(256) latent_finish_warp_kernel(
     const int half = rot / 2, d = kv_rank + rot, pos = positions[t];
     const int e0 = interleaved ? 2 * lane : lane, e1 = interleaved ? e0 + 1 : lane + half;
     const bool turns = lane < half;
-    // the query rows: [q_abs | rotated part] per head
     bf16* qf = q_full + (size_t)t * H * d;
     const int pieces = kv_rank / 8;
-#pragma unroll 8
-    for (int idx = lane; idx < H * pieces; idx += 32) {
-        const int h = idx / pieces, i = (idx - h * pieces) * 8;
-        *reinterpret_cast<uint4*>(qf + (size_t)h * d + i) = *reinterpret_cast<const uint4*>(q_abs + ((size_t)h * Ttot + t) * kv_rank + i);
+    // What the first rows need is asked for at once, in front of the first store and of the sines (which take as long as a trip to memory):
+    // one trip after the other took 32 us where this takes 27.
+    struct alignas(16) Eight { bf16 v[8]; };
+    const bf16* dkv = dkv_src ? dkv_src + (size_t)t * dkv_stride : nullptr;
+    Eight c[2];                                           // the cache row: kv_rank of up to 512
+    bf16 ka = from_float<bf16>(0.f), kb = ka;
+    int page = -1;
+    if (dkv) {
+        page = block_table[(size_t)token_seq[t] * max_blocks + pos / block_size];
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+            if ((m * 32 + lane) * 8 < kv_rank) c[m] = *reinterpret_cast<const Eight*>(dkv + (m * 32 + lane) * 8);
+        if (turns) { ka = dkv[kv_rank + e0]; kb = dkv[kv_rank + e1]; }
+    }
+    const bf16* q = q_src + (size_t)t * q_stride + dim;
+    bf16 qa[LF_HEADS], qb[LF_HEADS];
+#pragma unroll
+    for (int h = 0; h < LF_HEADS; ++h)
+        if (turns && h < H) { qa[h] = q[(size_t)h * (dim + rot) + e0]; qb[h] = q[(size_t)h * (dim + rot) + e1]; }
+    // the query rows: [q_abs | rotated part] per head
+    for (int i0 = lane; i0 < H * pieces; i0 += 32 * LF_PIECES) {
+        uint4 raw[LF_PIECES];
+#pragma unroll
+        for (int k = 0; k < LF_PIECES; ++k) {
+            const int idx = i0 + 32 * k, h = idx / pieces, i = (idx - h * pieces) * 8;
+            if (idx < H * pieces) raw[k] = *reinterpret_cast<const uint4*>(q_abs + ((size_t)h * Ttot + t) * kv_rank + i);
+        }
+#pragma unroll
+        for (int k = 0; k < LF_PIECES; ++k) {
+            const int idx = i0 + 32 * k, h = idx / pieces, i = (idx - h * pieces) * 8;
+            if (idx < H * pieces) *reinterpret_cast<uint4*>(qf + (size_t)h * d + i) = raw[k];
+        }
     }
     float cs = 1.f, sn = 0.f;
     if (turns) {
@@ -137,34 +165,33 @@ __global__ void __launch_bounds__(256) latent_finish_warp_kernel(
         sincos((double)pos * freq[lane], &s64, &c64);
         cs = (float)c64;
         sn = (float)s64;
-    }
-    const bf16* q = q_src + (size_t)t * q_stride + dim;
-#pragma unroll 4
-    for (int h = 0; h < H; ++h) {
-        if (turns) {
-            const bf16* qr = q + (size_t)h * (dim + rot);
-            const float a = to_float(qr[e0]), b = to_float(qr[e1]);
-            bf16* to = qf + (size_t)h * d + kv_rank;
-            to[e0] = from_float<bf16>(a * cs - b * sn);
-            to[e1] = from_float<bf16>(b * cs + a * sn);
+        for (int h0 = 0; h0 < H; h0 += LF_HEADS) {
+            if (h0 > 0) {
+#pragma unroll
+                for (int h = 0; h < LF_HEADS; ++h)
+                    if (h0 + h < H) { qa[h] = q[(size_t)(h0 + h) * (dim + rot) + e0]; qb[h] = q[(size_t)(h0 + h) * (dim + rot) + e1]; }
+            }
+#pragma unroll
+            for (int h = 0; h < LF_HEADS; ++h)
+                if (h0 + h < H) {
+                    const float a = to_float(qa[h]), b = to_float(qb[h]);
+                    bf16* to = qf + (size_t)(h0 + h) * d + kv_rank;
+                    to[e0] = from_float<bf16>(a * cs - b * sn);
+                    to[e1] = from_float<bf16>(b * cs + a * sn);
+                }
         }
     }
-    if (!dkv_src) return;
+    if (!dkv) return;
     // the cache row
-    const bf16* dkv = dkv_src + (size_t)t * dkv_stride;
-    const int page = block_table[(size_t)token_seq[t] * max_blocks + pos / block_size];
     if (page < 0 || page >= num_blocks) {
         if (lane == 0) atomicExch(status, 2);
         return;
     }
-    struct alignas(16) Eight { bf16 v[8]; };
-    Eight c[2];                                           // kv_rank of up to 512
     float ss = 0.f;
 #pragma unroll
     for (int m = 0; m < 2; ++m) {
         const int i = (m * 32 + lane) * 8;
         if (i < kv_rank) {
-            c[m] = *reinterpret_cast<const Eight*>(dkv + i);
 #pragma unroll
             for (int e = 0; e < 8; ++e) { const float v = to_float(c[m].v[e]); ss += v * v; }
         }
@@ -182,7 +209,7 @@ __global__ void __launch_bounds__(256) latent_finish_warp_kernel(
         }
     }
     if (turns) {
-        const float a = to_float(dkv[kv_rank + e0]), b = to_float(dkv[kv_rank + e1]);
+        const float a = to_float(ka), b = to_float(kb);
         krow[kv_rank + e0] = from_float<bf16>(a * cs - b * sn);
         krow[kv_rank + e1] = from_float<bf16>(b * cs + a * sn);
     }
