@@ -799,7 +799,7 @@ __global__ void __launch_bounds__(32 * CF_WARPS) channel_decay_prepare_kernel(Sc
 // A thread keeps one channel's row of w in registers (up to LRD_R of it at a time) and walks a tile of tokens, LRD_U of
 // them at once, whose low rows stand in shared memory, two tokens side by side for the instructions that take two sums.
 // Bound by instructions: 96 a token and channel with one sum an instruction and softplus of expf and logf, now some 35, and
-// by weights that were asked for two bytes at a time.  3140 tokens of 1024 channels 19.6 us, now 12.5; 1000 tokens 8.6, now 4.8.
+// by weights that were asked for two bytes at a time.  4140 tokens of 1024 channels 19.6 us, now 12.5; 1000 tokens 8.6, now 4.8.
 constexpr int LRD_TOK = 32, LRD_U = 4, LRD_THREADS = 128, LRD_R = 16;
 
 // SHORT: softplus with the fast exponential and logarithm, together within 4.2e-7 of it absolutely, which is a relative
