@@ -898,8 +898,10 @@ def paged_attention(q: torch.Tensor, q_stride: int, pages: torch.Tensor, table: 
             def portions(parts: int) -> None:
                 attn_tc(q, q_stride, pages, table_t, cu_q_t, ctx_lens_t, n - n_dec, tiles, out, nq, nkv, d, scale, window, ctx.status,
                         shares=shares, dist_bias=dist_bias, softcap=softcap, sink=sink, two_tiles=two_tiles, parts=parts)
-            if not n_dec:
+            if not n_dec or not tiles:
                 portions(BOTH_PARTS)
+                if n_dec:                        # portions without a token launch nothing that the single tokens could run beside
+                    single_tokens(BOTH_PARTS)
             else:
                 # The two attentions need nothing of one another: the single tokens' blocks run in the places that the portions' leave
                 # and need not wait for their end (one after the other they took 69 us a layer for 2 x 256 + 24 tokens, now 63, and 66 for 2048 + 1, now 60),

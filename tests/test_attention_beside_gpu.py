@@ -10,7 +10,8 @@ pytestmark = pytest.mark.gpu
 
 # portions: many row tiles (two a block), few (keys shared out over blocks), shorter than a tile; single tokens in fixed ranges and by length
 @pytest.mark.parametrize("q_lens,before", [([1] * 24 + [256, 256], [60 * i for i in range(24)] + [1536, 1500]), ([1, 2048], [0, 0]),
-                                           ([1, 1, 3], [2000, 5, 700]), ([1] * 64 + [1500, 2], [31 * i for i in range(64)] + [0, 64])])
+                                           ([1, 1, 3], [2000, 5, 700]), ([1] * 64 + [1500, 2], [31 * i for i in range(64)] + [0, 64]),
+                                           ([1, 1, 0], [100, 30, 5])])            # a portion without a token: nothing to run beside
 @pytest.mark.parametrize("d,by_length", [(128, False), (128, True), (64, False)])
 def test_single_tokens_beside_portions(q_lens, before, d, by_length):
     from firefly_b200.engine.context import Workspace
