@@ -166,21 +166,6 @@ __device__ __forceinline__ float query_temperature(int pos, float coef, int ever
     return 1.0f + coef * logf((float)((pos + 1) / every) + 1.0f);
 }
 
-// Sigmoid and SiLU for a result of type T.  32-bit results take the exact division; what is rounded to 16 bits takes the exponential and
-// the reciprocal instruction, five in all instead of some thirty (relative error up to 2^-21 for |z| <= 8, and |z| 2^-24 beyond; 0 where
-// e^-z overflows, the true sigmoid being below 2^-127): the element-wise kernels are bound by their instructions otherwise.
-template <typename T> __device__ __forceinline__ float sigmoid_for(float z) {
-    if constexpr (sizeof(T) == 4) return 1.0f / (1.0f + expf(-z));
-    float e, r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(z * -1.4426950408889634f));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(e + 1.0f));
-    return r;
-}
-template <typename T> __device__ __forceinline__ float silu_for(float z) {
-    if constexpr (sizeof(T) == 4) return z / (1.0f + expf(-z));
-    return z * sigmoid_for<T>(z);
-}
-
 __device__ __forceinline__ float to_float(float x) { return x; }
 __device__ __forceinline__ float to_float(bf16 x) { return __bfloat162float(x); }
 

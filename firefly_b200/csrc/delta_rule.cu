@@ -380,7 +380,7 @@ __global__ void head_norm_gate_kernel(const float* o, const TG* gate, int gate_s
     ss = warp_sum(ss);
     const float inv = 1.0f / sqrtf(ss / (float)V + eps);
     for (int i = lane; i < V; i += 32) {
-        const float g = to_float(grow[i]), sg = sigmoid_for<T>(g);
+        const float g = to_float(grow[i]), sg = 1.0f / (1.0f + expf(-g));
         y[(size_t)row * V + i] = from_float<T>(orow[i] * inv * w[i] * (gate_act ? g * sg : sg));
     }
 }
@@ -416,7 +416,7 @@ __global__ void __launch_bounds__(256) head_norm_gate_vec_kernel(const float* o,
     Four out;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-        const float g = to_float(gv.v[e]), sg = sigmoid_for<T>(g);
+        const float g = to_float(gv.v[e]), sg = 1.0f / (1.0f + expf(-g));
         out.v[e] = from_float<T>(v[e] * inv * wv[e] * (gate_act ? g * sg : sg));
     }
     *reinterpret_cast<Four*>(y + (size_t)row * V + i) = out;

@@ -242,7 +242,7 @@ __global__ void silu_mul_vec8_kernel(const bf16* __restrict__ gu, bf16* __restri
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
         const float x = __bfloat162float(g[j]);
-        o[j] = __float2bfloat16_rn(silu_for<bf16>(x) * __bfloat162float(u[j]));
+        o[j] = __float2bfloat16_rn(x / (1.0f + expf(-x)) * __bfloat162float(u[j]));
     }
     *reinterpret_cast<uint4*>(out + (size_t)t * I + i) = ov;
 }

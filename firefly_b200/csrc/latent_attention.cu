@@ -229,7 +229,7 @@ __global__ void latent_gate_kernel(const T* val /*[H,T,vdim]*/, const T* g, int 
     const int c = (int)(idx - t * hv);
     const int h = c / vdim, j = c - h * vdim;
     const float gv = to_float(g[t * g_stride + (per_head ? h : c)]);
-    y[idx] = from_float<T>(to_float(val[((size_t)h * Ttot + t) * vdim + j]) * sigmoid_for<T>(gv));
+    y[idx] = from_float<T>(to_float(val[((size_t)h * Ttot + t) * vdim + j]) / (1.0f + expf(-gv)));
 }
 
 // The same in bfloat16, eight values a thread (vdim in steps of 8, everything on 16 bytes); bound by the loads and stores of
@@ -245,13 +245,13 @@ __global__ void __launch_bounds__(256) latent_gate_vec_kernel(const bf16* val /*
     struct alignas(16) Eight { bf16 v[8]; };
     Eight x = *reinterpret_cast<const Eight*>(val + ((size_t)h * Ttot + t) * vdim + j);
     if (per_head) {
-        const float sg = sigmoid_for<bf16>(to_float(g[(size_t)t * g_stride + h]));
+        const float div = 1.0f + expf(-to_float(g[(size_t)t * g_stride + h]));
 #pragma unroll
-        for (int e = 0; e < 8; ++e) x.v[e] = from_float<bf16>(to_float(x.v[e]) * sg);
+        for (int e = 0; e < 8; ++e) x.v[e] = from_float<bf16>(to_float(x.v[e]) / div);
     } else {
         const Eight gv = *reinterpret_cast<const Eight*>(g + (size_t)t * g_stride + c);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) x.v[e] = from_float<bf16>(to_float(x.v[e]) * sigmoid_for<bf16>(to_float(gv.v[e])));
+        for (int e = 0; e < 8; ++e) x.v[e] = from_float<bf16>(to_float(x.v[e]) / (1.0f + expf(-to_float(gv.v[e]))));
     }
     *reinterpret_cast<Eight*>(y + idx * 8) = x;
 }

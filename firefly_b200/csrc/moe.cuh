@@ -16,12 +16,12 @@ __device__ __forceinline__ float clamped_glu(float g, float u, float limit, int 
     return g / (1.0f + expf(-1.702f * g)) * (u + 1.0f);
 }
 
-// The same for results that are rounded to bfloat16.
+// The same on the fast exponential and division, for results that are rounded to bfloat16.
 __device__ __forceinline__ float clamped_glu_fast(float g, float u, float limit, int act) {
-    if (act == 1) return silu_for<bf16>(g) * u;
+    if (act == 1) return __fdividef(g, 1.0f + __expf(-g)) * u;
     g = fminf(g, limit);
     u = fminf(fmaxf(u, -limit), limit);
-    return g * sigmoid_for<bf16>(1.702f * g) * (u + 1.0f);
+    return __fdividef(g, 1.0f + __expf(-1.702f * g)) * (u + 1.0f);
 }
 
 constexpr int GROUPED_TC_ROWS = 128;      // rows of a row tile of the tensor-core product

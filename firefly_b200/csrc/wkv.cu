@@ -302,7 +302,7 @@ __global__ void wkv_out_kernel(const float* __restrict__ o, const T* __restrict_
     const float inv = 1.0f / sqrtf(ss / (float)dim + eps);
     for (int i = lane; i < dim; i += 32) {
         const float gv = to_float(g[base + i]);
-        y[base + i] = from_float<T>(o[base + i] * inv * norm[h * dim + i] * silu_for<T>(gv));
+        y[base + i] = from_float<T>(o[base + i] * inv * norm[h * dim + i] * (gv / (1.0f + expf(-gv))));
     }
 }
 
@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(256) wkv_out_vec_kernel(const float* o, const 
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
         const float z = to_float(gv.v[e]);
-        out.v[e] = from_float<T>(v[e] * inv * wv[e] * silu_for<T>(z));
+        out.v[e] = from_float<T>(v[e] * inv * wv[e] * (z / (1.0f + expf(-z))));
     }
     *reinterpret_cast<Four*>(y + (size_t)row * D + i) = out;
 }

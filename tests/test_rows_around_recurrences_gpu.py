@@ -138,6 +138,40 @@ def test_gate_of_latent_attention(T, heads, vdim, shift, per_head):
     _close(y, val.double().transpose(0, 1).reshape(T, -1) * gate)
 
 
+@pytest.mark.parametrize("kernel", ["gated_norm", "gated_norm_behind", "head_norm_sigmoid", "head_norm_silu", "wkv_out", "latent_gate", "swiglu"])
+@pytest.mark.parametrize("W", [128, 100])
+def test_gates_far_below_zero(kernel, W):
+    """Gates down to where e^-z leaves 32 bits (z of -88.7): exponential and division are the 32-bit ones, so the result, a normal number, has
+    all its bits; a reciprocal that flushes small numbers gives 0 from -87.3 on."""
+    z = torch.linspace(-88.5, -80.0, 9 * W, device="cuda").to(BF).view(9, W)
+    sig, x = torch.sigmoid(z.double()), 1e6 * (1.5 + torch.rand(9, W, device="cuda"))
+    w, y, xd = torch.ones(W, device="cuda"), torch.empty(9, W, dtype=BF, device="cuda"), x.double()
+    unit = xd / (xd.square().mean(-1, keepdim=True)).sqrt()
+    if kernel == "gated_norm":                       # x silu(z) in front of the norm: the largest of a row has to count in its own size
+        eps = 1e-30
+        K.gated_rms_norm(x, (z, 0), w, eps, y, 1, True)
+        v = xd * z.double() * sig
+        want = v / (v.square().mean(-1, keepdim=True) + eps).sqrt()
+    elif kernel == "gated_norm_behind":
+        K.gated_rms_norm(x, (z, 0), 1e6 * w, 0.0, y, 1, False)
+        want = 1e6 * unit * sig
+    elif kernel.startswith("head_norm"):
+        K.head_norm_gate(x, (z, 0), 1e6 * w, 0.0, y, 1, W, kernel[10:])
+        want = 1e6 * unit * sig * (z.double() if kernel.endswith("silu") else 1)
+    elif kernel == "wkv_out":
+        K.wkv_out(x, z, 1e6 * w, 0.0, y, 1, W)
+        want = 1e6 * unit * sig * z.double()
+    elif kernel == "latent_gate":
+        val = x.to(BF).view(1, 9, W)
+        K.latent_gate(val, z, y, 1, W)
+        want = val[0].double() * sig
+    else:
+        u = x.to(BF)
+        K.silu_mul(torch.cat([z, u], 1), y)
+        want = z.double() * sig * u.double()
+    assert bool(((y.double() - want).abs() <= 2.0 ** -8 * want.abs()).all()) and bool((y != 0).all())
+
+
 @pytest.mark.parametrize("H,dim,rot,rank,planes,shift", [(3, 16, 64, 200, 1, 0), (8, 128, 64, 512, 1, 8), (2, 24, 8, 8, 1, 0), (5, 16, 48, 264, 1, 0),
                                                          (3, 16, 64, 200, 2, 0), (2, 16, 72, 64, 1, 0), (2, 16, 64, 520, 1, 0), (3, 16, 64, 200, 1, 1)])
 @pytest.mark.parametrize("interleaved", [False, True])
