@@ -805,9 +805,7 @@ __global__ void __launch_bounds__(32 * CF_WARPS) channel_decay_prepare_kernel(Sc
 // by weights that were asked for two bytes at a time.  4140 tokens of 1024 channels 19.6 us, now 12.5; 1000 tokens 8.6, now 4.8.
 constexpr int LRD_TOK = 32, LRD_U = 4, LRD_THREADS = 128, LRD_R = 16;
 
-// SHORT: softplus with the fast exponential and logarithm, together within 4.2e-7 of it absolutely, which is a relative
-// 4.2e-7 / tau of alpha: from tau = 16 on below half a unit in its last place.
-template <typename T, bool SHORT>
+template <typename T>
 __global__ void __launch_bounds__(LRD_THREADS) low_rank_decay_kernel(const T* low, int low_stride, int low_off,
                                                                      const T* __restrict__ w, const float* __restrict__ bias,
                                                                      float inv_tau, float* __restrict__ alpha, int Ttot, int C,
@@ -867,8 +865,9 @@ __global__ void __launch_bounds__(LRD_THREADS) low_rank_decay_kernel(const T* lo
         for (int u = 0; u < LRD_U; ++u)
             if (u0 + u < n) {
                 const float z = (u & 1 ? f2_high(acc[u / 2]) : f2_low(acc[u / 2])) + b;
-                // softplus(-z) = -ln sigmoid(z)
-                const float sp = fmaxf(-z, 0.f) + (SHORT ? __logf(1.0f + __expf(-fabsf(z))) : logf(1.0f + expf(-fabsf(z))));
+                // softplus(-z) = -ln sigmoid(z), right to about 1e-7 absolutely, which is a relative 1e-7 / tau of alpha: the decays of
+                // thousands of tokens are multiplied, so not with the fast exponential and logarithm (4e-7)
+                const float sp = fmaxf(-z, 0.f) + logf(1.0f + expf(-fabsf(z)));
                 to[(size_t)u * C] = expf(-sp * inv_tau);
             }
     }
@@ -1219,16 +1218,14 @@ FF_EXPORT int ff_low_rank_decay(const void* low, int dtype, int low_stride, int 
     const size_t smem = (size_t)Rp * tile * sizeof(float);
     if (smem > 48 * 1024) return FF_ERR_UNSUPPORTED;
     dim3 grid((T + tile - 1) / tile, cols);
-    const bool close = tau >= 16.f;
-#define FF_LOW_RANK(TT, SHORT)                                                                                                       \
-    FF_LAUNCH((low_rank_decay_kernel<TT, SHORT>), grid, LRD_THREADS, smem, stream, (const TT*)low, low_stride, low_off, (const TT*)w, \
-              bias, 1.0f / tau, alpha, T, C, R, tile, ((uintptr_t)w & 15) == 0 && R % (16 / (int)sizeof(TT)) == 0 ? 1 : 0)
-    if (dtype == 0 && close) FF_LOW_RANK(float, true);
-    else if (dtype == 0) FF_LOW_RANK(float, false);
-    else if (dtype == 1 && close) FF_LOW_RANK(bf16, true);
-    else if (dtype == 1) FF_LOW_RANK(bf16, false);
+    auto w_pieces = [&](int n) { return ((uintptr_t)w & 15) == 0 && R % n == 0 ? 1 : 0; };
+    if (dtype == 0)
+        FF_LAUNCH((low_rank_decay_kernel<float>), grid, LRD_THREADS, smem, stream, (const float*)low, low_stride, low_off,
+                  (const float*)w, bias, 1.0f / tau, alpha, T, C, R, tile, w_pieces(4));
+    else if (dtype == 1)
+        FF_LAUNCH((low_rank_decay_kernel<bf16>), grid, LRD_THREADS, smem, stream, (const bf16*)low, low_stride, low_off,
+                  (const bf16*)w, bias, 1.0f / tau, alpha, T, C, R, tile, w_pieces(8));
     else return FF_ERR_BAD_ARG;
-#undef FF_LOW_RANK
     FF_LAUNCH_CHECK();
     return 0;
 }
