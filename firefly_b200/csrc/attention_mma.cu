@@ -1069,19 +1069,19 @@ FF_EXPORT int ff_attn_decode(const void* q, int q_stride, const void* cache, con
                              int max_blocks, const int* cu_q, const int* ctx_lens, int n_seqs, void* out,
                              int out_stride, float* part_o, float* part_ml, int nq, int nkv,
                              int block_size, int num_blocks, float scale, int window, int num_splits,
-                             const float* dist_bias, int bias_len, float softcap, const float* sink, int parts, int beside,
+                             const float* dist_bias, int bias_len, float softcap, const float* sink, int beside,
                              int* status, cudaStream_t stream) {
     if (n_seqs <= 0) return 0;
     if (nkv <= 0 || nq % nkv || num_splits < 1 || (dist_bias && (window <= 0 || bias_len < window))) return FF_ERR_BAD_ARG;
     if (nq / nkv > 16) return FF_ERR_UNSUPPORTED;
     FF_SMEM_LIMIT(attn_decode_kernel, DECODE_SMEM);
     dim3 grid(n_seqs, nkv, num_splits);
-    if (parts & 1) FF_LAUNCH((attn_decode_kernel), grid, NTHREADS, DECODE_SMEM, stream, 
+    FF_LAUNCH((attn_decode_kernel), grid, NTHREADS, DECODE_SMEM, stream, 
         (const bf16*)q, q_stride, (const bf16*)cache, block_table, max_blocks, cu_q, ctx_lens, (bf16*)out,
         out_stride, part_o, part_ml, nq, nkv, block_size, num_blocks, scale * LOG2E, window, num_splits, dist_bias,
         bias_len, softcap * LOG2E, sink, beside, longest_first(n_seqs, nkv, num_splits), status);
     FF_LAUNCH_CHECK();
-    if (num_splits > 1 && (parts & 2)) {
+    if (num_splits > 1) {
         dim3 cgrid(n_seqs, nq);
         if (num_splits > 8)
             FF_LAUNCH((attn_combine_many_kernel), cgrid, COMBINE_THREADS, 0, stream, part_o, part_ml, cu_q, (bf16*)out,
@@ -1150,7 +1150,7 @@ FF_EXPORT int ff_attn_decode_units(const void* q, int q_stride, void* cache, con
                                    int max_ranges, int finish_heads, const float* q_norm_w,
                                    const float* k_norm_w, float eps, const float* cos_sin, int max_positions,
                                    const float* dist_bias, int bias_len, float softcap, const float* sink, float temp_coef,
-                                   int temp_every, int value_is_key, int parts, int beside, int* status, cudaStream_t stream) {
+                                   int temp_every, int value_is_key, int beside, int* status, cudaStream_t stream) {
     if (finish_heads && beside) return FF_ERR_BAD_ARG;
     if (finish_heads && temp_every > 0 && !q_norm_w) return FF_ERR_BAD_ARG;
     if (FF_KV_PLANES != 2 && finish_heads) return FF_ERR_UNSUPPORTED;
@@ -1170,8 +1170,7 @@ FF_EXPORT int ff_attn_decode_units(const void* q, int q_stride, void* cache, con
                    softcap * LOG2E, sink, temp_coef, temp_every, value_is_key, beside, 0};
     DecodeUnits un{n_seqs, max_ranges, seq_ranges, units};
     dim3 grid(nkv, units);
-    if (!(parts & 1)) {}
-    else if (finish_heads && (sink || temp_every > 0 || value_is_key))
+    if (finish_heads && (sink || temp_every > 0 || value_is_key))
         FF_LAUNCH((attn_decode_units_kernel<true, true>), grid, NTHREADS, DECODE_SMEM, stream,
             (const bf16*)q, q_stride, (const bf16*)cache, block_table, max_blocks, cu_q, ctx_lens, (bf16*)out,
             out_stride, part_o, part_ml, nq, nkv, block_size, num_blocks, scale * LOG2E, window, hd, un);
@@ -1184,7 +1183,7 @@ FF_EXPORT int ff_attn_decode_units(const void* q, int q_stride, void* cache, con
             (const bf16*)q, q_stride, (const bf16*)cache, block_table, max_blocks, cu_q, ctx_lens, (bf16*)out,
             out_stride, part_o, part_ml, nq, nkv, block_size, num_blocks, scale * LOG2E, window, hd, un);
     FF_LAUNCH_CHECK();
-    if (units > n_seqs && max_ranges > 1 && (parts & 2)) {
+    if (units > n_seqs && max_ranges > 1) {
         dim3 cgrid(n_seqs, nq);
         // a sequence gets at most this many ranges: many of them take the form that spreads them over warps
         const int most = max_ranges < units - n_seqs + 1 ? max_ranges : units - n_seqs + 1;

@@ -1145,20 +1145,31 @@ using namespace ff;
 
 FF_EXPORT int ff_attn_tc_block_m() { return BM; }
 
+// The kernel that joins the shares of n_tokens rows from tok_base on (see below).
+FF_EXPORT int ff_attn_tc_join(const float* part_o, const float* part_ml, void* out, int out_stride, int nq, int num_splits, int tok_base,
+                              int n_tokens, cudaStream_t stream) {
+    if (!part_o || !part_ml || nq <= 0 || num_splits < 2 || n_tokens <= 0 || tok_base < 0) return FF_ERR_BAD_ARG;
+    const int n_pairs = n_tokens * nq, per_block = JOIN_THREADS / (D / 4);
+    FF_LAUNCH((attn_tc_join_kernel), dim3((unsigned)((n_pairs + per_block - 1) / per_block)), JOIN_THREADS, 0, stream,
+              part_o, part_ml, (bf16*)out, out_stride, nq, num_splits, tok_base, n_pairs);
+    FF_LAUNCH_CHECK();
+    return 0;
+}
+
 // total_tiles = sum over sequences of ceil(q_len * G / 128).  Needs a block size that divides 64
 // (8, 16, 32 or 64), a 128-byte aligned cache and q rows aligned to 16 bytes.
 // num_splits > 1: every row tile's keys are shared out over that many blocks, which leave partial
 // results in part_o (float [tokens * nq * num_splits * D]) and part_ml (float [tokens * nq * num_splits * 2]),
 // indexed by the token's row in q/out; a second kernel joins them for the n_tokens rows from tok_base on
 // (the rows of the sequences given here).
-// parts: 1 the attention itself, 2 the kernel that joins the shares, 3 both (a caller may put another kernel between them).
+// join 0: without that kernel; the caller asks for it by ff_attn_tc_join, behind another kernel that runs beside this one.
 // two_tiles: two row tiles a block where that kernel takes the call (heads of 64 and 128, one share, neither bias nor cap), as the caller
 // finds it faster.
 FF_EXPORT int ff_attn_tc(const void* q, int q_stride, const void* cache, const int* block_table, int max_blocks,
                          const int* cu_q, const int* ctx_lens, int n_seqs, int total_tiles, void* out,
                          int out_stride, int nq, int nkv, int block_size, int num_blocks, float scale, int window,
                          int* status, int num_splits, float* part_o, float* part_ml, int tok_base, int n_tokens,
-                         const float* dist_bias, int bias_len, float softcap, const float* sink, int two_tiles, int parts, cudaStream_t stream) {
+                         const float* dist_bias, int bias_len, float softcap, const float* sink, int two_tiles, int join, cudaStream_t stream) {
     if (n_seqs <= 0 || total_tiles <= 0) return 0;
     if (nkv <= 0 || nq % nkv || (dist_bias && (window <= 0 || bias_len < window))) return FF_ERR_BAD_ARG;
     if (num_splits < 1 || (num_splits > 1 && (!part_o || !part_ml || n_tokens <= 0 || tok_base < 0))) return FF_ERR_BAD_ARG;
@@ -1177,7 +1188,6 @@ FF_EXPORT int ff_attn_tc(const void* q, int q_stride, const void* cache, const i
 #if FF_ATC_PAIR
     const long long pairs = (((long long)total_tiles + n_seqs) / 2) * nkv;    // at least ceil(row tiles of a sequence / 2), summed
     if (two_tiles && num_splits == 1 && !dist_bias && softcap == 0.f && pairs < (1ll << 31)) {
-        if (!(parts & 1)) return 0;
         FF_SMEM_LIMIT(attn_tc_pair_kernel, PAIR_SMEM);
         FF_LAUNCH((attn_tc_pair_kernel), dim3((unsigned)pairs), PAIR_THREADS, PAIR_SMEM, stream, arg, (const bf16*)q, q_stride,
                   block_table, max_blocks, cu_q, ctx_lens, n_seqs, (bf16*)out, out_stride, nq, nkv, block_size, num_blocks,
@@ -1186,14 +1196,8 @@ FF_EXPORT int ff_attn_tc(const void* q, int q_stride, const void* cache, const i
     }
 #endif
     if ((long long)total_tiles * nkv * num_splits >= (1ll << 31)) return FF_ERR_UNSUPPORTED;
-    if (parts & 1) FF_LAUNCH((attn_tc_kernel), dim3((unsigned)(total_tiles * nkv * num_splits)), ATC_THREADS, ATC_SMEM, stream, arg,
+    FF_LAUNCH((attn_tc_kernel), dim3((unsigned)(total_tiles * nkv * num_splits)), ATC_THREADS, ATC_SMEM, stream, arg,
               (const bf16*)q, q_stride, block_table, max_blocks, cu_q, ctx_lens, n_seqs, (bf16*)out, out_stride, nq, nkv,
               block_size, num_blocks, scale * LOG2E, window, status, num_splits, part_o, part_ml, dist_bias, bias_len, softcap * LOG2E, sink);
-    if (num_splits > 1 && (parts & 2)) {
-        const int n_pairs = n_tokens * nq, per_block = JOIN_THREADS / (D / 4);
-        FF_LAUNCH((attn_tc_join_kernel), dim3((unsigned)((n_pairs + per_block - 1) / per_block)), JOIN_THREADS, 0, stream,
-                  (const float*)part_o, (const float*)part_ml, (bf16*)out, out_stride, nq, num_splits, tok_base, n_pairs);
-        FF_LAUNCH_CHECK();
-    }
-    return 0;
+    return join && num_splits > 1 ? ff_attn_tc_join(part_o, part_ml, out, out_stride, nq, num_splits, tok_base, n_tokens, stream) : 0;
 }

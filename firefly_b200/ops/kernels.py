@@ -586,25 +586,23 @@ def attn_tiled(q, q_stride, pages, table, cu_q, ctx_lens, n_seqs, total_tiles, o
         c_float(softcap), _sink_arg(sink, nq), _p(status), _stream()), "attn_tiled")
 
 
-BOTH_PARTS, ATTENTION_PART, JOIN_PART = 3, 1, 2     # of an attention whose keys are shared out over blocks
-
-
 def attn_decode(q, q_stride, pages, table, cu_q, ctx_lens, n_seqs, out, part_o, part_ml, nq, nkv, d,
                 scale, window, num_splits, status: Optional[torch.Tensor] = None,
                 dist_bias: Optional[torch.Tensor] = None, softcap: float = 0.0, sink: Sink = None,
-                parts: int = BOTH_PARTS, beside: bool = False) -> None:
+                beside: bool = False) -> None:
     """Split-KV tensor-core attention when every sequence has one token (bfloat16).  ``status``,
-    ``dist_bias`` and ``sink`` as for `attn_tiled`; ``parts``, ``beside``: as `paged_attention` uses them."""
+    ``dist_bias`` and ``sink`` as for `attn_tiled`.  ``beside``: the launch in front of this one is `attn_tc` over other sequences of the
+    same step, and nothing here waits for it (`paged_attention`)."""
     _need_cuda(pages, table, cu_q, ctx_lens, out, part_o, part_ml, status, dist_bias)
     num_blocks, planes, _, block_size, _ = pages.shape
     _check(_attn_lib(d, planes).ff_attn_decode(
         _p(q), c_int(q_stride), _p(pages), _p(table), c_int(table.shape[1]), _p(cu_q), _p(ctx_lens),
         c_int(n_seqs), _p(out), c_int(out.shape[1]), _p(part_o), _p(part_ml), c_int(nq), c_int(nkv),
         c_int(block_size), c_int(num_blocks), c_float(scale), c_int(window), c_int(num_splits),
-        *_bias_args(dist_bias, nq, window), c_float(softcap), _sink_arg(sink, nq), c_int(parts), c_int(1 if beside else 0),
+        *_bias_args(dist_bias, nq, window), c_float(softcap), _sink_arg(sink, nq), c_int(1 if beside else 0),
         _p(status), _stream()), "attn_decode")
     global LAUNCHES
-    if num_splits > 1 and parts == BOTH_PARTS:
+    if num_splits > 1:
         LAUNCHES += 1     # the kernel that joins the splits
 
 
@@ -677,14 +675,14 @@ def tc_attention_supported(dtype: torch.dtype, d: int, block_size: int, max_kv_l
 
 def attn_tc(q, q_stride, pages, table, cu_q, ctx_lens, n_seqs, total_tiles, out, nq, nkv, d, scale, window,
             status, page_list: Optional[int] = None, shares=None, dist_bias: Optional[torch.Tensor] = None,
-            softcap: float = 0.0, sink: Sink = None, two_tiles: bool = False, parts: int = BOTH_PARTS) -> None:
+            softcap: float = 0.0, sink: Sink = None, two_tiles: bool = False, join: bool = True) -> None:
     """tcgen05 flash attention over the paged cache (bfloat16); total_tiles counts row tiles of 128.
     ``shares`` = (count, part_o, part_ml, first row, rows): every row tile's keys are shared out over
     ``count`` blocks and a second kernel joins their partial results (for prompts so short that their
     row tiles alone would leave most SMs idle); the scratch tensors are float32 with at least
     (first row + rows) * nq * count * d and ... * 2 elements.  ``dist_bias``, ``sink``: as for `paged_attention_simt`.
     ``two_tiles``: two row tiles a block (`attn_tc_two_tiles`), where the kernel for that takes the call: heads of 64 and 128, no
-    shares, neither bias nor cap.  ``parts``: the attention, the join of its shares or both."""
+    shares, neither bias nor cap.  ``join`` False: the partial results are left to `attn_tc_join`."""
     _need_cuda(pages, table, cu_q, ctx_lens, out, status, dist_bias)
     num_blocks, planes, _, block_size, _ = pages.shape
     count, part_o, part_ml, row0, rows = shares if shares is not None else (1, None, None, 0, 0)
@@ -697,10 +695,17 @@ def attn_tc(q, q_stride, pages, table, cu_q, ctx_lens, n_seqs, total_tiles, out,
         c_int(n_seqs), c_int(total_tiles), _p(out), c_int(out.shape[1]), c_int(nq), c_int(nkv),
         c_int(block_size), c_int(num_blocks), c_float(scale), c_int(window), _p(status), c_int(count), _p(part_o),
         _p(part_ml), c_int(row0), c_int(rows), *_bias_args(dist_bias, nq, window), c_float(softcap),
-        _sink_arg(sink, nq), c_int(1 if two_tiles else 0), c_int(parts), _stream()), "attn_tc")
-    if count > 1 and parts == BOTH_PARTS:
+        _sink_arg(sink, nq), c_int(1 if two_tiles else 0), c_int(1 if join else 0), _stream()), "attn_tc")
+    if count > 1 and join:
         global LAUNCHES
         LAUNCHES += 1     # the kernel that joins the shares
+
+
+def attn_tc_join(out, nq, d, planes: int, shares) -> None:
+    """Joins the partial results that `attn_tc` with the same ``shares`` and ``join`` False left in them (which has looked at their sizes)."""
+    count, part_o, part_ml, row0, rows = shares
+    _check(_attn_tc_lib(d, None, planes).ff_attn_tc_join(_p(part_o), _p(part_ml), _p(out), c_int(out.shape[1]), c_int(nq), c_int(count),
+                                                         c_int(row0), c_int(rows), _stream()), "attn_tc_join")
 
 
 USE_TC_SHARES = True       # short portions behind long contexts share their keys out over several blocks
@@ -803,7 +808,7 @@ def _decode_scratch(ws, n: int, nq: int, nkv: int, d: int, splits: int):
 def attn_decode_units(q, q_stride, pages, table, cu_q, ctx_lens, n_seqs, out, part_o, part_ml, seq_ranges,
                       nq, nkv, d, scale, window, units, max_ranges, heads=None, status=None,
                       dist_bias: Optional[torch.Tensor] = None, softcap: float = 0.0, sink: Sink = None, q_temp=None,
-                      value_is_key: bool = False, parts: int = BOTH_PARTS, beside: bool = False) -> None:
+                      value_is_key: bool = False, beside: bool = False) -> None:
     """Split-KV decode attention with `units` blocks per kv head shared out among the sequences
     in proportion to their lengths.  ``heads = (q_norm_w, k_norm_w, eps, cos_sin)``: q is the raw
     q|k|v projection and the kernel finishes the heads itself (``q_temp``, ``value_is_key``: as for
@@ -819,11 +824,11 @@ def attn_decode_units(q, q_stride, pages, table, cu_q, ctx_lens, n_seqs, out, pa
         c_int(nkv), c_int(block_size), c_int(num_blocks), c_float(scale), c_int(window), c_int(units),
         c_int(max_ranges), c_int(1 if heads is not None else 0), _p(qw), _p(kw), c_float(eps), _p(cos_sin),
         c_int(cos_sin.shape[0] if cos_sin is not None else 0), *_bias_args(dist_bias, nq, window), c_float(softcap),
-        _sink_arg(sink, nq), *_temp_args(q_temp), c_int(1 if value_is_key else 0), c_int(parts), c_int(1 if beside else 0),
+        _sink_arg(sink, nq), *_temp_args(q_temp), c_int(1 if value_is_key else 0), c_int(1 if beside else 0),
         _p(status), _stream()), "attn_decode_units")
     global LAUNCHES, BY_LENGTH_CALLS
-    BY_LENGTH_CALLS += parts != JOIN_PART
-    if units > n_seqs and max_ranges > 1 and parts == BOTH_PARTS:
+    BY_LENGTH_CALLS += 1
+    if units > n_seqs and max_ranges > 1:
         LAUNCHES += 1     # the kernel that joins the ranges
 
 
@@ -852,16 +857,16 @@ def paged_attention(q: torch.Tensor, q_stride: int, pages: torch.Tensor, table: 
         units = decode_units(n_dec, nkv, d, ctx.ranges_by_length)
         part_o, part_ml, seq_ranges = _decode_scratch(ctx.workspace, n_dec, nq, nkv, d, splits)
 
-    def single_tokens(parts: int, beside: bool = False) -> None:
+    def single_tokens(beside: bool = False) -> None:
         if units:
             attn_decode_units(q, q_stride, pages, table, ctx.cu_q, ctx.ctx_lens, n_dec, out, part_o, part_ml,
                               seq_ranges, nq, nkv, d, scale, window, units, DECODE_MAX_RANGES, status=ctx.status,
-                              dist_bias=dist_bias, softcap=softcap, sink=sink, parts=parts, beside=beside)
-        elif parts != JOIN_PART or splits > 1:
+                              dist_bias=dist_bias, softcap=softcap, sink=sink, beside=beside)
+        else:
             attn_decode(q, q_stride, pages, table, ctx.cu_q, ctx.ctx_lens, n_dec, out, part_o, part_ml, nq, nkv,
-                        d, scale, window, splits, ctx.status, dist_bias, softcap, sink, parts=parts, beside=beside)
+                        d, scale, window, splits, ctx.status, dist_bias, softcap, sink, beside=beside)
     if n_dec and not tc:
-        single_tokens(BOTH_PARTS)
+        single_tokens()
     if n_dec < n:
         # portions of prompts: tiled kernel over the remaining sequences (token offsets in cu_q are absolute)
         # every layer of a step asks the same of the step's arrays: worked out once and kept with the step
@@ -895,22 +900,23 @@ def paged_attention(q: torch.Tensor, q_stride: int, pages: torch.Tensor, table: 
                 cells = (row0 + rows) * nq * count
                 shares = (count, ctx.workspace.get("attn.tc_part_o", (cells * d,), torch.float32),
                           ctx.workspace.get("attn.tc_part_ml", (cells * 2,), torch.float32), row0, rows)
-            def portions(parts: int) -> None:
+
+            def portions(join: bool) -> None:
                 attn_tc(q, q_stride, pages, table_t, cu_q_t, ctx_lens_t, n - n_dec, tiles, out, nq, nkv, d, scale, window, ctx.status,
-                        shares=shares, dist_bias=dist_bias, softcap=softcap, sink=sink, two_tiles=two_tiles, parts=parts)
+                        shares=shares, dist_bias=dist_bias, softcap=softcap, sink=sink, two_tiles=two_tiles, join=join)
             if not n_dec or not tiles:
-                portions(BOTH_PARTS)
+                portions(join=True)
                 if n_dec:                        # portions without a token launch nothing that the single tokens could run beside
-                    single_tokens(BOTH_PARTS)
+                    single_tokens()
             else:
                 # The two attentions need nothing of one another: the single tokens' blocks run in the places that the portions' leave
                 # and need not wait for their end (one after the other they took 69 us a layer for 2 x 256 + 24 tokens, now 63, and 66 for 2048 + 1, now 60),
-                # and the kernels that join partial results come behind both.
-                portions(ATTENTION_PART)
-                single_tokens(ATTENTION_PART, beside=True)
+                # and the kernels that join partial results come behind both.  A step that the host bounds pays for every call: two, as one after
+                # the other, or three where the portions' keys are shared out (28 layers of the 0.6B shape, 2 x 100 + 24 tokens: 4.8 ms, with four calls 5.4).
+                portions(join=False)
+                single_tokens(beside=True)
                 if count > 1:
-                    portions(JOIN_PART)
-                single_tokens(JOIN_PART)
+                    attn_tc_join(out, nq, d, pages.shape[1], shares)
         else:
             tiles = sum(-(-(ql * G) // 64) for ql in ctx.q_lens[n_dec:])
             attn_tiled(q, q_stride, pages, table_t, cu_q_t, ctx_lens_t, n - n_dec,
