@@ -410,8 +410,8 @@ struct DecodeHeads {
     float temp_coef;           // heads finished here: q also times 1 + temp_coef ln(floor((pos + 1) / temp_every) + 1)
     int temp_every;            // (0: no such factor; it needs q_norm_w)
     int value_is_key;          // heads finished here: the row is q heads | k heads and the raw key is the value
-    int beside;                // the kernel in front is the same step's attention over prompts (attention_tc.cu): nothing here
-                               // depends on it, and it lets this one start only when what both read is there
+    int beside;                // the kernel in front is the same step's attention over prompts (attention_tc.cu), on which nothing here
+                               // depends: no wait for it before the end (see there what the loads count on)
     int longest_first;         // fixed ranges: the blocks are handed out sequence by sequence, the longest first (at most NTHREADS sequences)
 };
 constexpr int HC = D / 64;     // elements of each half of a head that a lane holds (heads finished in a warp)
@@ -651,7 +651,12 @@ attn_decode_body(const bf16* __restrict__ q, int q_stride, const bf16* __restric
         for (int c = G * CHUNKS + threadIdx.x; c < 16 * CHUNKS; c += NTHREADS)
             *reinterpret_cast<uint4*>(Qs + (c / CHUNKS) * KSTR + (c % CHUNKS) * 8) = make_uint4(0, 0, 0, 0);
     }
+    // Beside the attention over prompts: q and the newest keys come from the kernels in front of *that* kernel.  Each of its blocks lets this one
+    // start only behind its own griddepcontrol.wait, so those kernels have ended, but PTX promises what they wrote to the grid that waits and
+    // to no other.  So what the step has produced is read behind this fence and from the L2 cache (cp.async.cg below), never by a
+    // plain or read-only load nor in front of it, and no other kernel may be launched between the two.
     if (HEADS || !hd.beside) asm volatile("griddepcontrol.wait;" ::: "memory");
+    else asm volatile("fence.acq_rel.gpu;" ::: "memory");
     if constexpr (UNITS) {
         if (split == 0 && kh == 0 && threadIdx.x == 0) un.seq_ranges[seq] = ranges;
     }

@@ -320,8 +320,8 @@ attn_tc_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __restri
                      ::"r"(sa(&s_tmem)), "r"((uint32_t)TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    // The next kernel may start once every block is behind this wait (and here, so that it may count on what the kernels in front
-    // wrote without a wait of its own: the decode attention beside this one, attention_mma.cu).
+    // The next kernel may start once every block is behind this wait, and not before: the decode attention beside this one (attention_mma.cu)
+    // has no wait of its own in front of its loads and reads what the kernels in front of this one wrote.
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // Row tiles are handed out last first, for all kv heads before the next tile: in a prompt the
@@ -773,7 +773,7 @@ attn_tc_pair_kernel(const __grid_constant__ TensorMapArg kv_map, const bf16* __r
     tc_before();
     __syncthreads();
     tc_after();
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");    // behind the wait above, as in attn_tc_kernel
     const uint32_t tmem = s_tmem;
     const uint32_t tm_S = tmem, tm_O = tmem + 2 * PN;                // S (then P) of either row tile, O of either
     const int seq = s_seq;

@@ -913,6 +913,7 @@ def paged_attention(q: torch.Tensor, q_stride: int, pages: torch.Tensor, table: 
                 # and need not wait for their end (one after the other they took 69 us a layer for 2 x 256 + 24 tokens, now 63, and 66 for 2048 + 1, now 60),
                 # and the kernels that join partial results come behind both.  A step that the host bounds pays for every call: two, as one after
                 # the other, or three where the portions' keys are shared out (28 layers of the 0.6B shape, 2 x 100 + 24 tokens: 4.8 ms, with four calls 5.4).
+                # The second kernel counts on the first one to start it only when q and the newest keys are there: nothing may be launched between them.
                 portions(join=False)
                 single_tokens(beside=True)
                 if count > 1:
