@@ -486,6 +486,68 @@ struct DecodeUnits {
     int part_stride;           // partial results of a (sequence, head) lie this many apart
 };
 
+// More blocks than the GPU holds at once are started longest first: in the order of the sequences' numbers, long ranges begin in the last
+// round and most SMs wait for them.  Every block finds its sequence for itself (number `rank` by tiles of keys, ties by their number; a sequence's
+// kv heads come together), by halving the range of lengths, a barrier each time.  It pays for one barrier where the order makes no difference: lengths within
+// an eighth of the longest, or this of fewer than LONG_TILES tiles; then seq, pos and tok stay those of the block's own number, else they become
+// those of the sequence found.  All threads of the block; n at most NTHREADS.
+// us of kernel and join, 32 / 8 heads of 128, three ranges, in order / now (and with every length compared with every other): 64 sequences of 2100 equal 113.0 / 112.7
+// (115.2), of 420 to 2100 76.8 / 72.2 (73.0), 8 of 2100 among 56 of 262 55.0 / 44.1 (44.8); 32 of 420 to 2100 44.5 / 35.7; 128 of 400 to 2000 134 / 130.  What it
+// costs many short ones: 64 of 500 43.6 / 44.6 (46.2), 128 of 1000 113.4 / 114.4 (121.7), of 200 to 1000 84.2 / 86.7 (91.0), of 200 52.5 / 54.9 (60.0).
+constexpr int LONG_TILES = 12;
+__device__ __forceinline__ bool sequence_by_length(const int* __restrict__ ctx_lens, const int* __restrict__ cu_q, int n, int rank, int window, int& seq,
+                                                   int& pos, int& tok) {
+    constexpr int WARPS = NTHREADS / 32;
+    __shared__ int s_low[WARPS], s_high[WARPS], s_same[WARPS], s_found[3];
+    const int i = threadIdx.x, lane = i & 31, warp = i >> 5;
+    int tiles = -1, p = 0, t = 0;
+    if (i < n) {
+        p = ctx_lens[i];
+        t = cu_q[i];
+    }
+    seq = blockIdx.x;                                              // asked for beside the others
+    pos = ctx_lens[seq];
+    tok = cu_q[seq];
+    if (i < n) tiles = (max(p, 0) + BN) / BN - first_visible_key(max(p, 0), window) / BN;
+    int low = __reduce_min_sync(0xffffffffu, i < n ? tiles : 0x7fffffff), high = __reduce_max_sync(0xffffffffu, tiles);
+    if (lane == 0) {
+        s_low[warp] = low;
+        s_high[warp] = high;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) {
+        low = min(low, s_low[w]);
+        high = max(high, s_high[w]);
+    }
+    if (high < LONG_TILES || high - low <= high / 8) return false;
+    int longer = 0;                                                // sequences of more than `high` tiles; more than `rank` have at least `low`
+    while (low < high) {
+        const int mid = (low + high + 1) / 2, at_least = __syncthreads_count(tiles >= mid);
+        if (at_least > rank) low = mid;
+        else {
+            high = mid - 1;
+            longer = at_least;
+        }
+    }
+    const unsigned same = __ballot_sync(0xffffffffu, tiles == low);
+    if (lane == 0) s_same[warp] = __popc(same);
+    __syncthreads();
+    int at = longer + __popc(same & ((1u << lane) - 1));
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) at += w < warp ? s_same[w] : 0;
+    if (tiles == low && at == rank) {
+        s_found[0] = i;
+        s_found[1] = p;
+        s_found[2] = t;
+    }
+    __syncthreads();
+    seq = s_found[0];
+    pos = s_found[1];
+    tok = s_found[2];
+    return true;
+}
+
 // XHEADS: the form that finishes the heads may have a sink, a temperature and raw keys as values (a build of its own, so
 // that the plain form's registers and latency stay what they are).
 template <bool HEADS, bool UNITS, bool XHEADS>
@@ -507,7 +569,7 @@ attn_decode_body(const bf16* __restrict__ q, int q_stride, const bf16* __restric
     bf16* Vs = Ks + 2 * BN * KSTR;                                // [2][BN][KSTR]
     const int G = nq / nkv;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int seq, kh, split, ranges, part_stride, pos;
+    int seq, kh, split, ranges, part_stride, pos, tok;
     if constexpr (UNITS) {
         __shared__ int s_warp_tiles[NTHREADS / 32];
         __shared__ int s_mine[4];
@@ -554,42 +616,24 @@ attn_decode_body(const bf16* __restrict__ q, int q_stride, const bf16* __restric
         part_stride = un.part_stride;
         if (seq < 0 || split >= ranges) return;                    // a unit without work
         pos = s_mine[3];
+        tok = cu_q[seq];
     } else {
+        kh = blockIdx.y;
+        split = blockIdx.z;
         if (hd.longest_first) {
-            // Three and more rounds of blocks on the GPU: started in the order of the sequences' numbers, long ranges begin in the last round
-            // and most SMs wait for them.  Every block ranks the sequences for itself; a sequence's kv heads come together.
-            // 64 requests of 600 to 3000 tokens, 8 kv heads of 128: 101 us in order, 95 now.
-            __shared__ __align__(16) unsigned s_key[NTHREADS];
-            __shared__ int s_ranked;
-            const int n = gridDim.x, i = threadIdx.x, of_seq = gridDim.y * gridDim.z;
-            const int block = blockIdx.x + n * (blockIdx.y + gridDim.y * blockIdx.z), rank = block / of_seq, rest = block % of_seq;
-            unsigned key = 0;
-            if (i < n) {
-                const int p = ctx_lens[i];
-                key = (unsigned)((p + BN) / BN - first_visible_key(p, window) / BN) * NTHREADS + (NTHREADS - 1 - i);
+            const int of_seq = gridDim.y * gridDim.z, block = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z), rank = block / of_seq;
+            if (sequence_by_length(ctx_lens, cu_q, gridDim.x, rank, window, seq, pos, tok)) {
+                kh = (block - rank * of_seq) % gridDim.y;
+                split = (block - rank * of_seq) / gridDim.y;
             }
-            s_key[i] = key;
-            __syncthreads();
-            int above = 0;
-            for (int j = 0; j < n; j += 4) {                       // keys behind the last sequence are 0
-                const uint4 o = *reinterpret_cast<const uint4*>(&s_key[j]);
-                above += (o.x > key) + (o.y > key) + (o.z > key) + (o.w > key);
-            }
-            if (i < n && above == rank) s_ranked = i;
-            __syncthreads();
-            seq = s_ranked;
-            kh = rest % gridDim.y;
-            split = rest / gridDim.y;
         } else {
             seq = blockIdx.x;
-            kh = blockIdx.y;
-            split = blockIdx.z;
+            pos = ctx_lens[seq];
+            tok = cu_q[seq];
         }
         ranges = num_splits;
         part_stride = num_splits;
-        pos = ctx_lens[seq];
     }
-    const int tok = cu_q[seq];
     const int kv_hi = pos + 1;
     const int kv_lo = first_visible_key(pos, window);
     const int* bt = block_table + (size_t)seq * max_blocks;
