@@ -12,16 +12,22 @@
 // -> 2.9 / 2.2 / 3.8 / 2.6 us, with the rows in registers 3.6 / 2.7 / 4.3 / 3.7; its decode step of 28 layers 938 -> 657 us, 836 in registers.
 //
 // The epilogues and the RMSNorm folded in on both sides are those of gemm_tcgen05.cu; a sum of squares stands for the rows of a block.
+// A product behind it that gemm_tcgen05.cu takes adds eight times as many of them, one thread a token: o here or there with gate|up there, us a pair, one
+// token: 2048 x 2048 with 12288 x 2048 17.9 / 18.8, 2560 x 2560 with 19456 x 2560 23.6 / 25.7, of the 2.8 that o alone is faster.  (32 of them asked
+// for at once there instead of eight gave 16.8 of these 17.9, but cost every other product behind a norm 0.1 to 0.7.)
 #include "chunk_mma.cuh"
+
+#include <algorithm>
 
 namespace ff {
 
 enum FewEpilogue { FEW_BF16 = 0, FEW_F32 = 1, FEW_RESIDUAL_ADD = 2, FEW_SWIGLU = 3, FEW_RELU2 = 4 };
 constexpr int FEW_TOKENS = 8, FEW_K = 32;                    // tokens at most; k of a step: 16 bytes of a row in each of four lanes
 constexpr int FEW_ROWS = 16;                                 // rows of W a block takes
+constexpr int FEW_PITCH = FEW_ROWS + 4;                      // of the shares of a sum: four tokens' eight rows lie in different banks
 constexpr int FEW_SQ = 4;                                    // sums of squares a lane asks for at once: those of 128 blocks
 constexpr int FEW_AHEAD = 4;                                 // steps of x a lane asks for at once
-constexpr int FEW_MAX_K = 3584;                              // a block's rows are at most half of an SM's shared memory
+constexpr int FEW_MAX_K = 3584;                              // a block's rows take 112 KB at most
 
 struct FewArgs {
     const bf16* x; const bf16* w; void* out;
@@ -37,9 +43,11 @@ __device__ __forceinline__ uint4 few_rows(const bf16* p) {
     return v;
 }
 
+constexpr int FEW_THREADS_SM = 1024;                         // threads an SM that its registers are shared out for
+
 template <int NW>
-__global__ void __launch_bounds__(32 * NW, NW == 8 ? 4 : 2) gemm_few_kernel(const FewArgs a) {
-    constexpr int RP = FEW_ROWS + 4;                          // the rows' pitch puts four tokens' eight rows in different banks
+__global__ void __launch_bounds__(32 * NW, FEW_THREADS_SM / (32 * NW)) gemm_few_kernel(const FewArgs a) {
+    constexpr int RP = FEW_PITCH;
     extern __shared__ __align__(16) uint4 w_rows[];           // [step of the warp][row half][thread]
     __shared__ float part[NW][FEW_TOKENS][RP];
     __shared__ float s_inv[FEW_TOKENS];
@@ -135,12 +143,19 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 4 : 2) gemm_few_kernel(cons
     }
 }
 
+static int few_blocks(int N) { return (N + FEW_ROWS - 1) / FEW_ROWS; }
+template <int NW> static size_t few_rows_bytes(int K) { return (size_t)((K / FEW_K + NW - 1) / NW) * 2 * 32 * NW * 16; }
+// blocks that an SM holds: its 228 KB, of which every block takes 1 KB besides its rows and its static part
+template <int NW> static int few_blocks_per_sm(int K) {
+    const size_t block = few_rows_bytes<NW>(K) + (size_t)NW * FEW_TOKENS * FEW_PITCH * sizeof(float) + FEW_TOKENS * sizeof(float) + 1024;
+    return (int)std::min<size_t>(228 * 1024 / block, FEW_THREADS_SM / (32 * NW));
+}
+
 template <int NW>
 static int few_launch(const FewArgs& a, cudaStream_t stream) {
     static_assert(32 * NW >= FEW_TOKENS * FEW_ROWS && NW >= FEW_TOKENS, "a thread an output, a warp a token's sum of squares");
     FF_SMEM_LIMIT(gemm_few_kernel<NW>, FEW_ROWS * FEW_MAX_K * 2);
-    const int steps = (a.K / FEW_K + NW - 1) / NW;
-    FF_LAUNCH(gemm_few_kernel<NW>, (a.N + FEW_ROWS - 1) / FEW_ROWS, 32 * NW, (size_t)steps * 2 * 32 * NW * 16, stream, a);
+    FF_LAUNCH(gemm_few_kernel<NW>, few_blocks(a.N), 32 * NW, few_rows_bytes<NW>(a.K), stream, a);
     FF_LAUNCH_CHECK();
     return 0;
 }
@@ -151,12 +166,19 @@ using namespace ff;
 
 FF_EXPORT int ff_gemm_few_rows() { return FEW_ROWS; }
 
-// Whether a product takes this kernel: a block's rows of W at most half of an SM's shared memory, and all blocks on the GPU at once (four
-// an SM; the head of the 0.6B shape, 64 blocks an SM, takes 53 us here and 51 through gemm_tcgen05.cu's rings).  Every block reads all
-// of x: with a second eight of tokens the wide products took longer than there (16 tokens, us there / here: q|k|v 5.5 / 6.3, gate|up
-// 7.1 / 6.9), and a step with only the narrow ones here (o 5.4 / 4.0, down 6.1 / 4.6) 10 % longer.
-FF_EXPORT int ff_gemm_few_usable(int T, int N, int K) {
-    return T <= FEW_TOKENS && K % FEW_K == 0 && K <= FEW_MAX_K && N <= 4 * 148 * FEW_ROWS;
+// Whether a product takes this kernel on a GPU of so many SMs: where all its blocks are there at once.  Then it is 1.2 to 1.6 times as fast as
+// gemm_tcgen05.cu (alone, 1 and 8 tokens, K of 1792 to 3584).  A second round of blocks has nothing under way while it copies its rows, 2.5 us: us here / there, 8
+// tokens: K = 2560, N = 4736 (one round) 6.1 / 8.3, 5008 9.1 / 8.6, 7104 (a round and a half) 10.0 / 10.9; K = 3328 7.8 / 9.5, 12.0 / 9.9, 13.1 / 12.9; K = 3584, of which
+// an SM holds one block, 2368 4.9 / 7.1, 3072 8.5 / 8.1, 5120 13.6 / 10.4.  It pays where the rows are short (K = 2304, N = 5008 8.0 / 8.3; 2048, 9232 10.3 / 10.6)
+// or the second round is half full.  Every block reads all of x: with a second eight of tokens the wide products took longer than there
+// (16 tokens: q|k|v 5.5 there / 6.3, gate|up 7.1 / 6.9), and a step with only the narrow ones here (o 5.4 / 4.0, down 6.1 / 4.6) 10 % longer.
+FF_EXPORT int ff_gemm_few_usable(int T, int N, int K, int sms) {
+    if (T > FEW_TOKENS || K <= 0 || K % FEW_K || K > FEW_MAX_K) return 0;
+    const int blocks = few_blocks(N);
+    if (blocks <= sms) return 1;                               // 16 warps a block, one an SM
+    const int places = sms * few_blocks_per_sm<8>(K);
+    if (blocks <= places) return 1;
+    return blocks <= 4 * sms && (K <= 2304 || (K <= 3072 && 2 * blocks >= 3 * places));
 }
 
 // x: bfloat16 [T, K], T <= 8; w: bfloat16 [N, K]; K a multiple of 32 up to FEW_MAX_K; both on 16 bytes.  Epilogues, norm folded in: as
@@ -170,6 +192,10 @@ FF_EXPORT int ff_gemm_few(const void* x, const void* w, void* out, int ldo, int 
         return FF_ERR_BAD_ARG;
     if (epilogue == FEW_SWIGLU && N % 32) return FF_ERR_UNSUPPORTED;
     const FewArgs a{(const bf16*)x, (const bf16*)w, out, ldo, T, N, K, epilogue, (bf16*)xw_out, xw_w, ssq_out, ssq_in, ssq_parts, norm_dim, norm_eps};
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return (int)e;
     // with a block an SM and fewer, more warps share its rows
-    return N <= FEW_ROWS * 148 ? few_launch<16>(a, stream) : few_launch<8>(a, stream);
+    return few_blocks(N) <= sms ? few_launch<16>(a, stream) : few_launch<8>(a, stream);
 }

@@ -427,13 +427,13 @@ USE_GEMM_FEW = True        # tests flip this to compare with `gemm_tc`
 
 
 @functools.lru_cache(maxsize=4096)
-def _gemm_few_takes(T: int, N: int, Kd: int) -> bool:
-    return bool(_lib("gemm_few").ff_gemm_few_usable(c_int(T), c_int(N), c_int(Kd)))
+def _gemm_few_takes(T: int, N: int, Kd: int, sms: int) -> bool:
+    return bool(_lib("gemm_few").ff_gemm_few_usable(c_int(T), c_int(N), c_int(Kd), c_int(sms)))
 
 
 def gemm_few_usable(T: int, N: int, Kd: int) -> bool:
     """True if the product of a few tokens with a small matrix (csrc/gemm_few.cu) takes this size."""
-    return USE_GEMM_FEW and _gemm_few_takes(T, N, Kd)
+    return USE_GEMM_FEW and _gemm_few_takes(T, N, Kd, sm_count())
 
 
 @functools.lru_cache(maxsize=None)

@@ -5,7 +5,9 @@ import torch
 pytestmark = pytest.mark.gpu
 
 # K: one step of a warp, less than a step for some, a ring that wraps, the longest; N: parts of a block, both numbers of warps
-SIZES = [(16, 32), (7, 96), (33, 288), (1000, 1024), (2368, 2080), (2369, 512), (4096, 1024), (640, 3584)]
+SIZES = [(16, 32), (7, 96), (33, 288), (1000, 1024), (2368, 2080), (2369, 512), (4096, 1024), (640, 3584),
+         # eight warps a block with long rows: three and two blocks an SM, and a second round of blocks that is half full
+         (4200, 2048), (4736, 3328), (7104, 2560)]
 
 
 def _K():
@@ -85,7 +87,11 @@ def test_limits():
     """Sizes that it does not take go to `gemm_tc`."""
     K = _K()
     assert not K.gemm_few_usable(9, 512, 512) and not K.gemm_few_usable(1, 512, 72) and not K.gemm_few_usable(1, 512, 4096)
-    assert not K.gemm_few_usable(1, 16 * 4 * 148 + 1, 512)
+    # the rows of all blocks on the GPU at once, whatever K: 4, 3, 2 and 1 blocks of 16 rows an SM; a second round where the rows are short or it is half full
+    row = 16 * K.sm_count()
+    for Kd, most in ((1536, 4 * row), (1568, 4 * row), (2304, 4 * row), (2816, 2 * row), (3328, 2 * row), (3552, row), (3584, row)):
+        assert K.gemm_few_usable(1, most, Kd) and not K.gemm_few_usable(1, most + 1, Kd), Kd
+    assert K.gemm_few_usable(8, 3 * row, 3072) and not K.gemm_few_usable(8, 3 * row - 16, 3072) and not K.gemm_few_usable(1, 3 * row, 3104)
     x, w = torch.zeros(9, 64, dtype=torch.bfloat16, device="cuda"), torch.zeros(16, 64, dtype=torch.bfloat16, device="cuda")
     with pytest.raises(K.KernelError, match="bad argument"):
         K.gemm_few(x, w, torch.zeros(9, 16, device="cuda"), K.EPI_F32)
