@@ -262,25 +262,9 @@ struct GroupWalk {
     __device__ __forceinline__ int row0(int m) const { return lo + (m - base) * GP_ROWS; }
 };
 
-// Loads, MMA and completion over the pair (as in gemm_pair.cu): a load is counted on the barrier of the pair's first block.
-__device__ __forceinline__ void gp_load_2d(bool issue, uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t"
-                 "@q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}"
-                 ::"r"(dst), "l"(map), "r"(bar & 0xFEFFFFFFu), "r"(x), "r"(y), "r"((uint32_t)issue) : "memory");
-}
 __device__ __forceinline__ void gp_store_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
     asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(map), "r"(src), "r"(x), "r"(y) : "memory");
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-}
-__device__ __forceinline__ void gp_mma(bool issue, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
-                 "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                 ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"((uint32_t)issue) : "memory");
-}
-__device__ __forceinline__ void gp_commit(bool issue, uint32_t bar) {   // arrives in both blocks
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
-                 "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
-                 ::"r"(bar), "h"((uint16_t)3), "r"((uint32_t)issue) : "memory");
 }
 __device__ __forceinline__ void gp_arrive_leader(uint32_t bar) {
     uint32_t peer;
@@ -355,8 +339,8 @@ moe_grouped_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
                 const uint32_t full = smem_addr(&bars[FULL + s]), sa = smem_addr(tiles + (size_t)s * GP_STAGE_BYTES);
                 if (half == 0) mbar_expect_tx(issue, full, 2 * GP_STAGE_BYTES);            // both blocks' bytes
                 __syncwarp();
-                gp_load_2d(issue, sa, &map_a, it * BK, row0, full);
-                gp_load_2d(issue, sa + GM * BK * 2, mb, it * BK, y, full);
+                tma_load_2d_pair(issue, sa, &map_a, it * BK, row0, full);
+                tma_load_2d_pair(issue, sa + GM * BK * 2, mb, it * BK, y, full);
             }
         }
         // the last stages' releases, which come from the first block's MMAs, have arrived before this block goes
@@ -389,12 +373,12 @@ moe_grouped_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
                     const uint32_t sa = smem_addr(tiles + (size_t)s * GP_STAGE_BYTES), sb = sa + GM * BK * 2;
 #pragma unroll
                     for (int k = 0; k < BK / UMMA_K; ++k)
-                        gp_mma(issue, tmem_base + buf * GP_BC, smem_desc_sw128(sa + k * UMMA_K * 2), smem_desc_sw128(sb + k * UMMA_K * 2), idesc,
+                        tc_mma_bf16_pair(issue, tmem_base + buf * GP_BC, smem_desc_sw128(sa + k * UMMA_K * 2), smem_desc_sw128(sb + k * UMMA_K * 2), idesc,
                                (it > 0 || k > 0) ? 1u : 0u);
-                    gp_commit(issue, smem_addr(&bars[EMPTY + s]));     // the stage is free in both blocks
+                    tc_commit_pair(issue, smem_addr(&bars[EMPTY + s]), 3);     // the stage is free in both blocks
                     __syncwarp();
                 }
-                if (ok) gp_commit(issue, smem_addr(&bars[READY + buf]));
+                if (ok) tc_commit_pair(issue, smem_addr(&bars[READY + buf]), 3);
             }
         }
     } else {

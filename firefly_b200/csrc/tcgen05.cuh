@@ -73,6 +73,28 @@ __device__ __forceinline__ void tc_mma_bf16(bool issue, uint32_t tmem_d, uint64_
                  "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
                  ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"((uint32_t)issue) : "memory");
 }
+// ---- the same over a pair of blocks (cta_group::2)
+// TMA load whose completion is counted on the barrier at the same place in the pair's first block
+// (the barrier's address with the pair bit cleared).
+__device__ __forceinline__ void tma_load_2d_pair(bool issue, uint32_t dst, const CUtensorMap* map, int x, int y,
+                                                 uint32_t bar_local) {
+    const uint32_t bar = bar_local & 0xFEFFFFFFu;
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+                 "@q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}"
+                 ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"((uint32_t)issue) : "memory");
+}
+__device__ __forceinline__ void tc_mma_bf16_pair(bool issue, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,
+                                                 uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+                 "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                 ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"((uint32_t)issue) : "memory");
+}
+// the MMAs issued so far are complete: arrive on the barrier at this place in both blocks of the pair
+__device__ __forceinline__ void tc_commit_pair(bool issue, uint32_t bar_local, uint16_t cta_mask) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
+                 "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+                 ::"r"(bar_local), "h"(cta_mask), "r"((uint32_t)issue) : "memory");
+}
 // 16 consecutive accumulator columns of this warp's 32 lanes
 __device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&v)[16]) {
     uint32_t r[16];
