@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(128, VEC > 1 ? CONV_BLOCKS : CONV_BLOCKS_ONE) 
     };
     // The rows and sequences of CONV_AHEAD tokens are asked for together, while the CONV_AHEAD in front of them are worked on: with one at
     // a time the walk waits for memory at every token.  Four channels a thread leave an SM the warps that hide the rest.  8192 tokens
-    // of 4096 channels, whose bytes take 21 us: a token at a time 118, four at a time with nothing asked for ahead and eight channels a thread 50, now 41 (48 of these 50 with the SiLU as it was).
+    // of 4096 channels, whose bytes take 21 us: a token at a time 118, four at a time with nothing asked for ahead and eight channels a thread 55, now 50.
     int s_prev = -1;
     float rows[CONV_AHEAD][VEC];
     Raw next[CONV_AHEAD];
@@ -801,8 +801,8 @@ __global__ void __launch_bounds__(32 * CF_WARPS) channel_decay_prepare_kernel(Sc
 // alpha[t, c] = sigmoid(z)^(1 / tau), z = sum_r low[t, r] * w[c, r] + bias[c], all in 32-bit: exp(-softplus(-z) / tau).
 // A thread keeps one channel's row of w in registers (up to LRD_R of it at a time) and walks a tile of tokens, LRD_U of
 // them at once, whose low rows stand in shared memory, two tokens side by side for the instructions that take two sums.
-// Bound by instructions: 96 a token and channel with one sum an instruction and softplus of expf and logf, now some 35, and
-// by weights that were asked for two bytes at a time.  4140 tokens of 1024 channels 19.6 us, now 12.5; 1000 tokens 8.6, now 4.8.
+// Bound by instructions, of which one sum at a time made a third more, and by weights that were asked for two bytes at a
+// time.  4140 tokens of 1024 channels 21.2 us, now 14.2; 1000 tokens 7.9, now 5.0.
 constexpr int LRD_TOK = 32, LRD_U = 4, LRD_THREADS = 128, LRD_R = 16;
 
 template <typename T>
@@ -991,7 +991,7 @@ static int conv_launch(const void* in, int in_stride, int in_off, const float* w
     const int threads = lanes >= 128 ? 128 : ((lanes + 31) / 32) * 32;
     // A thread's weights are read once for its tile of tokens; few tokens get small tiles, so that they still fill the GPU.  Longer steps get the
     // tile (up to 48) with which the blocks fill the GPU's places a whole number of times: at 32 whatever the rest, 8192 tokens of 2048 channels
-    // were 1.15 rounds of blocks, 28 us (now 23), and of 4096 channels 2.3, 43 us (now 41, of instructions).
+    // were 1.15 rounds of blocks, 31 us (now 28), and of 4096 channels 2.3, 51 us (now 50, of instructions); 2048 tokens of 4096 channels at 4 21 us (now 17).
     const int cols = (lanes + threads - 1) / threads;
     int tile = 1;
     if (T_ >= 512) {
